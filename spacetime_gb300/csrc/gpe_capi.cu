@@ -18,10 +18,10 @@ cudaError_t launch_hyper(const StepArgs& a, int kind, cudaStream_t s);
 template <typename R, int C>
 cudaError_t launch_observe(const StepArgs& a, double* out, bool node_fp32, cudaStream_t s);
 template <typename R, int C>
-cudaError_t launch_scale(const StepArgs& a, const double* norm_sum, double dv, cudaStream_t s);
+cudaError_t launch_scale(const StepArgs& a, cudaStream_t s);
 template <typename R, int C>
-cudaError_t launch_norm(const StepArgs& a, double* out, cudaStream_t s);
-cudaError_t launch_dot(const StepArgs& a, int precision, int C, double* out, cudaStream_t s);
+cudaError_t launch_norm(const StepArgs& a, cudaStream_t s);
+cudaError_t launch_dot(const StepArgs& a, int precision, int C, cudaStream_t s);
 struct InitArgs {
     double zeta[5][2];
     double mu, c0inv, noise_abs, noise_rel;
@@ -54,6 +54,8 @@ cudaError_t launch_parabolic_observe(const StepArgs& a, double* out, cudaStream_
 template <int C>
 cudaError_t launch_il_step(const StepArgs& a, const ILGrid& G, int deg, size_t max_blocks, bool obs, double* out,
                            cudaStream_t s);
+template <int C>
+cudaError_t launch_il_itp(const StepArgs& a, const ILGrid& G, int deg, size_t max_blocks, cudaStream_t s);
 template <int C>
 unsigned il_blocks(const ILGrid& G, int deg, bool obs, size_t max_blocks);
 cudaError_t launch_il_convert(char* aos, const Grid& g, char* il, const ILGrid& G, bool to_il, cudaStream_t s);
@@ -203,6 +205,7 @@ static void release(gpe_handle* h) {
     for (void* p : h->dev_tables) cudaFree(p);
     if (h->partials) cudaFree(h->partials);
     if (h->obs_out) cudaFree(h->obs_out);
+    if (h->itp_scale) cudaFree(h->itp_scale);
     if (h->stage) cudaFree(h->stage);
     if (h->field_buf) cudaFree(h->field_buf);
     if (h->err) cudaFree(h->err);
@@ -391,6 +394,8 @@ extern "C" gpe_status gpe_create(const gpe_lattice* lat, const gpe_params* p, gp
     h->partial_blocks = std::max<size_t>((sites + 255) / 256, 2048);
     if (cudaMalloc(&h->partials, h->partial_blocks * OBS_COUNT * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&h->obs_out, OBS_COUNT * sizeof(double)) != cudaSuccess ||
+        cudaMalloc(&h->itp_scale, 2 * sizeof(ItpScale)) != cudaSuccess ||
+        cudaMemset(h->itp_scale, 0, 2 * sizeof(ItpScale)) != cudaSuccess ||
         cudaMalloc(&h->err, sizeof(int)) != cudaSuccess || cudaMemset(h->err, 0, sizeof(int)) != cudaSuccess) {
         release(h);
         delete h;
@@ -608,6 +613,7 @@ StepArgs gpe::make_args(const gpe_handle* h, const gpe_fields& B, double t) {
     a.divRowE = make_fastdiv(a.row_items_e ? a.row_items_e : 1);
     a.total = (uint64_t)g.X * g.Y * g.Z * g.V;
     a.partials = h->partials;
+    a.dv = cell_dv(h);
     a.err = h->err;
     fill_phys(a.pf, a.ph, B, t);
     fill_phys(a.pd, a.ph, B, t);
@@ -664,27 +670,40 @@ static cudaError_t dispatch_observe(const gpe_handle* h, const StepArgs& a, doub
     }
 }
 template <int C>
-static cudaError_t dispatch_norm_c(const gpe_handle* h, const StepArgs& a, double* out, cudaStream_t s) {
-    return h->real_bytes == 8 ? launch_norm<double, C>(a, out, s) : launch_norm<float, C>(a, out, s);
+static cudaError_t dispatch_norm_c(const gpe_handle* h, const StepArgs& a, cudaStream_t s) {
+    return h->real_bytes == 8 ? launch_norm<double, C>(a, s) : launch_norm<float, C>(a, s);
 }
-// sum |psi|^2 of a.prev into out[OBS_NORM] (the other entries zero)
-static cudaError_t dispatch_norm(const gpe_handle* h, const StepArgs& a, double* out, cudaStream_t s) {
+// the normalisation of a.prev into *a.scale_out
+static cudaError_t dispatch_norm(const gpe_handle* h, const StepArgs& a, cudaStream_t s) {
     switch (h->g.C) {
-        case 1: return dispatch_norm_c<1>(h, a, out, s);
-        case 3: return dispatch_norm_c<3>(h, a, out, s);
-        default: return dispatch_norm_c<5>(h, a, out, s);
+        case 1: return dispatch_norm_c<1>(h, a, s);
+        case 3: return dispatch_norm_c<3>(h, a, s);
+        default: return dispatch_norm_c<5>(h, a, s);
     }
 }
 template <int C>
-static cudaError_t dispatch_scale_c(const gpe_handle* h, const StepArgs& a, const double* n, double dv, cudaStream_t s) {
-    return h->real_bytes == 8 ? launch_scale<double, C>(a, n, dv, s) : launch_scale<float, C>(a, n, dv, s);
+static cudaError_t dispatch_scale_c(const gpe_handle* h, const StepArgs& a, cudaStream_t s) {
+    return h->real_bytes == 8 ? launch_scale<double, C>(a, s) : launch_scale<float, C>(a, s);
 }
-static cudaError_t dispatch_scale(const gpe_handle* h, const StepArgs& a, const double* n, double dv, cudaStream_t s) {
+// a.next scaled by *a.scale_in
+static cudaError_t dispatch_scale(const gpe_handle* h, const StepArgs& a, cudaStream_t s) {
     switch (h->g.C) {
-        case 1: return dispatch_scale_c<1>(h, a, n, dv, s);
-        case 3: return dispatch_scale_c<3>(h, a, n, dv, s);
-        default: return dispatch_scale_c<5>(h, a, n, dv, s);
+        case 1: return dispatch_scale_c<1>(h, a, s);
+        case 3: return dispatch_scale_c<3>(h, a, s);
+        default: return dispatch_scale_c<5>(h, a, s);
     }
+}
+// The state in `slot` normalised to norm 1 (two launches).
+static cudaError_t normalize_slot(gpe_handle* h, int slot, cudaStream_t s) {
+    gpe_fields zero;
+    std::memset(&zero, 0, sizeof zero);
+    StepArgs a = make_args(h, zero, 0.0);
+    a.prev = a.next = h->interior[slot];
+    a.scale_in = a.scale_out = h->itp_scale;
+    cudaError_t e = dispatch_norm(h, a, s);
+    if (e == cudaSuccess) e = dispatch_scale(h, a, s);
+    h->launches += 2;
+    return e;
 }
 
 // Shape of the 2.5-D z-march kernel (T = 0: not used).
@@ -1612,6 +1631,78 @@ extern "C" gpe_status gpe_observe(gpe_handle* h, int32_t slot, double t, gpe_obs
     return fill_observables(h, r, out);
 }
 
+static cudaError_t dispatch_il_itp(const gpe_handle* h, const StepArgs& a, cudaStream_t s) {
+    switch (h->g.C) {
+        case 1: return launch_il_itp<1>(a, h->ilg, il_deg(h), h->partial_blocks, s);
+        case 3: return launch_il_itp<3>(a, h->ilg, il_deg(h), h->partial_blocks, s);
+        default: return launch_il_itp<5>(a, h->ilg, il_deg(h), h->partial_blocks, s);
+    }
+}
+
+// Whether the iterations of an imaginary-time call run in the interleaved layout:
+// the leapfrog's rule for a call of n steps, where the interleaved copies exist or
+// can be allocated now (gpe_itp needs no memory of its own otherwise, and a stream
+// that is being captured takes no allocation).
+static bool itp_interleaved(gpe_handle* h, int32_t n, cudaStream_t s) {
+    if (!use_interleaved(h, n)) return false;
+    if (!h->il[0] || !h->il[1]) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+    }
+    return ensure_il(h, s) == GPE_OK;
+}
+
+// n iterations of parabolic imaginary time (itp + normalisation,
+// Spin1GpeBCC.cu:1470-1473) from the newest psi slot, H psi left out.  Each is one
+// launch that also sums |next|^2: with FP32 storage the launch after it reads the
+// iterate times the normalisation factor, rounded as the normalised state would be
+// stored, and one pass at the end scales the last; FP64 storage, whose launches the
+// FP64 pipe bounds, scales after each.
+static gpe_status itp_iterations(gpe_handle* h, int32_t n, cudaStream_t s) {
+    gpe_fields zero;
+    std::memset(&zero, 0, sizeof zero);
+    const bool deferred = h->real_bytes == 4;
+    const bool il = deferred && itp_interleaved(h, n, s);
+    cudaError_t e;
+    if (il) {
+        e = launch_il_convert(h->interior[h->cur], h->g, h->il[h->cur], h->ilg, true, s);
+        if (e != cudaSuccess) return cuda_fail(e, "layout change (in)");
+        h->launches += 1;
+    }
+    StepArgs a = make_args(h, zero, 0.0);
+    for (int32_t k = 0; k < n; ++k) {
+        const int prev = h->cur, next = h->cur == GPE_PSI_EVEN ? GPE_PSI_ODD : GPE_PSI_EVEN;
+        a.prev = il ? h->il[prev] : h->interior[prev];
+        a.next = il ? h->il[next] : h->interior[next];
+        a.scale_in = deferred && k > 0 ? h->itp_scale + (k & 1) : nullptr;
+        a.scale_out = h->itp_scale + ((k + 1) & 1);
+        e = il ? dispatch_il_itp(h, a, s) : dispatch_parabolic(h, a, kModeItpNorm, s);
+        h->launches += 1;
+        h->epoch += 1;
+        if (e != cudaSuccess) return cuda_fail(e, "itp launch");
+        h->cur = next;
+        if (!deferred) {
+            a.scale_in = a.scale_out;
+            e = dispatch_scale(h, a, s);
+            h->launches += 1;
+            if (e != cudaSuccess) return cuda_fail(e, "itp scale");
+        }
+    }
+    if (il) {
+        e = launch_il_convert(h->interior[h->cur], h->g, h->il[h->cur], h->ilg, false, s);
+        if (e != cudaSuccess) return cuda_fail(e, "layout change (out)");
+        h->launches += 1;
+    }
+    if (deferred) {
+        a.next = h->interior[h->cur];
+        a.scale_in = a.scale_out;
+        e = dispatch_scale(h, a, s);
+        h->launches += 1;
+        if (e != cudaSuccess) return cuda_fail(e, "itp scale");
+    }
+    return GPE_OK;
+}
+
 extern "C" gpe_status gpe_itp(gpe_handle* h, int32_t n, double* mu_out, void* stream) {
     if (!h) return fail(GPE_ERR_INVALID_ARG, "null handle");
     if (h->p.scheme == GPE_SCHEME_SPLIT) return fail(GPE_ERR_UNSUPPORTED, "imaginary time is not built for the split scheme");
@@ -1621,20 +1712,21 @@ extern "C" gpe_status gpe_itp(gpe_handle* h, int32_t n, double* mu_out, void* st
     gpe_fields zero;
     std::memset(&zero, 0, sizeof zero);
     const double dv = cell_dv(h);
-    for (int32_t k = 0; k < n; ++k) {
+    int32_t k = 0;
+    if (h->p.scheme == GPE_SCHEME_PARABOLIC && n > 1) {
+        // the iterations whose H psi nobody sees
+        st = itp_iterations(h, n - 1, s);
+        if (st) return st;
+        k = n - 1;
+    }
+    for (; k < n; ++k) {
         const int prev = h->cur, next = h->cur == GPE_PSI_EVEN ? GPE_PSI_ODD : GPE_PSI_EVEN;
         // itp(H psi, next <- prev) then normalize(next) (Spin1GpeBCC.cu:1470-1473;
         // hyperbolic: itp_q + itp_psi, normalize_h, RelativisticSpin2Gpe.cu:1712-1715)
         st = one_step(h, next, prev, zero, 0.0, GPE_MODE_ITP, s);
         if (st) return st;
-        StepArgs a = make_args(h, zero, 0.0);
-        a.prev = h->interior[next];
-        a.next = h->interior[next];
-        cudaError_t e = dispatch_norm(h, a, h->obs_out, s);
-        if (e != cudaSuccess) return cuda_fail(e, "itp norm");
-        e = dispatch_scale(h, a, h->obs_out, dv, s);
-        if (e != cudaSuccess) return cuda_fail(e, "itp scale");
-        h->launches += 3;
+        cudaError_t e = normalize_slot(h, next, s);
+        if (e != cudaSuccess) return cuda_fail(e, "itp normalisation");
         h->cur = next;
     }
     if (mu_out) {
@@ -1642,13 +1734,14 @@ extern "C" gpe_status gpe_itp(gpe_handle* h, int32_t n, double* mu_out, void* st
         StepArgs a = make_args(h, zero, 0.0);
         a.prev = h->interior[h->cur];
         a.next = h->interior[GPE_HPSI];
-        cudaError_t e = launch_dot(a, h->p.precision, h->g.C, h->obs_out, s);
+        a.scale_out = h->itp_scale;
+        cudaError_t e = launch_dot(a, h->p.precision, h->g.C, s);
         if (e != cudaSuccess) return cuda_fail(e, "itp dot");
-        h->launches += 2;
-        double r[OBS_COUNT];
-        CUDA_TRY(cudaMemcpyAsync(r, h->obs_out, sizeof r, cudaMemcpyDeviceToHost, s));
+        h->launches += 1;
+        double r = 0;
+        CUDA_TRY(cudaMemcpyAsync(&r, &h->itp_scale->sum, sizeof r, cudaMemcpyDeviceToHost, s));
         CUDA_TRY(cudaStreamSynchronize(s));
-        *mu_out = r[OBS_NORM] * dv;
+        *mu_out = r * dv;
     }
     return GPE_OK;
 }
@@ -1952,11 +2045,8 @@ extern "C" gpe_status gpe_init_state(gpe_handle* h, int32_t slot, const gpe_init
     h->launches += 1;
     h->epoch += 1;
     if (init->normalize) {
-        a.prev = h->interior[slot];
-        e = dispatch_norm(h, a, h->obs_out, s);
-        if (e == cudaSuccess) e = dispatch_scale(h, a, h->obs_out, cell_dv(h), s);
+        e = normalize_slot(h, slot, s);
         if (e != cudaSuccess) return cuda_fail(e, "init normalisation");
-        h->launches += 3;
     }
     h->cur = slot;
     return GPE_OK;

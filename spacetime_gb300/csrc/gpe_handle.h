@@ -58,6 +58,7 @@ struct gpe_handle {
     double* partials = nullptr;
     size_t partial_blocks = 0;
     double* obs_out = nullptr;
+    gpe::ItpScale* itp_scale = nullptr;  // two: the iterations' factors in turn
     double* stage = nullptr;   // FP64 staging for uploads/downloads (allocated on first use)
     double* field_buf = nullptr;  // per-node output fields (gpe_node_fields; allocated on first use)
     size_t field_count = 0;

@@ -185,11 +185,14 @@ __device__ __forceinline__ bool il_lane_group(const ILGrid& G, uint32_t u, uint3
 // One lane's node of an interleaved leapfrog step: node l of cell gx CELLS + sub
 // of row (y, z), next <- next + 2 dt (-i H prev), with the arithmetic and its order of
 // parabolic_node_t + node_finish.  F: where the step's fields come from (P if
-// null); oa: where the observables of prev go.
+// null); oa: where the observables of prev go.  With a NormAcc for oa: an imaginary-
+// time iteration (kModeItpNorm), next = prev - dt H prev with prev read times inv.
 template <int C, int D, int CELLS, class OA>
 __device__ __forceinline__ void il_task(const ILGrid& G, const PhysR<float>& P, const PhysR<float>* F, const char* prev,
                                         char* next, const int32_t* off, const float* w, int nd, const float* pos,
-                                        uint32_t sub, uint32_t l, uint32_t gx, uint32_t y, uint32_t z, OA* oa) {
+                                        uint32_t sub, uint32_t l, uint32_t gx, uint32_t y, uint32_t z, OA* oa,
+                                        float inv = 1.f) {
+    constexpr bool kItp = std::is_same<OA, NormAcc<float>>::value;
     constexpr uint32_t kComp = CELLS * 8;   // bytes between a record's components
     const uint32_t x = gx * CELLS + sub;
     if (x >= G.X) return;
@@ -199,7 +202,7 @@ __device__ __forceinline__ void il_task(const ILGrid& G, const PhysR<float>& P, 
 #pragma unroll
     for (int s = 0; s < C; ++s) {
         prv[s] = ldc<float>(prev + own + s * kComp);
-        nv[s] = ldc_rw<float>(next + own + s * kComp);
+        if constexpr (!kItp) nv[s] = ldc_rw<float>(next + own + s * kComp);
     }
 #pragma unroll
     for (int s = 0; s < C; ++s) H[s] = cx<float>(0.f, 0.f);
@@ -224,18 +227,33 @@ __device__ __forceinline__ void il_task(const ILGrid& G, const PhysR<float>& P, 
             for (int s = 0; s < C; ++s) H[s] += w[k0 + k] * (v[k][s] - prv[s]);
         }
     }
+    if constexpr (kItp) {
+        scale_record(prv, C, inv);
+        scale_record(H, C, inv);
+    }
     // local terms and the leapfrog update, as node_finish
     float rr[3];
     rr[0] = P.p0[0] + P.bs * ((float)x * P.bw[0] + pos[0]);
     rr[1] = P.p0[1] + P.bs * ((float)y * P.bw[1] + pos[1]);
     rr[2] = P.p0[2] + P.bs * ((float)z * P.bw[2] + pos[2]);
     const float pot = trap<float>(P, rr, F);
+    if constexpr (kItp) {
+        local_terms<float, C>(P, rr, pot, GPE_MODE_ITP, false, prv, H, F);
+#pragma unroll
+        for (int s = 0; s < C; ++s) {
+            nv[s] = prv[s] - P.dt * H[s];
+            stc<float>(next + own + s * kComp, nv[s]);
+        }
+        oa->template add<C>(nv);
+        return;
+    } else {
     local_terms<float, C>(P, rr, pot, GPE_MODE_LEAPFROG, false, prv, H, F);
     if constexpr (!std::is_same<OA, NoObs>::value) oa->template node<float, C>(P, rr, prv, H);
 #pragma unroll
     for (int s = 0; s < C; ++s) {
         nv[s] += (2.f * P.dt) * cx<float>(H[s].y, -H[s].x);
         stc<float>(next + own + s * kComp, nv[s]);
+    }
     }
 }
 
@@ -246,6 +264,9 @@ __host__ __device__ inline uint32_t il_warp_tasks(const ILGrid& G) {
     return (G.Y * G.Z * G.GX + wg - 1) / wg;
 }
 
+constexpr unsigned kIlPlainThreads = 128;
+constexpr unsigned kIlObsThreads = 256;
+
 // One FP32 leapfrog step in the interleaved layout: next <- next + 2 dt (-i H prev).
 // D = 4: every node has 4 stencil entries (BCC, A15, C15, Z); D = 8: rows of 4 or 8
 // entries (FCC's tetrahedra and octahedra).  Warp task t = u V + l: node l of the
@@ -253,14 +274,16 @@ __host__ __device__ inline uint32_t il_warp_tasks(const ILGrid& G) {
 // of V, so a warp keeps its node, and with it its entries and position, in
 // registers; the row length is the same in every lane of a warp, so the second
 // group of 4 entries is a uniform branch.  OBS: the observables of prev are summed
-// on the way (ObsAcc, as the gather kernels' observed step).
-template <int C, int D, int CELLS, bool OBS>
+// on the way (ObsAcc, as the gather kernels' observed step).  MODE kModeItpNorm: an
+// imaginary-time iteration instead.
+template <int C, int D, int CELLS, bool OBS, int MODE = GPE_MODE_LEAPFROG>
 __device__ __forceinline__ void il_step_body(const StepArgs& a, const ILGrid& G, uint32_t tasks, FastDiv dGX) {
     static_assert(D == 4 || D == 8, "rows of 4, or of 4 and 8 entries");
     const PhysR<float>& P = make_phys<float>(a);
-    using OA = typename ObsOf<OBS, float>::type;
+    using OA = typename AccOf<MODE, OBS, float>::type;
     __shared__ double obs_sums[OBS ? kObsSums * 256 : 1];
-    OA oa = ObsOf<OBS, float>::make(obs_sums);
+    OA oa = AccOf<MODE, OBS, float>::make(obs_sums);
+    const float inv = MODE == kModeItpNorm && a.scale_in ? a.scale_in->inv : 1.f;
     const uint32_t sub = threadIdx.x & (CELLS - 1);
     const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
@@ -282,11 +305,15 @@ __device__ __forceinline__ void il_step_body(const StepArgs& a, const ILGrid& G,
         const uint32_t u = fdiv(t, a.divV);
         uint32_t gx, y, z;
         if (il_lane_group<CELLS>(G, u, nq, 0, dGX, a.divY, gx, y, z))
-            il_task<C, D, CELLS, OA>(G, P, nullptr, a.prev, a.next, off, w, nd, pos, sub, l, gx, y, z, &oa);
+            il_task<C, D, CELLS, OA>(G, P, nullptr, a.prev, a.next, off, w, nd, pos, sub, l, gx, y, z, &oa, inv);
     }
     if constexpr (OBS) {
         __shared__ double red[8][OBS_COUNT];
         oa.block_reduce(red, a.partials);
+    }
+    if constexpr (MODE == kModeItpNorm) {
+        __shared__ double nred[kIlPlainThreads / 32];
+        oa.finish(nred, a.partials, a.dv, a.scale_out);
     }
 }
 
@@ -294,8 +321,6 @@ __device__ __forceinline__ void il_step_body(const StepArgs& a, const ILGrid& G,
 // IlBounds<C>::kMin of them per SM (the register cap that keeps the most warps in
 // flight without spills), the observed step in blocks of 256 (its FP64 sums take
 // shared memory per thread).
-constexpr unsigned kIlPlainThreads = 128;
-constexpr unsigned kIlObsThreads = 256;
 template <int C, int D>
 struct IlBounds {
     // D = 4: spin-1 BCC 96^3 (the cap 7 blocks lets it use 64 registers, 8 blocks):
@@ -320,22 +345,23 @@ __global__ void __launch_bounds__(kIlObsThreads, IlBounds<C, D>::kMinObs) il_ste
     il_step_body<C, D, CELLS, true>(a, G, tasks, dGX);
 }
 
+// One imaginary-time iteration of gpe_itp before its last: next = prev - dt H prev
+// with prev read times the factor of the normalisation before (a.scale_in), the sum
+// |next|^2 and the next factor left in a.scale_out.  Reads prev and writes next, 16 C
+// bytes per site, where the separate step, norm and scale passes of the handle's
+// layout move 48 C.
+template <int C, int D, int CELLS>
+__global__ void __launch_bounds__(kIlPlainThreads, IlBounds<C, D>::kMin) il_itp_kernel(StepArgs a, ILGrid G, uint32_t tasks,
+                                                                                   FastDiv dGX) {
+    il_step_body<C, D, CELLS, false, kModeItpNorm>(a, G, tasks, dGX);
+}
+
 // Blocks of one interleaved step (rows of D entries at most): one wave at the
 // kernel's occupancy or one warp per task if that is fewer, as a multiple of m =
 // V / gcd(V, warps per block) (the grid's warp count a multiple of V), and at most
 // `max_blocks` (the handle's partial-sum rows); 0 if no such grid.
-template <int C, int D, int CELLS>
-unsigned il_blocks_d(const ILGrid& G, bool obs, size_t max_blocks) {
-    static int occ[2] = {0, 0};
-    const unsigned threads = obs ? kIlObsThreads : kIlPlainThreads;
+inline unsigned il_wave(const ILGrid& G, unsigned threads, int occ, size_t max_blocks) {
     const unsigned wpb = threads / 32;
-    int& o = occ[obs ? 1 : 0];
-    if (o == 0) {
-        auto k = obs ? il_step_obs_kernel<C, D, CELLS> : il_step_kernel<C, D, CELLS>;
-        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, obs ? 50 : 0);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k, (int)threads, 0);
-        if (o < 1) o = 1;
-    }
     uint32_t gv = G.V, gb = wpb;
     while (gb) {
         const uint32_t r = gv % gb;
@@ -344,12 +370,26 @@ unsigned il_blocks_d(const ILGrid& G, bool obs, size_t max_blocks) {
     }
     const uint64_t m = G.V / gv;
     const uint64_t tasks = (uint64_t)il_warp_tasks(G) * G.V;
-    uint64_t nb = std::min<uint64_t>((uint64_t)o * (unsigned)device_sm_count(), (tasks + wpb - 1) / wpb);
+    uint64_t nb = std::min<uint64_t>((uint64_t)occ * (unsigned)device_sm_count(), (tasks + wpb - 1) / wpb);
     // rounded down (a block past the wave would start only when another ends);
     // grids of fewer tasks than m blocks' warps take m blocks, some warps idle
     nb = nb >= m ? nb / m * m : m;
     if (nb > max_blocks) nb = max_blocks / m * m;
     return (unsigned)nb;
+}
+
+template <int C, int D, int CELLS>
+unsigned il_blocks_d(const ILGrid& G, bool obs, size_t max_blocks) {
+    static int occ[2] = {0, 0};
+    const unsigned threads = obs ? kIlObsThreads : kIlPlainThreads;
+    int& o = occ[obs ? 1 : 0];
+    if (o == 0) {
+        auto k = obs ? il_step_obs_kernel<C, D, CELLS> : il_step_kernel<C, D, CELLS>;
+        cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, obs ? 50 : 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k, (int)threads, 0);
+        if (o < 1) o = 1;
+    }
+    return il_wave(G, threads, o, max_blocks);
 }
 
 template <int C>
@@ -390,8 +430,35 @@ cudaError_t launch_il_step(const StepArgs& a, const ILGrid& G, int deg, size_t m
     return cudaErrorInvalidValue;
 }
 
+template <int C, int D, int CELLS>
+cudaError_t launch_il_itp_d(const StepArgs& a, const ILGrid& G, size_t max_blocks, cudaStream_t s) {
+    static int occ = 0;
+    if (occ == 0) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, il_itp_kernel<C, D, CELLS>, (int)kIlPlainThreads, 0);
+        if (occ < 1) occ = 1;
+    }
+    const unsigned nb = il_wave(G, kIlPlainThreads, occ, max_blocks);
+    if (nb == 0) return cudaErrorInvalidConfiguration;
+    il_itp_kernel<C, D, CELLS><<<nb, kIlPlainThreads, 0, s>>>(a, G, il_warp_tasks(G) * G.V, make_fastdiv(G.GX));
+    return cudaGetLastError();
+}
+
+// One imaginary-time iteration (a.prev / a.next: interleaved buffers).
+template <int C>
+cudaError_t launch_il_itp(const StepArgs& a, const ILGrid& G, int deg, size_t max_blocks, cudaStream_t s) {
+    if (G.cells == 32) {
+        if (deg == 4) return launch_il_itp_d<C, 4, 32>(a, G, max_blocks, s);
+        if (deg == 8) return launch_il_itp_d<C, 8, 32>(a, G, max_blocks, s);
+    } else if (G.cells == 16) {
+        if (deg == 4) return launch_il_itp_d<C, 4, 16>(a, G, max_blocks, s);
+        if (deg == 8) return launch_il_itp_d<C, 8, 16>(a, G, max_blocks, s);
+    }
+    return cudaErrorInvalidValue;
+}
+
 #define GPE_INSTANTIATE_IL(C)                                                                                           \
     template cudaError_t launch_il_step<C>(const StepArgs&, const ILGrid&, int, size_t, bool, double*, cudaStream_t); \
+    template cudaError_t launch_il_itp<C>(const StepArgs&, const ILGrid&, int, size_t, cudaStream_t);                 \
     template unsigned il_blocks<C>(const ILGrid&, int, bool, size_t);                                                 \
     template cudaError_t launch_il_hyper<C>(const StepArgs&, const ILGrid&, const ILGrid&, const int32_t*, cudaStream_t);
 

@@ -20,15 +20,15 @@ GPE_INSTANTIATE_HYPER_TILE(double, 1)
 template cudaError_t launch_split<float>(const StepArgs&, int, double, cudaStream_t);
 template cudaError_t launch_split<double>(const StepArgs&, int, double, cudaStream_t);
 
-cudaError_t launch_dot(const StepArgs& a, int precision, int C, double* out, cudaStream_t s) {
+cudaError_t launch_dot(const StepArgs& a, int precision, int C, cudaStream_t s) {
     if (precision == GPE_FP64) {
-        if (C == 1) return launch_dot_t<double, 1>(a, out, s);
-        if (C == 3) return launch_dot_t<double, 3>(a, out, s);
-        return launch_dot_t<double, 5>(a, out, s);
+        if (C == 1) return launch_dot_t<double, 1>(a, s);
+        if (C == 3) return launch_dot_t<double, 3>(a, s);
+        return launch_dot_t<double, 5>(a, s);
     }
-    if (C == 1) return launch_dot_t<float, 1>(a, out, s);
-    if (C == 3) return launch_dot_t<float, 3>(a, out, s);
-    return launch_dot_t<float, 5>(a, out, s);
+    if (C == 1) return launch_dot_t<float, 1>(a, s);
+    if (C == 3) return launch_dot_t<float, 3>(a, s);
+    return launch_dot_t<float, 5>(a, s);
 }
 
 cudaError_t launch_pack_any(int precision, double* packed, char* dev_base, uint32_t X, uint32_t Y, uint32_t Z,

@@ -18,6 +18,21 @@ namespace gpe {
 // reads the old value from StepArgs::hpsi and writes next, leaving the old buffer
 // as it was (the adjoint's recomputation keeps every state of a segment).
 constexpr int kModeLeapfrogFrom = 3;
+// An imaginary-time step that also sums |next|^2 (ItpScale): the iterations of
+// gpe_itp before its last.  FP32: prev is read times ItpScale::inv, so that the
+// normalisation of the iteration before needs no pass of its own.
+constexpr int kModeItpNorm = 4;
+
+// The normalisation of one imaginary-time iterate: sum |psi|^2 over the nodes, the
+// factor sqrt(sum dv) the state is divided by and (FP32 storage) its reciprocal
+// rounded once; written by the last block of a NormAcc kernel (`count` blocks
+// arrived so far, zero between launches).
+struct ItpScale {
+    double sum;
+    double sq;
+    float inv;
+    uint32_t count;
+};
 
 constexpr int kMaxNodes = 160;
 constexpr int kMaxEntries = 640;
@@ -199,6 +214,9 @@ struct StepArgs {
     uint32_t row_items_e; // X*E
     uint64_t total;       // total threads of work
     double* partials;     // observables
+    double dv;            // bs0^3 VOLUME
+    const ItpScale* scale_in;  // kModeItpNorm, FP32: the scale of prev (null: 1)
+    ItpScale* scale_out;       // NormAcc kernels: the scale of what was summed
     int* err;             // device error flag (bounded waits that ran out)
 };
 

@@ -545,6 +545,130 @@ struct ObsOf<true, R> {
     __device__ static ObsAcc<R> make(double* sums) { return ObsAcc<R>(sums); }
 };
 
+// A sum of products of FP32 values kept as an unevaluated pair of FP32 values: each
+// product is split exactly by a fused multiply-add, each addition's rounding error
+// is recovered exactly (Knuth's two-sum), and only the sum of those errors is
+// rounded (Ogita, Rump and Oishi, "Accurate sum and dot product", 2005), to about
+// n 2^-48 of the sum of magnitudes of a thread's n terms at worst, sqrt(n) times less
+// in practice.  GB300 runs 64 FP32 operations for each FP64 one, and its conversions from
+// FP32 share the FP64 pipe.
+struct PairSum {
+    float h, l;
+    __device__ __forceinline__ PairSum() : h(0.f), l(0.f) {}
+    __device__ __forceinline__ void add(float v) {
+        const float s = __fadd_rn(h, v), b = __fsub_rn(s, h);
+        l = __fadd_rn(l, __fadd_rn(__fsub_rn(h, __fsub_rn(s, b)), __fsub_rn(v, b)));
+        h = s;
+    }
+    __device__ __forceinline__ void add_prod(float a, float b) {
+        const float p = __fmul_rn(a, b);
+        l = __fadd_rn(l, __fmaf_rn(a, b, -p));
+        add(p);
+    }
+    // (an overflow or an infinity leaves NaN in l)
+    __device__ __forceinline__ double value() const { return isfinite(l) ? (double)h + (double)l : (double)h; }
+    // the sum over the warp's lanes, in lane 0
+    __device__ __forceinline__ void warp_sum() {
+        for (int o = 16; o > 0; o >>= 1) {
+            const float uh = __shfl_down_sync(0xffffffffu, h, o), ul = __shfl_down_sync(0xffffffffu, l, o);
+            add(uh);
+            l = __fadd_rn(l, ul);
+        }
+    }
+};
+
+// Sum of |v|^2 over the records a thread passes to add(), the per-node terms in R
+// and their sum in FP64 (FP64 storage) or as a pair of FP32 values (PairSum: no FP64
+// operation per node), and the normalisation factor from the whole grid's sum: every
+// block writes its FP64 sum to partials[blockIdx.x] and the last block to arrive adds
+// them in an order that depends only on the grid and writes *out, so no launch is
+// spent on it (a one-block finalize launch took 36 us of a 290 us iteration on
+// spin-1 BCC 72^3).
+template <typename R>
+struct NormAcc {
+    double acc;
+    PairSum pair;
+    __device__ __forceinline__ NormAcc() : acc(0.0) {}
+    template <int C>
+    __device__ __forceinline__ void add(const Cx<R>* v) {
+        R n2 = 0;
+#pragma unroll
+        for (int s = 0; s < C; ++s) n2 += v[s].x * v[s].x + v[s].y * v[s].y;
+        if constexpr (sizeof(R) == 4) pair.add(n2);
+        else acc += n2;
+    }
+    // every thread of the block must call it; red: a double per warp of the block
+    __device__ __forceinline__ void finish(double* red, double* partials, double dv, ItpScale* out) {
+        if constexpr (sizeof(R) == 4) {
+            pair.warp_sum();
+            acc = pair.value();
+        } else {
+            acc = warp_sum(acc);
+        }
+        grid_sum(acc, red, partials, dv, out);
+    }
+    __device__ static __forceinline__ double warp_sum(double v) {
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        return v;
+    }
+    // v: the warp's sum, in its lane 0
+    __device__ static __forceinline__ void grid_sum(double v, double* red, double* partials, double dv, ItpScale* out) {
+        const double s = block_sum(v, red);
+        __shared__ bool last;
+        if (threadIdx.x == 0) {
+            partials[blockIdx.x] = s;
+            __threadfence();
+            last = atomicAdd(&out->count, 1u) == gridDim.x - 1;
+        }
+        __syncthreads();
+        if (!last) return;
+        __threadfence();
+        // four loads in flight per thread: the chain of L2 latencies is the last block's time
+        double t[4] = {0.0, 0.0, 0.0, 0.0};
+        for (uint32_t b = threadIdx.x; b < gridDim.x; b += 4 * blockDim.x) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (b + k * blockDim.x < gridDim.x) t[k] += __ldcg(partials + b + k * blockDim.x);
+        }
+        const double sum = block_sum(warp_sum((t[0] + t[1]) + (t[2] + t[3])), red);
+        if (threadIdx.x == 0) {
+            out->sum = sum;
+            out->sq = sqrt(sum * dv);
+            out->inv = (float)(1.0 / out->sq);
+            out->count = 0;
+        }
+    }
+    // the sum of the warps' sums, in thread 0
+    __device__ static __forceinline__ double block_sum(double v, double* red) {
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v += red[w];
+        return v;
+    }
+};
+
+// What a step kernel of MODE sums on the way: NormAcc (kModeItpNorm), else ObsOf.
+template <int MODE, bool OBS, typename R>
+struct AccOf {
+    using type = typename ObsOf<OBS, R>::type;
+    __device__ static type make(double* sums) { return ObsOf<OBS, R>::make(sums); }
+};
+template <bool OBS, typename R>
+struct AccOf<kModeItpNorm, OBS, R> {
+    using type = NormAcc<R>;
+    __device__ static type make(double*) { return NormAcc<R>(); }
+};
+
+// The previous iterate's record times its normalisation factor (kModeItpNorm),
+// rounded as the normalised state would be stored (no fused multiply-add with what
+// follows); the Laplacian, linear in it, is scaled once as a whole.
+__device__ __forceinline__ void scale_record(Cx<float>* v, int C, float inv) {
+#pragma unroll
+    for (int s = 0; s < C; ++s) v[s] = cx<float>(__fmul_rn(inv, v[s].x), __fmul_rn(inv, v[s].y));
+}
+
 // The local terms and the time update of one node, given its Laplacian sum in H
 // (Spin1GpeBCC.cu:867-916).  nv: the old next record (leapfrog).  oa: where the
 // observables of prv go (ObsAcc), or nothing (NoObs).
@@ -557,6 +681,14 @@ __device__ __forceinline__ void node_finish(const PhysR<R>& P, const R pos[3], u
     r[1] = P.p0[1] + P.bs * ((R)y * P.bw[1] + pos[1]);
     r[2] = P.p0[2] + P.bs * ((R)z * P.bw[2] + pos[2]);
     const R pot = trap<R>(P, r, F);
+    if constexpr (MODE == kModeItpNorm) {
+        local_terms<R, C>(P, r, pot, GPE_MODE_ITP, false, prv, H, F);
+#pragma unroll
+        for (int s = 0; s < C; ++s) nv[s] = prv[s] - P.dt * H[s];
+        st_node<R, C>(nxt, nv);
+        oa->template add<C>(nv);
+        return;
+    } else {
     local_terms<R, C>(P, r, pot, MODE, false, prv, H, F);
     if constexpr (!std::is_same<OA, NoObs>::value) oa->template node<R, C>(P, r, prv, H);
     if constexpr (MODE == GPE_MODE_LEAPFROG || MODE == kModeLeapfrogFrom) {
@@ -566,6 +698,7 @@ __device__ __forceinline__ void node_finish(const PhysR<R>& P, const R pos[3], u
         st_node<R, C>(nxt, nv);
     } else {
         write_update<R, C>(MODE, P.dt, nxt, hp, prv, H);
+    }
     }
 }
 
@@ -580,7 +713,9 @@ __device__ __forceinline__ void parabolic_node_t(const Grid& g, const NodeTab<R,
                                                  const char* prev, char* next, char* hpsi, uint32_t x, uint32_t y,
                                                  uint32_t z, uint32_t l, const SmemTables<R>* st = nullptr,
                                                  int f_more = 0, int f_end = 0, const PhysR<R>* F = nullptr,
-                                                 OA* oa = nullptr) {
+                                                 OA* oa = nullptr, R inv = (R)1) {
+    // FP32 imaginary time: prev is read scaled (kModeItpNorm)
+    constexpr bool kScale = MODE == kModeItpNorm && sizeof(R) == 4;
     const size_t cell_off = (size_t)z * g.slice + (size_t)y * g.pitch + (size_t)x * g.cell_bytes;
     const char* base = prev + cell_off;
     const uint32_t node_bytes = C * 2 * sizeof(R);
@@ -628,11 +763,15 @@ __device__ __forceinline__ void parabolic_node_t(const Grid& g, const NodeTab<R,
                 for (int k = 0; k < G; ++k) ld_node<R, C, true>(base + o[h + k], v[k]);
 #pragma unroll
                 for (int k = 0; k < G; ++k) {
-#pragma unroll
+    #pragma unroll
                     for (int s = 0; s < C; ++s) H[s] += w[h + k] * (v[k][s] - prv[s]);
                 }
             }
         }
+    }
+    if constexpr (kScale) {
+        scale_record(prv, C, inv);
+        scale_record(H, C, inv);
     }
     char* hp = (MODE == GPE_MODE_ITP && hpsi) ? hpsi + cell_off + l * node_bytes : nullptr;
     node_finish<R, C, MODE, OA>(P, t.pos, x, y, z, prv, H, nv, nxt, hp, F, oa);
@@ -647,14 +786,15 @@ __device__ __forceinline__ void parabolic_node_t(const Grid& g, const NodeTab<R,
 template <typename R, int C, int MODE, int D = 0, int G = D, bool MORE = false, class OA = NoObs>
 __device__ __forceinline__ void parabolic_node(const Grid& g, const SmemTables<R>& st, const PhysR<R>& P, const char* prev,
                                                char* next, char* hpsi, uint32_t x, uint32_t y, uint32_t z, uint32_t l,
-                                               const PhysR<R>* F = nullptr, OA* oa = nullptr) {
+                                               const PhysR<R>* F = nullptr, OA* oa = nullptr, R inv = (R)1) {
+    constexpr bool kScale = MODE == kModeItpNorm && sizeof(R) == 4;
     if constexpr (D > 0 && MORE) {
         const int f0 = st.row_ptr[l];
         parabolic_node_t<R, C, MODE, D, G, true, OA>(g, node_tab<R, D>(st, l, f0), P, prev, next, hpsi, x, y, z, l, &st,
-                                                     f0 + D, st.row_ptr[l + 1], F, oa);
+                                                     f0 + D, st.row_ptr[l + 1], F, oa, inv);
     } else if constexpr (D > 0) {
         parabolic_node_t<R, C, MODE, D, G, false, OA>(g, node_tab<R, D>(st, l), P, prev, next, hpsi, x, y, z, l, nullptr, 0,
-                                                      0, F, oa);
+                                                      0, F, oa, inv);
     } else {
         const size_t cell_off = (size_t)z * g.slice + (size_t)y * g.pitch + (size_t)x * g.cell_bytes;
         const char* base = prev + cell_off;
@@ -679,7 +819,7 @@ __device__ __forceinline__ void parabolic_node(const Grid& g, const SmemTables<R
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     if (f + k < f1) {
-                        const R w = st.w[f + k];
+                                const R w = st.w[f + k];
 #pragma unroll
                         for (int s = 0; s < C; ++s) H[s] += w * (v[k][s] - prv[s]);
                     }
@@ -695,6 +835,10 @@ __device__ __forceinline__ void parabolic_node(const Grid& g, const SmemTables<R
             }
         }
         const R pos[3] = {st.pos[3 * l + 0], st.pos[3 * l + 1], st.pos[3 * l + 2]};
+        if constexpr (kScale) {
+            scale_record(prv, C, inv);
+            scale_record(H, C, inv);
+        }
         char* hp = (MODE == GPE_MODE_ITP && hpsi) ? hpsi + cell_off + l * node_bytes : nullptr;
         node_finish<R, C, MODE, OA>(P, pos, x, y, z, prv, H, nv, nxt, hp, F, oa);
     }
@@ -708,9 +852,10 @@ __device__ __forceinline__ void parabolic_step_body(const StepArgs& a) {
     load_tables<R>(st, a);
     __syncthreads();
     const PhysR<R>& P = make_phys<R>(a);
-    using OA = typename ObsOf<OBS, R>::type;
+    using OA = typename AccOf<MODE, OBS, R>::type;
     __shared__ double obs_sums[OBS ? kObsSums * 256 : 1];
-    OA oa = ObsOf<OBS, R>::make(obs_sums);
+    OA oa = AccOf<MODE, OBS, R>::make(obs_sums);
+    const R inv = MODE == kModeItpNorm && a.scale_in ? (R)a.scale_in->inv : (R)1;
     for (uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < a.total;
          gid += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t i = (uint32_t)gid;
@@ -720,11 +865,15 @@ __device__ __forceinline__ void parabolic_step_body(const StepArgs& a) {
         const uint32_t l = within - x * a.g.V;
         const uint32_t z = fdiv(row, a.divY);
         const uint32_t y = row - z * a.g.Y;
-        parabolic_node<R, C, MODE, D, D, false, OA>(a.g, st, P, a.prev, a.next, a.hpsi, x, y, z, l, nullptr, &oa);
+        parabolic_node<R, C, MODE, D, D, false, OA>(a.g, st, P, a.prev, a.next, a.hpsi, x, y, z, l, nullptr, &oa, inv);
     }
     if constexpr (OBS) {
         __shared__ double red[8][OBS_COUNT];
         oa.block_reduce(red, a.partials);
+    }
+    if constexpr (MODE == kModeItpNorm) {
+        __shared__ double nred[8];
+        oa.finish(nred, a.partials, a.dv, a.scale_out);
     }
 }
 template <typename R, int C, int MODE, int D>
@@ -748,11 +897,13 @@ __device__ __forceinline__ void parabolic_fixed_body(const StepArgs& a) {
     load_tables<R>(st, a);
     __syncthreads();
     const PhysR<R>& P = make_phys<R>(a);
-    using OA = typename ObsOf<OBS, R>::type;
+    constexpr bool kAll = OBS || MODE == kModeItpNorm;   // every thread takes part in the block's sums
+    using OA = typename AccOf<MODE, OBS, R>::type;
     __shared__ double obs_sums[OBS ? kObsSums * 256 : 1];
-    OA oa = ObsOf<OBS, R>::make(obs_sums);
+    OA oa = AccOf<MODE, OBS, R>::make(obs_sums);
+    const R inv = MODE == kModeItpNorm && a.scale_in ? (R)a.scale_in->inv : (R)1;
     uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (!OBS && gid >= a.total) return;
+    if (!kAll && gid >= a.total) return;
     const uint32_t l = (uint32_t)gid - fdiv((uint32_t)gid, a.divV) * a.g.V;
     const int f0 = MORE ? st.row_ptr[l] : (int)l * D;
     const int f_end = MORE ? st.row_ptr[l + 1] : 0;
@@ -764,11 +915,15 @@ __device__ __forceinline__ void parabolic_fixed_body(const StepArgs& a) {
         const uint32_t z = fdiv(row, a.divY);
         const uint32_t y = row - z * a.g.Y;
         parabolic_node_t<R, C, MODE, D, G, MORE, OA>(a.g, t, P, a.prev, a.next, a.hpsi, x, y, z, l, &st, f0 + D, f_end,
-                                                     nullptr, &oa);
+                                                     nullptr, &oa, inv);
     }
     if constexpr (OBS) {
         __shared__ double red[8][OBS_COUNT];
         oa.block_reduce(red, a.partials);
+    }
+    if constexpr (MODE == kModeItpNorm) {
+        __shared__ double nred[8];
+        oa.finish(nred, a.partials, a.dv, a.scale_out);
     }
 }
 template <typename R, int C, int MODE, int D, int G, bool MORE>
@@ -1197,19 +1352,13 @@ static __global__ void __launch_bounds__(256) observe_finalize_kernel(const doub
     }
 }
 
-// The squared norm sum_nodes |psi|^2 of a psi buffer alone (density + integrate,
-// Spin1GpeBCC.cu:191-211, 328-348, for normalize_h :955-975): grid-stride, whole-
-// record loads, the per-node terms in the storage precision (FP32 storage: groups
-// of 8 nodes summed in FP32, each group added in FP64), FP64 block sums written to
-// the OBS_NORM column of the partials (the other columns zero) for
-// observe_finalize_kernel.
+// The normalisation of a psi buffer (density + integrate, Spin1GpeBCC.cu:191-211,
+// 328-348, for normalize_h :955-975): grid-stride, whole-record loads, NormAcc's
+// sums and factor.
 template <typename R, int C>
 __global__ void __launch_bounds__(256) norm_kernel(StepArgs a) {
     __shared__ double red[8];
-    constexpr int kGroup = sizeof(R) == 4 ? 8 : 1;
-    double acc = 0.0;
-    R grp = (R)0;
-    int in_group = 0;
+    NormAcc<R> acc;
     const uint32_t node_bytes = C * 2 * sizeof(R);
     for (uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < a.total;
          gid += (uint64_t)gridDim.x * blockDim.x) {
@@ -1223,61 +1372,40 @@ __global__ void __launch_bounds__(256) norm_kernel(StepArgs a) {
         Cx<R> v[C];
         ld_node<R, C, true>(a.prev + (size_t)z * a.g.slice + (size_t)y * a.g.pitch + (size_t)x * a.g.cell_bytes +
                                 l * node_bytes, v);
-        R n2 = 0;
-#pragma unroll
-        for (int s = 0; s < C; ++s) n2 += v[s].x * v[s].x + v[s].y * v[s].y;
-        grp += n2;
-        if (++in_group == kGroup) {
-            acc += (double)grp;
-            grp = (R)0;
-            in_group = 0;
-        }
+        acc.template add<C>(v);
     }
-    acc += (double)grp;
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) red[warp] = acc;
-    __syncthreads();
-    if (threadIdx.x < OBS_COUNT) {
-        double v = 0.0;
-        if (threadIdx.x == OBS_NORM)
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += red[w];
-        a.partials[(size_t)blockIdx.x * OBS_COUNT + threadIdx.x] = v;
-    }
+    acc.finish(red, a.partials, a.dv, a.scale_out);
 }
 
-// Scale every interior value of a psi buffer by 1/sqrt(norm) where norm is read
-// from device memory (normalize, Spin1GpeBCC.cu:412-434: FP64 storage divides by
-// the square root as the reference does; FP32 storage multiplies by its
-// reciprocal, computed in FP64 and rounded once).
+// Scale every interior value of a psi buffer by the factor of a.scale_in
+// (normalize, Spin1GpeBCC.cu:412-434: FP64 storage divides by the square root as
+// the reference does; FP32 storage multiplies by its reciprocal, computed in FP64
+// and rounded once).  The factor is computed once per normalisation: a square root
+// and a division in FP64 per thread took this pass from 25 to 125 us on spin-1 BCC
+// 72^3.
 template <typename R, int C>
-__global__ void __launch_bounds__(256) scale_kernel(StepArgs a, const double* norm_sum, double dv) {
-    const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid >= a.total) return;
-    const uint32_t i = (uint32_t)gid;
-    const uint32_t row = fdiv(i, a.divRow);
-    const uint32_t within = i - row * a.row_items;
-    const uint32_t x = fdiv(within, a.divV);
-    const uint32_t l = within - x * a.g.V;
-    const uint32_t z = fdiv(row, a.divY);
-    const uint32_t y = row - z * a.g.Y;
-    const size_t cell_off = (size_t)z * a.g.slice + (size_t)y * a.g.pitch + (size_t)x * a.g.cell_bytes;
-    char* p = a.next + cell_off + l * (C * 2 * sizeof(R));
-    const double sq = sqrt(norm_sum[OBS_NORM] * dv);
-    if constexpr (sizeof(R) == 8) {
-#pragma unroll
-        for (int s = 0; s < C; ++s) {
-            Cx<R> v = ldc_rw<R>(p + s * 2 * sizeof(R));
-            v.x = v.x / sq;
-            v.y = v.y / sq;
-            stc<R>(p + s * 2 * sizeof(R), v);
-        }
-    } else {
-        const R inv = (R)(1.0 / sq);
+__global__ void __launch_bounds__(256) scale_kernel(StepArgs a) {
+    const double sq = a.scale_in->sq;
+    const float inv = a.scale_in->inv;
+    for (uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < a.total;
+         gid += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t i = (uint32_t)gid;
+        const uint32_t row = fdiv(i, a.divRow);
+        const uint32_t within = i - row * a.row_items;
+        const uint32_t x = fdiv(within, a.divV);
+        const uint32_t l = within - x * a.g.V;
+        const uint32_t z = fdiv(row, a.divY);
+        const uint32_t y = row - z * a.g.Y;
+        char* p = a.next + (size_t)z * a.g.slice + (size_t)y * a.g.pitch + (size_t)x * a.g.cell_bytes +
+                  l * (C * 2 * sizeof(R));
         Cx<R> v[C];
         ld_node<R, C, false>(p, v);
+        if constexpr (sizeof(R) == 8) {
 #pragma unroll
-        for (int s = 0; s < C; ++s) v[s] = inv * v[s];
+            for (int s = 0; s < C; ++s) v[s] = cx<R>(v[s].x / sq, v[s].y / sq);
+        } else {
+            scale_record(v, C, inv);
+        }
         st_node<R, C>(p, v);
     }
 }
@@ -1293,7 +1421,10 @@ cudaError_t launch_parabolic_m(const StepArgs& a, cudaStream_t s, unsigned* grid
     if constexpr (D > 0) {
         // the largest multiple of V / gcd(V, 256) blocks within one wave: the grid
         // stride is then a multiple of V
-        auto kf = OBS ? parabolic_fixed_obs_kernel<R, C, MODE, D, G, MORE> : parabolic_fixed_kernel<R, C, MODE, D, G, MORE>;
+        auto kf = [] {
+            if constexpr (OBS) return &parabolic_fixed_obs_kernel<R, C, MODE, D, G, MORE>;
+            else return &parabolic_fixed_kernel<R, C, MODE, D, G, MORE>;
+        }();
         static int occ_f = 0;
         if (occ_f == 0) {
             // a small shared-memory share leaves the rest of L1 to cache the gathers; the
@@ -1320,7 +1451,10 @@ cudaError_t launch_parabolic_m(const StepArgs& a, cudaStream_t s, unsigned* grid
     // grids smaller than V / gcd(V, 256) blocks: the grid-stride kernel (the
     // 4-entry form where every node has 4 entries)
     constexpr int DS = (D == 4 && !MORE) ? 4 : 0;
-    auto ks = OBS ? parabolic_step_obs_kernel<R, C, MODE, DS> : parabolic_step_kernel<R, C, MODE, DS>;
+    auto ks = [] {
+        if constexpr (OBS) return &parabolic_step_obs_kernel<R, C, MODE, DS>;
+        else return &parabolic_step_kernel<R, C, MODE, DS>;
+    }();
     static int occ = 0;
     if (occ == 0) {
         // a small shared-memory share leaves the rest of L1 to cache the gathers
@@ -1340,6 +1474,7 @@ cudaError_t launch_parabolic_d(const StepArgs& a, int mode, cudaStream_t s) {
         case GPE_MODE_LEAPFROG: return launch_parabolic_m<R, C, GPE_MODE_LEAPFROG, D, G, MORE>(a, s);
         case GPE_MODE_EULER: return launch_parabolic_m<R, C, GPE_MODE_EULER, D, G, MORE>(a, s);
         case kModeLeapfrogFrom: return launch_parabolic_m<R, C, kModeLeapfrogFrom, D, G, MORE>(a, s);
+        case kModeItpNorm: return launch_parabolic_m<R, C, kModeItpNorm, D, G, MORE>(a, s);
         default: return launch_parabolic_m<R, C, GPE_MODE_ITP, D, G, MORE>(a, s);
     }
 }
@@ -1581,8 +1716,9 @@ cudaError_t launch_observe(const StepArgs& a, double* out, bool node_fp32, cudaS
     return cudaGetLastError();
 }
 
+// The normalisation of a.prev into *a.scale_out.
 template <typename R, int C>
-cudaError_t launch_norm(const StepArgs& a, double* out, cudaStream_t s) {
+cudaError_t launch_norm(const StepArgs& a, cudaStream_t s) {
     static int occ = 0;
     if (occ == 0) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, norm_kernel<R, C>, 256, 0);
@@ -1590,13 +1726,14 @@ cudaError_t launch_norm(const StepArgs& a, double* out, cudaStream_t s) {
     }
     const unsigned nb = std::min<unsigned>(nblocks(a.total, 256), (unsigned)occ * (unsigned)device_sm_count());
     norm_kernel<R, C><<<nb, 256, 0, s>>>(a);
-    observe_finalize_kernel<<<1, 256, 0, s>>>(a.partials, nb, out);
     return cudaGetLastError();
 }
 
+// a.next scaled by *a.scale_in.
 template <typename R, int C>
-cudaError_t launch_scale(const StepArgs& a, const double* norm_sum, double dv, cudaStream_t s) {
-    scale_kernel<R, C><<<nblocks(a.total, 256), 256, 0, s>>>(a, norm_sum, dv);
+cudaError_t launch_scale(const StepArgs& a, cudaStream_t s) {
+    const unsigned nb = std::min<unsigned>(nblocks(a.total, 256), 8u * (unsigned)device_sm_count());
+    scale_kernel<R, C><<<nb, 256, 0, s>>>(a);
     return cudaGetLastError();
 }
 
@@ -1605,21 +1742,23 @@ cudaError_t launch_scale(const StepArgs& a, const double* norm_sum, double dv, c
     template cudaError_t launch_parabolic_observe<R, C>(const StepArgs&, double*, cudaStream_t); \
     template cudaError_t launch_hyper<R, C>(const StepArgs&, int, cudaStream_t);           \
     template cudaError_t launch_observe<R, C>(const StepArgs&, double*, bool, cudaStream_t);     \
-    template cudaError_t launch_scale<R, C>(const StepArgs&, const double*, double, cudaStream_t); \
-    template cudaError_t launch_norm<R, C>(const StepArgs&, double*, cudaStream_t);
+    template cudaError_t launch_scale<R, C>(const StepArgs&, cudaStream_t);                \
+    template cudaError_t launch_norm<R, C>(const StepArgs&, cudaStream_t);
 
 }  // namespace gpe
 
 namespace gpe {
 
-// sum_interior Re(conj(a) b) into partials[.][OBS_NORM] (innerProduct,
-// Spin1GpeBCC.cu:213-233); a = StepArgs::prev, b = StepArgs::next.
+// sum_interior Re(conj(a) b) into scale_out->sum (innerProduct, Spin1GpeBCC.cu:
+// 213-233); a = StepArgs::prev, b = StepArgs::next.  FP32 storage: a pair sum per
+// thread.
 template <typename R, int C>
 __global__ void __launch_bounds__(256) dot_kernel(StepArgs a) {
     __shared__ double red[8];
     double acc = 0;
-    const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid < a.total) {
+    PairSum pair;
+    for (uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < a.total;
+         gid += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t i = (uint32_t)gid;
         const uint32_t row = fdiv(i, a.divRow);
         const uint32_t within = i - row * a.row_items;
@@ -1628,29 +1767,33 @@ __global__ void __launch_bounds__(256) dot_kernel(StepArgs a) {
         const uint32_t z = fdiv(row, a.divY);
         const uint32_t y = row - z * a.g.Y;
         const size_t off = (size_t)z * a.g.slice + (size_t)y * a.g.pitch + (size_t)x * a.g.cell_bytes + l * (C * 2 * sizeof(R));
+        Cx<R> u[C], v[C];
+        ld_node<R, C, true>(a.prev + off, u);
+        ld_node<R, C, true>(a.next + off, v);
+        if constexpr (sizeof(R) == 8) {
 #pragma unroll
-        for (int s = 0; s < C; ++s) {
-            const Cx<R> u = ldc<R>(a.prev + off + s * 2 * sizeof(R));
-            const Cx<R> v = ldc<R>(a.next + off + s * 2 * sizeof(R));
-            acc += (double)u.x * (double)v.x + (double)u.y * (double)v.y;
+            for (int s = 0; s < C; ++s) acc += u[s].x * v[s].x + u[s].y * v[s].y;
+        } else {
+#pragma unroll
+            for (int s = 0; s < C; ++s) {
+                pair.add_prod(u[s].x, v[s].x);
+                pair.add_prod(u[s].y, v[s].y);
+            }
         }
     }
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x < OBS_COUNT) {
-        double v = 0;
-        if (threadIdx.x == OBS_NORM)
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += red[w];
-        a.partials[(size_t)blockIdx.x * OBS_COUNT + threadIdx.x] = v;
+    if constexpr (sizeof(R) == 4) {
+        pair.warp_sum();
+        acc = pair.value();
+    } else {
+        acc = NormAcc<R>::warp_sum(acc);
     }
+    NormAcc<R>::grid_sum(acc, red, a.partials, a.dv, a.scale_out);
 }
 
 template <typename R, int C>
-cudaError_t launch_dot_t(const StepArgs& a, double* out, cudaStream_t s) {
-    const unsigned nb = nblocks(a.total, 256);
+cudaError_t launch_dot_t(const StepArgs& a, cudaStream_t s) {
+    const unsigned nb = std::min<unsigned>(nblocks(a.total, 256), 4u * (unsigned)device_sm_count());
     dot_kernel<R, C><<<nb, 256, 0, s>>>(a);
-    observe_finalize_kernel<<<1, 256, 0, s>>>(a.partials, nb, out);
     return cudaGetLastError();
 }
 
