@@ -241,7 +241,7 @@ __device__ __forceinline__ void batch_rows_c1x2(const MK& M, const SmemTables<R>
 
 // Rows row0 .. row0 + rows - 1 of a member in the interleaved layout (FP32).
 // Warp task t = u V + l within the item: node l of the item's u-th group
-// (il_lane_group, counted row after row): the 8 warps of a block take
+// (ILWalk, counted row after row): the 8 warps of a block take
 // consecutive nodes of the same groups, as the single-condensate interleaved
 // kernel's warps do, so the neighbour records they gather are read while they are
 // still in L2.  A node's stencil comes from the shared tables for every task:
@@ -264,22 +264,27 @@ __device__ __forceinline__ void batch_il_rows(const BatchMember& M, const SmemTa
     for (uint32_t t = threadIdx.x >> 5; t < tasks; t += kWarps) {
         const uint32_t u = fdiv(t, M.divV);
         const uint32_t l = t - u * G.V;
-        uint32_t gx, y, z;
-        if (!il_lane_group<CELLS>(G, u, nq, row0, M.divGX, M.divY, gx, y, z)) continue;
+        const ILWalk<CELLS> g(G, u, 0, row0, M.divGX, M.divY);
+        const uint32_t x = g.gx * CELLS + sub;
+        if (g.q >= nq || x >= G.X) continue;
         const int f0 = st.row_ptr[l];
         const int nd = D == 4 ? 4 : st.row_ptr[l + 1] - f0;
         int32_t off[D];
+        uint32_t outside = 0;
 #pragma unroll
         for (int k = 0; k < D; ++k) {
-            off[k] = 1;
+            off[k] = 0;
             if (k < nd) {
                 const int32_t b = st.nb_off[f0 + k];
-                const int xl = (int)sub + (b & 3) - 1;
+                const int dx = (b & 3) - 1, xl = (int)sub + dx;
                 const int32_t gs = xl < 0 ? -1 : (xl >= CELLS ? 1 : 0);
-                off[k] = ((b & ~3) + (int32_t)sub * 8 + gs * wrap) | (b & 3);
+                off[k] = (b & ~3) + (int32_t)sub * 8 + gs * wrap;
+                outside |= (uint32_t)((unsigned)((int)x + dx) >= G.X) << k;
             }
         }
-        il_task<C, D, CELLS, NoObs>(G, P, F, prev, next, off, st.w + f0, nd, st.pos + 3 * l, sub, l, gx, y, z, &no);
+        const size_t base = g.base(G);
+        il_task<C, D, CELLS, NoObs>(P, F, prev + base, next + base, l * (C * CELLS * 8) + sub * 8, off, outside, g.zero(G),
+                                    st.w + f0, nd, st.pos + 3 * l, x, g.y, g.z, &no);
     }
 }
 

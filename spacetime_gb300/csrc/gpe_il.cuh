@@ -137,94 +137,125 @@ __global__ void __launch_bounds__(kIlConvThreads, 4) il_convert_kernel(char* aos
     }
 }
 
-// Node l's stencil in the interleaved layout, for cell `sub` of a group (the
-// lane's cell in its group): neighbour k is node e.w of the cells shifted by (dx,
-// dy, dz), a fixed offset from the group base: the rows (dz, dy), the node, and
-// sub + dx within the group or (first / last cell) the last / first cell of the
-// group before / after it.  The offset is a multiple of 8, so its two low bits carry dx
-// + 1 (|dx| <= 1, checked on the host) for the halo test of cells x + dx outside
-// [0, X).  ent / wt: the node's table entries and weights; nd (4, or 4 or 8 for
-// D = 8) of them.
-template <int D, int CELLS>
-__device__ __forceinline__ void il_node_stencil(const ILGrid& G, const int4* ent, const float* wt, int nd, uint32_t sub,
-                                                int32_t* off, float* w) {
-    const uint32_t node_run = G.C * CELLS * 8;   // bytes between nodes of a group
-#pragma unroll
-    for (int k = 0; k < D; ++k) {
-        off[k] = 1;
-        w[k] = 0.f;
-        if (k < nd) {
-            const int4 e = ent[k];
-            const int xl = (int)sub + e.x;                        // -1 .. CELLS
-            const int64_t gshift = xl < 0 ? -1 : (xl >= CELLS ? 1 : 0);
-            const int64_t cell = xl - gshift * (int64_t)CELLS;
-            off[k] = (int32_t)(((int64_t)e.z * (G.Y + 2) + e.y) * (int64_t)G.row + (int64_t)e.w * node_run +
-                               gshift * (int64_t)G.gb + cell * 8) |
-                     (e.x + 1);
-            w[k] = wt[k];
+// A neighbour in the interleaved layout, for cell `sub` of a group (the lane's cell in
+// its group): node (or edge) `item` of the cells shifted by (dx, dy, dz), at a fixed
+// byte offset from the group's base: the rows (dz, dy), the item's run, and sub + dx
+// within the group or (first / last cell) the last / first cell of the group before /
+// after it.
+template <int CELLS>
+__device__ __forceinline__ int32_t il_lane_off(const ILGrid& G, int dx, int dy, int dz, uint32_t item, uint32_t sub) {
+    const int xl = (int)sub + dx;   // -1 .. CELLS
+    const int64_t gshift = xl < 0 ? -1 : (xl >= CELLS ? 1 : 0);
+    const int64_t cell = xl - gshift * (int64_t)CELLS;
+    return (int32_t)(((int64_t)dz * (G.Y + 2) + dy) * (int64_t)G.row + (int64_t)item * (G.C * CELLS * 8) +
+                     gshift * (int64_t)G.gb + cell * 8);
+}
+
+// Which of a lane's neighbours lie outside [0, X): only the cell x = 0 has some to the
+// left and only x = X - 1 to the right, so one bit per neighbour for each side, fixed
+// for the launch, that count in the first and the last group of a row.
+struct ILEdge {
+    uint32_t left, right;
+    __device__ __forceinline__ ILEdge() : left(0), right(0) {}
+    __device__ __forceinline__ void add(int k, int dx, bool first, bool last) {
+        left |= (uint32_t)(dx < 0 && first) << k;
+        right |= (uint32_t)(dx > 0 && last) << k;
+    }
+    __device__ __forceinline__ uint32_t outside(uint32_t gx, uint32_t GX) const {
+        return (gx == 0 ? left : 0u) | (gx == GX - 1 ? right : 0u);
+    }
+};
+
+// The group a lane works on: the q-th group of the rows row0 .. (counted row after
+// row), as (gx, y, z), stepped through the rows without divisions: a warp's next task
+// is a fixed number of groups further on.
+template <int CELLS>
+struct ILWalk {
+    uint32_t q, gx, y, z;   // this task's group
+    uint32_t dq, dgx, dy, dz;
+    // warp task u (32 / CELLS groups) of `step` tasks apart
+    __device__ __forceinline__ ILWalk(const ILGrid& G, uint32_t u, uint32_t step, uint32_t row0, FastDiv dGX, FastDiv dY) {
+        constexpr uint32_t kWG = 32 / CELLS;
+        q = kWG * u + (threadIdx.x & 31) / CELLS;
+        const uint32_t r = fdiv(q, dGX), row = row0 + r;
+        gx = q - r * G.GX;
+        z = fdiv(row, dY);
+        y = row - z * G.Y;
+        dq = kWG * step;
+        const uint32_t dr = fdiv(dq, dGX);
+        dgx = dq - dr * G.GX;
+        dz = fdiv(dr, dY);
+        dy = dr - dz * G.Y;
+    }
+    __device__ __forceinline__ void next(const ILGrid& G) {
+        q += dq;
+        gx += dgx;
+        y += dy;
+        z += dz;
+        if (gx >= G.GX) {
+            gx -= G.GX;
+            ++y;
+        }
+        if (y >= G.Y) {
+            y -= G.Y;
+            ++z;
         }
     }
-}
+    // byte offset of the group in its buffer (a plane of rows is below 2^31 bytes)
+    __device__ __forceinline__ size_t base(const ILGrid& G) const {
+        const uint32_t r = (z + 1) * (G.Y + 2) + (y + 1);
+        return (size_t)r * (uint32_t)G.row + (size_t)gx * (uint32_t)G.gb;
+    }
+    // from the group's base to the first value of the plane's zero row y = -1
+    __device__ __forceinline__ int32_t zero(const ILGrid& G) const {
+        return -(int32_t)((y + 1) * (uint32_t)G.row + gx * (uint32_t)G.gb);
+    }
+};
 
-// The group a lane works on in warp task u: the q-th group of the rows row0 ..
-// (q = u 32 / CELLS + the lane's group within its warp, counted row after row),
-// as (gx, y, z); false past the last group (nq groups).
-template <int CELLS>
-__device__ __forceinline__ bool il_lane_group(const ILGrid& G, uint32_t u, uint32_t nq, uint32_t row0, FastDiv dGX,
-                                              FastDiv dY, uint32_t& gx, uint32_t& y, uint32_t& z) {
-    const uint32_t q = (32 / CELLS) * u + (threadIdx.x & 31) / CELLS;
-    if (q >= nq) return false;
-    const uint32_t r = fdiv(q, dGX);
-    gx = q - r * G.GX;
-    const uint32_t row = row0 + r;
-    z = fdiv(row, dY);
-    y = row - z * G.Y;
-    return true;
-}
-
-// One lane's node of an interleaved leapfrog step: node l of cell gx CELLS + sub
-// of row (y, z), next <- next + 2 dt (-i H prev), with the arithmetic and its order of
-// parabolic_node_t + node_finish.  F: where the step's fields come from (P if
-// null); oa: where the observables of prev go.  With a NormAcc for oa: an imaginary-
-// time iteration (kModeItpNorm), next = prev - dt H prev with prev read times inv.
+// One lane's node of an interleaved leapfrog step, cell (x, y, z): next <- next + 2 dt
+// (-i H prev), with the arithmetic and its order of parabolic_node_t + node_finish.
+// prev, next: the group's base in the two buffers; own: the node's offset from it; off:
+// its neighbours', those with their bit set in `outside` read the zero row at `zero`
+// instead.  F: where the step's fields come from (P if null); oa: where the observables
+// of prev go.  With a NormAcc for oa: an imaginary-time iteration (kModeItpNorm), next =
+// prev - dt H prev with prev read times inv.
+//
+// What bounds the plain step is the instruction count and the latency of the loads
+// together (spin-1 BCC 96^3: warps issue on 63 % of the cycles, DRAM at 72 %), so
+// nothing is computed here that is the same for the whole launch or row.
 template <int C, int D, int CELLS, class OA>
-__device__ __forceinline__ void il_task(const ILGrid& G, const PhysR<float>& P, const PhysR<float>* F, const char* prev,
-                                        char* next, const int32_t* off, const float* w, int nd, const float* pos,
-                                        uint32_t sub, uint32_t l, uint32_t gx, uint32_t y, uint32_t z, OA* oa,
+__device__ __forceinline__ void il_task(const PhysR<float>& P, const PhysR<float>* F, const char* prev, char* next,
+                                        uint32_t own, const int32_t* off, uint32_t outside, int32_t zero, const float* w,
+                                        int nd, const float* pos, uint32_t x, uint32_t y, uint32_t z, OA* oa,
                                         float inv = 1.f) {
     constexpr bool kItp = std::is_same<OA, NormAcc<float>>::value;
     constexpr uint32_t kComp = CELLS * 8;   // bytes between a record's components
-    const uint32_t x = gx * CELLS + sub;
-    if (x >= G.X) return;
-    const size_t gbase = il_row(G, y, z) + (size_t)gx * G.gb;
-    const size_t own = gbase + (size_t)l * (G.C * kComp) + (size_t)sub * 8;
     Cx<float> prv[C], nv[C], H[C];
+    const char* pp = prev + own;
+    char* np = next + own;
 #pragma unroll
     for (int s = 0; s < C; ++s) {
-        prv[s] = ldc<float>(prev + own + s * kComp);
-        if constexpr (!kItp) nv[s] = ldc_rw<float>(next + own + s * kComp);
+        prv[s] = ldc<float>(pp + s * kComp);
+        if constexpr (!kItp) nv[s] = ldc_rw<float>(np + s * kComp);
     }
 #pragma unroll
     for (int s = 0; s < C; ++s) H[s] = cx<float>(0.f, 0.f);
     // DEC Laplacian, sum_f w_f (psi_nb - psi) in entry order (Spin1GpeBCC.cu:835-865),
-    // the loads of a group of 4 entries issued together; cells x + dx outside
-    // [0, X) are the zero halo
+    // the loads of a group of 4 entries issued together
 #pragma unroll
     for (int k0 = 0; k0 < D; k0 += 4) {
         if (k0 >= nd) break;
         Cx<float> v[4][C];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            const int32_t o = off[k0 + k];
-            const bool in = (unsigned)((int)x + (o & 3) - 1) < G.X;
-            const char* p = prev + gbase + (in ? (o & ~3) : 0);
+            const char* p = prev + ((outside >> (k0 + k)) & 1 ? zero : off[k0 + k]);
 #pragma unroll
-            for (int s = 0; s < C; ++s) v[k][s] = in ? ldc<float>(p + s * kComp) : cx<float>(0.f, 0.f);
+            for (int s = 0; s < C; ++s) v[k][s] = ldc<float>(p + s * kComp);
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
 #pragma unroll
-            for (int s = 0; s < C; ++s) H[s] += w[k0 + k] * (v[k][s] - prv[s]);
+            for (int s = 0; s < C; ++s) add_scaled(H[s], w[k0 + k], v[k][s] - prv[s]);
         }
     }
     if constexpr (kItp) {
@@ -233,27 +264,25 @@ __device__ __forceinline__ void il_task(const ILGrid& G, const PhysR<float>& P, 
     }
     // local terms and the leapfrog update, as node_finish
     float rr[3];
-    rr[0] = P.p0[0] + P.bs * ((float)x * P.bw[0] + pos[0]);
-    rr[1] = P.p0[1] + P.bs * ((float)y * P.bw[1] + pos[1]);
-    rr[2] = P.p0[2] + P.bs * ((float)z * P.bw[2] + pos[2]);
+    node_pos(P, x, y, z, pos, rr);
     const float pot = trap<float>(P, rr, F);
     if constexpr (kItp) {
         local_terms<float, C>(P, rr, pot, GPE_MODE_ITP, false, prv, H, F);
 #pragma unroll
         for (int s = 0; s < C; ++s) {
-            nv[s] = prv[s] - P.dt * H[s];
-            stc<float>(next + own + s * kComp, nv[s]);
+            nv[s] = prv[s];
+            add_scaled(nv[s], -P.dt, H[s]);
+            stc<float>(np + s * kComp, nv[s]);
         }
         oa->template add<C>(nv);
-        return;
     } else {
-    local_terms<float, C>(P, rr, pot, GPE_MODE_LEAPFROG, false, prv, H, F);
-    if constexpr (!std::is_same<OA, NoObs>::value) oa->template node<float, C>(P, rr, prv, H);
+        local_terms<float, C>(P, rr, pot, GPE_MODE_LEAPFROG, false, prv, H, F);
+        if constexpr (!std::is_same<OA, NoObs>::value) oa->template node<float, C>(P, rr, prv, H);
 #pragma unroll
-    for (int s = 0; s < C; ++s) {
-        nv[s] += (2.f * P.dt) * cx<float>(H[s].y, -H[s].x);
-        stc<float>(next + own + s * kComp, nv[s]);
-    }
+        for (int s = 0; s < C; ++s) {
+            add_scaled(nv[s], 2.f * P.dt, cx<float>(H[s].y, -H[s].x));
+            stc<float>(np + s * kComp, nv[s]);
+        }
     }
 }
 
@@ -270,14 +299,14 @@ constexpr unsigned kIlObsThreads = 256;
 // One FP32 leapfrog step in the interleaved layout: next <- next + 2 dt (-i H prev).
 // D = 4: every node has 4 stencil entries (BCC, A15, C15, Z); D = 8: rows of 4 or 8
 // entries (FCC's tetrahedra and octahedra).  Warp task t = u V + l: node l of the
-// u-th group (il_lane_group).  The grid's warp count is a multiple
+// u-th group (or groups, ILWalk).  The grid's warp count is a multiple
 // of V, so a warp keeps its node, and with it its entries and position, in
 // registers; the row length is the same in every lane of a warp, so the second
 // group of 4 entries is a uniform branch.  OBS: the observables of prev are summed
 // on the way (ObsAcc, as the gather kernels' observed step).  MODE kModeItpNorm: an
 // imaginary-time iteration instead.
 template <int C, int D, int CELLS, bool OBS, int MODE = GPE_MODE_LEAPFROG>
-__device__ __forceinline__ void il_step_body(const StepArgs& a, const ILGrid& G, uint32_t tasks, FastDiv dGX) {
+__device__ __forceinline__ void il_step_body(const StepArgs& a, const ILGrid& G, FastDiv dGX) {
     static_assert(D == 4 || D == 8, "rows of 4, or of 4 and 8 entries");
     const PhysR<float>& P = make_phys<float>(a);
     using OA = typename AccOf<MODE, OBS, float>::type;
@@ -287,25 +316,36 @@ __device__ __forceinline__ void il_step_body(const StepArgs& a, const ILGrid& G,
     const uint32_t sub = threadIdx.x & (CELLS - 1);
     const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
-    const uint32_t l = warp - fdiv(warp, a.divV) * G.V;
+    const uint32_t u0 = fdiv(warp, a.divV), l = warp - u0 * G.V;
     const uint32_t nq = G.Y * G.Z * G.GX;
     // the warp's node's table, read once from global memory (no shared tables: the
     // block then needs no shared memory, which left the plain kernel at 7 blocks per
     // SM); weights h / bs^2 of the step's block scale, as load_tables scales them
     const int f0 = a.tab.row_ptr[l];
     const int nd = D == 4 ? 4 : a.tab.row_ptr[l + 1] - f0;   // 4 or 8, the same in the whole warp
-    float wt[D];
-#pragma unroll
-    for (int k = 0; k < D; ++k) wt[k] = k < nd ? a.tab.w32[f0 + k] * P.ks : 0.f;
     int32_t off[D];
     float w[D];
-    il_node_stencil<D, CELLS>(G, a.tab.ent4 + f0, wt, nd, sub, off, w);
+    ILEdge edge;
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+        off[k] = 0;
+        w[k] = 0.f;
+        if (k < nd) {
+            const int4 e = a.tab.ent4[f0 + k];
+            off[k] = il_lane_off<CELLS>(G, e.x, e.y, e.z, (uint32_t)e.w, sub);
+            w[k] = a.tab.w32[f0 + k] * P.ks;
+            edge.add(k, e.x, sub == 0, sub == (G.X - 1) % CELLS);
+        }
+    }
     const float pos[3] = {a.tab.pos32[3 * l], a.tab.pos32[3 * l + 1], a.tab.pos32[3 * l + 2]};
-    for (uint32_t t = warp; t < tasks; t += nwarps) {
-        const uint32_t u = fdiv(t, a.divV);
-        uint32_t gx, y, z;
-        if (il_lane_group<CELLS>(G, u, nq, 0, dGX, a.divY, gx, y, z))
-            il_task<C, D, CELLS, OA>(G, P, nullptr, a.prev, a.next, off, w, nd, pos, sub, l, gx, y, z, &oa, inv);
+    const uint32_t own = l * (C * CELLS * 8) + sub * 8;
+    // the grid's warp count is a multiple of V
+    for (ILWalk<CELLS> g(G, u0, fdiv(nwarps, a.divV), 0, dGX, a.divY); g.q < nq; g.next(G)) {
+        const uint32_t x = g.gx * CELLS + sub;
+        if (x >= G.X) continue;
+        const size_t base = g.base(G);
+        il_task<C, D, CELLS, OA>(P, nullptr, a.prev + base, a.next + base, own, off, edge.outside(g.gx, G.GX), g.zero(G), w,
+                                 nd, pos, x, g.y, g.z, &oa, inv);
     }
     if constexpr (OBS) {
         __shared__ double red[8][OBS_COUNT];
@@ -323,26 +363,23 @@ __device__ __forceinline__ void il_step_body(const StepArgs& a, const ILGrid& G,
 // shared memory per thread).
 template <int C, int D>
 struct IlBounds {
-    // D = 4: spin-1 BCC 96^3 (the cap 7 blocks lets it use 64 registers, 8 blocks):
-    // 0.130 ms per step; capped at 72 registers before the offsets carried dx, 7
-    // blocks 0.131, 8 (64) 0.147, 9 (56) 0.145; spin-2 BCC 96^3: 4 blocks (105)
-    // 0.222 ms, 5 (96) 0.211, 6 (80) 0.218.  D = 8 keeps 12 more registers for the
-    // second group of entries (FCC 96^3, fraction of the copy peak): spin-1 at 5
-    // blocks (95 registers) 0.58, at 6 (80, 16 bytes of spills) 0.58, at 4 0.52;
-    // spin-2 at 4 blocks (128) 0.58, at 3 0.52, at 5 0.49.
-    static constexpr int kMin = D == 8 ? (C == 5 ? 4 : (C == 3 ? 5 : 8)) : (C == 5 ? 5 : (C == 3 ? 7 : 8));
+    // D = 4: spin-1 BCC 96^3 at 7 blocks (72 registers) 0.125 ms per step, at 8 (64)
+    // 0.132; spin-2 BCC 64^3 at 5 blocks (96) 0.065 ms, at 6 (80) 0.067.  D = 8 keeps
+    // 12 more registers for the second group of entries: spin-1 FCC 64^3 at 6 blocks
+    // (80) 0.0563 ms, at 5 (96) 0.0595; spin-2 at 4 blocks (128).
+    static constexpr int kMin = D == 8 ? (C == 5 ? 4 : (C == 3 ? 6 : 8)) : (C == 5 ? 5 : (C == 3 ? 7 : 8));
     static constexpr int kMinObs = (C == 5 || (C == 3 && D == 8)) ? 2 : 3;
 };
 
 template <int C, int D, int CELLS>
-__global__ void __launch_bounds__(kIlPlainThreads, IlBounds<C, D>::kMin) il_step_kernel(StepArgs a, ILGrid G, uint32_t tasks,
+__global__ void __launch_bounds__(kIlPlainThreads, IlBounds<C, D>::kMin) il_step_kernel(StepArgs a, ILGrid G,
                                                                                     FastDiv dGX) {
-    il_step_body<C, D, CELLS, false>(a, G, tasks, dGX);
+    il_step_body<C, D, CELLS, false>(a, G, dGX);
 }
 template <int C, int D, int CELLS>
 __global__ void __launch_bounds__(kIlObsThreads, IlBounds<C, D>::kMinObs) il_step_obs_kernel(StepArgs a, ILGrid G,
-                                                                                        uint32_t tasks, FastDiv dGX) {
-    il_step_body<C, D, CELLS, true>(a, G, tasks, dGX);
+                                                                                        FastDiv dGX) {
+    il_step_body<C, D, CELLS, true>(a, G, dGX);
 }
 
 // One imaginary-time iteration of gpe_itp before its last: next = prev - dt H prev
@@ -351,9 +388,9 @@ __global__ void __launch_bounds__(kIlObsThreads, IlBounds<C, D>::kMinObs) il_ste
 // bytes per site, where the separate step, norm and scale passes of the handle's
 // layout move 48 C.
 template <int C, int D, int CELLS>
-__global__ void __launch_bounds__(kIlPlainThreads, IlBounds<C, D>::kMin) il_itp_kernel(StepArgs a, ILGrid G, uint32_t tasks,
+__global__ void __launch_bounds__(kIlPlainThreads, IlBounds<C, D>::kMin) il_itp_kernel(StepArgs a, ILGrid G,
                                                                                    FastDiv dGX) {
-    il_step_body<C, D, CELLS, false, kModeItpNorm>(a, G, tasks, dGX);
+    il_step_body<C, D, CELLS, false, kModeItpNorm>(a, G, dGX);
 }
 
 // Blocks of one interleaved step (rows of D entries at most): one wave at the
@@ -406,13 +443,12 @@ template <int C, int D, int CELLS>
 cudaError_t launch_il_step_d(const StepArgs& a, const ILGrid& G, size_t max_blocks, bool obs, double* out, cudaStream_t s) {
     const unsigned nb = il_blocks_d<C, D, CELLS>(G, obs, max_blocks);
     if (nb == 0) return cudaErrorInvalidConfiguration;
-    const uint32_t tasks = il_warp_tasks(G) * G.V;
     const FastDiv dGX = make_fastdiv(G.GX);
     if (obs) {
-        il_step_obs_kernel<C, D, CELLS><<<nb, kIlObsThreads, 0, s>>>(a, G, tasks, dGX);
+        il_step_obs_kernel<C, D, CELLS><<<nb, kIlObsThreads, 0, s>>>(a, G, dGX);
         observe_finalize_kernel<<<1, 256, 0, s>>>(a.partials, nb, out);
     } else {
-        il_step_kernel<C, D, CELLS><<<nb, kIlPlainThreads, 0, s>>>(a, G, tasks, dGX);
+        il_step_kernel<C, D, CELLS><<<nb, kIlPlainThreads, 0, s>>>(a, G, dGX);
     }
     return cudaGetLastError();
 }
@@ -439,7 +475,7 @@ cudaError_t launch_il_itp_d(const StepArgs& a, const ILGrid& G, size_t max_block
     }
     const unsigned nb = il_wave(G, kIlPlainThreads, occ, max_blocks);
     if (nb == 0) return cudaErrorInvalidConfiguration;
-    il_itp_kernel<C, D, CELLS><<<nb, kIlPlainThreads, 0, s>>>(a, G, il_warp_tasks(G) * G.V, make_fastdiv(G.GX));
+    il_itp_kernel<C, D, CELLS><<<nb, kIlPlainThreads, 0, s>>>(a, G, make_fastdiv(G.GX));
     return cudaGetLastError();
 }
 
@@ -481,12 +517,12 @@ cudaError_t launch_il_itp(const StepArgs& a, const ILGrid& G, int deg, size_t ma
 // states bit for bit.
 template <int C, int CELLS>
 __device__ __forceinline__ void il_hyper_body(const StepArgs& a, const ILGrid& G, const ILGrid& Gq, const int32_t* tab,
-                                              uint32_t tasks, FastDiv dGX) {
+                                              FastDiv dGX) {
     const uint32_t V = G.V, E = Gq.V;
     const uint32_t sub = threadIdx.x & (CELLS - 1);
     const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
-    const uint32_t j = warp - fdiv(warp, a.divV) * V;
+    const uint32_t u0 = fdiv(warp, a.divV), j = warp - u0 * V;
     const PhysR<float>& P = make_phys<float>(a);
     constexpr uint32_t kComp = CELLS * 8;
     const uint32_t nq = G.Y * G.Z * G.GX;
@@ -496,30 +532,32 @@ __device__ __forceinline__ void il_hyper_body(const StepArgs& a, const ILGrid& G
     auto lane_off = [&](int32_t b, int32_t wrap) {
         const int xl = (int)sub + (b & 3) - 1;
         const int32_t gs = xl < 0 ? -1 : (xl >= CELLS ? 1 : 0);
-        return ((b & ~3) + (int32_t)sub * 8 + gs * wrap) | (b & 3);
+        return (b & ~3) + (int32_t)sub * 8 + gs * wrap;
     };
     int32_t off[4], eto[2], efrom[2];
     float w[4];
+    ILEdge edge;   // bits 0..3 the incidences, 4 and 5 the to-nodes
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        off[k] = lane_off(tab[4 * j + k], (int32_t)Gq.gb - (int32_t)kComp);
+        const int32_t b = tab[4 * j + k];
+        off[k] = lane_off(b, (int32_t)Gq.gb - (int32_t)kComp);
+        edge.add(k, (b & 3) - 1, sub == 0, sub == (G.X - 1) % CELLS);
         w[k] = a.tab.inc_w32[4 * j + k];
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-        eto[r] = lane_off(tab[4 * V + 2 * j + r], (int32_t)G.gb - (int32_t)kComp);
+        const int32_t b = tab[4 * V + 2 * j + r];
+        eto[r] = lane_off(b, (int32_t)G.gb - (int32_t)kComp);
+        edge.add(4 + r, (b & 3) - 1, sub == 0, sub == (G.X - 1) % CELLS);
         efrom[r] = tab[4 * V + E + 2 * j + r] + (int32_t)sub * 8;
     }
     const float pos[3] = {a.tab.pos32[3 * j], a.tab.pos32[3 * j + 1], a.tab.pos32[3 * j + 2]};
     const float dts = P.dts;
-    for (uint32_t t = warp; t < tasks; t += nwarps) {
-        const uint32_t u = fdiv(t, a.divV);
-        uint32_t gx, y, z;
-        if (!il_lane_group<CELLS>(G, u, nq, 0, dGX, a.divY, gx, y, z)) continue;
-        const uint32_t x = gx * CELLS + sub;
+    for (ILWalk<CELLS> g(G, u0, fdiv(nwarps, a.divV), 0, dGX, a.divY); g.q < nq; g.next(G)) {
+        const uint32_t x = g.gx * CELLS + sub, y = g.y, z = g.z;
         if (x >= G.X) continue;
-        const size_t gbase = il_row(G, y, z) + (size_t)gx * G.gb;
-        const size_t qbase = il_row(Gq, y, z) + (size_t)gx * Gq.gb;
+        const size_t gbase = g.base(G), qbase = g.base(Gq);
+        const uint32_t outside = edge.outside(g.gx, G.GX);
         {
             // node j
             const size_t own = gbase + (size_t)j * (C * kComp) + (size_t)sub * 8;
@@ -534,21 +572,18 @@ __device__ __forceinline__ void il_hyper_body(const StepArgs& a, const ILGrid& G
             Cx<float> qv[4][C];
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const int32_t o = off[k];
-                const bool in = (unsigned)((int)x + (o & 3) - 1) < G.X;
-                const char* p = a.q + qbase + (in ? (o & ~3) : 0);
+                const bool in = !((outside >> k) & 1);
+                const char* p = a.q + qbase + off[k];
 #pragma unroll
                 for (int s = 0; s < C; ++s) qv[k][s] = in ? ldc<float>(p + s * kComp) : cx<float>(0.f, 0.f);
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
 #pragma unroll
-                for (int s = 0; s < C; ++s) H[s] += w[k] * qv[k][s];
+                for (int s = 0; s < C; ++s) add_scaled(H[s], w[k], qv[k][s]);
             }
             float r[3];
-            r[0] = P.p0[0] + P.bs * ((float)x * P.bw[0] + pos[0]);
-            r[1] = P.p0[1] + P.bs * ((float)y * P.bw[1] + pos[1]);
-            r[2] = P.p0[2] + P.bs * ((float)z * P.bw[2] + pos[2]);
+            node_pos(P, x, y, z, pos, r);
             const float pot = trap<float>(P, r);
             if constexpr (C == 1) {
                 local_scalar<float>(P, pot, false, true, prv, H);
@@ -560,7 +595,7 @@ __device__ __forceinline__ void il_hyper_body(const StepArgs& a, const ILGrid& G
             // the leapfrog update, as write_update
 #pragma unroll
             for (int s = 0; s < C; ++s) {
-                nv[s] += (2.f * P.dt) * cx<float>(H[s].y, -H[s].x);
+                add_scaled(nv[s], 2.f * P.dt, cx<float>(H[s].y, -H[s].x));
                 stc<float>(a.next + own + s * kComp, nv[s]);
             }
         }
@@ -569,9 +604,8 @@ __device__ __forceinline__ void il_hyper_body(const StepArgs& a, const ILGrid& G
             // edge 2j + e: q_update, hyperbolic leapfrog: next_q += i 2 (dt/sigma)(prev_q + d0 psi)
             const size_t own = qbase + (size_t)(2 * j + e) * (C * kComp) + (size_t)sub * 8;
             Cx<float> to[C], fr[C], pq[C], v[C];
-            const int32_t o = eto[e];
-            const bool in = (unsigned)((int)x + (o & 3) - 1) < G.X;
-            const char* pt = a.prev + gbase + (in ? (o & ~3) : 0);
+            const bool in = !((outside >> (4 + e)) & 1);
+            const char* pt = a.prev + gbase + eto[e];
 #pragma unroll
             for (int s = 0; s < C; ++s) {
                 to[s] = in ? ldc<float>(pt + s * kComp) : cx<float>(0.f, 0.f);
@@ -582,8 +616,8 @@ __device__ __forceinline__ void il_hyper_body(const StepArgs& a, const ILGrid& G
 #pragma unroll
             for (int s = 0; s < C; ++s) {
                 const Cx<float> d0psi = to[s] - fr[s];
-                const Cx<float> qq = (2.f * dts) * (pq[s] + d0psi);
-                v[s] += cx<float>(-qq.y, qq.x);
+                const Cx<float> qq = pq[s] + d0psi;
+                add_scaled(v[s], 2.f * dts, cx<float>(-qq.y, qq.x));
                 stc<float>(a.qnext + own + s * kComp, v[s]);
             }
         }
@@ -591,9 +625,10 @@ __device__ __forceinline__ void il_hyper_body(const StepArgs& a, const ILGrid& G
 }
 
 // Register caps: spin-2 at 5 blocks of 128 threads (96 registers, no spills),
-// spin-1 at 6 (80 registers).  Measured against 6 blocks (80 registers) for
-// spin-2: BCC 96^3 0.98 / 1.03, C15 48^3 0.93 / 0.97, but C15 128^3 (285 M sites)
-// 0.87 / 0.73 of peak; spin-1 at 8 blocks (64 registers) within 1 %.
+// spin-1 at 6 (80 registers).  At 6 blocks (80 registers) spin-2 is within 1 % on
+// C15 40^3 and 48^3 and BCC 64^3 (0.545 / 0.544, 0.818 / 0.819, 0.172 / 0.170 ms), but on
+// C15 128^3 (285 M sites) it fell from 0.87 to 0.73 of peak; spin-1 BCC 64^3 at 7
+// blocks 0.109 ms, at 6 0.107.
 template <int C>
 struct IlHyperBounds {
     static constexpr int kMin = C == 5 ? 5 : (C == 3 ? 6 : 8);
@@ -601,8 +636,8 @@ struct IlHyperBounds {
 
 template <int C, int CELLS>
 __global__ void __launch_bounds__(kIlPlainThreads, IlHyperBounds<C>::kMin)
-    il_hyper_kernel(StepArgs a, ILGrid G, ILGrid Gq, const int32_t* tab, uint32_t tasks, FastDiv dGX) {
-    il_hyper_body<C, CELLS>(a, G, Gq, tab, tasks, dGX);
+    il_hyper_kernel(StepArgs a, ILGrid G, ILGrid Gq, const int32_t* tab, FastDiv dGX) {
+    il_hyper_body<C, CELLS>(a, G, Gq, tab, dGX);
 }
 
 template <int C, int CELLS>
@@ -634,14 +669,13 @@ template <int C>
 cudaError_t launch_il_hyper(const StepArgs& a, const ILGrid& G, const ILGrid& Gq, const int32_t* tab, cudaStream_t s) {
     const uint64_t tasks64 = (uint64_t)il_warp_tasks(G) * G.V;
     if (tasks64 > 0xffffffffu || G.cells != Gq.cells || G.GX != Gq.GX || Gq.V != 2 * G.V) return cudaErrorInvalidValue;
-    const uint32_t tasks = (uint32_t)tasks64;
     const FastDiv dGX = make_fastdiv(G.GX);
     if (G.cells == 32) {
         const unsigned nb = il_hyper_blocks_c<C, 32>(G, Gq);
-        il_hyper_kernel<C, 32><<<nb, kIlPlainThreads, 0, s>>>(a, G, Gq, tab, tasks, dGX);
+        il_hyper_kernel<C, 32><<<nb, kIlPlainThreads, 0, s>>>(a, G, Gq, tab, dGX);
     } else {
         const unsigned nb = il_hyper_blocks_c<C, 16>(G, Gq);
-        il_hyper_kernel<C, 16><<<nb, kIlPlainThreads, 0, s>>>(a, G, Gq, tab, tasks, dGX);
+        il_hyper_kernel<C, 16><<<nb, kIlPlainThreads, 0, s>>>(a, G, Gq, tab, dGX);
     }
     return cudaGetLastError();
 }

@@ -162,6 +162,34 @@ __device__ __forceinline__ const PhysR<R>& make_phys(const StepArgs& a) {
 // kernel keeps its members' constants in constant memory and the fields of the
 // step in shared memory.
 
+// a b + c, one rounding (float, double); dual numbers multiply and add.  The step's
+// arithmetic is written out in it where a product meets a sum, so that every kernel
+// that shares it rounds alike whatever the compiler makes of the code around it.
+template <typename R>
+__device__ __forceinline__ R fm(R a, R b, R c) {
+    if constexpr (std::is_same<R, float>::value) return __fmaf_rn(a, b, c);
+    else if constexpr (std::is_same<R, double>::value) return __fma_rn(a, b, c);
+    else return a * b + c;
+}
+template <typename R>
+__device__ __forceinline__ R norm_sq(Cx<R> a) { return fm(a.y, a.y, a.x * a.x); }
+// acc += conj(a) b, acc += a b, acc += s a (real s), written out in multiply-adds
+template <typename R>
+__device__ __forceinline__ void add_conj_mul(Cx<R>& acc, Cx<R> a, Cx<R> b) {
+    acc.x = fm(a.y, b.y, fm(a.x, b.x, acc.x));
+    acc.y = fm(-a.y, b.x, fm(a.x, b.y, acc.y));
+}
+template <typename R>
+__device__ __forceinline__ void add_mul(Cx<R>& acc, Cx<R> a, Cx<R> b) {
+    acc.x = fm(-a.y, b.y, fm(a.x, b.x, acc.x));
+    acc.y = fm(a.y, b.x, fm(a.x, b.y, acc.y));
+}
+template <typename R>
+__device__ __forceinline__ void add_scaled(Cx<R>& acc, R s, Cx<R> a) {
+    acc.x = fm(s, a.x, acc.x);
+    acc.y = fm(s, a.y, acc.y);
+}
+
 // trap (Spin1GpeBCC.cu:112-122)
 template <typename R>
 __device__ __forceinline__ R trap(const PhysR<R>& P, const R r[3], const PhysR<R>* F = nullptr) {
@@ -169,132 +197,193 @@ __device__ __forceinline__ R trap(const PhysR<R>& P, const R r[3], const PhysR<R
     R x = r[0] * P.lambda[0];
     R y = r[1] * P.lambda[1];
     R z = r[2] * P.lambda[2];
-    return (R)0.5 * (x * x + y * y + z * z) + P.trap_offset;
+    return fm((R)0.5, fm(z, z, fm(y, y, x * x)), P.trap_offset);
+}
+
+// Position of a node at pos in cell (x, y, z) (globalPos, Spin1GpeBCC.cu:871-874).
+template <typename R>
+__device__ __forceinline__ void node_pos(const PhysR<R>& P, uint32_t x, uint32_t y, uint32_t z, const R* pos, R r[3]) {
+    r[0] = fm(P.bs, fm((R)x, P.bw[0], pos[0]), P.p0[0]);
+    r[1] = fm(P.bs, fm((R)y, P.bw[1], pos[1]), P.p0[1]);
+    r[2] = fm(P.bs, fm((R)z, P.bw[2], pos[2]), P.p0[2]);
 }
 
 // magneticField (Spin1GpeBCC.cu:128-142)
 template <typename R>
 __device__ __forceinline__ void mag_field(const PhysR<R>& P, const R r[3], R Bq, const R Bb[3], R B[3]) {
     if (P.flags & GPE_FLAG_QUADRUPOLE_OFFSET) {
-        B[0] = Bq * (r[0] - P.qc[0]) + Bb[0];
-        B[1] = Bq * (r[1] - P.qc[1]) + Bb[1];
-        B[2] = (R)-2 * Bq * (r[2] - P.qc[2]) + Bb[2];
+        B[0] = fm(Bq, r[0] - P.qc[0], Bb[0]);
+        B[1] = fm(Bq, r[1] - P.qc[1], Bb[1]);
+        B[2] = fm((R)-2 * Bq, r[2] - P.qc[2], Bb[2]);
     } else {
-        B[0] = Bq * r[0] + Bb[0];
-        B[1] = Bq * r[1] + Bb[1];
-        B[2] = (R)-2 * Bq * r[2] + Bb[2];
+        B[0] = fm(Bq, r[0], Bb[0]);
+        B[1] = fm(Bq, r[1], Bb[1]);
+        B[2] = fm((R)-2 * Bq, r[2], Bb[2]);
+    }
+}
+
+// The local terms are written as multiply-adds onto H with the real potential kept
+// real: the reference multiplies each component by a complex potential whose
+// imaginary part only three-body loss sets, and by matrix elements of which some
+// are equal.  Spin-1: 76 FP operations a node instead of 118, spin-2 140 instead of
+// 265; the interleaved spin-1 step, whose warps issue on 63 % of the cycles, is
+// bound by its instruction count as much as by DRAM, and the FP64 step by the FP64
+// pipe alone.
+
+// Three-body loss, -i alpha n^2 psi (Spin1GpeBCC.cu:877-880).
+template <typename R, int C>
+__device__ __forceinline__ void add_loss(const PhysR<R>& P, R n, const Cx<R>* ps, Cx<R>* H) {
+    const R an2 = P.alpha * n * n;
+#pragma unroll
+    for (int s = 0; s < C; ++s) {
+        H[s].x = fm(an2, ps[s].y, H[s].x);
+        H[s].y = fm(-an2, ps[s].x, H[s].y);
     }
 }
 
 // Local (non-kinetic) part of H for spin-1 (Spin1GpeBCC.cu:867-912).  ext: use the
 // external field (leapfrog / Euler); the imaginary-time kernel uses only c2<F>
 // (Spin1GpeBCC.cu:645-646).  pot = trap value; lossqz: loss and quadratic Zeeman
-// allowed.  totalPot_out receives trap + c0 rho for the hyperbolic c_K.
+// allowed.  hyper: H scaled by -c_K first (RelativisticSpin1Gpe/common_kernels.h:
+// 229-235).
 template <typename R>
 __device__ __forceinline__ void local_spin1(const PhysR<R>& P, const R r[3], R pot, bool ext, bool lossqz,
                                             bool hyper, const Cx<R>* ps, Cx<R>* H, const PhysR<R>* F = nullptr) {
     const PhysR<R>& Fs = F ? *F : P;
-    const R n1 = ps[0].x * ps[0].x + ps[0].y * ps[0].y;
-    const R n_1 = ps[2].x * ps[2].x + ps[2].y * ps[2].y;
-    const R normSq = n1 + (ps[1].x * ps[1].x + ps[1].y * ps[1].y) + n_1;
-    Cx<R> totalPot = cx<R>(pot + P.c0 * normSq, (R)0);
-    if (lossqz && (P.flags & GPE_FLAG_THREE_BODY_LOSS)) totalPot.y = -P.alpha * normSq * normSq;
+    const R n1 = norm_sq(ps[0]), n_1 = norm_sq(ps[2]);
+    const R n = n1 + norm_sq(ps[1]) + n_1;
+    const R T = fm(P.c0, n, pot);
     if (hyper) {
-        // RelativisticSpin1Gpe/common_kernels.h:229-235
-        const R cK = (R)1 + P.sigma * totalPot.x;
+        const R cK = fm(P.sigma, T, (R)1);
+#pragma unroll
         for (int s = 0; s < 3; ++s) H[s] = (-cK) * H[s];
     }
-    H[0] += totalPot * ps[0];
-    H[1] += totalPot * ps[1];
-    H[2] += totalPot * ps[2];
-    const Cx<R> magXY = (R)GPE_REF_SQRT_2 * (conj(ps[0]) * ps[1] + conj(ps[1]) * ps[2]);
-    R B[3];
+    // B = B_ext + c2 <F> with <F_x> + i <F_y> = sqrt2 m, m = conj(psi_1) psi_0 +
+    // conj(psi_0) psi_-1; the matrix elements off the diagonal are b = (Bx + i By) /
+    // sqrt2 = B_ext / sqrt2 + c2 m and its conjugate
+    Cx<R> m = cx<R>(ps[0].x * ps[1].x, ps[0].x * ps[1].y);
+    m.x = fm(ps[0].y, ps[1].y, m.x);
+    m.y = fm(-ps[0].y, ps[1].x, m.y);
+    add_conj_mul(m, ps[1], ps[2]);
+    R Bz;
+    Cx<R> b = P.c2 * m;
     if (ext) {
+        R B[3];
         mag_field(P, r, Fs.bq, Fs.bb, B);
-        B[0] += P.c2 * magXY.x;
-        B[1] += P.c2 * magXY.y;
-        B[2] += P.c2 * (n1 - n_1);
+        b.x = fm((R)GPE_REF_INV_SQRT_2, B[0], b.x);
+        b.y = fm((R)GPE_REF_INV_SQRT_2, B[1], b.y);
+        Bz = fm(P.c2, n1 - n_1, B[2]);
     } else {
-        B[0] = P.c2 * magXY.x;
-        B[1] = P.c2 * magXY.y;
-        B[2] = P.c2 * (n1 - n_1);
+        Bz = P.c2 * (n1 - n_1);
     }
-    Cx<R> Bxy = (R)GPE_REF_INV_SQRT_2 * cx<R>(B[0], B[1]);
-    Cx<R> BxyConj = conj(Bxy);
-    H[0] += (B[2] * ps[0] + BxyConj * ps[1]);
-    H[1] += (Bxy * ps[0] + BxyConj * ps[2]);
-    H[2] += (Bxy * ps[1] - B[2] * ps[2]);
+    add_scaled(H[0], T + Bz, ps[0]);
+    add_conj_mul(H[0], b, ps[1]);
+    add_scaled(H[1], T, ps[1]);
+    add_mul(H[1], b, ps[0]);
+    add_conj_mul(H[1], b, ps[2]);
+    add_scaled(H[2], T - Bz, ps[2]);
+    add_mul(H[2], b, ps[1]);
+    if (lossqz && (P.flags & GPE_FLAG_THREE_BODY_LOSS)) add_loss<R, 3>(P, n, ps, H);
     if (lossqz && (P.flags & GPE_FLAG_QUADRATIC_ZEEMAN)) {
         // Spin1GpeBCC.cu:897-912
         R Q[3];
         mag_field(P, r, Fs.bqq, Fs.bbq, Q);
-        Bxy = (R)GPE_REF_INV_SQRT_2 * cx<R>(Q[0], Q[1]);
-        BxyConj = conj(Bxy);
-        const R BxyNormSq = (BxyConj * Bxy).x;
-        const Cx<R> BxySq = Bxy * Bxy;
-        const Cx<R> BxyConjSq = BxyConj * BxyConj;
-        const R BzSq = Q[2] * Q[2];
-        const Cx<R> BzBxy = Q[2] * Bxy;
-        const Cx<R> BzBxyConj = Q[2] * BxyConj;
-        H[0] += (BzSq + BxyNormSq) * ps[0] + BzBxyConj * ps[1] + BxyConjSq * ps[2];
-        H[1] += BzBxy * ps[0] + ((R)2 * BxyNormSq) * ps[1] - BzBxyConj * ps[2];
-        H[2] += BxySq * ps[0] - BzBxy * ps[1] + (BzSq + BxyNormSq) * ps[2];
+        const Cx<R> q = (R)GPE_REF_INV_SQRT_2 * cx<R>(Q[0], Q[1]);
+        const R n2 = norm_sq(q), zz = fm(Q[2], Q[2], n2);
+        const Cx<R> sq = cx<R>(fm(-q.y, q.y, q.x * q.x), (R)2 * q.x * q.y);
+        const Cx<R> zq = Q[2] * q, mzq = (-Q[2]) * q;
+        add_scaled(H[0], zz, ps[0]);
+        add_conj_mul(H[0], zq, ps[1]);
+        add_conj_mul(H[0], sq, ps[2]);
+        add_mul(H[1], zq, ps[0]);
+        add_scaled(H[1], (R)2 * n2, ps[1]);
+        add_conj_mul(H[1], mzq, ps[2]);
+        add_mul(H[2], sq, ps[0]);
+        add_mul(H[2], mzq, ps[1]);
+        add_scaled(H[2], zz, ps[2]);
     }
 }
 
-// Local part of H for spin-2 (Spin2GpeBCC.cu:923-970; RelativisticSpin2Gpe.cu:1068-1125).
+// Local part of H for spin-2 (Spin2GpeBCC.cu:923-970; RelativisticSpin2Gpe.cu:1068-1125):
+// with g = c2 <F_z> - B_z, d = c2 conj(<F_+>) - (B_x - i B_y) and the singlet sum
+// theta = psi_0^2 - 2 psi_1 psi_-1 + 2 psi_2 psi_-2, H psi_m = (T + m g) psi_m + (the
+// F_+ and F_- neighbours of m with d and conj(d)) + (-1)^m (c4 / 5) theta conj(psi_-m),
+// which collects the reference's products of three components.
 template <typename R>
 __device__ __forceinline__ void local_spin2(const PhysR<R>& P, const R r[3], R pot, bool ext, bool loss, bool hyper,
                                             const Cx<R>* ps, Cx<R>* H, const PhysR<R>* F = nullptr) {
     const PhysR<R>& Fs = F ? *F : P;
     R n[5];
-    for (int s = 0; s < 5; ++s) n[s] = ps[s].x * ps[s].x + ps[s].y * ps[s].y;
+#pragma unroll
+    for (int s = 0; s < 5; ++s) n[s] = norm_sq(ps[s]);
     const R normSq = n[0] + n[1] + n[2] + n[3] + n[4];
-    Cx<R> ab = cx<R>(pot + P.c0 * normSq, (R)0);
-    if (loss && (P.flags & GPE_FLAG_THREE_BODY_LOSS)) ab.y = -P.alpha * normSq * normSq;
+    const R T = fm(P.c0, normSq, pot);
     if (hyper) {
-        const R cK = (R)1 + P.sigma * ab.x;
+        const R cK = fm(P.sigma, T, (R)1);
+#pragma unroll
         for (int s = 0; s < 5; ++s) H[s] = (-cK) * H[s];
     }
-    R B[3] = {(R)0, (R)0, (R)0};
-    if (ext) mag_field(P, r, Fs.bq, Fs.bb, B);
-    const R c2 = P.c2, c4 = P.c4;
-    const R Fz = c2 * ((R)2 * n[0] + n[1] - n[3] - (R)2 * n[4]);
-    Cx<R> d[5];
-    d[0] = cx<R>((R)2 * Fz + (R)0.4 * c4 * n[4] - (R)2 * B[2], (R)0) + ab;
-    d[1] = cx<R>(Fz + (R)0.4 * c4 * n[3] - B[2], (R)0) + ab;
-    d[2] = cx<R>((R)0.2 * c4 * n[2], (R)0) + ab;
-    d[3] = cx<R>(-Fz + (R)0.4 * c4 * n[1] + B[2], (R)0) + ab;
-    d[4] = cx<R>((R)-2 * Fz + (R)0.4 * c4 * n[0] + (R)2 * B[2], (R)0) + ab;
-    for (int s = 0; s < 5; ++s) H[s] += d[s] * ps[s];
     const Cx<R> s2 = ps[0], s1 = ps[1], s0 = ps[2], s_1 = ps[3], s_2 = ps[4];
+    const Cx<R> zero = cx<R>((R)0, (R)0);
+    // <F_+> / 2 without its sqrt6 part: conj(psi_2) psi_1 + conj(psi_-1) psi_-2, and
+    // the part with it, conj(psi_1) psi_0 + conj(psi_0) psi_-1
+    Cx<R> f2 = zero, f6 = zero;
+    add_conj_mul(f2, s2, s1);
+    add_conj_mul(f2, s_1, s_2);
+    add_conj_mul(f6, s1, s0);
+    add_conj_mul(f6, s0, s_1);
     const R sq6 = (R)2.449489742783178098, sq15 = (R)1.224744871391589049;  // sqrt(6), sqrt(1.5)
-    const Cx<R> den = c2 * ((R)2 * (s2 * conj(s1) + s_1 * conj(s_2)) + sq6 * (s1 * conj(s0) + s0 * conj(s_1))) -
-                      cx<R>(B[0], -B[1]);
-    const Cx<R> c12 = den - ((R)0.4 * c4 * s_1) * conj(s_2);
-    const Cx<R> c45 = den - ((R)0.4 * c4 * s2) * conj(s1);
-    const Cx<R> c13 = ((R)0.2 * c4 * s0) * conj(s_2);
-    const Cx<R> c35 = ((R)0.2 * c4 * s2) * conj(s0);
-    const Cx<R> c23 = sq15 * den - ((R)0.2 * c4 * s0) * conj(s_1);
-    const Cx<R> c34 = sq15 * den - ((R)0.2 * c4 * s1) * conj(s0);
-    H[0] += (c12 * s1 + c13 * s0);
-    H[1] += (conj(c12) * s2 + c23 * s0);
-    H[2] += (conj(c13) * s2 + c35 * s_2 + c34 * s_1 + conj(c23) * s1);
-    H[3] += (conj(c34) * s0 + c45 * s_2);
-    H[4] += (conj(c35) * s0 + conj(c45) * s_1);
+    R g = fm((R)2, n[0] - n[4], n[1] - n[3]);
+    const R c2x2 = (R)2 * P.c2, c2x6 = sq6 * P.c2;
+    Cx<R> d = cx<R>(fm(c2x6, f6.x, c2x2 * f2.x), fm(-c2x6, f6.y, -(c2x2 * f2.y)));
+    if (ext) {
+        R B[3];
+        mag_field(P, r, Fs.bq, Fs.bb, B);
+        g = fm(P.c2, g, -B[2]);
+        d.x = d.x - B[0];
+        d.y = d.y + B[1];
+    } else {
+        g = P.c2 * g;
+    }
+    Cx<R> th = zero;
+    add_mul(th, s2, s_2);
+    add_mul(th, cx<R>(-s1.x, -s1.y), s_1);
+    th = (R)2 * th;
+    add_mul(th, s0, s0);
+    th = ((R)0.2 * P.c4) * th;
+    const Cx<R> e = sq15 * d, mth = cx<R>(-th.x, -th.y);
+    add_scaled(H[0], fm((R)2, g, T), s2);
+    add_mul(H[0], d, s1);
+    add_conj_mul(H[0], s_2, th);
+    add_scaled(H[1], T + g, s1);
+    add_conj_mul(H[1], d, s2);
+    add_mul(H[1], e, s0);
+    add_conj_mul(H[1], s_1, mth);
+    add_scaled(H[2], T, s0);
+    add_conj_mul(H[2], e, s1);
+    add_mul(H[2], e, s_1);
+    add_conj_mul(H[2], s0, th);
+    add_scaled(H[3], T - g, s_1);
+    add_conj_mul(H[3], e, s0);
+    add_mul(H[3], d, s_2);
+    add_conj_mul(H[3], s1, mth);
+    add_scaled(H[4], fm((R)-2, g, T), s_2);
+    add_conj_mul(H[4], d, s_1);
+    add_conj_mul(H[4], s2, th);
+    if (loss && (P.flags & GPE_FLAG_THREE_BODY_LOSS)) add_loss<R, 5>(P, normSq, ps, H);
 }
 
 template <typename R>
 __device__ __forceinline__ void local_scalar(const PhysR<R>& P, R pot, bool loss, bool hyper, const Cx<R>* ps, Cx<R>* H) {
     // GPUGrossPitaevskii_BCC.cu:198-199; RelativisticGpeBCC.cu:244-253
-    const R normsq = ps[0].x * ps[0].x + ps[0].y * ps[0].y;
-    Cx<R> tp = cx<R>(pot + P.c0 * normsq, (R)0);
-    if (loss && (P.flags & GPE_FLAG_THREE_BODY_LOSS)) tp.y = -P.alpha * normsq * normsq;
+    const R n = norm_sq(ps[0]);
+    const R T = fm(P.c0, n, pot);
     if (hyper) {
-        const R cK = (R)1 + P.sigma * tp.x;
+        const R cK = fm(P.sigma, T, (R)1);
         H[0] = (-cK) * H[0];
     }
-    H[0] += tp * ps[0];
+    add_scaled(H[0], T, ps[0]);
+    if (loss && (P.flags & GPE_FLAG_THREE_BODY_LOSS)) add_loss<R, 1>(P, n, ps, H);
 }
 
 template <typename R, int C>
@@ -344,7 +433,7 @@ __device__ __forceinline__ void write_update(int mode, R dt, char* nxt, char* hp
         char* p = nxt + s * 2 * sizeof(R);
         if (mode == GPE_MODE_LEAPFROG) {
             Cx<R> v = ldc_rw<R>(p);
-            v += ((R)2 * dt) * cx<R>(H[s].y, -H[s].x);
+            add_scaled(v, (R)2 * dt, cx<R>(H[s].y, -H[s].x));
             stc<R>(p, v);
         } else if (mode == GPE_MODE_EULER) {
             stc<R>(p, prv[s] + dt * cx<R>(H[s].y, -H[s].x));
@@ -677,14 +766,15 @@ __device__ __forceinline__ void node_finish(const PhysR<R>& P, const R pos[3], u
                                             const Cx<R>* prv, Cx<R>* H, Cx<R>* nv, char* nxt, char* hp,
                                             const PhysR<R>* F = nullptr, OA* oa = nullptr) {
     R r[3];
-    r[0] = P.p0[0] + P.bs * ((R)x * P.bw[0] + pos[0]);
-    r[1] = P.p0[1] + P.bs * ((R)y * P.bw[1] + pos[1]);
-    r[2] = P.p0[2] + P.bs * ((R)z * P.bw[2] + pos[2]);
+    node_pos(P, x, y, z, pos, r);
     const R pot = trap<R>(P, r, F);
     if constexpr (MODE == kModeItpNorm) {
         local_terms<R, C>(P, r, pot, GPE_MODE_ITP, false, prv, H, F);
 #pragma unroll
-        for (int s = 0; s < C; ++s) nv[s] = prv[s] - P.dt * H[s];
+        for (int s = 0; s < C; ++s) {
+            nv[s] = prv[s];
+            add_scaled(nv[s], -P.dt, H[s]);
+        }
         st_node<R, C>(nxt, nv);
         oa->template add<C>(nv);
         return;
@@ -694,7 +784,7 @@ __device__ __forceinline__ void node_finish(const PhysR<R>& P, const R pos[3], u
     if constexpr (MODE == GPE_MODE_LEAPFROG || MODE == kModeLeapfrogFrom) {
         // next = old + 2 dt (-i H), the whole record written at once
 #pragma unroll
-        for (int s = 0; s < C; ++s) nv[s] += ((R)2 * P.dt) * cx<R>(H[s].y, -H[s].x);
+        for (int s = 0; s < C; ++s) add_scaled(nv[s], (R)2 * P.dt, cx<R>(H[s].y, -H[s].x));
         st_node<R, C>(nxt, nv);
     } else {
         write_update<R, C>(MODE, P.dt, nxt, hp, prv, H);
@@ -738,7 +828,7 @@ __device__ __forceinline__ void parabolic_node_t(const Grid& g, const NodeTab<R,
         for (int k = 0; k < G; ++k) {
             if (k0 + k < D) {
 #pragma unroll
-                for (int s = 0; s < C; ++s) H[s] += t.w[k0 + k] * (v[k][s] - prv[s]);
+                for (int s = 0; s < C; ++s) add_scaled(H[s], t.w[k0 + k], v[k][s] - prv[s]);
             }
         }
     }
@@ -764,7 +854,7 @@ __device__ __forceinline__ void parabolic_node_t(const Grid& g, const NodeTab<R,
 #pragma unroll
                 for (int k = 0; k < G; ++k) {
     #pragma unroll
-                    for (int s = 0; s < C; ++s) H[s] += w[h + k] * (v[k][s] - prv[s]);
+                    for (int s = 0; s < C; ++s) add_scaled(H[s], w[h + k], v[k][s] - prv[s]);
                 }
             }
         }
@@ -821,7 +911,7 @@ __device__ __forceinline__ void parabolic_node(const Grid& g, const SmemTables<R
                     if (f + k < f1) {
                                 const R w = st.w[f + k];
 #pragma unroll
-                        for (int s = 0; s < C; ++s) H[s] += w * (v[k][s] - prv[s]);
+                        for (int s = 0; s < C; ++s) add_scaled(H[s], w, v[k][s] - prv[s]);
                     }
                 }
             }
@@ -831,7 +921,7 @@ __device__ __forceinline__ void parabolic_node(const Grid& g, const SmemTables<R
                 ld_node<R, C, true>(base + st.nb_off[f], v);
                 const R w = st.w[f];
 #pragma unroll
-                for (int s = 0; s < C; ++s) H[s] += w * (v[s] - prv[s]);
+                for (int s = 0; s < C; ++s) add_scaled(H[s], w, v[s] - prv[s]);
             }
         }
         const R pos[3] = {st.pos[3 * l + 0], st.pos[3 * l + 1], st.pos[3 * l + 2]};
@@ -1006,8 +1096,8 @@ __device__ __forceinline__ void q_update(const StepArgs& a, const SmemHyper<R>& 
         if constexpr (QM == 1) {
             v[s] = d0psi;
         } else if constexpr (QM == 0) {
-            const Cx<R> qq = ((R)2 * dts) * (pq[s] + d0psi);
-            v[s] += cx<R>(-qq.y, qq.x);
+            const Cx<R> qq = pq[s] + d0psi;
+            add_scaled(v[s], (R)2 * dts, cx<R>(-qq.y, qq.x));
         } else if constexpr (QM == 3) {
             v[s] = pq[s] - dts * (pq[s] - d0psi);
         } else {
@@ -1087,7 +1177,7 @@ __global__ void __launch_bounds__(256) hyper_step_kernel(StepArgs a, uint32_t no
                 Cx<R> qv[C];
                 ld_node<R, C, true>(qb + off[k], qv);
 #pragma unroll
-                for (int s = 0; s < C; ++s) H[s] += w[k] * qv[s];
+                for (int s = 0; s < C; ++s) add_scaled(H[s], w[k], qv[s]);
             }
         } else {
             for (int k = 0; k < F; ++k) {
@@ -1095,13 +1185,11 @@ __global__ void __launch_bounds__(256) hyper_step_kernel(StepArgs a, uint32_t no
                 ld_node<R, C, true>(qb + sh.inc_off[l * F + k], qv);
                 const R w = sh.inc_w[l * F + k];
 #pragma unroll
-                for (int s = 0; s < C; ++s) H[s] += w * qv[s];
+                for (int s = 0; s < C; ++s) add_scaled(H[s], w, qv[s]);
             }
         }
         R r[3];
-        r[0] = P.p0[0] + P.bs * ((R)x * P.bw[0] + sh.pos[3 * l + 0]);
-        r[1] = P.p0[1] + P.bs * ((R)y * P.bw[1] + sh.pos[3 * l + 1]);
-        r[2] = P.p0[2] + P.bs * ((R)z * P.bw[2] + sh.pos[3 * l + 2]);
+        node_pos(P, x, y, z, sh.pos + 3 * l, r);
         const R pot = trap<R>(P, r);
         if constexpr (C == 1) {
             local_scalar<R>(P, pot, false, HYPERB, prv, H);
@@ -1224,9 +1312,7 @@ __global__ void __launch_bounds__(256) observe_kernel(StepArgs a) {
         }
         const PhysR<A>& P = make_phys<A>(a);
         A r[3];
-        r[0] = P.p0[0] + P.bs * ((A)x * P.bw[0] + st.pos[3 * l + 0]);
-        r[1] = P.p0[1] + P.bs * ((A)y * P.bw[1] + st.pos[3 * l + 1]);
-        r[2] = P.p0[2] + P.bs * ((A)z * P.bw[2] + st.pos[3 * l + 2]);
+        node_pos(P, x, y, z, st.pos + 3 * l, r);
         local_terms<A, C>(P, r, trap<A>(P, r), GPE_MODE_LEAPFROG, false, ps, Hl);
         // interaction-only part: no trap, no external field, no loss / quadratic
         // Zeeman.  Scalars: psi^H (c0 n) psi = c0 n^2; spin-1: psi^H [c0 n +
@@ -1641,9 +1727,7 @@ __global__ void __launch_bounds__(256) split_step_kernel(StepArgs a, uint32_t no
             for (int k = 0; k < F; ++k) d1q += sh.inc_w[l * F + k] * *reinterpret_cast<const R*>(qb + sh.inc_off[l * F + k]);
         }
         R r[3];
-        r[0] = P.p0[0] + P.bs * ((R)x * P.bw[0] + sh.pos[3 * l + 0]);
-        r[1] = P.p0[1] + P.bs * ((R)y * P.bw[1] + sh.pos[3 * l + 1]);
-        r[2] = P.p0[2] + P.bs * ((R)z * P.bw[2] + sh.pos[3 * l + 2]);
+        node_pos(P, x, y, z, sh.pos + 3 * l, r);
         const R tp = trap<R>(P, r) + P.c0 * (v.x * v.x + v.y * v.y);
         if constexpr (PART == 0) *reinterpret_cast<R*>(own + wr) = v.y - P.dt * (tp * v.x - d1q);
         else *reinterpret_cast<R*>(own + wr) = v.x + P.dt * (tp * v.y - d1q);
