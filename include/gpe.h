@@ -392,7 +392,7 @@ gpe_status gpe_node_fields_reduce(gpe_handle* h, int32_t slot, int32_t kind, dou
  *                      hyperbolic scheme with 4 edges per node and 2 edges per
  *                      node of a cell -- BCC, C15).  The call changes the two psi
  *                      slots (and q) into a cell-interleaved layout (node l,
- *                      component s of 32 or 16 cells along x contiguous), steps
+ *                      component s of 32, 16 or 8 cells along x contiguous), steps
  *                      there and changes them back; the states are those of the
  *                      gather kernel, bit for bit.  Single explicit steps
  *                      (gpe_step_explicit, imaginary time) take the gather kernel.

@@ -298,14 +298,16 @@ __device__ __forceinline__ void batch_item(const BatchMember& M, const MK& K, co
                                            uint32_t row0, uint32_t rows) {
     if constexpr (IL && sizeof(R) == 4) {
         if (M.il_deg) {
-            const bool c32 = M.ilg.cells == 32;
             if ((CMASK & 2) && M.C == 3) {
+                const uint32_t c = M.ilg.cells;
                 if (M.il_deg == 4) {
-                    if (c32) batch_il_rows<3, 4, 32>(M, st, P, F, prev, next, row0, rows);
-                    else batch_il_rows<3, 4, 16>(M, st, P, F, prev, next, row0, rows);
+                    if (c == 32) batch_il_rows<3, 4, 32>(M, st, P, F, prev, next, row0, rows);
+                    else if (c == 16) batch_il_rows<3, 4, 16>(M, st, P, F, prev, next, row0, rows);
+                    else batch_il_rows<3, 4, 8>(M, st, P, F, prev, next, row0, rows);
                 } else {
-                    if (c32) batch_il_rows<3, 8, 32>(M, st, P, F, prev, next, row0, rows);
-                    else batch_il_rows<3, 8, 16>(M, st, P, F, prev, next, row0, rows);
+                    if (c == 32) batch_il_rows<3, 8, 32>(M, st, P, F, prev, next, row0, rows);
+                    else if (c == 16) batch_il_rows<3, 8, 16>(M, st, P, F, prev, next, row0, rows);
+                    else batch_il_rows<3, 8, 8>(M, st, P, F, prev, next, row0, rows);
                 }
             }
             return;

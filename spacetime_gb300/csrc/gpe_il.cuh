@@ -429,11 +429,24 @@ unsigned il_blocks_d(const ILGrid& G, bool obs, size_t max_blocks) {
     return il_wave(G, threads, o, max_blocks);
 }
 
+// f(<cells of a group>, <entries of a row>) as compile-time constants; bad where the
+// kernels have no such form.
+template <class T, class F>
+T il_form(const ILGrid& G, int deg, T bad, F f) {
+    auto with = [&](auto cells) {
+        if (deg == 4) return f(cells, std::integral_constant<int, 4>());
+        if (deg == 8) return f(cells, std::integral_constant<int, 8>());
+        return bad;
+    };
+    if (G.cells == 32) return with(std::integral_constant<int, 32>());
+    if (G.cells == 16) return with(std::integral_constant<int, 16>());
+    if (G.cells == 8) return with(std::integral_constant<int, 8>());
+    return bad;
+}
+
 template <int C>
 unsigned il_blocks(const ILGrid& G, int deg, bool obs, size_t max_blocks) {
-    if (G.cells == 32)
-        return deg == 4 ? il_blocks_d<C, 4, 32>(G, obs, max_blocks) : il_blocks_d<C, 8, 32>(G, obs, max_blocks);
-    return deg == 4 ? il_blocks_d<C, 4, 16>(G, obs, max_blocks) : il_blocks_d<C, 8, 16>(G, obs, max_blocks);
+    return il_form(G, deg, 0u, [&](auto cells, auto d) { return il_blocks_d<C, d(), cells()>(G, obs, max_blocks); });
 }
 
 // One interleaved leapfrog step (a.prev / a.next: interleaved buffers) on rows of
@@ -456,14 +469,9 @@ cudaError_t launch_il_step_d(const StepArgs& a, const ILGrid& G, size_t max_bloc
 template <int C>
 cudaError_t launch_il_step(const StepArgs& a, const ILGrid& G, int deg, size_t max_blocks, bool obs, double* out,
                            cudaStream_t s) {
-    if (G.cells == 32) {
-        if (deg == 4) return launch_il_step_d<C, 4, 32>(a, G, max_blocks, obs, out, s);
-        if (deg == 8) return launch_il_step_d<C, 8, 32>(a, G, max_blocks, obs, out, s);
-    } else if (G.cells == 16) {
-        if (deg == 4) return launch_il_step_d<C, 4, 16>(a, G, max_blocks, obs, out, s);
-        if (deg == 8) return launch_il_step_d<C, 8, 16>(a, G, max_blocks, obs, out, s);
-    }
-    return cudaErrorInvalidValue;
+    return il_form(G, deg, cudaErrorInvalidValue, [&](auto cells, auto d) {
+        return launch_il_step_d<C, d(), cells()>(a, G, max_blocks, obs, out, s);
+    });
 }
 
 template <int C, int D, int CELLS>
@@ -482,14 +490,8 @@ cudaError_t launch_il_itp_d(const StepArgs& a, const ILGrid& G, size_t max_block
 // One imaginary-time iteration (a.prev / a.next: interleaved buffers).
 template <int C>
 cudaError_t launch_il_itp(const StepArgs& a, const ILGrid& G, int deg, size_t max_blocks, cudaStream_t s) {
-    if (G.cells == 32) {
-        if (deg == 4) return launch_il_itp_d<C, 4, 32>(a, G, max_blocks, s);
-        if (deg == 8) return launch_il_itp_d<C, 8, 32>(a, G, max_blocks, s);
-    } else if (G.cells == 16) {
-        if (deg == 4) return launch_il_itp_d<C, 4, 16>(a, G, max_blocks, s);
-        if (deg == 8) return launch_il_itp_d<C, 8, 16>(a, G, max_blocks, s);
-    }
-    return cudaErrorInvalidValue;
+    return il_form(G, deg, cudaErrorInvalidValue,
+                   [&](auto cells, auto d) { return launch_il_itp_d<C, d(), cells()>(a, G, max_blocks, s); });
 }
 
 #define GPE_INSTANTIATE_IL(C)                                                                                           \
@@ -670,12 +672,17 @@ cudaError_t launch_il_hyper(const StepArgs& a, const ILGrid& G, const ILGrid& Gq
     const uint64_t tasks64 = (uint64_t)il_warp_tasks(G) * G.V;
     if (tasks64 > 0xffffffffu || G.cells != Gq.cells || G.GX != Gq.GX || Gq.V != 2 * G.V) return cudaErrorInvalidValue;
     const FastDiv dGX = make_fastdiv(G.GX);
-    if (G.cells == 32) {
-        const unsigned nb = il_hyper_blocks_c<C, 32>(G, Gq);
-        il_hyper_kernel<C, 32><<<nb, kIlPlainThreads, 0, s>>>(a, G, Gq, tab, dGX);
-    } else {
-        const unsigned nb = il_hyper_blocks_c<C, 16>(G, Gq);
-        il_hyper_kernel<C, 16><<<nb, kIlPlainThreads, 0, s>>>(a, G, Gq, tab, dGX);
+    switch (G.cells) {
+        case 32:
+            il_hyper_kernel<C, 32><<<il_hyper_blocks_c<C, 32>(G, Gq), kIlPlainThreads, 0, s>>>(a, G, Gq, tab, dGX);
+            break;
+        case 16:
+            il_hyper_kernel<C, 16><<<il_hyper_blocks_c<C, 16>(G, Gq), kIlPlainThreads, 0, s>>>(a, G, Gq, tab, dGX);
+            break;
+        case 8:
+            il_hyper_kernel<C, 8><<<il_hyper_blocks_c<C, 8>(G, Gq), kIlPlainThreads, 0, s>>>(a, G, Gq, tab, dGX);
+            break;
+        default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }

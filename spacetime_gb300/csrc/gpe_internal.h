@@ -99,26 +99,34 @@ struct Grid {
 
 // Geometry of an FP32 state in the cell-interleaved layout.  Rows (y, z) run from
 // -1 to Y and -1 to Z (the halo rows and planes are zero); a row holds GX groups of
-// `cells` (32 or 16) consecutive cells along x; a group holds [node l][component
+// `cells` (32, 16 or 8) consecutive cells along x; a group holds [node l][component
 // s][cell of the group][re, im], so that node l's component s of a group's cells
 // is one contiguous run of 8 cells bytes.  Cells x >= X of the last group, and the
 // cells x = -1 and x = X, read as zero.  A warp takes node l of 32 / cells groups,
-// the grid's groups counted row after row.  The group width is chosen per grid:
-// 32 where that leaves no more lanes idle than 16 would (X a multiple of 32, or
-// X mod 32 > 16), 16 otherwise.  Measured (FP32 leapfrog, fraction of the copy
-// peak, 32 / 16): spin-1 BCC 96^3 0.860 / 0.833, A15 64^3 0.857 / 0.832, Z 56^3
-// 0.774 / 0.750, C15 48^3 0.700 / 0.829; the 256-member ensemble 0.555 / 0.568.
+// the grid's groups counted row after row.
 struct ILGrid {
     uint32_t X, Y, Z, V, C, GX;
-    uint32_t cells; // cells per group: 32 or 16
+    uint32_t cells; // cells per group: 32, 16 or 8
     size_t gb;      // bytes per group: V * C * cells * 8
     size_t row;     // bytes per row: GX * gb
     size_t bytes;   // the buffer: (Y + 2) (Z + 2) rows
 };
 
-inline uint32_t il_group_cells(uint32_t X) {
-    const uint32_t g32 = (X + 31) / 32, g16 = (X + 15) / 16;
-    return 32 * g32 <= 16 * g16 ? 32 : 16;
+// The group width, per grid: narrow groups leave fewer lanes idle in a row's last
+// group, but a warp's loads then fall into 2 (16 cells) or 4 (8 cells) shorter runs.
+// What that costs where no lane is idle (FP32, one launch, 32 / 16 / 8 cells): spin-1
+// BCC 96^3 124.7 / 129.2 / 141.6 us, A15 64^3 142.1 / 147.6 / 164.0; spin-2 BCC 64^3
+// 64.9 / 67.2 / 68.9, C15 32^3 90.3 / 94.2 / 99.4; hyperbolic spin-2 BCC 64^3 171.9 /
+// 174.1 / 180.5 -- taken as 3 % and 15 % (6 % for the spin-2's longer records) on the
+// lanes' count.  Where lanes are idle: spin-1 C15 40^3 141.6 / 124.3 / 120.9, Z 40^3
+// 85.9 / 75.9 / 71.6, BCC 72^3 67.3 / 62.6 / 63.6; hyperbolic spin-2 C15 40^3 620.5 /
+// 545.4 / 501.3, 48^3 923.7 / 818.3 / 863.9.
+inline uint32_t il_group_cells(uint32_t X, uint32_t C) {
+    auto cost = [X](uint32_t cells, uint32_t percent) { return (uint64_t)((X + cells - 1) / cells) * cells * percent; };
+    uint32_t best = 32;
+    if (cost(16, 103) < cost(32, 100)) best = 16;
+    if (cost(8, C == 3 ? 115 : 106) < (best == 32 ? cost(32, 100) : cost(16, 103))) best = 8;
+    return best;
 }
 
 // The interleaved kernels keep a neighbour's offset from its group's base in 32
@@ -134,7 +142,7 @@ inline ILGrid make_il_grid(const Grid& g) {
     G.Z = g.Z;
     G.V = g.V;
     G.C = g.C;
-    G.cells = il_group_cells(g.X);
+    G.cells = il_group_cells(g.X, g.C);
     G.GX = (g.X + G.cells - 1) / G.cells;
     G.gb = (size_t)g.V * g.C * G.cells * 8;
     G.row = G.GX * G.gb;
