@@ -18,6 +18,8 @@ cudaError_t launch_hyper(const StepArgs& a, int kind, cudaStream_t s);
 template <typename R, int C>
 cudaError_t launch_observe(const StepArgs& a, double* out, bool node_fp32, cudaStream_t s);
 template <typename R, int C>
+cudaError_t launch_observe_columns(const StepArgs& a, double* out, cudaStream_t s);
+template <typename R, int C>
 cudaError_t launch_scale(const StepArgs& a, cudaStream_t s);
 template <typename R, int C>
 cudaError_t launch_norm(const StepArgs& a, cudaStream_t s);
@@ -657,17 +659,30 @@ static gpe_status split_launch(gpe_handle* h, int part, double t, cudaStream_t s
     return GPE_OK;
 }
 
+// `columns`: the kernel that sums columns of cells (observe_columns_kernel)
 template <int C>
-static cudaError_t dispatch_observe_c(const gpe_handle* h, const StepArgs& a, double* out, cudaStream_t s) {
+static cudaError_t dispatch_observe_c(const gpe_handle* h, const StepArgs& a, bool columns, double* out, cudaStream_t s) {
+    if (columns)
+        return h->real_bytes == 8 ? launch_observe_columns<double, C>(a, out, s) : launch_observe_columns<float, C>(a, out, s);
     return h->real_bytes == 8 ? launch_observe<double, C>(a, out, false, s)
                               : launch_observe<float, C>(a, out, h->tune_observe != 0, s);
 }
-static cudaError_t dispatch_observe(const gpe_handle* h, const StepArgs& a, double* out, cudaStream_t s) {
+static cudaError_t dispatch_observe(const gpe_handle* h, const StepArgs& a, bool columns, double* out, cudaStream_t s) {
     switch (h->g.C) {
-        case 1: return dispatch_observe_c<1>(h, a, out, s);
-        case 3: return dispatch_observe_c<3>(h, a, out, s);
-        default: return dispatch_observe_c<5>(h, a, out, s);
+        case 1: return dispatch_observe_c<1>(h, a, columns, out, s);
+        case 3: return dispatch_observe_c<3>(h, a, columns, out, s);
+        default: return dispatch_observe_c<5>(h, a, columns, out, s);
     }
+}
+// Where gpe_observe takes the columns kernel: FP64 node terms, rows of up to 4, 6 or 8
+// entries, and no quadratic Zeeman term (its field products would need moments of
+// their own).  FP32 node terms (GPE_TUNE_OBSERVE_ARITH 1) keep observe_kernel, which
+// is bound by its loads there.
+static bool observe_columns_applies(const gpe_handle* h) {
+    const int d = h->tab.max_deg;
+    if (h->real_bytes == 4 && h->tune_observe) return false;
+    if (h->g.C == 3 && (h->p.flags & GPE_FLAG_QUADRATIC_ZEEMAN)) return false;
+    return d <= 4 || d == 6 || d == 8;
 }
 template <int C>
 static cudaError_t dispatch_norm_c(const gpe_handle* h, const StepArgs& a, cudaStream_t s) {
@@ -1620,12 +1635,16 @@ extern "C" gpe_status gpe_observe(gpe_handle* h, int32_t slot, double t, gpe_obs
     cudaStream_t s = (cudaStream_t)stream;
     StepArgs a = make_args(h, fields_at(h, t), t);
     a.prev = h->interior[slot];
-    cudaError_t e = dispatch_observe(h, a, h->obs_out, s);
-    if (e != cudaSuccess) return cuda_fail(e, "observe launch");
-    h->launches += 2;
     double r[OBS_COUNT];
-    CUDA_TRY(cudaMemcpyAsync(r, h->obs_out, sizeof r, cudaMemcpyDeviceToHost, s));
-    CUDA_TRY(cudaStreamSynchronize(s));
+    for (bool columns = observe_columns_applies(h);; columns = false) {
+        cudaError_t e = dispatch_observe(h, a, columns, h->obs_out, s);
+        if (e != cudaSuccess) return cuda_fail(e, "observe launch");
+        h->launches += 2;
+        CUDA_TRY(cudaMemcpyAsync(r, h->obs_out, sizeof r, cudaMemcpyDeviceToHost, s));
+        CUDA_TRY(cudaStreamSynchronize(s));
+        // a state out of the range of the pairs is summed again in FP64
+        if (!columns || h->real_bytes == 8 || pair_range(r[OBS_MAXABS])) break;
+    }
     gpe_status dst = check_device_error(h, s);
     if (dst) return dst;
     return fill_observables(h, r, out);

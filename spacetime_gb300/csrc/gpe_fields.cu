@@ -22,6 +22,9 @@
 
 namespace gpe {
 
+template <typename R, int C>
+cudaError_t launch_field_sums(const StepArgs& a, bool spin, bool fp64, double* out, cudaStream_t s);
+
 static int field_width(int kind) {
     switch (kind) {
         case GPE_FIELD_DENSITY: return 1;
@@ -140,45 +143,18 @@ __global__ void __launch_bounds__(256) node_fields_kernel(StepArgs a, double* ou
     }
 }
 
-// Block partials of a field buffer: DENSITY sum; SPIN (spin norm, rho s_x, rho s_y,
-// rho s_z, rho) sums, the weighting of integrateVecWithDensity; MAX_HAMILTON max.
-__global__ void __launch_bounds__(256) fields_reduce_kernel(const double* buf, uint64_t n, int kind, double* partials) {
-    __shared__ double red[8][5];
-    const bool is_max = kind == GPE_FIELD_MAX_HAMILTON;
-    double acc[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) acc[k] = is_max ? -INFINITY : 0.0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        if (kind == GPE_FIELD_SPIN) {
-            const double* v = buf + i * 5;
-            acc[0] += v[0];
-            acc[1] += v[4] * v[1];
-            acc[2] += v[4] * v[2];
-            acc[3] += v[4] * v[3];
-            acc[4] += v[4];
-        } else if (is_max) {
-            acc[0] = fmax(acc[0], buf[i]);
-        } else {
-            acc[0] += buf[i];
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-        double v = acc[k];
-        for (int off = 16; off > 0; off >>= 1) {
-            const double u = __shfl_down_sync(0xffffffffu, v, off);
-            v = is_max ? fmax(v, u) : v + u;
-        }
-        acc[k] = v;
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0)
-        for (int k = 0; k < 5; ++k) red[warp][k] = acc[k];
+// Block maxima of a field buffer (MAX_HAMILTON).
+__global__ void __launch_bounds__(256) fields_max_kernel(const double* buf, uint64_t n, double* partials) {
+    __shared__ double red[8];
+    double v = -INFINITY;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        v = fmax(v, buf[i]);
+    for (int off = 16; off > 0; off >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, off));
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
-    if (threadIdx.x < 5) {
-        double v = red[0][threadIdx.x];
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = is_max ? fmax(v, red[w][threadIdx.x]) : v + red[w][threadIdx.x];
-        partials[(size_t)blockIdx.x * 5 + threadIdx.x] = v;
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) v = fmax(v, red[w]);
+        partials[blockIdx.x] = v;
     }
 }
 
@@ -220,18 +196,24 @@ static cudaError_t launch_fields(const StepArgs& a, int C, int kind, double* out
     return launch_fields_c<R, 5>(a, kind, out, s);
 }
 
-// Checks the request and writes the field of every interior node into the
-// handle's field buffer (grown on demand).
-static gpe_status compute_fields(gpe_handle* h, int32_t slot, int32_t kind, double t, cudaStream_t s, int* width) {
+static gpe_status check_request(const gpe_handle* h, int32_t slot, int32_t kind) {
     if (slot != GPE_PSI_EVEN && slot != GPE_PSI_ODD && slot != GPE_HPSI) return fail(GPE_ERR_INVALID_ARG, "psi slot");
     if (!h->alloc[slot]) return fail(GPE_ERR_INVALID_ARG, "slot not allocated");
-    const int w = field_width(kind);
-    if (w == 0) return fail(GPE_ERR_INVALID_ARG, "unknown field kind");
+    if (field_width(kind) == 0) return fail(GPE_ERR_INVALID_ARG, "unknown field kind");
     const int C = h->g.C;
     if ((kind == GPE_FIELD_SPIN || kind == GPE_FIELD_UV_THETA) && C == 1)
         return fail(GPE_ERR_UNSUPPORTED, "spin fields need a spinor (C = 3 or 5)");
     if ((kind == GPE_FIELD_MAX_HAMILTON || kind == GPE_FIELD_PROJ_X || kind == GPE_FIELD_PROJ_Y) && C != 3)
         return fail(GPE_ERR_UNSUPPORTED, "this field is defined for spin-1 (C = 3)");
+    return GPE_OK;
+}
+
+// Checks the request and writes the field of every interior node into the
+// handle's field buffer (grown on demand).
+static gpe_status compute_fields(gpe_handle* h, int32_t slot, int32_t kind, double t, cudaStream_t s, int* width) {
+    gpe_status st = check_request(h, slot, kind);
+    if (st) return st;
+    const int w = field_width(kind), C = h->g.C;
     const uint64_t nodes = (uint64_t)h->g.X * h->g.Y * h->g.Z * h->g.V;
     const size_t need = (size_t)nodes * w;
     if (need > h->field_count) {
@@ -284,37 +266,58 @@ extern "C" gpe_status gpe_node_fields(gpe_handle* h, int32_t slot, int32_t kind,
     return GPE_OK;
 }
 
+// DENSITY and SPIN integrated straight from the state.
+static gpe_status reduce_sums(gpe_handle* h, int32_t slot, bool spin, double t, double* out, cudaStream_t s) {
+    gpe_fields B;
+    std::memset(&B, 0, sizeof B);
+    StepArgs a = make_args(h, B, t);
+    a.prev = h->interior[slot];
+    double r[6];
+    for (bool fp64 = h->real_bytes == 8;; fp64 = true) {
+        cudaError_t e;
+        if (h->real_bytes == 8)
+            e = h->g.C == 1   ? launch_field_sums<double, 1>(a, spin, fp64, h->obs_out, s)
+                : h->g.C == 3 ? launch_field_sums<double, 3>(a, spin, fp64, h->obs_out, s)
+                              : launch_field_sums<double, 5>(a, spin, fp64, h->obs_out, s);
+        else
+            e = h->g.C == 1   ? launch_field_sums<float, 1>(a, spin, fp64, h->obs_out, s)
+                : h->g.C == 3 ? launch_field_sums<float, 3>(a, spin, fp64, h->obs_out, s)
+                              : launch_field_sums<float, 5>(a, spin, fp64, h->obs_out, s);
+        if (e != cudaSuccess) return cuda_fail(e, "node fields reduction");
+        h->launches += 2;
+        e = cudaMemcpyAsync(r, h->obs_out, sizeof r, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return cuda_fail(e, "node fields reduction copy");
+        if (fp64 || pair_range(r[5])) break;
+    }
+    for (int k = 0; k < (spin ? 5 : 1); ++k) out[k] = r[k] * cell_dv(h);
+    return GPE_OK;
+}
+
 extern "C" gpe_status gpe_node_fields_reduce(gpe_handle* h, int32_t slot, int32_t kind, double t, double* out,
                                              void* stream) {
     if (!h || !out) return fail(GPE_ERR_INVALID_ARG, "null argument");
     if (kind != GPE_FIELD_DENSITY && kind != GPE_FIELD_SPIN && kind != GPE_FIELD_MAX_HAMILTON)
         return fail(GPE_ERR_UNSUPPORTED, "reductions exist for DENSITY, SPIN and MAX_HAMILTON");
     cudaStream_t s = (cudaStream_t)stream;
-    int w = 0;
-    gpe_status st = compute_fields(h, slot, kind, t, s, &w);
+    gpe_status st = check_request(h, slot, kind);
     if (st) return st;
+    if (kind != GPE_FIELD_MAX_HAMILTON) return reduce_sums(h, slot, kind == GPE_FIELD_SPIN, t, out, s);
+    int w = 0;
+    if ((st = compute_fields(h, slot, kind, t, s, &w))) return st;
     const uint64_t nodes = (uint64_t)h->g.X * h->g.Y * h->g.Z * h->g.V;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    unsigned nb = (unsigned)std::min<uint64_t>((nodes + 255) / 256, 8ull * (uint64_t)(sms > 0 ? sms : 1));
-    nb = (unsigned)std::min<size_t>(nb, h->partial_blocks * OBS_COUNT / 5);
-    if (nb == 0) nb = 1;
-    fields_reduce_kernel<<<nb, 256, 0, s>>>(h->field_buf, nodes, kind, h->partials);
+    unsigned nb = (unsigned)std::min<uint64_t>((nodes + 255) / 256, 8ull * (uint64_t)device_sm_count());
+    nb = (unsigned)std::min<size_t>(nb, h->partial_blocks * OBS_COUNT);
+    fields_max_kernel<<<nb, 256, 0, s>>>(h->field_buf, nodes, h->partials);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "node fields reduction");
     h->launches += 1;
-    std::vector<double> part((size_t)nb * 5);
+    std::vector<double> part(nb);
     e = cudaMemcpyAsync(part.data(), h->partials, part.size() * sizeof(double), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(e, "node fields reduction copy");
-    const int nout = kind == GPE_FIELD_SPIN ? 5 : 1;
-    const bool is_max = kind == GPE_FIELD_MAX_HAMILTON;
-    const double dv = cell_dv(h);
-    for (int k = 0; k < nout; ++k) {
-        double v = is_max ? -INFINITY : 0.0;
-        for (unsigned b = 0; b < nb; ++b) v = is_max ? std::fmax(v, part[(size_t)b * 5 + k]) : v + part[(size_t)b * 5 + k];
-        out[k] = is_max ? v : v * dv;
-    }
+    double v = -INFINITY;
+    for (double u : part) v = std::fmax(v, u);
+    out[0] = v;
     return GPE_OK;
 }

@@ -116,6 +116,10 @@ bool leapfrog_from_supported(const gpe_handle* h);
 gpe_status leapfrog_from(gpe_handle* h, char* next, const char* cur, const char* old, const gpe_fields& B, double t,
                          cudaStream_t s);
 double cell_dv(const gpe_handle* h);
+// Whether sums in pairs of FP32 values (gpe_observe.cuh) hold a state whose largest
+// value is m: its fourth powers keep their full precision, and stay finite, between
+// 2^-20 and 2^27.
+inline bool pair_range(double m) { return m == 0.0 || (m >= 0x1p-20 && m <= 0x1p27); }
 size_t host_count(const gpe_handle* h, bool is_q);
 gpe_status ensure_stage(gpe_handle* h, size_t count);
 gpe_status check_device_error(gpe_handle* h, cudaStream_t s);

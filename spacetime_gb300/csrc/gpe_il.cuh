@@ -459,7 +459,7 @@ cudaError_t launch_il_step_d(const StepArgs& a, const ILGrid& G, size_t max_bloc
     const FastDiv dGX = make_fastdiv(G.GX);
     if (obs) {
         il_step_obs_kernel<C, D, CELLS><<<nb, kIlObsThreads, 0, s>>>(a, G, dGX);
-        observe_finalize_kernel<<<1, 256, 0, s>>>(a.partials, nb, out);
+        finalize_observables(a.partials, nb, out, s);
     } else {
         il_step_kernel<C, D, CELLS><<<nb, kIlPlainThreads, 0, s>>>(a, G, dGX);
     }

@@ -1,9 +1,12 @@
 // Explicit instantiation of the C=1 kernels (one translation unit per spinor
 // size so that the build compiles them in parallel).
 #include "gpe_kernels.cuh"
+#include "gpe_observe.cuh"
 
 namespace gpe {
 GPE_INSTANTIATE(float, 1)
+GPE_INSTANTIATE_OBSERVE(float, 1)
+GPE_INSTANTIATE_OBSERVE(double, 1)
 GPE_INSTANTIATE(double, 1)
 GPE_INSTANTIATE_TILE(float, 1)
 GPE_INSTANTIATE_TILE(double, 1)

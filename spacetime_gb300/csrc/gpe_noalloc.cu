@@ -290,7 +290,7 @@ extern "C" gpe_status gpe_observe_noalloc(const gpe_lattice_desc* lat, const gpe
             else observe_noalloc_kernel<float, 5><<<nb, 256, 0, s>>>(a, tab, scratch);
             break;
     }
-    observe_finalize_kernel<<<1, 256, 0, s>>>(scratch, nb, result);
+    finalize_observables(scratch, nb, result, s);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return noalloc_fail(GPE_ERR_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     double r[OBS_COUNT];
