@@ -1022,6 +1022,42 @@ __device__ __forceinline__ void parabolic_fixed_body(const StepArgs& a) {
         oa.finish(nred, a.partials, a.dv, a.scale_out);
     }
 }
+// The same update with a thread walking up a column of cells (node l of the cells (x, y,
+// z0 .. z0 + zc - 1), a column per pass): x, y and what depends on them alone -- two
+// thirds of the position, the trap and the field -- are computed once per column.  The
+// FP64 step's form: the FP64 pipe bounds it (87 % busy, DRAM at 5 %), and per node it
+// had some 20 of 139 FP64 operations for those (spin-1 BCC 40^3 0.170 -> 0.157 ms).  The FP32
+// step is bound by its loads and measured no faster in columns.
+template <typename R, int C, int MODE, int D, int G, bool MORE>
+__global__ void __launch_bounds__(256) parabolic_columns_kernel(StepArgs a, uint32_t zc, uint32_t columns, uint32_t total,
+                                                                FastDiv dcol) {
+    __shared__ SmemTables<R> st;
+    load_tables<R>(st, a);
+    __syncthreads();
+    const PhysR<R>& P = make_phys<R>(a);
+    using OA = typename AccOf<MODE, false, R>::type;
+    OA oa = AccOf<MODE, false, R>::make(nullptr);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const uint32_t chunk = fdiv(i, dcol);
+        const uint32_t col = i - chunk * columns;   // (y X + x) V + l
+        const uint32_t y = fdiv(col, a.divRow);
+        const uint32_t within = col - y * a.row_items;
+        const uint32_t x = fdiv(within, a.divV);
+        const uint32_t l = within - x * a.g.V;
+        const int f0 = MORE ? st.row_ptr[l] : (int)l * D;
+        const int f_end = MORE ? st.row_ptr[l + 1] : 0;
+        const NodeTab<R, D> t = node_tab<R, D>(st, l, f0);
+        const uint32_t z1 = min((chunk + 1) * zc, a.g.Z);
+#pragma unroll 1
+        for (uint32_t z = chunk * zc; z < z1; ++z)
+            parabolic_node_t<R, C, MODE, D, G, MORE, OA>(a.g, t, P, a.prev, a.next, a.hpsi, x, y, z, l, &st, f0 + D, f_end,
+                                                         nullptr, &oa);
+    }
+    if constexpr (MODE == kModeItpNorm) {
+        __shared__ double nred[8];
+        oa.finish(nred, a.partials, a.dv, a.scale_out);
+    }
+}
 template <typename R, int C, int MODE, int D, int G, bool MORE>
 __global__ void __launch_bounds__(256) parabolic_fixed_kernel(StepArgs a) {
     parabolic_fixed_body<R, C, MODE, D, G, MORE, false>(a);
@@ -1490,11 +1526,50 @@ __global__ void __launch_bounds__(256) scale_kernel(StepArgs a) {
 
 inline unsigned nblocks(uint64_t items, unsigned bs) { return (unsigned)((items + bs - 1) / bs); }
 
+// The launch of a kernel whose threads walk up columns of cells (256 threads a block,
+// occ blocks per SM): the cells of z per column that leave the busiest thread the least
+// work, with what is done once per column counted as `overhead` nodes.
+struct ColumnGrid {
+    uint32_t zc, columns, total;   // total: columns times chunks of z
+    unsigned blocks;
+};
+inline ColumnGrid column_grid(const StepArgs& a, unsigned occ, uint32_t overhead) {
+    constexpr uint32_t kMost = 64;   // cells per column
+    const uint64_t threads = (uint64_t)occ * (unsigned)device_sm_count() * 256;
+    ColumnGrid g;
+    g.columns = a.row_items * a.g.Y;
+    g.zc = std::min(kMost, a.g.Z);
+    uint64_t best = ~0ull;
+    for (uint32_t c = (a.g.Z + kMost - 1) / kMost; c <= a.g.Z && c <= 4 * kMost; ++c) {
+        const uint32_t z = (a.g.Z + c - 1) / c;
+        const uint64_t cost = ((uint64_t)g.columns * c + threads - 1) / threads * (z + overhead);
+        if (cost < best) {
+            best = cost;
+            g.zc = z;
+        }
+    }
+    const uint64_t total = (uint64_t)g.columns * ((a.g.Z + g.zc - 1) / g.zc);
+    g.total = (uint32_t)total;   // at most the grid's sites
+    g.blocks = (unsigned)std::min<uint64_t>((total + 255) / 256, threads / 256);
+    return g;
+}
+
 // One wave of resident blocks (the kernel's occupancy x SMs), fewer for small grids.
 // D > 0: the fixed-node kernel (see parabolic_fixed_kernel for D, G, MORE).
 template <typename R, int C, int MODE, int D, int G, bool MORE, bool OBS = false>
 cudaError_t launch_parabolic_m(const StepArgs& a, cudaStream_t s, unsigned* grid = nullptr) {
-    if constexpr (D > 0) {
+    if constexpr (D > 0 && sizeof(R) == 8 && !OBS) {
+        auto kc = parabolic_columns_kernel<R, C, MODE, D, G, MORE>;
+        static int occ_c = 0;
+        if (occ_c == 0) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, kc, 256, 0);
+            if (occ_c < 1) occ_c = 1;
+        }
+        const ColumnGrid g = column_grid(a, (unsigned)occ_c, 1);
+        kc<<<g.blocks, 256, 0, s>>>(a, g.zc, g.columns, g.total, make_fastdiv(g.columns));
+        if (grid) *grid = g.blocks;
+        return cudaGetLastError();
+    } else if constexpr (D > 0) {
         // the largest multiple of V / gcd(V, 256) blocks within one wave: the grid
         // stride is then a multiple of V
         auto kf = [] {

@@ -59,12 +59,22 @@ __device__ __forceinline__ Pair twice(Pair a) {
     a.l = __fadd_rn(a.l, a.l);
     return a;
 }
+// Newton's step from the correctly rounded root: what it leaves out is below 2^-51.
 __device__ __forceinline__ Pair square_root(Pair a) {
     if (!(a.h > 0.f)) return Pair{a.h, 0.f};
-    const float q = rsqrtf(a.h), s = __fmul_rn(a.h, q);
+    const float s = __fsqrt_rn(a.h);
     const float r = __fadd_rn(__fmaf_rn(-s, s, a.h), a.l);   // a - s^2
-    return pair_norm(s, __fmul_rn(__fmul_rn(0.5f, q), r));
+    return pair_norm(s, __fmul_rn(__fmul_rn(0.5f, rsqrtf(a.h)), r));
 }
+// sqrt(6) a: the constant in three parts, since two leave an error of 1e-15 that is the
+// same for every node
+__device__ __forceinline__ Pair times_sqrt6(Pair a) {
+    constexpr double c = 2.449489742783178098;
+    constexpr float c1 = (float)c, c2 = (float)(c - (double)c1), c3 = (float)(c - (double)c1 - (double)c2);
+    const Pair p = two_prod(c1, a.h);
+    return pair_norm(p.h, __fadd_rn(p.l, __fmaf_rn(c3, a.h, __fmaf_rn(c2, a.h, __fmul_rn(c1, a.l)))));
+}
+__device__ __forceinline__ double times_sqrt6(double a) { return 2.449489742783178098 * a; }
 __device__ __forceinline__ double twice(double a) { return 2.0 * a; }
 __device__ __forceinline__ double square_root(double a) { return sqrt(a); }
 
@@ -261,10 +271,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_k
                 const T re2 = A::dot2(p[0].x, p[1].x, p[0].y, p[1].y) + A::dot2(p[3].x, p[4].x, p[3].y, p[4].y);
                 const T im2 = A::cross2(p[0].x, p[1].y, p[0].y, p[1].x) + A::cross2(p[3].x, p[4].y, p[3].y, p[4].x);
                 const T f = twice(t.n[0] - t.n[4]) + (t.n[1] - t.n[3]);
-                T sq6;
-                if constexpr (sizeof(R) == 4) sq6 = pair_norm(2.4494898f, (float)(2.449489742783178098 - (double)2.4494898f));
-                else sq6 = 2.449489742783178098;
-                const T fx = twice(re2) + sq6 * re6, fy = twice(im2) + sq6 * im6;
+                const T fx = twice(re2) + times_sqrt6(re6), fy = twice(im2) + times_sqrt6(im6);
                 const T ff = fx * fx + fy * fy + f * f;
                 A::add(mx, re2);
                 A::add(my, im2);
@@ -426,26 +433,10 @@ cudaError_t launch_observe_columns_d(const StepArgs& a, double* out, cudaStream_
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, 256, 0);
         occ = std::max(occ, 1);
     }
-    // cells of z per column: the split with the least work for the busiest thread, a
-    // column's FP64 part (about 100 operations) counted as 9 nodes
-    const uint64_t columns = (uint64_t)a.row_items * a.g.Y;
-    const uint64_t threads = (uint64_t)occ * (unsigned)device_sm_count() * 256;
-    uint32_t zc = 1;
-    uint64_t best = ~0ull;
-    for (uint32_t c = 1; c <= a.g.Z && c <= 64; ++c) {
-        const uint32_t z = (a.g.Z + c - 1) / c;
-        const uint64_t cost = (columns * c + threads - 1) / threads * (z + 9);
-        if (z <= 64 && cost < best) {
-            best = cost;
-            zc = z;
-        }
-    }
-    if (best == ~0ull) zc = 64;   // more than 4096 planes
-    const uint32_t chunks = (a.g.Z + zc - 1) / zc;
-    const uint64_t total = columns * chunks;
-    const unsigned nb = (unsigned)std::min<uint64_t>((total + 255) / 256, (uint64_t)occ * (unsigned)device_sm_count());
-    k<<<nb, 256, 0, s>>>(a, zc, (uint32_t)columns, (uint32_t)total, make_fastdiv((uint32_t)columns));
-    finalize_observables(a.partials, nb, out, s);
+    // a column's FP64 part, about 100 operations, costs what 9 nodes cost
+    const ColumnGrid g = column_grid(a, (unsigned)occ, 9);
+    k<<<g.blocks, 256, 0, s>>>(a, g.zc, g.columns, g.total, make_fastdiv(g.columns));
+    finalize_observables(a.partials, g.blocks, out, s);
     return cudaGetLastError();
 }
 
