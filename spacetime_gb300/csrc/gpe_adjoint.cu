@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(256, (sizeof(R) == 4 && C <= 3) ? 4 : 1) adjoi
             if constexpr (sizeof(R) == 4) fac = j.factor32;
             else fac = j.factor;
             Cx<R> v[C];
-            ld_node<R, C, false>(o, v);
+            ld_node<R, C>(o, v);
 #pragma unroll
             for (int c = 0; c < C; ++c) {
                 v[c].x += fac * (K[c].x - diag * b[c].x + g[c].x);
@@ -409,8 +409,8 @@ __global__ void __launch_bounds__(256) adjoint_final_kernel(StepArgs a) {
         Cx<double> u[C];
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            const Cx<R> t = ldc<R>(a.prev + off + c * 2 * sizeof(R));
-            const Cx<R> p = ldc<R>(a.next + off + c * 2 * sizeof(R));
+            const Cx<R> t = ldc_nc<R>(a.prev + off + c * 2 * sizeof(R));
+            const Cx<R> p = ldc_nc<R>(a.next + off + c * 2 * sizeof(R));
             u[c] = cx<double>((double)p.x, (double)p.y);
             v[0] += (double)t.x * p.x + (double)t.y * p.y;
             v[1] += (double)t.x * p.y - (double)t.y * p.x;
@@ -438,8 +438,8 @@ __global__ void __launch_bounds__(256) adjoint_seed_kernel(StepArgs a, const cha
     Cx<double> u[C], g[C];
 #pragma unroll
     for (int c = 0; c < C; ++c) {
-        const Cx<R> t = ldc<R>(a.prev + off + c * 2 * sizeof(R));
-        const Cx<R> p = ldc<R>(psi + off + c * 2 * sizeof(R));
+        const Cx<R> t = ldc_nc<R>(a.prev + off + c * 2 * sizeof(R));
+        const Cx<R> p = ldc_nc<R>(psi + off + c * 2 * sizeof(R));
         u[c] = cx<double>((double)p.x, (double)p.y);
         g[c] = cx<double>(s0 * t.x - s1 * t.y, s0 * t.y + s1 * t.x);
     }

@@ -221,10 +221,10 @@ __device__ __forceinline__ void batch_rows_c1x2(const MK& M, const SmemTables<R>
             own[q] = cell_off + l[q] * node_bytes;
             const int4 o4 = *reinterpret_cast<const int4*>(st.nb_off + 4 * l[q]);
             const int32_t off[4] = {o4.x, o4.y, o4.z, o4.w};
-            ld_node<R, 1, true>(prev + own[q], prv[q]);
-            ld_node<R, 1, false>(next + own[q], nv[q]);
+            ld_node<R, 1>(prev + own[q], prv[q]);
+            ld_node<R, 1>(next + own[q], nv[q]);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) ld_node<R, 1, true>(prev + cell_off + off[k], v[q][k]);
+            for (int k = 0; k < 4; ++k) ld_node<R, 1>(prev + cell_off + off[k], v[q][k]);
         }
 #pragma unroll
         for (int q = 0; q < 2; ++q) {

@@ -54,7 +54,7 @@ __global__ void __launch_bounds__(256) node_fields_kernel(StepArgs a, double* ou
     double rho = 0;
 #pragma unroll
     for (int s = 0; s < C; ++s) {
-        const Cx<R> v = ldc<R>(p + s * 2 * sizeof(R));
+        const Cx<R> v = ldc_nc<R>(p + s * 2 * sizeof(R));
         re[s] = (double)v.x;
         im[s] = (double)v.y;
         rho += re[s] * re[s] + im[s] * im[s];

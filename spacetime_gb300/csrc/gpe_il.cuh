@@ -236,7 +236,7 @@ __device__ __forceinline__ void il_task(const PhysR<float>& P, const PhysR<float
 #pragma unroll
     for (int s = 0; s < C; ++s) {
         prv[s] = ldc<float>(pp + s * kComp);
-        if constexpr (!kItp) nv[s] = ldc_rw<float>(np + s * kComp);
+        if constexpr (!kItp) nv[s] = ldc<float>(np + s * kComp);
     }
 #pragma unroll
     for (int s = 0; s < C; ++s) H[s] = cx<float>(0.f, 0.f);
@@ -312,7 +312,6 @@ __device__ __forceinline__ void il_step_body(const StepArgs& a, const ILGrid& G,
     using OA = typename AccOf<MODE, OBS, float>::type;
     __shared__ double obs_sums[OBS ? kObsSums * 256 : 1];
     OA oa = AccOf<MODE, OBS, float>::make(obs_sums);
-    const float inv = MODE == kModeItpNorm && a.scale_in ? a.scale_in->inv : 1.f;
     const uint32_t sub = threadIdx.x & (CELLS - 1);
     const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
@@ -339,6 +338,8 @@ __device__ __forceinline__ void il_step_body(const StepArgs& a, const ILGrid& G,
     }
     const float pos[3] = {a.tab.pos32[3 * l], a.tab.pos32[3 * l + 1], a.tab.pos32[3 * l + 2]};
     const uint32_t own = l * (C * CELLS * 8) + sub * 8;
+    after_previous_kernel<false>();
+    const float inv = MODE == kModeItpNorm && a.scale_in ? a.scale_in->inv : 1.f;
     // the grid's warp count is a multiple of V
     for (ILWalk<CELLS> g(G, u0, fdiv(nwarps, a.divV), 0, dGX, a.divY); g.q < nq; g.next(G)) {
         const uint32_t x = g.gx * CELLS + sub;
@@ -461,7 +462,7 @@ cudaError_t launch_il_step_d(const StepArgs& a, const ILGrid& G, size_t max_bloc
         il_step_obs_kernel<C, D, CELLS><<<nb, kIlObsThreads, 0, s>>>(a, G, dGX);
         finalize_observables(a.partials, nb, out, s);
     } else {
-        il_step_kernel<C, D, CELLS><<<nb, kIlPlainThreads, 0, s>>>(a, G, dGX);
+        return launch_overlapped(il_step_kernel<C, D, CELLS>, nb, kIlPlainThreads, 0, s, a, G, dGX);
     }
     return cudaGetLastError();
 }
@@ -483,8 +484,7 @@ cudaError_t launch_il_itp_d(const StepArgs& a, const ILGrid& G, size_t max_block
     }
     const unsigned nb = il_wave(G, kIlPlainThreads, occ, max_blocks);
     if (nb == 0) return cudaErrorInvalidConfiguration;
-    il_itp_kernel<C, D, CELLS><<<nb, kIlPlainThreads, 0, s>>>(a, G, make_fastdiv(G.GX));
-    return cudaGetLastError();
+    return launch_overlapped(il_itp_kernel<C, D, CELLS>, nb, kIlPlainThreads, 0, s, a, G, make_fastdiv(G.GX));
 }
 
 // One imaginary-time iteration (a.prev / a.next: interleaved buffers).
@@ -566,8 +566,8 @@ __device__ __forceinline__ void il_hyper_body(const StepArgs& a, const ILGrid& G
             Cx<float> prv[C], H[C], nv[C];
 #pragma unroll
             for (int s = 0; s < C; ++s) {
-                prv[s] = ldc<float>(a.prev + own + s * kComp);
-                nv[s] = ldc_rw<float>(a.next + own + s * kComp);   // in flight with the q loads
+                prv[s] = ldc_nc<float>(a.prev + own + s * kComp);
+                nv[s] = ldc<float>(a.next + own + s * kComp);   // in flight with the q loads
             }
 #pragma unroll
             for (int s = 0; s < C; ++s) H[s] = cx<float>(0.f, 0.f);
@@ -577,7 +577,7 @@ __device__ __forceinline__ void il_hyper_body(const StepArgs& a, const ILGrid& G
                 const bool in = !((outside >> k) & 1);
                 const char* p = a.q + qbase + off[k];
 #pragma unroll
-                for (int s = 0; s < C; ++s) qv[k][s] = in ? ldc<float>(p + s * kComp) : cx<float>(0.f, 0.f);
+                for (int s = 0; s < C; ++s) qv[k][s] = in ? ldc_nc<float>(p + s * kComp) : cx<float>(0.f, 0.f);
             }
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
@@ -610,10 +610,10 @@ __device__ __forceinline__ void il_hyper_body(const StepArgs& a, const ILGrid& G
             const char* pt = a.prev + gbase + eto[e];
 #pragma unroll
             for (int s = 0; s < C; ++s) {
-                to[s] = in ? ldc<float>(pt + s * kComp) : cx<float>(0.f, 0.f);
-                fr[s] = ldc<float>(a.prev + gbase + efrom[e] + s * kComp);
-                pq[s] = ldc<float>(a.q + own + s * kComp);
-                v[s] = ldc_rw<float>(a.qnext + own + s * kComp);
+                to[s] = in ? ldc_nc<float>(pt + s * kComp) : cx<float>(0.f, 0.f);
+                fr[s] = ldc_nc<float>(a.prev + gbase + efrom[e] + s * kComp);
+                pq[s] = ldc_nc<float>(a.q + own + s * kComp);
+                v[s] = ldc<float>(a.qnext + own + s * kComp);
             }
 #pragma unroll
             for (int s = 0; s < C; ++s) {

@@ -60,26 +60,19 @@ __device__ __forceinline__ Cx<R> conj(Cx<R> a) { return cx<R>(a.x, -a.y); }
 template <typename R>
 __device__ __forceinline__ void operator+=(Cx<R>& a, Cx<R> b) { a.x += b.x; a.y += b.y; }
 
+// Loads of the state are plain: a kernel of the time loop may start before the one that
+// writes what it reads has ended (after_previous_kernel), which the read-only path does
+// not allow for.
 template <typename R>
 __device__ __forceinline__ Cx<R> ldc(const char* p) {
-    if constexpr (sizeof(R) == 4) {
-        float2 v = __ldg(reinterpret_cast<const float2*>(p));
-        return cx<R>(v.x, v.y);
-    } else {
-        double2 v = __ldg(reinterpret_cast<const double2*>(p));
-        return cx<R>(v.x, v.y);
-    }
+    const auto v = *reinterpret_cast<const typename Vec2<R>::type*>(p);
+    return cx<R>(v.x, v.y);
 }
-// plain (coherent) load for buffers the kernel also writes
+// the read-only path, for kernels that start when everything before them is done
 template <typename R>
-__device__ __forceinline__ Cx<R> ldc_rw(const char* p) {
-    if constexpr (sizeof(R) == 4) {
-        float2 v = *reinterpret_cast<const float2*>(p);
-        return cx<R>(v.x, v.y);
-    } else {
-        double2 v = *reinterpret_cast<const double2*>(p);
-        return cx<R>(v.x, v.y);
-    }
+__device__ __forceinline__ Cx<R> ldc_nc(const char* p) {
+    const auto v = __ldg(reinterpret_cast<const typename Vec2<R>::type*>(p));
+    return cx<R>(v.x, v.y);
 }
 template <typename R>
 __device__ __forceinline__ void stc(char* p, Cx<R> c) {
@@ -95,8 +88,8 @@ __device__ __forceinline__ void stc(char* p, Cx<R> c) {
 // 16-byte loads plus one 8-byte load, in an order set by bit 3 of the address
 // (which half of the record is 16-byte aligned): a warp's load instructions, and
 // with them the L1 wavefronts they cost, drop from C to (C+1)/2 per record.
-// NC: the read-only path (buffers the kernel does not write).
-template <typename R, int C, bool NC>
+// NC: the read-only path (see ldc_nc).
+template <typename R, int C, bool NC = false>
 __device__ __forceinline__ void ld_node(const char* p, Cx<R>* v) {
     if constexpr (sizeof(R) == 4 && C > 1 && (C % 2) == 1) {
         const bool odd = (reinterpret_cast<uintptr_t>(p) & 8) != 0;
@@ -123,7 +116,7 @@ __device__ __forceinline__ void ld_node(const char* p, Cx<R>* v) {
         }
     } else {
 #pragma unroll
-        for (int s = 0; s < C; ++s) v[s] = NC ? ldc<R>(p + s * 2 * sizeof(R)) : ldc_rw<R>(p + s * 2 * sizeof(R));
+        for (int s = 0; s < C; ++s) v[s] = NC ? ldc_nc<R>(p + s * 2 * sizeof(R)) : ldc<R>(p + s * 2 * sizeof(R));
     }
 }
 
@@ -149,6 +142,20 @@ __device__ __forceinline__ void st_node(char* p, const Cx<R>* v) {
 #pragma unroll
         for (int s = 0; s < C; ++s) stc<R>(p + s * 2 * sizeof(R), v[s]);
     }
+}
+
+// To be called before the first access to anything a kernel before this one writes (see
+// launch_overlapped; a no-op in a kernel launched otherwise), once the block's own
+// start is done.  LET_IN: the next kernel's blocks may take slots as this kernel's blocks
+// end, instead of when all have ended, and read their tables while the last ones
+// finish.  Measured per step, let in / not: gather kernel, scalar C15 41 x 37 x 35 39.3 /
+// 40.6 us, split C15 36^3 194 / 199, scalar BCC 32^3 3.97 / 3.85; interleaved kernels
+// (no tables to stage) equal or slower, imaginary time 2 % slower.  (Deciding it by the
+// grid's size inside the kernel cost 10-25 % of the scalar steps.)
+template <bool LET_IN>
+__device__ __forceinline__ void after_previous_kernel() {
+    if constexpr (LET_IN) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 template <typename R>
@@ -432,7 +439,7 @@ __device__ __forceinline__ void write_update(int mode, R dt, char* nxt, char* hp
     for (int s = 0; s < C; ++s) {
         char* p = nxt + s * 2 * sizeof(R);
         if (mode == GPE_MODE_LEAPFROG) {
-            Cx<R> v = ldc_rw<R>(p);
+            Cx<R> v = ldc<R>(p);
             add_scaled(v, (R)2 * dt, cx<R>(H[s].y, -H[s].x));
             stc<R>(p, v);
         } else if (mode == GPE_MODE_EULER) {
@@ -816,11 +823,11 @@ __device__ __forceinline__ void parabolic_node_t(const Grid& g, const NodeTab<R,
     const char* base = prev + cell_off;
     const uint32_t node_bytes = C * 2 * sizeof(R);
     Cx<R> prv[C], H[C], nv[C];
-    ld_node<R, C, true>(base + l * node_bytes, prv);
+    ld_node<R, C>(base + l * node_bytes, prv);
     char* nxt = next + cell_off + l * node_bytes;
     // leapfrog: the old next record is loaded up front, in flight with the gathers
-    if constexpr (MODE == GPE_MODE_LEAPFROG) ld_node<R, C, false>(nxt, nv);
-    if constexpr (MODE == kModeLeapfrogFrom) ld_node<R, C, true>(hpsi + cell_off + l * node_bytes, nv);
+    if constexpr (MODE == GPE_MODE_LEAPFROG) ld_node<R, C>(nxt, nv);
+    if constexpr (MODE == kModeLeapfrogFrom) ld_node<R, C>(hpsi + cell_off + l * node_bytes, nv);
     // DEC Laplacian, sum_f w_f (psi_nb - psi) in entry order (Spin1GpeBCC.cu:835-865)
 #pragma unroll
     for (int s = 0; s < C; ++s) H[s] = cx<R>((R)0, (R)0);
@@ -829,7 +836,7 @@ __device__ __forceinline__ void parabolic_node_t(const Grid& g, const NodeTab<R,
         Cx<R> v[G][C];
 #pragma unroll
         for (int k = 0; k < G; ++k)
-            if (k0 + k < D) ld_node<R, C, true>(base + t.off[k0 + k], v[k]);
+            if (k0 + k < D) ld_node<R, C>(base + t.off[k0 + k], v[k]);
 #pragma unroll
         for (int k = 0; k < G; ++k) {
             if (k0 + k < D) {
@@ -856,7 +863,7 @@ __device__ __forceinline__ void parabolic_node_t(const Grid& g, const NodeTab<R,
             for (int h = 0; h < 4; h += G) {
                 Cx<R> v[G][C];
 #pragma unroll
-                for (int k = 0; k < G; ++k) ld_node<R, C, true>(base + o[h + k], v[k]);
+                for (int k = 0; k < G; ++k) ld_node<R, C>(base + o[h + k], v[k]);
 #pragma unroll
                 for (int k = 0; k < G; ++k) {
     #pragma unroll
@@ -896,12 +903,12 @@ __device__ __forceinline__ void parabolic_node(const Grid& g, const SmemTables<R
         const char* base = prev + cell_off;
         const uint32_t node_bytes = C * 2 * sizeof(R);
         Cx<R> prv[C], H[C], nv[C];
-        ld_node<R, C, true>(base + l * node_bytes, prv);
+        ld_node<R, C>(base + l * node_bytes, prv);
 #pragma unroll
         for (int s = 0; s < C; ++s) H[s] = cx<R>((R)0, (R)0);
         char* nxt = next + cell_off + l * node_bytes;
-        if constexpr (MODE == GPE_MODE_LEAPFROG) ld_node<R, C, false>(nxt, nv);
-        if constexpr (MODE == kModeLeapfrogFrom) ld_node<R, C, true>(hpsi + cell_off + l * node_bytes, nv);
+        if constexpr (MODE == GPE_MODE_LEAPFROG) ld_node<R, C>(nxt, nv);
+        if constexpr (MODE == kModeLeapfrogFrom) ld_node<R, C>(hpsi + cell_off + l * node_bytes, nv);
         const int f0 = st.row_ptr[l], f1 = st.row_ptr[l + 1];
         if constexpr (C == 1) {
             // scalars: groups of 4 entries, the loads of a group issued together (rows
@@ -911,7 +918,7 @@ __device__ __forceinline__ void parabolic_node(const Grid& g, const SmemTables<R
                 Cx<R> v[4][C];
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    if (f + k < f1) ld_node<R, C, true>(base + st.nb_off[f + k], v[k]);
+                    if (f + k < f1) ld_node<R, C>(base + st.nb_off[f + k], v[k]);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     if (f + k < f1) {
@@ -924,7 +931,7 @@ __device__ __forceinline__ void parabolic_node(const Grid& g, const SmemTables<R
         } else {
             for (int f = f0; f < f1; ++f) {
                 Cx<R> v[C];
-                ld_node<R, C, true>(base + st.nb_off[f], v);
+                ld_node<R, C>(base + st.nb_off[f], v);
                 const R w = st.w[f];
 #pragma unroll
                 for (int s = 0; s < C; ++s) add_scaled(H[s], w, v[s] - prv[s]);
@@ -947,6 +954,7 @@ __device__ __forceinline__ void parabolic_step_body(const StepArgs& a) {
     __shared__ SmemTables<R> st;
     load_tables<R>(st, a);
     __syncthreads();
+    after_previous_kernel<true>();
     const PhysR<R>& P = make_phys<R>(a);
     using OA = typename AccOf<MODE, OBS, R>::type;
     __shared__ double obs_sums[OBS ? kObsSums * 256 : 1];
@@ -992,6 +1000,7 @@ __device__ __forceinline__ void parabolic_fixed_body(const StepArgs& a) {
     __shared__ SmemTables<R> st;
     load_tables<R>(st, a);
     __syncthreads();
+    after_previous_kernel<true>();
     const PhysR<R>& P = make_phys<R>(a);
     constexpr bool kAll = OBS || MODE == kModeItpNorm;   // every thread takes part in the block's sums
     using OA = typename AccOf<MODE, OBS, R>::type;
@@ -1034,6 +1043,7 @@ __global__ void __launch_bounds__(256) parabolic_columns_kernel(StepArgs a, uint
     __shared__ SmemTables<R> st;
     load_tables<R>(st, a);
     __syncthreads();
+    after_previous_kernel<true>();
     const PhysR<R>& P = make_phys<R>(a);
     using OA = typename AccOf<MODE, false, R>::type;
     OA oa = AccOf<MODE, false, R>::make(nullptr);
@@ -1066,6 +1076,25 @@ __global__ void __launch_bounds__(256) parabolic_fixed_kernel(StepArgs a) {
 template <typename R, int C, int MODE, int D, int G, bool MORE>
 __global__ void __launch_bounds__(256, 3) parabolic_fixed_obs_kernel(StepArgs a) {
     parabolic_fixed_body<R, C, MODE, D, G, MORE, true>(a);
+}
+
+// Launch of a kernel of the time loop that may start while the kernel before it in the
+// stream is still finishing (programmatic dependent launch): its blocks take the slots
+// that become free, read their tables and then wait in after_previous_kernel() until
+// everything the kernels before have written is there.
+template <class... P, class... T>
+cudaError_t launch_overlapped(void (*kernel)(P...), unsigned blocks, unsigned threads, size_t smem, cudaStream_t s, T&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 // SM count of the current device (cached per device).
@@ -1128,10 +1157,10 @@ __device__ __forceinline__ void q_update(const StepArgs& a, const SmemHyper<R>& 
     const R dts = make_phys<R>(a).dts;
     // whole records: (C+1)/2 loads each in FP32
     Cx<R> to[C], from[C], pq[C], v[C];
-    ld_node<R, C, true>(otherp, to);
-    ld_node<R, C, true>(thisp, from);
-    if constexpr (QM != 1) ld_node<R, C, false>(qprev, pq);
-    if constexpr (QM == 0) ld_node<R, C, false>(qnext, v);
+    ld_node<R, C>(otherp, to);
+    ld_node<R, C>(thisp, from);
+    if constexpr (QM != 1) ld_node<R, C>(qprev, pq);
+    if constexpr (QM == 0) ld_node<R, C>(qnext, v);
 #pragma unroll
     for (int s = 0; s < C; ++s) {
         const Cx<R> d0psi = to[s] - from[s];
@@ -1178,6 +1207,7 @@ __global__ void __launch_bounds__(256) hyper_step_kernel(StepArgs a, uint32_t no
     }
     __syncthreads();
 
+    after_previous_kernel<true>();
     for (uint32_t vb = blockIdx.x; vb < vblocks; vb += gridDim.x) {
     uint32_t group, sub;
     if (DO_PSI && QM >= 0) {
@@ -1205,7 +1235,7 @@ __global__ void __launch_bounds__(256) hyper_step_kernel(StepArgs a, uint32_t no
         const size_t qcell_off = (size_t)z * a.g.qslice + (size_t)y * a.g.qpitch + (size_t)x * a.g.qcell_bytes;
         const char* own = a.prev + cell_off + l * node_bytes;
         Cx<R> prv[C], H[C];
-        ld_node<R, C, true>(own, prv);
+        ld_node<R, C>(own, prv);
 #pragma unroll
         for (int s = 0; s < C; ++s) H[s] = cx<R>((R)0, (R)0);
         // d1 of q (RelativisticSpin2Gpe.cu:1051-1066), whole edge records
@@ -1217,14 +1247,14 @@ __global__ void __launch_bounds__(256) hyper_step_kernel(StepArgs a, uint32_t no
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 Cx<R> qv[C];
-                ld_node<R, C, true>(qb + off[k], qv);
+                ld_node<R, C>(qb + off[k], qv);
 #pragma unroll
                 for (int s = 0; s < C; ++s) add_scaled(H[s], w[k], qv[s]);
             }
         } else {
             for (int k = 0; k < F; ++k) {
                 Cx<R> qv[C];
-                ld_node<R, C, true>(qb + sh.inc_off[l * F + k], qv);
+                ld_node<R, C>(qb + sh.inc_off[l * F + k], qv);
                 const R w = sh.inc_w[l * F + k];
 #pragma unroll
                 for (int s = 0; s < C; ++s) add_scaled(H[s], w, qv[s]);
@@ -1511,7 +1541,7 @@ __global__ void __launch_bounds__(256) scale_kernel(StepArgs a) {
         char* p = a.next + (size_t)z * a.g.slice + (size_t)y * a.g.pitch + (size_t)x * a.g.cell_bytes +
                   l * (C * 2 * sizeof(R));
         Cx<R> v[C];
-        ld_node<R, C, false>(p, v);
+        ld_node<R, C>(p, v);
         if constexpr (sizeof(R) == 8) {
 #pragma unroll
             for (int s = 0; s < C; ++s) v[s] = cx<R>(v[s].x / sq, v[s].y / sq);
@@ -1566,7 +1596,8 @@ cudaError_t launch_parabolic_m(const StepArgs& a, cudaStream_t s, unsigned* grid
             if (occ_c < 1) occ_c = 1;
         }
         const ColumnGrid g = column_grid(a, (unsigned)occ_c, 1);
-        kc<<<g.blocks, 256, 0, s>>>(a, g.zc, g.columns, g.total, make_fastdiv(g.columns));
+        const cudaError_t e = launch_overlapped(kc, g.blocks, 256, 0, s, a, g.zc, g.columns, g.total, make_fastdiv(g.columns));
+        if (e != cudaSuccess) return e;
         if (grid) *grid = g.blocks;
         return cudaGetLastError();
     } else if constexpr (D > 0) {
@@ -1594,9 +1625,8 @@ cudaError_t launch_parabolic_m(const StepArgs& a, cudaStream_t s, unsigned* grid
         const uint64_t wave = std::min<uint64_t>((uint64_t)occ_f * (unsigned)device_sm_count(), (a.total + 255) / 256);
         const unsigned nb = (unsigned)(wave / m * m);
         if (nb > 0) {
-            kf<<<nb, 256, 0, s>>>(a);
             if (grid) *grid = nb;
-            return cudaGetLastError();
+            return launch_overlapped(kf, nb, 256, 0, s, a);
         }
     }
     // grids smaller than V / gcd(V, 256) blocks: the grid-stride kernel (the
@@ -1614,9 +1644,8 @@ cudaError_t launch_parabolic_m(const StepArgs& a, cudaStream_t s, unsigned* grid
         if (occ < 1) occ = 1;
     }
     const unsigned nb = std::min<unsigned>(nblocks(a.total, 256), (unsigned)occ * (unsigned)device_sm_count());
-    if (nb) ks<<<nb, 256, 0, s>>>(a);
     if (grid) *grid = nb;
-    return cudaGetLastError();
+    return nb ? launch_overlapped(ks, nb, 256, 0, s, a) : cudaSuccess;
 }
 
 template <typename R, int C, int D, int G = D, bool MORE = false>
@@ -1688,8 +1717,8 @@ cudaError_t launch_hyper_k(const StepArgs& a, uint32_t nn, uint32_t ne, uint32_t
         if (occ < 1) occ = 1;
     }
     const unsigned nb = std::min(vb, (unsigned)occ * (unsigned)device_sm_count());
-    if (nb) hyper_step_kernel<R, C, DO_PSI, MODE, HYPERB, QM><<<nb, 256, 0, s>>>(a, nn, ne, ratio, vb);
-    return cudaGetLastError();
+    if (nb == 0) return cudaSuccess;
+    return launch_overlapped(hyper_step_kernel<R, C, DO_PSI, MODE, HYPERB, QM>, nb, 256, 0, s, a, nn, ne, ratio, vb);
 }
 
 template <typename R, int C>
@@ -1750,6 +1779,7 @@ __global__ void __launch_bounds__(256) split_step_kernel(StepArgs a, uint32_t no
         else sh.pos[i] = a.tab.pos64[i];
     }
     __syncthreads();
+    after_previous_kernel<true>();
     constexpr bool kNodes = PART != 2;
     const PhysR<R>& P = make_phys<R>(a);
     // the half read by the psi update and by d0 (R for PARTs 0 and 2, I for PART 1)
@@ -1776,7 +1806,7 @@ __global__ void __launch_bounds__(256) split_step_kernel(StepArgs a, uint32_t no
         const size_t cell_off = (size_t)z * a.g.slice + (size_t)y * a.g.pitch + (size_t)x * a.g.cell_bytes;
         const size_t qcell_off = (size_t)z * a.g.qslice + (size_t)y * a.g.qpitch + (size_t)x * a.g.qcell_bytes;
         char* own = a.next + cell_off + l * 2 * sizeof(R);
-        const Cx<R> v = ldc_rw<R>(own);
+        const Cx<R> v = ldc<R>(own);
         const char* qb = a.qnext + qcell_off + rd;
         R d1q = (R)0;
         if (F == 4) {
@@ -1837,11 +1867,10 @@ cudaError_t launch_split(const StepArgs& a, int part, double qinit, cudaStream_t
     const unsigned vb = part == 2 ? nbe : groups * (1 + ratio);
     const unsigned nb = std::min(vb, wave);
     switch (part) {
-        case 0: split_step_kernel<R, 0><<<nb, 256, 0, s>>>(a, nn, ne, ratio, (R)0, vb); break;
-        case 1: split_step_kernel<R, 1><<<nb, 256, 0, s>>>(a, nn, ne, ratio, (R)0, vb); break;
-        default: split_step_kernel<R, 2><<<nb, 256, 0, s>>>(a, nn, ne, ratio, (R)qinit, vb); break;
+        case 0: return launch_overlapped(split_step_kernel<R, 0>, nb, 256, 0, s, a, nn, ne, ratio, (R)0, vb);
+        case 1: return launch_overlapped(split_step_kernel<R, 1>, nb, 256, 0, s, a, nn, ne, ratio, (R)0, vb);
+        default: return launch_overlapped(split_step_kernel<R, 2>, nb, 256, 0, s, a, nn, ne, ratio, (R)qinit, vb);
     }
-    return cudaGetLastError();
 }
 
 // node_fp32: per-node terms in FP32 (FP32 storage only); sums are FP64 either way.
@@ -2142,7 +2171,7 @@ __global__ void __launch_bounds__(256) leapfrog_tile_kernel(StepArgs a, uint32_t
                 // off-row neighbour: read-only global path (L2)
                 const char* g = g_cell + s_goff[f];
 #pragma unroll
-                for (int c = 0; c < C; ++c) H[c] += w * (ldc<R>(g + c * 2 * sizeof(R)) - prv[c]);
+                for (int c = 0; c < C; ++c) H[c] += w * (ldc_nc<R>(g + c * 2 * sizeof(R)) - prv[c]);
             }
         }
         const PhysR<R>& P = make_phys<R>(a);
@@ -2760,7 +2789,7 @@ __global__ void __launch_bounds__(256) respin_kernel(StepArgs a, RespinArgs r) {
         const uint32_t y = row - z * a.g.Y;
         char* p = a.next + (size_t)z * a.g.slice + (size_t)y * a.g.pitch + (size_t)x * a.g.cell_bytes + l * node_bytes;
         Cx<R> v[C];
-        ld_node<R, C, false>(p, v);
+        ld_node<R, C>(p, v);
         R rho = 0;
 #pragma unroll
         for (int m = 0; m < C; ++m) rho += v[m].x * v[m].x + v[m].y * v[m].y;
@@ -2892,7 +2921,7 @@ __global__ void __launch_bounds__(kHyperTileThreads, sizeof(R) == 4 ? 5 : 2)
                 } else {
                     const char* g = so != INT32_MIN ? g_q + tgt : g_q + qrow + s_inc_goff[l * F + k];
 #pragma unroll
-                    for (int c = 0; c < C; ++c) H[c] += w * ldc<R>(g + c * 2 * sizeof(R));
+                    for (int c = 0; c < C; ++c) H[c] += w * ldc_nc<R>(g + c * 2 * sizeof(R));
                 }
             }
             R r[3];
@@ -2939,7 +2968,7 @@ __global__ void __launch_bounds__(kHyperTileThreads, sizeof(R) == 4 ? 5 : 2)
                     const V2 w2 = reinterpret_cast<const V2*>(otherp)[c];
                     ov = cx<R>(w2.x, w2.y);
                 } else {
-                    ov = ldc<R>(otherp + c * 2 * sizeof(R));
+                    ov = ldc_nc<R>(otherp + c * 2 * sizeof(R));
                 }
                 const Cx<R> d0psi = ov - cx<R>(tv.x, tv.y);
                 const V2 pq = reinterpret_cast<const V2*>(qprev)[c];

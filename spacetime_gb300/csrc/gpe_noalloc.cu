@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(256) observe_noalloc_kernel(StepArgs a, NoAllo
         double rho = 0, maxabs = 0, bad = 0;
 #pragma unroll
         for (int s = 0; s < C; ++s) {
-            const Cx<R> v = ldc<R>(base + l * node_bytes + s * 2 * sizeof(R));
+            const Cx<R> v = ldc_nc<R>(base + l * node_bytes + s * 2 * sizeof(R));
             ps[s] = cx<double>((double)v.x, (double)v.y);
             L[s] = Hl[s] = Hn[s] = cx<double>(0.0, 0.0);
             const double n2 = ps[s].x * ps[s].x + ps[s].y * ps[s].y;
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(256) observe_noalloc_kernel(StepArgs a, NoAllo
             const char* nb = base + tab.nb_off[f];
 #pragma unroll
             for (int s = 0; s < C; ++s) {
-                const Cx<R> v = ldc<R>(nb + s * 2 * sizeof(R));
+                const Cx<R> v = ldc_nc<R>(nb + s * 2 * sizeof(R));
                 L[s] += tab.w[f] * (cx<double>((double)v.x, (double)v.y) - ps[s]);
             }
         }

@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kSlabMaxThreads, 2) parabolic_slab_kernel(Step
     };
     for (uint32_t z = 0; z < Z; ++z) {
         Cx<R> nv[C];
-        if (!ring_n && active) ld_node<R, C, false>(nxt, nv);
+        if (!ring_n && active) ld_node<R, C>(nxt, nv);
         // loads z, z+1, z+2 and tile load z must have landed
         while (ok && waited < z + 3) {
             ok = wait_on(&full[wp.slot], wp.par);
