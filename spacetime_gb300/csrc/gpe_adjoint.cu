@@ -30,6 +30,7 @@
 
 #include "gpe_handle.h"
 #include "gpe_kernels.cuh"
+#include "gpe_observe.cuh"
 
 namespace gpe {
 
@@ -88,28 +89,6 @@ __device__ __forceinline__ PhysR<Dual<R>> dual_phys(const PhysR<R>& P) {
     return Q;
 }
 
-// Local spin density <F> (unnormalised), the quantity gpe_observe integrates.
-template <typename R, int C>
-__device__ __forceinline__ void local_mag(const Cx<R>* ps, R M[3]) {
-    if constexpr (C == 3) {
-        const Cx<R> m = (R)GPE_REF_SQRT_2 * (conj(ps[0]) * ps[1] + conj(ps[1]) * ps[2]);
-        M[0] = m.x;
-        M[1] = m.y;
-        M[2] = (ps[0].x * ps[0].x + ps[0].y * ps[0].y) - (ps[2].x * ps[2].x + ps[2].y * ps[2].y);
-    } else if constexpr (C == 5) {
-        const Cx<R> fp = (R)2 * (conj(ps[0]) * ps[1] + conj(ps[3]) * ps[4]) +
-                         (R)2.449489742783178098 * (conj(ps[1]) * ps[2] + conj(ps[2]) * ps[3]);
-        R n[5];
-#pragma unroll
-        for (int s = 0; s < 5; ++s) n[s] = ps[s].x * ps[s].x + ps[s].y * ps[s].y;
-        M[0] = fp.x;
-        M[1] = fp.y;
-        M[2] = (R)2 * n[0] + n[1] - n[3] - (R)2 * n[4];
-    } else {
-        M[0] = M[1] = M[2] = (R)0;
-    }
-}
-
 // Re(b^H (e_k . F) u) for k = x, y, z: the spin-1 Zeeman term of local_spin1
 // (Spin1GpeBCC.cu:884-896: H0 += Bz u0 + conj(Bxy) u1, H1 += Bxy u0 + conj(Bxy) u2,
 // H2 += Bxy u1 - Bz u2 with Bxy = (Bx + i By)/sqrt2) for a unit field along each
@@ -138,26 +117,41 @@ __device__ __forceinline__ void zeeman_proj_spin1(const Cx<R>* b, const Cx<R>* u
 template <typename R>
 __device__ __forceinline__ void jvp_spin1(const PhysR<R>& P, const R r[3], R pot, const Cx<R>* u, const Cx<R>* b,
                                           Cx<R>* g) {
-    const R n1 = u[0].x * u[0].x + u[0].y * u[0].y;
-    const R n_1 = u[2].x * u[2].x + u[2].y * u[2].y;
-    const R n = n1 + (u[1].x * u[1].x + u[1].y * u[1].y) + n_1;
-    const R d1 = (R)2 * (u[0].x * b[0].x + u[0].y * b[0].y);
-    const R d_1 = (R)2 * (u[2].x * b[2].x + u[2].y * b[2].y);
-    const R dn = d1 + (R)2 * (u[1].x * b[1].x + u[1].y * b[1].y) + d_1;
-    const R T = pot + P.c0 * n, dT = P.c0 * dn;
-    const Cx<R> m = (R)GPE_REF_SQRT_2 * (conj(u[0]) * u[1] + conj(u[1]) * u[2]);
-    const Cx<R> dm = (R)GPE_REF_SQRT_2 * (conj(b[0]) * u[1] + conj(u[0]) * b[1] + conj(b[1]) * u[2] + conj(u[1]) * b[2]);
+    const R n1 = norm_sq(u[0]), n_1 = norm_sq(u[2]);
+    const R n = n1 + norm_sq(u[1]) + n_1;
+    // half the derivatives of n_m
+    const R d1 = fm(u[0].y, b[0].y, u[0].x * b[0].x);
+    const R d_1 = fm(u[2].y, b[2].y, u[2].x * b[2].x);
+    const R dn = d1 + fm(u[1].y, b[1].y, fm(u[1].x, b[1].x, d_1));
+    const R T = fm(P.c0, n, pot), dT = (R)2 * P.c0 * dn;
+    const Cx<R> zero = cx<R>((R)0, (R)0);
+    Cx<R> m = zero, dm = zero;   // conj(u1) u0 + conj(u0) u-1 and its derivative
+    add_conj_mul(m, u[0], u[1]);
+    add_conj_mul(m, u[1], u[2]);
+    add_conj_mul(dm, b[0], u[1]);
+    add_conj_mul(dm, u[0], b[1]);
+    add_conj_mul(dm, b[1], u[2]);
+    add_conj_mul(dm, u[1], b[2]);
     R B[3];
     mag_field(P, r, P.bq, P.bb, B);
-    B[0] += P.c2 * m.x;
-    B[1] += P.c2 * m.y;
-    B[2] += P.c2 * (n1 - n_1);
-    const R dBz = P.c2 * (d1 - d_1);
-    const Cx<R> Bxy = (R)GPE_REF_INV_SQRT_2 * cx<R>(B[0], B[1]);
-    const Cx<R> dBxy = ((R)GPE_REF_INV_SQRT_2 * P.c2) * dm;
-    g[0] = (dT + dBz) * u[0] + (T + B[2]) * b[0] + conj(dBxy) * u[1] + conj(Bxy) * b[1];
-    g[1] = dT * u[1] + T * b[1] + dBxy * u[0] + Bxy * b[0] + conj(dBxy) * u[2] + conj(Bxy) * b[2];
-    g[2] = (dT - dBz) * u[2] + (T - B[2]) * b[2] + dBxy * u[1] + Bxy * b[1];
+    const R Bz = fm(P.c2, n1 - n_1, B[2]), dBz = (R)2 * P.c2 * (d1 - d_1);
+    // the matrix elements off the diagonal, as in local_spin1
+    const Cx<R> q = cx<R>(fm((R)GPE_REF_INV_SQRT_2, B[0], P.c2 * m.x), fm((R)GPE_REF_INV_SQRT_2, B[1], P.c2 * m.y));
+    const Cx<R> dq = P.c2 * dm;
+    g[0] = (dT + dBz) * u[0];
+    add_scaled(g[0], T + Bz, b[0]);
+    add_conj_mul(g[0], dq, u[1]);
+    add_conj_mul(g[0], q, b[1]);
+    g[1] = dT * u[1];
+    add_scaled(g[1], T, b[1]);
+    add_mul(g[1], dq, u[0]);
+    add_mul(g[1], q, b[0]);
+    add_conj_mul(g[1], dq, u[2]);
+    add_conj_mul(g[1], q, b[2]);
+    g[2] = (dT - dBz) * u[2];
+    add_scaled(g[2], T - Bz, b[2]);
+    add_mul(g[2], dq, u[1]);
+    add_mul(g[2], q, b[1]);
     if (P.flags & GPE_FLAG_QUADRATIC_ZEEMAN) {
         // linear in u: the same matrix applied to b
         R Q[3];
@@ -169,6 +163,83 @@ __device__ __forceinline__ void jvp_spin1(const PhysR<R>& P, const R r[3], R pot
         g[0] += (bz2 + nsq) * b[0] + (Q[2] * qc) * b[1] + (qc * qc) * b[2];
         g[1] += (Q[2] * qxy) * b[0] + ((R)2 * nsq) * b[1] - (Q[2] * qc) * b[2];
         g[2] += (qxy * qxy) * b[0] - (Q[2] * qxy) * b[1] + (bz2 + nsq) * b[2];
+    }
+}
+
+// The transposed Jacobian of three-body loss: h_loss = -i alpha n^2 u, J^T b = i alpha
+// n^2 b + 4 alpha n Im(b^H u) u, added to g.
+template <typename R, int C>
+__device__ __forceinline__ void add_loss_transpose(const PhysR<R>& P, const Cx<R>* u, const Cx<R>* b, Cx<R>* g) {
+    R n = 0, im = 0;
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        n += u[c].x * u[c].x + u[c].y * u[c].y;
+        im += b[c].x * u[c].y - b[c].y * u[c].x;
+    }
+    const R an2 = P.alpha * n * n, k4 = (R)4 * P.alpha * n * im;
+#pragma unroll
+    for (int c = 0; c < C; ++c) g[c] += cx<R>(-an2 * b[c].y + k4 * u[c].x, an2 * b[c].x + k4 * u[c].y);
+}
+
+// (dh/du)^T b.  Apart from three-body loss, h = dE/d(conj u) for a real energy E (trap,
+// c0 n^2/2, Zeeman B.<F>, c2 <F>^2/2, quadratic Zeeman, spin-2 singlet |A00|^2), so its
+// real Jacobian is half the Hessian of E, symmetric: J^T b = J b, one dual evaluation
+// along b.
+template <typename R, int C>
+__device__ __forceinline__ void local_jvp(const PhysR<R>& P, const R r[3], R pot, const Cx<R>* u, const Cx<R>* b, Cx<R>* g) {
+    if constexpr (C == 3) {
+        jvp_spin1<R>(P, r, pot, u, b, g);
+    } else {
+        PhysR<Dual<R>> PD = dual_phys<R>(P);
+        PD.flags &= ~GPE_FLAG_THREE_BODY_LOSS;
+        const Dual<R> rD[3] = {cd<R>(r[0]), cd<R>(r[1]), cd<R>(r[2])};
+        Cx<Dual<R>> psD[C], H[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            psD[c] = cx<Dual<R>>(Dual<R>(u[c].x, b[c].x), Dual<R>(u[c].y, b[c].y));
+            H[c] = cx<Dual<R>>(cd<R>((R)0), cd<R>((R)0));
+        }
+        local_terms<Dual<R>, C>(PD, rD, cd<R>(pot), GPE_MODE_LEAPFROG, false, psD, H);
+#pragma unroll
+        for (int c = 0; c < C; ++c) g[c] = cx<R>(H[c].x.d, H[c].y.d);
+    }
+}
+
+// The field parameters' gradients added to gsum (Bq, Bb).  h depends on Bb only through
+// the Zeeman term (B.F) u, so dh/dBb_k = F_k u: the local terms with every coefficient
+// zero except Bb = e_k.  dB/dBq is mag_field's B at Bq = 1, Bb = 0.
+template <typename R, int C>
+__device__ __forceinline__ void add_field_gradient(const PhysR<R>& P, const R r[3], const Cx<R>* b, const Cx<R>* u, R* gsum) {
+    if constexpr (C > 1) {
+        R s3[3];
+        if constexpr (C == 3) {
+            zeeman_proj_spin1<R>(b, u, s3);
+        } else {
+            PhysR<R> Z = P;
+            Z.c0 = Z.c2 = Z.c4 = Z.alpha = Z.bq = Z.bqq = (R)0;
+            Z.flags = 0;
+            Z.trap_on = 0;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+#pragma unroll
+                for (int i = 0; i < 3; ++i) Z.bb[i] = (R)(i == k);
+                Cx<R> H[C];
+#pragma unroll
+                for (int c = 0; c < C; ++c) H[c] = cx<R>((R)0, (R)0);
+                local_terms<R, C>(Z, r, (R)0, GPE_MODE_LEAPFROG, false, u, H);
+                R d = 0;
+#pragma unroll
+                for (int c = 0; c < C; ++c) d += b[c].x * H[c].x + b[c].y * H[c].y;
+                s3[k] = d;
+            }
+        }
+        const R zero3[3] = {(R)0, (R)0, (R)0};
+        R w[3];
+        mag_field<R>(P, r, (R)1, zero3, w);
+        gsum[0] += w[0] * s3[0] + w[1] * s3[1] + w[2] * s3[2];
+        gsum[1] += s3[0];
+        gsum[2] += s3[1];
+        gsum[3] += s3[2];
     }
 }
 
@@ -278,39 +349,9 @@ __global__ void __launch_bounds__(256, (sizeof(R) == 4 && C <= 3) ? 4 : 1) adjoi
                     for (int c = 0; c < C; ++c) K[c] += wt * cx<R>(-av[c].y, av[c].x);
                 }
             }
-            // (dh/du)^T b.  Apart from three-body loss, h = dE/d(conj u) for a real
-            // energy E (trap, c0 n^2/2, Zeeman B.<F>, c2 <F>^2/2, quadratic Zeeman,
-            // spin-2 singlet |A00|^2), so its real Jacobian is half the Hessian of E,
-            // symmetric: J^T b = J b, one dual evaluation along b.
             Cx<R> g[C];
-            if constexpr (C == 3) {
-                jvp_spin1<R>(P, r, pot, u, b, g);
-            } else {
-                PhysR<Dual<R>> PD = dual_phys<R>(P);
-                PD.flags &= ~GPE_FLAG_THREE_BODY_LOSS;
-                const Dual<R> rD[3] = {cd<R>(r[0]), cd<R>(r[1]), cd<R>(r[2])};
-                Cx<Dual<R>> psD[C], H[C];
-#pragma unroll
-                for (int c = 0; c < C; ++c) {
-                    psD[c] = cx<Dual<R>>(Dual<R>(u[c].x, b[c].x), Dual<R>(u[c].y, b[c].y));
-                    H[c] = cx<Dual<R>>(cd<R>((R)0), cd<R>((R)0));
-                }
-                local_terms<Dual<R>, C>(PD, rD, cd<R>(pot), GPE_MODE_LEAPFROG, false, psD, H);
-#pragma unroll
-                for (int c = 0; c < C; ++c) g[c] = cx<R>(H[c].x.d, H[c].y.d);
-            }
-            if (P.flags & GPE_FLAG_THREE_BODY_LOSS) {
-                // h_loss = -i alpha n^2 u: J^T b = i alpha n^2 b + 4 alpha n Im(b^H u) u
-                R n = 0, im = 0;
-#pragma unroll
-                for (int c = 0; c < C; ++c) {
-                    n += u[c].x * u[c].x + u[c].y * u[c].y;
-                    im += b[c].x * u[c].y - b[c].y * u[c].x;
-                }
-                const R an2 = P.alpha * n * n, k4 = (R)4 * P.alpha * n * im;
-#pragma unroll
-                for (int c = 0; c < C; ++c) g[c] += cx<R>(-an2 * b[c].y + k4 * u[c].x, an2 * b[c].x + k4 * u[c].y);
-            }
+            local_jvp<R, C>(P, r, pot, u, b, g);
+            if (P.flags & GPE_FLAG_THREE_BODY_LOSS) add_loss_transpose<R, C>(P, u, b, g);
             char* o = j.a_next + cell_off + l * node_bytes;
             R fac;
             if constexpr (sizeof(R) == 4) fac = j.factor32;
@@ -324,42 +365,100 @@ __global__ void __launch_bounds__(256, (sizeof(R) == 4 && C <= 3) ? 4 : 1) adjoi
             }
             st_node<R, C>(o, v);
         }
-        // field parameters.  h depends on Bb only through the Zeeman term (B.F) u,
-        // so dh/dBb_k = F_k u: the local terms with every coefficient zero except
-        // Bb = e_k.  dB/dBq is mag_field's B at Bq = 1, Bb = 0.
-        if constexpr (C > 1) {
-            R s3[3];
-            if constexpr (C == 3) {
-                zeeman_proj_spin1<R>(b, u, s3);
-            } else {
-            PhysR<R> Z = P;
-            Z.c0 = Z.c2 = Z.c4 = Z.alpha = Z.bq = Z.bqq = (R)0;
-            Z.flags = 0;
-            Z.trap_on = 0;
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-#pragma unroll
-                for (int i = 0; i < 3; ++i) Z.bb[i] = (R)(i == k);
-                Cx<R> H[C];
-#pragma unroll
-                for (int c = 0; c < C; ++c) H[c] = cx<R>((R)0, (R)0);
-                local_terms<R, C>(Z, r, (R)0, GPE_MODE_LEAPFROG, false, u, H);
-                R d = 0;
-#pragma unroll
-                for (int c = 0; c < C; ++c) d += b[c].x * H[c].x + b[c].y * H[c].y;
-                s3[k] = d;
-            }
-            }
-            const R zero3[3] = {(R)0, (R)0, (R)0};
-            R w[3];
-            mag_field<R>(P, r, (R)1, zero3, w);
-            gsum[0] += w[0] * s3[0] + w[1] * s3[1] + w[2] * s3[2];
-            gsum[1] += s3[0];
-            gsum[2] += s3[1];
-            gsum[3] += s3[2];
-        }
+        add_field_gradient<R, C>(P, r, b, u, gsum);
     }
     block_partials<kGradCount, R>(gsum, j.factor, a.partials);
+}
+
+// The reverse step of FP32 states in the interleaved layout (gpe_il.cuh): a warp keeps
+// one node of the lattice for the launch, its offsets, weights and transposed weights
+// in registers, and every load and store is one run of full lines.  The handle-layout
+// form above spends its time on L1 (67 %), index arithmetic and table reads.  Spin-1 BCC
+// 40^3, 200 steps forward and back: 10.7 ms with every state in the handle's layout, 7.75
+// with all of them in this one (a reverse step 20.4 -> 16 us, a forward or recomputed
+// step 15.0 -> 11.9).  Registers: 6 blocks per SM (80) 7.75 ms, 5 (96) 7.85, 7 (72) 7.85.
+constexpr unsigned kIlAdjThreads = 128;
+template <int C, int D, int CELLS>
+__global__ void __launch_bounds__(kIlAdjThreads, C == 5 ? 3 : D == 8 ? 4 : 6) il_adjoint_kernel(StepArgs a, AdjArgs j, ILGrid G,
+                                                                                         FastDiv dGX) {
+    constexpr uint32_t kComp = CELLS * 8;
+    const PhysR<float>& P = a.pf;
+    const uint32_t sub = threadIdx.x & (CELLS - 1);
+    const uint32_t warp = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
+    const uint32_t u0 = fdiv(warp, a.divV), l = warp - u0 * G.V;
+    const uint32_t nq = G.Y * G.Z * G.GX;
+    const int f0 = a.tab.row_ptr[l];
+    const int nd = D == 4 ? 4 : a.tab.row_ptr[l + 1] - f0;
+    int32_t off[D];
+    float wT[D], diag = 0.f;
+    ILEdge edge;
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+        off[k] = 0;
+        wT[k] = 0.f;
+        if (k < nd) {
+            const int4 e = a.tab.ent4[f0 + k];
+            off[k] = il_lane_off<CELLS>(G, e.x, e.y, e.z, (uint32_t)e.w, sub);
+            wT[k] = j.wT32[f0 + k];
+            diag += a.tab.w32[f0 + k];
+            edge.add(k, e.x, sub == 0, sub == (G.X - 1) % CELLS);
+        }
+    }
+    const float pos[3] = {a.tab.pos32[3 * l], a.tab.pos32[3 * l + 1], a.tab.pos32[3 * l + 2]};
+    const uint32_t own = l * (C * kComp) + sub * 8;
+    float gsum[kGradCount] = {0.f, 0.f, 0.f, 0.f};
+    after_previous_kernel<false>();
+    for (ILWalk<CELLS> g(G, u0, fdiv(nwarps, a.divV), 0, dGX, a.divY); g.q < nq; g.next(G)) {
+        const uint32_t x = g.gx * CELLS + sub;
+        if (x >= G.X) continue;
+        const size_t base = g.base(G);
+        const uint32_t outside = edge.outside(g.gx, G.GX);
+        const int32_t zero = g.zero(G);
+        const char* lam = j.a_prev + base;
+        char* o = j.a_next + base + own;
+        Cx<float> b[C], u[C], v[C], K[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            const Cx<float> m = ldc<float>(lam + own + c * kComp);
+            b[c] = cx<float>(-m.y, m.x);   // b = i lambda
+            u[c] = ldc<float>(j.psi + base + own + c * kComp);
+            v[c] = ldc<float>(o + c * kComp);
+        }
+        float r[3];
+        node_pos(P, x, g.y, g.z, pos, r);
+        if (j.update) {
+            // L^T b = sum_f wT_f b_nb(f) - (sum_f w_f) b
+#pragma unroll
+            for (int c = 0; c < C; ++c) K[c] = cx<float>(-diag * b[c].x, -diag * b[c].y);
+#pragma unroll
+            for (int k0 = 0; k0 < D; k0 += 4) {
+                if (k0 >= nd) break;
+                Cx<float> n[4][C];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const char* p = lam + ((outside >> (k0 + k)) & 1 ? zero : off[k0 + k]);
+#pragma unroll
+                    for (int c = 0; c < C; ++c) n[k][c] = ldc<float>(p + c * kComp);
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+#pragma unroll
+                    for (int c = 0; c < C; ++c) add_scaled(K[c], wT[k0 + k], cx<float>(-n[k][c].y, n[k][c].x));
+                }
+            }
+            Cx<float> q[C];
+            local_jvp<float, C>(P, r, trap<float>(P, r), u, b, q);
+            if (P.flags & GPE_FLAG_THREE_BODY_LOSS) add_loss_transpose<float, C>(P, u, b, q);
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+                add_scaled(v[c], j.factor32, K[c] + q[c]);
+                stc<float>(o + c * kComp, v[c]);
+            }
+        }
+        add_field_gradient<float, C>(P, r, b, u, gsum);
+    }
+    block_partials<kGradCount, float>(gsum, j.factor, a.partials);
 }
 
 // Block g adds the nblocks x K partials at partials + g * nblocks * K into
@@ -395,39 +494,96 @@ __global__ void __launch_bounds__(kSumThreads) adjoint_sum_kernel(const double* 
 
 constexpr int kFinalCount = 5;  // Re <T|u>, Im <T|u>, Mx, My, Mz
 
-// Final-state quantities: the overlap sum conj(T) u and the spin density sums.
-// a.prev = target T, a.next = u_N.
+// Final-state quantities: the overlap sum conj(T) u and the spin density sums, to FP64's
+// precision in pairs of FP32 values (gpe_observe.cuh) for FP32 storage.  a.prev = target
+// T, a.next = u_N.
 template <typename R, int C>
 __global__ void __launch_bounds__(256) adjoint_final_kernel(StepArgs a) {
-    double v[kFinalCount] = {0, 0, 0, 0, 0};
-    const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gid < a.total) {
+    using A = ObsArith<R>;
+    typename A::S s[kFinalCount] = {}, f6[2] = {};
+    for (uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < a.total;
+         gid += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t x, y, z, l;
         node_coords(a, (uint32_t)gid, x, y, z, l);
         const size_t off = (size_t)z * a.g.slice + (size_t)y * a.g.pitch + (size_t)x * a.g.cell_bytes +
                            l * (C * 2 * sizeof(R));
-        Cx<double> u[C];
+        Cx<R> t[C], p[C];
+        ld_node<R, C, true>(a.prev + off, t);
+        ld_node<R, C, true>(a.next + off, p);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            const Cx<R> t = ldc_nc<R>(a.prev + off + c * 2 * sizeof(R));
-            const Cx<R> p = ldc_nc<R>(a.next + off + c * 2 * sizeof(R));
-            u[c] = cx<double>((double)p.x, (double)p.y);
-            v[0] += (double)t.x * p.x + (double)t.y * p.y;
-            v[1] += (double)t.x * p.y - (double)t.y * p.x;
+            A::add(s[0], A::dot2(t[c].x, p[c].x, t[c].y, p[c].y));
+            A::add(s[1], A::cross2(t[c].x, p[c].y, t[c].y, p[c].x));
         }
-        double M[3];
-        local_mag<double, C>(u, M);
-        v[2] = M[0];
-        v[3] = M[1];
-        v[4] = M[2];
+        if constexpr (C > 1) {
+            // the spin densities' sums: spin-1 sqrt2 (chain of its components), spin-2 twice its outer
+            // pairs and sqrt6 times its inner chain
+            const NodeTerms<R, C> n(p);
+            typename A::T re, im;
+            constexpr int b = C == 5 ? 1 : 0;
+            n.chain(p[b], p[b + 1], p[b + 2], re, im);
+            if constexpr (C == 3) {
+                A::add(s[2], re);
+                A::add(s[3], im);
+                A::add(s[4], n.n[0] - n.n[2]);
+            } else {
+                A::add(f6[0], re);
+                A::add(f6[1], im);
+                A::add(s[2], A::dot2(p[0].x, p[1].x, p[0].y, p[1].y) + A::dot2(p[3].x, p[4].x, p[3].y, p[4].y));
+                A::add(s[3], A::cross2(p[0].x, p[1].y, p[0].y, p[1].x) + A::cross2(p[3].x, p[4].y, p[3].y, p[4].x));
+                A::add(s[4], twice(n.n[0] - n.n[4]) + (n.n[1] - n.n[3]));
+            }
+        }
+    }
+    double v[kFinalCount];
+#pragma unroll
+    for (int k = 0; k < kFinalCount; ++k) v[k] = A::value(s[k]);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        if constexpr (C == 3) v[2 + k] *= GPE_REF_SQRT_2;
+        if constexpr (C == 5) v[2 + k] = 2.0 * v[2 + k] + 2.449489742783178098 * A::value(f6[k]);
     }
     block_partials<kFinalCount, double>(v, 1.0, a.partials);
 }
 
-// lambda_N = dv [ (s0 + i s1) T + sum_m s_{2+m} grad M_m(u_N) ].
-// a.prev = target T, a.next = lambda buffer, psi = u_N.
+// (grad M_m(u))_m weighted by s: d(s.M)/d(conj u) in the real sense, 2 (s.F) u, for the spin
+// densities M that gpe_observe integrates.
 template <typename R, int C>
-__global__ void __launch_bounds__(256) adjoint_seed_kernel(StepArgs a, const char* psi, double s0, double s1, double sx,
+__device__ __forceinline__ void add_mag_gradient(const R s[3], const Cx<R>* u, Cx<R>* g) {
+    if constexpr (C == 3) {
+        const Cx<R> b = cx<R>((R)GPE_REF_SQRT_2 * s[0], (R)GPE_REF_SQRT_2 * s[1]);
+        const R z = (R)2 * s[2];
+        add_scaled(g[0], z, u[0]);
+        add_conj_mul(g[0], b, u[1]);
+        add_mul(g[1], b, u[0]);
+        add_conj_mul(g[1], b, u[2]);
+        add_mul(g[2], b, u[1]);
+        add_scaled(g[2], -z, u[2]);
+    } else if constexpr (C == 5) {
+        const R q6 = (R)2.449489742783178098;
+        const Cx<R> b2 = cx<R>((R)2 * s[0], (R)2 * s[1]), b6 = cx<R>(q6 * s[0], q6 * s[1]);
+        const R z = (R)2 * s[2];
+        add_scaled(g[0], (R)2 * z, u[0]);
+        add_conj_mul(g[0], b2, u[1]);
+        add_scaled(g[1], z, u[1]);
+        add_mul(g[1], b2, u[0]);
+        add_conj_mul(g[1], b6, u[2]);
+        add_mul(g[2], b6, u[1]);
+        add_conj_mul(g[2], b6, u[3]);
+        add_scaled(g[3], -z, u[3]);
+        add_mul(g[3], b6, u[2]);
+        add_conj_mul(g[3], b2, u[4]);
+        add_scaled(g[4], (R)-2 * z, u[4]);
+        add_mul(g[4], b2, u[3]);
+    }
+}
+
+// lambda_N = dv [ (s0 + i s1) T + sum_m s_{2+m} grad M_m(u_N) ], in FP64.  a.prev = target
+// T and psi = u_N in the handle's layout, a.next = lambda's buffer, in that layout or (G
+// given) the interleaved one.  (The gradient by dual numbers, one evaluation of M per
+// real part of u, took 248 us of FP64 work on spin-1 BCC 40^3.)
+template <typename R, int C>
+__global__ void __launch_bounds__(256) adjoint_seed_kernel(StepArgs a, ILGrid G, const char* psi, double s0, double s1, double sx,
                                                            double sy, double sz, double dv) {
     const uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (gid >= a.total) return;
@@ -435,6 +591,14 @@ __global__ void __launch_bounds__(256) adjoint_seed_kernel(StepArgs a, const cha
     node_coords(a, (uint32_t)gid, x, y, z, l);
     const size_t off = (size_t)z * a.g.slice + (size_t)y * a.g.pitch + (size_t)x * a.g.cell_bytes +
                        l * (C * 2 * sizeof(R));
+    const bool il = G.cells != 0;
+    char* out = a.next + off;
+    size_t comp = 2 * sizeof(R);
+    if (il) {
+        const uint32_t gx = x / G.cells;
+        out = a.next + il_row(G, y, z) + (size_t)gx * G.gb + ((size_t)l * C * G.cells + (x - gx * G.cells)) * 8;
+        comp = (size_t)G.cells * 8;
+    }
     Cx<double> u[C], g[C];
 #pragma unroll
     for (int c = 0; c < C; ++c) {
@@ -443,23 +607,10 @@ __global__ void __launch_bounds__(256) adjoint_seed_kernel(StepArgs a, const cha
         u[c] = cx<double>((double)p.x, (double)p.y);
         g[c] = cx<double>(s0 * t.x - s1 * t.y, s0 * t.y + s1 * t.x);
     }
-    if (C > 1 && (sx != 0.0 || sy != 0.0 || sz != 0.0)) {
+    const double sm[3] = {sx, sy, sz};
+    if (C > 1 && (sx != 0.0 || sy != 0.0 || sz != 0.0)) add_mag_gradient<double, C>(sm, u, g);
 #pragma unroll
-        for (int k = 0; k < 2 * C; ++k) {
-            Cx<Dual<double>> uD[C];
-#pragma unroll
-            for (int c = 0; c < C; ++c)
-                uD[c] = cx<Dual<double>>(Dual<double>(u[c].x, (double)(k == 2 * c)),
-                                         Dual<double>(u[c].y, (double)(k == 2 * c + 1)));
-            Dual<double> M[3];
-            local_mag<Dual<double>, C>(uD, M);
-            const double d = sx * M[0].d + sy * M[1].d + sz * M[2].d;
-            if (k & 1) g[k >> 1].y += d;
-            else g[k >> 1].x += d;
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < C; ++c) stc<R>(a.next + off + c * 2 * sizeof(R), cx<R>((R)(dv * g[c].x), (R)(dv * g[c].y)));
+    for (int c = 0; c < C; ++c) stc<R>(out + c * comp, cx<R>((R)(dv * g[c].x), (R)(dv * g[c].y)));
 }
 
 // Blocks of a reverse step: one wave (the kernel's occupancy x SMs), fewer for
@@ -482,17 +633,40 @@ static cudaError_t launch_adjoint_step(const StepArgs& a, const AdjArgs& j, unsi
     return cudaGetLastError();
 }
 
+// Blocks of a reverse step on interleaved states (its partials are that many blocks x
+// kGradCount), and its launch.
+template <int C>
+static unsigned il_adjoint_blocks(const gpe_handle* h) {
+    return il_form(h->ilg, il_stencil_deg(h), 0u, [&](auto cells, auto d) {
+        static int occ = 0;
+        if (occ == 0) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, il_adjoint_kernel<C, d(), cells()>, (int)kIlAdjThreads, 0);
+            if (occ < 1) occ = 1;
+        }
+        return il_wave(h->ilg, kIlAdjThreads, occ, h->partial_blocks);
+    });
+}
+template <int C>
+static cudaError_t launch_il_adjoint(const gpe_handle* h, const StepArgs& a, const AdjArgs& j, unsigned nb, cudaStream_t s) {
+    return il_form(h->ilg, il_stencil_deg(h), cudaErrorInvalidValue, [&](auto cells, auto d) {
+        return launch_overlapped(il_adjoint_kernel<C, d(), cells()>, nb, kIlAdjThreads, 0, s, a, j, h->ilg, make_fastdiv(h->ilg.GX));
+    });
+}
+#define GPE_IL_ADJ_DISPATCH(FN, H, ...) ((H)->g.C == 1 ? FN<1>(__VA_ARGS__) : (H)->g.C == 3 ? FN<3>(__VA_ARGS__) : FN<5>(__VA_ARGS__))
+
 template <typename R, int C>
 static cudaError_t launch_adjoint_final(const StepArgs& a, double dv, double* out, cudaStream_t s) {
-    const unsigned nb = nblocks(a.total, 256);
+    const unsigned nb = std::min<unsigned>(nblocks(a.total, 256), 4u * (unsigned)device_sm_count());
     adjoint_final_kernel<R, C><<<nb, 256, 0, s>>>(a);
     adjoint_sum_kernel<kFinalCount><<<1, kSumThreads, 0, s>>>(a.partials, nb, dv, out);
     return cudaGetLastError();
 }
 
 template <typename R, int C>
-static cudaError_t launch_adjoint_seed(const StepArgs& a, const char* psi, const double* sd, double dv, cudaStream_t s) {
-    adjoint_seed_kernel<R, C><<<nblocks(a.total, 256), 256, 0, s>>>(a, psi, sd[0], sd[1], sd[2], sd[3], sd[4], dv);
+static cudaError_t launch_adjoint_seed(const StepArgs& a, const ILGrid* G, const char* psi, const double* sd, double dv,
+                                       cudaStream_t s) {
+    adjoint_seed_kernel<R, C><<<nblocks(a.total, 256), 256, 0, s>>>(a, G ? *G : ILGrid{}, psi, sd[0], sd[1], sd[2], sd[3], sd[4],
+                                                                    dv);
     return cudaGetLastError();
 }
 
@@ -528,7 +702,8 @@ void adjoint_release(gpe_handle* h) {
     A.target = nullptr;
     A.grad = A.out = A.wT64 = nullptr;
     A.wT32 = nullptr;
-    A.valid = false;
+    A.valid = A.il = false;
+    A.buf_bytes = 0;
     A.n = A.stride = A.segments = 0;
 }
 
@@ -575,10 +750,11 @@ static gpe_status build_transpose(gpe_handle* h) {
     return GPE_OK;
 }
 
-static gpe_status ensure_adjoint_buffers(gpe_handle* h, int n, int stride) {
+static gpe_status ensure_adjoint_buffers(gpe_handle* h, int n, int stride, bool il) {
     AdjointStore& A = h->adj;
     const int segments = (n + stride - 1) / stride;
-    const size_t bytes = h->alloc_bytes[GPE_PSI_EVEN];
+    const size_t bytes = il ? h->ilg.bytes : h->alloc_bytes[GPE_PSI_EVEN];
+    if (A.il != il || A.buf_bytes != bytes) adjoint_release(h);
     const size_t want_ckpt = (size_t)2 * segments, want_seg = stride > 2 ? (size_t)(stride - 2) : 0;
     auto resize = [&](std::vector<void*>& v, size_t want) -> bool {
         while (v.size() > want) {
@@ -604,8 +780,9 @@ static gpe_status ensure_adjoint_buffers(gpe_handle* h, int n, int stride) {
     for (void*& p : A.adj)
         if (!p && cudaMalloc(&p, bytes) != cudaSuccess) return fail(GPE_ERR_OOM, "cudaMalloc (adjoint state)");
     if (!A.target) {
-        if (cudaMalloc(&A.target, bytes) != cudaSuccess) return fail(GPE_ERR_OOM, "cudaMalloc (target)");
-        if (cudaMemset(A.target, 0, bytes) != cudaSuccess) return fail(GPE_ERR_CUDA, "cudaMemset (target)");
+        const size_t tb = h->alloc_bytes[GPE_PSI_EVEN];   // the target stays in the handle's layout
+        if (cudaMalloc(&A.target, tb) != cudaSuccess) return fail(GPE_ERR_OOM, "cudaMalloc (target)");
+        if (cudaMemset(A.target, 0, tb) != cudaSuccess) return fail(GPE_ERR_CUDA, "cudaMemset (target)");
     }
     if (A.grad && A.n < n) {
         cudaFree(A.grad);
@@ -628,6 +805,7 @@ static gpe_status ensure_adjoint_buffers(gpe_handle* h, int n, int stride) {
         if (st) return st;
     }
     A.buf_bytes = bytes;
+    A.il = il;
     A.segments = segments;
     return GPE_OK;
 }
@@ -652,9 +830,21 @@ extern "C" gpe_status gpe_adjoint_forward(gpe_handle* h, int32_t n_steps, const 
     if (stride > n_steps) stride = n_steps;
     AdjointStore& A = h->adj;
     A.valid = false;
-    gpe_status st = ensure_adjoint_buffers(h, n_steps, stride);
-    if (st) return st;
     cudaStream_t s = (cudaStream_t)stream;
+    // runs long enough for the interleaved step kernel keep all their states in its layout, where the memory for them can be had (its rows are padded to whole
+    // groups of cells); others in the handle's layout
+    gpe_status st = GPE_ERR_OOM;
+    if (n_steps > 1 && il_leapfrog_applies(h, n_steps)) {
+        st = il_ensure(h, s);
+        if (!st) st = ensure_adjoint_buffers(h, n_steps, stride, true);
+        if (st && st != GPE_ERR_OOM) return st;
+        if (st) {
+            adjoint_release(h);
+            cudaGetLastError();
+        }
+    }
+    if (st) st = ensure_adjoint_buffers(h, n_steps, stride, false);
+    if (st) return st;
     // target: host FP64 file layout -> device buffer in the handle's precision
     if ((st = ensure_stage(h, count))) return st;
     const Grid& g = h->g;
@@ -673,30 +863,42 @@ extern "C" gpe_status gpe_adjoint_forward(gpe_handle* h, int32_t n_steps, const 
     auto slot_of = [](int j) { return (j & 1) ? GPE_PSI_EVEN : GPE_PSI_ODD; };
     if ((st = step_buffers(h, h->interior[GPE_PSI_EVEN], h->interior[GPE_PSI_ODD], fields[0], A.t0, GPE_MODE_EULER, s)))
         return st;
-    if ((st = copy_state(h, A.ckpt[0], h->alloc[GPE_PSI_ODD], s))) return st;
-    if ((st = copy_state(h, A.ckpt[1], h->alloc[GPE_PSI_EVEN], s))) return st;
-    // steps j .. je up to the next checkpoint (after a step j that is a multiple of
-    // the stride), in the interleaved layout where that is the handle's kernel for a
-    // call of that length (the same states as step_buffers', bit for bit, so the
-    // recomputation in the handle's layout reproduces them)
-    for (int j = 1; j < n_steps;) {
-        int je = (j + stride - 1) / stride * stride;
-        if (je > n_steps - 1) je = n_steps - 1;
-        const int32_t cnt = je - j + 1;
-        if (il_leapfrog_applies(h, cnt)) {
-            if ((st = il_leapfrog_explicit(h, slot_of(j), cnt, fields + j, A.t0 + j * dt, dt, s))) return st;
-        } else {
-            for (int jj = j; jj <= je; ++jj)
-                if ((st = step_buffers(h, h->interior[slot_of(jj + 1)], h->interior[slot_of(jj)], fields[jj],
-                                       A.t0 + jj * dt, GPE_MODE_LEAPFROG, s)))
-                    return st;
+    if (A.il) {
+        // u_j goes where it is wanted: a checkpoint (u_{kS}, u_{kS+1}), or one of two work
+        // buffers, in place of u_{j-2} where that is no checkpoint
+        auto il_buffer = [&](void* p) { return static_cast<char*>(p); };
+        auto home = [&](int j) -> char* {
+            if (j == n_steps) return nullptr;
+            if (j % stride == 0) return il_buffer(A.ckpt[2 * (j / stride)]);
+            if (j % stride == 1) return il_buffer(A.ckpt[2 * (j / stride) + 1]);
+            return nullptr;
+        };
+        char *old = home(0), *cur = home(1) ? home(1) : h->il[0];
+        if ((st = il_convert(h, h->interior[GPE_PSI_ODD], old, true, s))) return st;
+        if ((st = il_convert(h, h->interior[GPE_PSI_EVEN], cur, true, s))) return st;
+        for (int j = 1; j < n_steps; ++j) {
+            const bool old_is_work = old == h->il[0] || old == h->il[1];
+            char* next = home(j + 1);
+            if (!next) next = old_is_work ? old : (cur == h->il[0] ? h->il[1] : h->il[0]);
+            if ((st = il_leapfrog(h, next, cur, old, fields[j], A.t0 + j * dt, s))) return st;
+            old = cur;
+            cur = next;
         }
-        if (je % stride == 0) {
-            const int k = je / stride;
-            if ((st = copy_state(h, A.ckpt[2 * k], h->alloc[slot_of(je)], s))) return st;
-            if ((st = copy_state(h, A.ckpt[2 * k + 1], h->alloc[slot_of(je + 1)], s))) return st;
+        if ((st = il_convert(h, h->interior[slot_of(n_steps - 1)], old, false, s))) return st;
+        if ((st = il_convert(h, h->interior[slot_of(n_steps)], cur, false, s))) return st;
+    } else {
+        if ((st = copy_state(h, A.ckpt[0], h->alloc[GPE_PSI_ODD], s))) return st;
+        if ((st = copy_state(h, A.ckpt[1], h->alloc[GPE_PSI_EVEN], s))) return st;
+        for (int j = 1; j < n_steps; ++j) {
+            if ((st = step_buffers(h, h->interior[slot_of(j + 1)], h->interior[slot_of(j)], fields[j], A.t0 + j * dt,
+                                   GPE_MODE_LEAPFROG, s)))
+                return st;
+            if (j % stride == 0) {
+                const int k = j / stride;
+                if ((st = copy_state(h, A.ckpt[2 * k], h->alloc[slot_of(j)], s))) return st;
+                if ((st = copy_state(h, A.ckpt[2 * k + 1], h->alloc[slot_of(j + 1)], s))) return st;
+            }
         }
-        j = je + 1;
     }
     h->cur = slot_of(n_steps);
     h->nstep = (uint64_t)(n_steps - 1);
@@ -730,16 +932,19 @@ extern "C" gpe_status gpe_adjoint_backward(gpe_handle* h, const double* seed, do
     cudaError_t e = cudaMemsetAsync(A.adj[0], 0, A.buf_bytes, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(A.adj[1], 0, A.buf_bytes, s);
     if (e != cudaSuccess) return cuda_fail(e, "adjoint clear");
+    // a state buffer's first interior value in the handle's layout, its start in the
+    // interleaved one
+    auto at = [&](void* p) { return A.il ? static_cast<char*>(p) : interior_of(h, p); };
     {
         StepArgs a = make_args(h, A.fields[n - 1], A.t0 + n * dt);
         a.prev = interior_of(h, A.target);
-        a.next = interior_of(h, A.adj[0]);
-        e = GPE_ADJ_DISPATCH(launch_adjoint_seed, h, a, h->interior[h->cur], seed, cell_dv(h), s);
+        a.next = at(A.adj[0]);
+        e = GPE_ADJ_DISPATCH(launch_adjoint_seed, h, a, A.il ? &h->ilg : nullptr, h->interior[h->cur], seed, cell_dv(h), s);
         if (e != cudaSuccess) return cuda_fail(e, "adjoint seed kernel");
         h->launches += 1;
     }
-    char* P = interior_of(h, A.adj[0]);  // lambda_{j+1}
-    char* Q = interior_of(h, A.adj[1]);  // lambda_{j+2} -> lambda_j
+    char* P = at(A.adj[0]);  // lambda_{j+1}
+    char* Q = at(A.adj[1]);  // lambda_{j+2} -> lambda_j
     std::vector<void*> state((size_t)S, nullptr);
     // the gather kernel recomputes a segment out of place; the tile kernels (which
     // the forward run then used) in place after a state copy, so that the states
@@ -752,6 +957,11 @@ extern "C" gpe_status gpe_adjoint_backward(gpe_handle* h, const double* seed, do
         for (int m = 2; m < len; ++m) {
             state[m] = A.seg[m - 2];
             const int jj = lo + m - 1;
+            if (A.il) {
+                if ((st = il_leapfrog(h, at(state[m]), at(state[m - 1]), at(state[m - 2]), A.fields[jj], A.t0 + jj * dt, s)))
+                    return st;
+                continue;
+            }
             if (oop) {
                 // u_{jj+1} = u_{jj-1} + F(u_jj) into a fresh buffer: no state copy
                 if ((st = leapfrog_from(h, interior_of(h, state[m]), interior_of(h, state[m - 1]),
@@ -764,20 +974,22 @@ extern "C" gpe_status gpe_adjoint_backward(gpe_handle* h, const double* seed, do
                                    A.t0 + jj * dt, GPE_MODE_LEAPFROG, s)))
                 return st;
         }
-        const unsigned nb = GPE_ADJ_DISPATCH(adjoint_step_blocks, h, h->g.X * (uint64_t)h->g.Y * h->g.Z * h->g.V);
+        const unsigned nb = A.il ? GPE_IL_ADJ_DISPATCH(il_adjoint_blocks, h, h)
+                                 : GPE_ADJ_DISPATCH(adjoint_step_blocks, h, h->g.X * (uint64_t)h->g.Y * h->g.Z * h->g.V);
         for (int j = hi - 1; j >= lo; --j) {
             StepArgs a = make_args(h, A.fields[j], A.t0 + j * dt);
             a.partials = A.part + (size_t)(j - lo) * nb * kGradCount;
             AdjArgs aj;
             aj.a_prev = P;
             aj.a_next = Q;
-            aj.psi = interior_of(h, state[j - lo]);
+            aj.psi = at(state[j - lo]);
             aj.wT64 = A.wT64;
             aj.wT32 = A.wT32;
             aj.factor = j >= 1 ? 2.0 * dt : dt;
             aj.factor32 = (float)aj.factor;
             aj.update = j >= 1 ? 1 : 0;
-            e = GPE_ADJ_DISPATCH(launch_adjoint_step, h, a, aj, nb, s);
+            e = A.il ? GPE_IL_ADJ_DISPATCH(launch_il_adjoint, h, h, a, aj, nb, s)
+                     : GPE_ADJ_DISPATCH(launch_adjoint_step, h, a, aj, nb, s);
             if (e != cudaSuccess) return cuda_fail(e, "adjoint step kernel");
             h->launches += 1;
             if (j >= 1) std::swap(P, Q);

@@ -283,7 +283,7 @@ __device__ __forceinline__ void batch_il_rows(const BatchMember& M, const SmemTa
             }
         }
         const size_t base = g.base(G);
-        il_task<C, D, CELLS, NoObs>(P, F, prev + base, next + base, l * (C * CELLS * 8) + sub * 8, off, outside, g.zero(G),
+        il_task<C, D, CELLS, NoObs>(P, F, prev + base, next + base, next + base, l * (C * CELLS * 8) + sub * 8, off, outside, g.zero(G),
                                     st.w + f0, nd, st.pos + 3 * l, x, g.y, g.z, &no);
     }
 }

@@ -59,6 +59,8 @@ cudaError_t launch_il_step(const StepArgs& a, const ILGrid& G, int deg, size_t m
 template <int C>
 cudaError_t launch_il_itp(const StepArgs& a, const ILGrid& G, int deg, size_t max_blocks, cudaStream_t s);
 template <int C>
+cudaError_t launch_il_step_from(const StepArgs& a, const ILGrid& G, int deg, size_t max_blocks, cudaStream_t s);
+template <int C>
 unsigned il_blocks(const ILGrid& G, int deg, bool obs, size_t max_blocks);
 cudaError_t launch_il_convert(char* aos, const Grid& g, char* il, const ILGrid& G, bool to_il, cudaStream_t s);
 template <int C>
@@ -1335,16 +1337,20 @@ static bool use_interleaved(const gpe_handle* h, int32_t n) {
 namespace gpe {
 gpe_status il_ensure(gpe_handle* h, cudaStream_t s) {
     const ILGrid G = make_il_grid(h->g);
+    void* fresh[2] = {nullptr, nullptr};
     for (int k = 0; k < 2; ++k) {
         if (h->il[k]) continue;
-        void* p = nullptr;
-        if (cudaMalloc(&p, G.bytes) != cudaSuccess) {
+        if (cudaMalloc(&fresh[k], G.bytes) != cudaSuccess) {
             cudaGetLastError();
+            if (fresh[0]) cudaFree(fresh[0]);
             return fail(GPE_ERR_OOM, "cudaMalloc (interleaved state)");
         }
-        h->il[k] = static_cast<char*>(p);
+    }
+    for (int k = 0; k < 2; ++k) {
+        if (!fresh[k]) continue;
+        h->il[k] = static_cast<char*>(fresh[k]);
         // the halo rows and the padding cells stay zero
-        CUDA_TRY(cudaMemsetAsync(p, 0, G.bytes, s));
+        CUDA_TRY(cudaMemsetAsync(fresh[k], 0, G.bytes, s));
     }
     h->ilg = G;
     return GPE_OK;
@@ -1436,34 +1442,34 @@ static cudaError_t dispatch_il_step(const gpe_handle* h, const StepArgs& a, bool
 static gpe_status fill_observables(const gpe_handle* h, const double* r, gpe_observables* out);
 
 namespace gpe {
-// n parabolic leapfrog steps through the interleaved layout with the fields of
-// every step given: step k reads slot `first_prev` (k even) or the other slot (k
-// odd), at time t_first + k dt with fields[k], as step_buffers does in the
-// handle's layout -- the same states, bit for bit.  False (nothing run) where the
-// interleaved kernel is not the handle's choice for a call of n steps.
 bool il_leapfrog_applies(const gpe_handle* h, int32_t n) {
     return h->p.scheme == GPE_SCHEME_PARABOLIC && use_interleaved(h, n);
 }
 
-gpe_status il_leapfrog_explicit(gpe_handle* h, int first_prev, int32_t n, const gpe_fields* fields, double t_first,
-                                double dt, cudaStream_t s) {
-    if (!il_leapfrog_applies(h, n)) return fail(GPE_ERR_UNSUPPORTED, "the interleaved kernel does not apply");
-    gpe_status st = ensure_il(h, s);
-    if (st) return st;
-    if ((st = il_convert_all(h, true, s))) return st;
-    int prev = first_prev;
-    for (int32_t k = 0; k < n; ++k) {
-        const int next = prev == GPE_PSI_EVEN ? GPE_PSI_ODD : GPE_PSI_EVEN;
-        StepArgs a = make_args(h, fields[k], t_first + k * dt);
-        a.prev = h->il[prev];
-        a.next = h->il[next];
-        cudaError_t e = dispatch_il_step(h, a, false, s);
-        if (e != cudaSuccess) return cuda_fail(e, "interleaved step launch");
-        h->launches += 1;
-        h->epoch += 1;
-        prev = next;
+gpe_status il_leapfrog(gpe_handle* h, char* next, const char* cur, const char* old, const gpe_fields& B, double t,
+                       cudaStream_t s) {
+    StepArgs a = make_args(h, B, t);
+    a.prev = cur;
+    a.next = next;
+    a.hpsi = const_cast<char*>(old);  // read only, by the out-of-place kernels
+    cudaError_t e;
+    if (old == next) e = dispatch_il_step(h, a, false, s);
+    else switch (h->g.C) {
+        case 1: e = launch_il_step_from<1>(a, h->ilg, il_deg(h), h->partial_blocks, s); break;
+        case 3: e = launch_il_step_from<3>(a, h->ilg, il_deg(h), h->partial_blocks, s); break;
+        default: e = launch_il_step_from<5>(a, h->ilg, il_deg(h), h->partial_blocks, s); break;
     }
-    return il_convert_all(h, false, s);
+    if (e != cudaSuccess) return cuda_fail(e, "interleaved step launch");
+    h->launches += 1;
+    h->epoch += 1;
+    return GPE_OK;
+}
+
+gpe_status il_convert(gpe_handle* h, char* aos, char* il, bool to_il, cudaStream_t s) {
+    const cudaError_t e = launch_il_convert(aos, h->g, il, h->ilg, to_il, s);
+    if (e != cudaSuccess) return cuda_fail(e, to_il ? "layout change (in)" : "layout change (out)");
+    h->launches += 1;
+    return GPE_OK;
 }
 }  // namespace gpe
 

@@ -32,7 +32,8 @@ struct AdjointStore {
     std::vector<void*> seg;         // stride buffers for the recomputed segment
     void* adj[2] = {nullptr, nullptr};
     void* target = nullptr;
-    size_t buf_bytes = 0;
+    size_t buf_bytes = 0;           // bytes of each state buffer above
+    bool il = false;                // checkpoints, segment and adjoint buffers in the interleaved layout
     double* grad = nullptr;         // device, n x 4
     double* out = nullptr;          // device, 8
     double* part = nullptr;         // device, stride x blocks x 4: block partials of one segment
@@ -131,11 +132,13 @@ void adjoint_release(gpe_handle* h);
 // and the handle's two interleaved psi copies, allocated (zeroed) on first use.
 int il_stencil_deg(const gpe_handle* h);
 gpe_status il_ensure(gpe_handle* h, cudaStream_t s);
-// n parabolic leapfrog steps with explicit fields in the interleaved layout (both
-// psi slots changed in and back), where the handle's kernel choice for a call of n
-// steps is the interleaved kernel (il_leapfrog_applies); the states step_buffers
-// would leave, bit for bit.
+// Whether a recorded run of n steps keeps its states in the interleaved layout: where
+// that is the handle's step kernel for a call of n steps.
 bool il_leapfrog_applies(const gpe_handle* h, int32_t n);
-gpe_status il_leapfrog_explicit(gpe_handle* h, int first_prev, int32_t n, const gpe_fields* fields, double t_first,
-                                double dt, cudaStream_t s);
+// One leapfrog step next <- old + F(cur) with explicit fields on interleaved buffers of
+// the handle's geometry, in place (old == next) or out of place: the same values.
+gpe_status il_leapfrog(gpe_handle* h, char* next, const char* cur, const char* old, const gpe_fields& B, double t,
+                       cudaStream_t s);
+// The layout change of one state (aos: an interior pointer of the handle's layout).
+gpe_status il_convert(gpe_handle* h, char* aos, char* il, bool to_il, cudaStream_t s);
 }  // namespace gpe

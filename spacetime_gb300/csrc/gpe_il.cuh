@@ -214,7 +214,8 @@ struct ILWalk {
 
 // One lane's node of an interleaved leapfrog step, cell (x, y, z): next <- next + 2 dt
 // (-i H prev), with the arithmetic and its order of parabolic_node_t + node_finish.
-// prev, next: the group's base in the two buffers; own: the node's offset from it; off:
+// prev, next: the group's base in the two buffers (old: in the buffer of the old next
+// values, next itself unless the step goes out of place); own: the node's offset from it; off:
 // its neighbours', those with their bit set in `outside` read the zero row at `zero`
 // instead.  F: where the step's fields come from (P if null); oa: where the observables
 // of prev go.  With a NormAcc for oa: an imaginary-time iteration (kModeItpNorm), next =
@@ -225,7 +226,7 @@ struct ILWalk {
 // nothing is computed here that is the same for the whole launch or row.
 template <int C, int D, int CELLS, class OA>
 __device__ __forceinline__ void il_task(const PhysR<float>& P, const PhysR<float>* F, const char* prev, char* next,
-                                        uint32_t own, const int32_t* off, uint32_t outside, int32_t zero, const float* w,
+                                        const char* old, uint32_t own, const int32_t* off, uint32_t outside, int32_t zero, const float* w,
                                         int nd, const float* pos, uint32_t x, uint32_t y, uint32_t z, OA* oa,
                                         float inv = 1.f) {
     constexpr bool kItp = std::is_same<OA, NormAcc<float>>::value;
@@ -236,7 +237,7 @@ __device__ __forceinline__ void il_task(const PhysR<float>& P, const PhysR<float
 #pragma unroll
     for (int s = 0; s < C; ++s) {
         prv[s] = ldc<float>(pp + s * kComp);
-        if constexpr (!kItp) nv[s] = ldc<float>(np + s * kComp);
+        if constexpr (!kItp) nv[s] = ldc<float>(old + own + s * kComp);
     }
 #pragma unroll
     for (int s = 0; s < C; ++s) H[s] = cx<float>(0.f, 0.f);
@@ -304,7 +305,8 @@ constexpr unsigned kIlObsThreads = 256;
 // registers; the row length is the same in every lane of a warp, so the second
 // group of 4 entries is a uniform branch.  OBS: the observables of prev are summed
 // on the way (ObsAcc, as the gather kernels' observed step).  MODE kModeItpNorm: an
-// imaginary-time iteration instead.
+// imaginary-time iteration instead; kModeLeapfrogFrom: the old next values are read
+// from a.hpsi and stay as they were.
 template <int C, int D, int CELLS, bool OBS, int MODE = GPE_MODE_LEAPFROG>
 __device__ __forceinline__ void il_step_body(const StepArgs& a, const ILGrid& G, FastDiv dGX) {
     static_assert(D == 4 || D == 8, "rows of 4, or of 4 and 8 entries");
@@ -345,7 +347,8 @@ __device__ __forceinline__ void il_step_body(const StepArgs& a, const ILGrid& G,
         const uint32_t x = g.gx * CELLS + sub;
         if (x >= G.X) continue;
         const size_t base = g.base(G);
-        il_task<C, D, CELLS, OA>(P, nullptr, a.prev + base, a.next + base, own, off, edge.outside(g.gx, G.GX), g.zero(G), w,
+        const char* old = MODE == kModeLeapfrogFrom ? a.hpsi + base : a.next + base;
+        il_task<C, D, CELLS, OA>(P, nullptr, a.prev + base, a.next + base, old, own, off, edge.outside(g.gx, G.GX), g.zero(G), w,
                                  nd, pos, x, g.y, g.z, &oa, inv);
     }
     if constexpr (OBS) {
@@ -392,6 +395,13 @@ template <int C, int D, int CELLS>
 __global__ void __launch_bounds__(kIlPlainThreads, IlBounds<C, D>::kMin) il_itp_kernel(StepArgs a, ILGrid G,
                                                                                    FastDiv dGX) {
     il_step_body<C, D, CELLS, false, kModeItpNorm>(a, G, dGX);
+}
+
+// The leapfrog step out of place (the adjoint's checkpoints and recomputed states).
+template <int C, int D, int CELLS>
+__global__ void __launch_bounds__(kIlPlainThreads, IlBounds<C, D>::kMin) il_step_from_kernel(StepArgs a, ILGrid G,
+                                                                                         FastDiv dGX) {
+    il_step_body<C, D, CELLS, false, kModeLeapfrogFrom>(a, G, dGX);
 }
 
 // Blocks of one interleaved step (rows of D entries at most): one wave at the
@@ -476,6 +486,25 @@ cudaError_t launch_il_step(const StepArgs& a, const ILGrid& G, int deg, size_t m
 }
 
 template <int C, int D, int CELLS>
+cudaError_t launch_il_step_from_d(const StepArgs& a, const ILGrid& G, size_t max_blocks, cudaStream_t s) {
+    static int occ = 0;
+    if (occ == 0) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, il_step_from_kernel<C, D, CELLS>, (int)kIlPlainThreads, 0);
+        if (occ < 1) occ = 1;
+    }
+    const unsigned nb = il_wave(G, kIlPlainThreads, occ, max_blocks);
+    if (nb == 0) return cudaErrorInvalidConfiguration;
+    return launch_overlapped(il_step_from_kernel<C, D, CELLS>, nb, kIlPlainThreads, 0, s, a, G, make_fastdiv(G.GX));
+}
+
+// One leapfrog step next <- hpsi + F(prev) (interleaved buffers).
+template <int C>
+cudaError_t launch_il_step_from(const StepArgs& a, const ILGrid& G, int deg, size_t max_blocks, cudaStream_t s) {
+    return il_form(G, deg, cudaErrorInvalidValue,
+                   [&](auto cells, auto d) { return launch_il_step_from_d<C, d(), cells()>(a, G, max_blocks, s); });
+}
+
+template <int C, int D, int CELLS>
 cudaError_t launch_il_itp_d(const StepArgs& a, const ILGrid& G, size_t max_blocks, cudaStream_t s) {
     static int occ = 0;
     if (occ == 0) {
@@ -497,6 +526,7 @@ cudaError_t launch_il_itp(const StepArgs& a, const ILGrid& G, int deg, size_t ma
 #define GPE_INSTANTIATE_IL(C)                                                                                           \
     template cudaError_t launch_il_step<C>(const StepArgs&, const ILGrid&, int, size_t, bool, double*, cudaStream_t); \
     template cudaError_t launch_il_itp<C>(const StepArgs&, const ILGrid&, int, size_t, cudaStream_t);                 \
+    template cudaError_t launch_il_step_from<C>(const StepArgs&, const ILGrid&, int, size_t, cudaStream_t);           \
     template unsigned il_blocks<C>(const ILGrid&, int, bool, size_t);                                                 \
     template cudaError_t launch_il_hyper<C>(const StepArgs&, const ILGrid&, const ILGrid&, const int32_t*, cudaStream_t);
 
