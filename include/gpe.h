@@ -540,7 +540,9 @@ gpe_status gpe_adjoint_backward(gpe_handle* h, const double* seed, double* grad,
  * (Spin1GpeBCC.cu:1574-1603).  A batch is built over existing handles of one
  * precision -- any lattices, grid sizes, component counts (1, 3, 5), traps and
  * ramps -- and advances all of them with one cooperative persistent kernel: the
- * members' rows are cut into work items of about GPE_BATCH_ITEM_NODES nodes, each
+ * members' rows are cut into work items of about GPE_BATCH_ITEM_NODES nodes (until it
+ * is set: at most 16384, fewer where that leaves a block of the grid less than seven
+ * items a step), each
  * block of the persistent grid processes its share of items, evaluates the next
  * step's fields of the members from their own ramps on the device, and meets the
  * other blocks at a grid barrier whose wait is bounded in time (GPE_ERR_TIMEOUT).

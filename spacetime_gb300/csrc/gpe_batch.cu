@@ -360,7 +360,12 @@ __global__ void __launch_bounds__(kBatchThreads, sizeof(R) == 8 ? 1 : (CMASK & 4
             // only where the member changes (w.member is the same in every thread)
             if (w.member != loaded) {
                 __syncthreads();  // every warp is done with the previous member's tables
-                if (threadIdx.x == 0) M = A.members[w.member];
+                // the member's description, a word per thread (one thread copying its 1.5 KB
+                // held the block for some 3 us)
+                static_assert(sizeof(BatchMember) % 4 == 0, "copied in words");
+                const uint32_t* src = reinterpret_cast<const uint32_t*>(A.members + w.member);
+                for (uint32_t i = threadIdx.x; i < sizeof(BatchMember) / 4; i += kBatchThreads)
+                    reinterpret_cast<uint32_t*>(&M)[i] = src[i];
                 __syncthreads();
                 const int V = M.g.V, nent = M.tab.entries;
                 for (int i = threadIdx.x; i <= V; i += kBatchThreads) st.row_ptr[i] = M.tab.row_ptr[i];
@@ -374,11 +379,15 @@ __global__ void __launch_bounds__(kBatchThreads, sizeof(R) == 8 ? 1 : (CMASK & 4
                     if constexpr (sizeof(R) == 4) st.pos[i] = M.tab.pos32[i];
                     else st.pos[i] = M.tab.pos64[i];
                 }
-                if (threadIdx.x == 0) {
-                    if constexpr (sizeof(R) == 4) P = M.pf;
-                    else P = M.pd;
-                    set_fields<R>(P, F[w.member]);
+                // constants from shared memory (with constant-memory members only the step's
+                // fields are read from P)
+                if constexpr (!CONSTP) {
+                    const uint32_t* ph = sizeof(R) == 4 ? reinterpret_cast<const uint32_t*>(&M.pf)
+                                                        : reinterpret_cast<const uint32_t*>(&M.pd);
+                    for (uint32_t i = threadIdx.x; i < sizeof(P) / 4; i += kBatchThreads) reinterpret_cast<uint32_t*>(&P)[i] = ph[i];
+                    __syncthreads();
                 }
+                if (threadIdx.x == 0) set_fields<R>(P, F[w.member]);
                 loaded = w.member;
                 __syncthreads();
             }
@@ -473,6 +482,7 @@ struct gpe_batch {
     int32_t steps_per_launch = 0;    // 0: all steps of a call in one launch
     std::vector<std::pair<uint64_t, int32_t>> item_nodes_by_lattice;  // (lattice key, target nodes per item)
     int32_t item_nodes = 16384;
+    bool item_nodes_set = false;     // GPE_BATCH_ITEM_NODES was set
     int32_t barrier_timeout_ms = 10000;
     int32_t extra_arrivals = 0;       // test hook: the barrier waits for arrivals that never come
     BatchMember* d_members = nullptr;
@@ -587,11 +597,13 @@ gpe_status upload_members(gpe_batch* b) {
 // The interleaved members' two psi slots changed into (to_il) or out of their
 // interleaved copies.
 gpe_status convert_members(gpe_batch* b, bool to_il, cudaStream_t s) {
+    bool beside = false;   // the first launch waits for what is before it, the others run side by side
     for (size_t i = 0; i < b->members.size(); ++i) {
         if (!b->il_deg[i]) continue;
         gpe_handle* h = b->members[i];
         for (int k = GPE_PSI_EVEN; k <= GPE_PSI_ODD; ++k) {
-            cudaError_t e = launch_il_convert(h->interior[k], h->g, h->il[k], h->ilg, to_il, s);
+            cudaError_t e = launch_il_convert(h->interior[k], h->g, h->il[k], h->ilg, to_il, beside, s);
+            beside = true;
             if (e != cudaSuccess) return cuda_fail(e, to_il ? "batch layout change (in)" : "batch layout change (out)");
         }
     }
@@ -607,10 +619,20 @@ uint64_t convert_launch_count(const gpe_batch* b) {
 // A lattice is told apart by its node and stencil-entry counts per cell.
 uint64_t lattice_key(const gpe_handle* h) { return ((uint64_t)h->g.V << 32) | (uint32_t)h->tab.entries; }
 
+// Nodes per work item: the autotuner's choice for the lattice, else the set size, else
+// what gives every block kItemsPerBlock items a step, at most 16384.  With three items
+// a block the blocks wait for those that took a fourth; many small ones cost their
+// turns at the counter.  24 members of 33M nodes, ten steps and their layout changes:
+// 16384 nodes (3.3 items a block) 6.49 ms, 4 items 5.92, 6 5.57, 8 5.57, 12 5.83, 24 6.09.
+constexpr int kItemsPerBlock = 7;
 int32_t target_nodes(const gpe_batch* b, const gpe_handle* h) {
     for (const auto& kv : b->item_nodes_by_lattice)
         if (kv.first == lattice_key(h)) return kv.second;
-    return b->item_nodes;
+    if (b->item_nodes_set) return b->item_nodes;
+    uint64_t nodes = 0;
+    for (const gpe_handle* m : b->members) nodes += (uint64_t)m->g.X * m->g.Y * m->g.Z * m->g.V;
+    const uint64_t share = nodes / ((uint64_t)std::max(b->grid, 1) * kItemsPerBlock);
+    return (int32_t)std::min<uint64_t>(b->item_nodes, std::max<uint64_t>(share, 1024));
 }
 
 // Work items of the members `which` (indices into b->members), sorted by lattice
@@ -951,6 +973,7 @@ extern "C" gpe_status gpe_batch_set_tuning(gpe_batch* b, int32_t key, int32_t va
     if (key == GPE_BATCH_ITEM_NODES) {
         if (value < 1) return fail(GPE_ERR_INVALID_ARG, "item nodes");
         b->item_nodes = value;
+        b->item_nodes_set = true;
         b->item_nodes_by_lattice.clear();
         return rebuild_items(b);
     }
@@ -1049,7 +1072,7 @@ extern "C" gpe_status gpe_batch_autotune(gpe_batch* b, int32_t steps, char* repo
                     }
                     scratch.push_back(p);
                     cudaMemsetAsync(p, 0, h->ilg.bytes, s);
-                    if (launch_il_convert(h->interior[slot], h->g, static_cast<char*>(p), h->ilg, true, s) != cudaSuccess) {
+                    if (launch_il_convert(h->interior[slot], h->g, static_cast<char*>(p), h->ilg, true, false, s) != cudaSuccess) {
                         ok = false;
                         break;
                     }

@@ -62,7 +62,7 @@ template <int C>
 cudaError_t launch_il_step_from(const StepArgs& a, const ILGrid& G, int deg, size_t max_blocks, cudaStream_t s);
 template <int C>
 unsigned il_blocks(const ILGrid& G, int deg, bool obs, size_t max_blocks);
-cudaError_t launch_il_convert(char* aos, const Grid& g, char* il, const ILGrid& G, bool to_il, cudaStream_t s);
+cudaError_t launch_il_convert(char* aos, const Grid& g, char* il, const ILGrid& G, bool to_il, bool beside, cudaStream_t s);
 template <int C>
 cudaError_t launch_il_hyper(const StepArgs& a, const ILGrid& G, const ILGrid& Gq, const int32_t* tab, cudaStream_t s);
 enum HyperKind {
@@ -1417,14 +1417,14 @@ static cudaError_t dispatch_il_hyper(const gpe_handle* h, const StepArgs& a, cud
 // handles (4 or 8 launches).
 static gpe_status il_convert_all(gpe_handle* h, bool to_il, cudaStream_t s) {
     for (int k = GPE_PSI_EVEN; k <= GPE_PSI_ODD; ++k) {
-        cudaError_t e = launch_il_convert(h->interior[k], h->g, h->il[k], h->ilg, to_il, s);
+        cudaError_t e = launch_il_convert(h->interior[k], h->g, h->il[k], h->ilg, to_il, k != GPE_PSI_EVEN, s);
         if (e != cudaSuccess) return cuda_fail(e, to_il ? "layout change (in)" : "layout change (out)");
     }
     h->launches += 2;
     if (h->p.scheme != GPE_SCHEME_HYPERBOLIC) return GPE_OK;
     const Grid gq = q_grid(h);
     for (int k = 0; k < 2; ++k) {
-        cudaError_t e = launch_il_convert(h->interior[GPE_Q_EVEN + k], gq, h->ilq[k], h->ilgq, to_il, s);
+        cudaError_t e = launch_il_convert(h->interior[GPE_Q_EVEN + k], gq, h->ilq[k], h->ilgq, to_il, true, s);
         if (e != cudaSuccess) return cuda_fail(e, to_il ? "layout change (in)" : "layout change (out)");
     }
     h->launches += 2;
@@ -1466,7 +1466,7 @@ gpe_status il_leapfrog(gpe_handle* h, char* next, const char* cur, const char* o
 }
 
 gpe_status il_convert(gpe_handle* h, char* aos, char* il, bool to_il, cudaStream_t s) {
-    const cudaError_t e = launch_il_convert(aos, h->g, il, h->ilg, to_il, s);
+    const cudaError_t e = launch_il_convert(aos, h->g, il, h->ilg, to_il, false, s);
     if (e != cudaSuccess) return cuda_fail(e, to_il ? "layout change (in)" : "layout change (out)");
     h->launches += 1;
     return GPE_OK;
@@ -1690,7 +1690,7 @@ static gpe_status itp_iterations(gpe_handle* h, int32_t n, cudaStream_t s) {
     const bool il = deferred && itp_interleaved(h, n, s);
     cudaError_t e;
     if (il) {
-        e = launch_il_convert(h->interior[h->cur], h->g, h->il[h->cur], h->ilg, true, s);
+        e = launch_il_convert(h->interior[h->cur], h->g, h->il[h->cur], h->ilg, true, false, s);
         if (e != cudaSuccess) return cuda_fail(e, "layout change (in)");
         h->launches += 1;
     }
@@ -1714,7 +1714,7 @@ static gpe_status itp_iterations(gpe_handle* h, int32_t n, cudaStream_t s) {
         }
     }
     if (il) {
-        e = launch_il_convert(h->interior[h->cur], h->g, h->il[h->cur], h->ilg, false, s);
+        e = launch_il_convert(h->interior[h->cur], h->g, h->il[h->cur], h->ilg, false, false, s);
         if (e != cudaSuccess) return cuda_fail(e, "layout change (out)");
         h->launches += 1;
     }

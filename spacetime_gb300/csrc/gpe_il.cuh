@@ -28,10 +28,9 @@ __host__ __device__ inline size_t il_row(const ILGrid& G, uint32_t y, uint32_t z
 // consecutive groups' cells (TC = KG cells of a row, contiguous in the handle's
 // layout) x JT complex values (j = l C + s) per pass, staged in shared memory (TC x
 // (JT + 1) float2, the padding against bank conflicts) so that both sides are read
-// and written in contiguous 16-byte runs.  KG is as many groups as keep a thread's
-// share of a tile within kIlConvLoads 16-byte loads (for J = 36, spin-1 BCC, three
-// groups of 32 cells: one group per pass left 2 loads per thread and ran at half
-// the copy rate).  aos: the slot's interior pointer.  J = V C and JT are even (every
+// and written in contiguous 16-byte runs.  The tile keeps a thread's share within
+// kIlConvLoads 16-byte loads (for J = 36, spin-1 BCC, three groups of 32 cells: one
+// group per pass left 2 loads per thread and ran at half the copy rate).  aos: the slot's interior pointer.  J = V C and JT are even (every
 // lattice with 4 entries per node has an even node count), so a cell's values and
 // the tiles start on 16-byte boundaries.  Each thread issues all its loads of a
 // tile before it stores any of them.  The interleaved halo rows and padding cells
@@ -44,6 +43,7 @@ __global__ void __launch_bounds__(kIlConvThreads, 4) il_convert_kernel(char* aos
                                                                     uint32_t tiles, FastDiv djt, FastDiv dgx,
                                                                     FastDiv dy) {
     extern __shared__ float2 il_tile[];  // TC x (JT + 1)
+    let_next_kernel_in();
     const uint32_t J = G.V * G.C;
     const uint32_t cells = G.cells;
     const uint32_t TC = KG * cells, htc = TC / 2;
@@ -135,6 +135,9 @@ __global__ void __launch_bounds__(kIlConvThreads, 4) il_convert_kernel(char* aos
         }
         __syncthreads();
     }
+    // a launch beside the one before it ends after that one, so that what follows may
+    // count on both
+    after_previous_kernel<false>();
 }
 
 // A neighbour in the interleaved layout, for cell `sub` of a group (the lane's cell in
@@ -717,19 +720,46 @@ cudaError_t launch_il_hyper(const StepArgs& a, const ILGrid& G, const ILGrid& Gq
     return cudaGetLastError();
 }
 
+// The tile of a layout change: KG groups x JT values with as few idle slots of the
+// threads' loads as can be (kIlConvLoads each, and 1024 cells): whole rows of cells
+// where they fit, runs of at least 32 values (256 bytes of the handle's layout).  Taking
+// as many groups as fit first left a row of five groups in tiles of four and one.
+struct IlTile {
+    uint32_t KG, JT;
+};
+inline IlTile il_convert_tile(const ILGrid& G) {
+    const uint32_t J = G.V * G.C, most = 2 * kIlConvLoads * kIlConvThreads;
+    IlTile best = {1, 2};
+    uint64_t slots = ~0ull;
+    for (uint32_t KG = 1; KG <= G.GX && KG * G.cells <= 1024; ++KG) {
+        uint32_t JT = std::min(J, most / (KG * G.cells) & ~1u);
+        if (JT < std::min(J, 32u)) break;
+        const uint32_t jt = (J + JT - 1) / JT, gt = (G.GX + KG - 1) / KG;
+        if (jt > 1) JT = ((J + jt - 1) / jt + 1) & ~1u;
+        const uint32_t k = (G.GX + gt - 1) / gt;
+        const uint64_t n = (uint64_t)jt * gt;
+        if (n <= slots) {
+            slots = n;
+            best = {k, JT};
+        }
+    }
+    return best;
+}
+
 // Both directions of the layout change for one state buffer (interior pointer aos).
+// beside: the launch may run beside the layout change launched before it, of other
+// buffers (a change of a small state is as long as its launch's ramp and tail).
 // Defined once (GPE_DEFINE_IL_CONVERT in one translation unit).
-cudaError_t launch_il_convert(char* aos, const Grid& g, char* il, const ILGrid& G, bool to_il, cudaStream_t s);
+cudaError_t launch_il_convert(char* aos, const Grid& g, char* il, const ILGrid& G, bool to_il, bool beside, cudaStream_t s);
 
 #define GPE_DEFINE_IL_CONVERT                                                                                        \
-    cudaError_t launch_il_convert(char* aos, const Grid& g, char* il, const ILGrid& G, bool to_il, cudaStream_t s) { \
+    cudaError_t launch_il_convert(char* aos, const Grid& g, char* il, const ILGrid& G, bool to_il, bool beside,      \
+                                  cudaStream_t s) {                                                                  \
         const uint32_t J = G.V * G.C;                                                                                \
         if (J % 2 || g.cell_bytes != J * 8) return cudaErrorInvalidValue;                                            \
-        const uint32_t JT = J < 128 ? J : 128;                                                                       \
+        const IlTile t = il_convert_tile(G);                                                                         \
+        const uint32_t JT = t.JT, KG = t.KG;                                                                         \
         const uint32_t jtiles = (J + JT - 1) / JT;                                                                   \
-        /* groups per tile: TC JT <= 2 kIlConvLoads kIlConvThreads values, TC <= 1024 cells */                       \
-        uint32_t KG = std::min<uint32_t>(2 * kIlConvLoads * kIlConvThreads / (G.cells * JT), 1024 / G.cells);      \
-        KG = std::max<uint32_t>(1, std::min<uint32_t>(KG, G.GX));                                                   \
         const uint32_t GXT = (G.GX + KG - 1) / KG;                                                                   \
         const uint64_t tiles = (uint64_t)G.Y * G.Z * GXT * jtiles;                                                   \
         if (tiles == 0) return cudaSuccess;                                                                          \
@@ -737,12 +767,11 @@ cudaError_t launch_il_convert(char* aos, const Grid& g, char* il, const ILGrid& 
         const size_t smem = (size_t)KG * G.cells * (JT + 1) * sizeof(float2);                                        \
         const unsigned nb = (unsigned)std::min<uint64_t>(tiles, (uint64_t)device_sm_count() * 8);                    \
         const FastDiv djt = make_fastdiv(jtiles), dgx = make_fastdiv(GXT), dy = make_fastdiv(G.Y);                   \
-        if (to_il)                                                                                                   \
-            il_convert_kernel<true><<<nb, kIlConvThreads, smem, s>>>(aos, g, il, G, JT, KG, GXT, jtiles, (uint32_t)tiles, \
-                                                                     djt, dgx, dy);                                  \
-        else                                                                                                         \
-            il_convert_kernel<false><<<nb, kIlConvThreads, smem, s>>>(aos, g, il, G, JT, KG, GXT, jtiles,            \
-                                                                      (uint32_t)tiles, djt, dgx, dy);                \
+        auto k = to_il ? il_convert_kernel<true> : il_convert_kernel<false>;                                         \
+        if (beside)                                                                                                  \
+            return launch_overlapped(k, nb, kIlConvThreads, smem, s, aos, g, il, G, JT, KG, GXT, jtiles,             \
+                                     (uint32_t)tiles, djt, dgx, dy);                                                 \
+        k<<<nb, kIlConvThreads, smem, s>>>(aos, g, il, G, JT, KG, GXT, jtiles, (uint32_t)tiles, djt, dgx, dy);       \
         return cudaGetLastError();                                                                                   \
     }
 

@@ -152,9 +152,10 @@ __device__ __forceinline__ void st_node(char* p, const Cx<R>* v) {
 // 40.6 us, split C15 36^3 194 / 199, scalar BCC 32^3 3.97 / 3.85; interleaved kernels
 // (no tables to stage) equal or slower, imaginary time 2 % slower.  (Deciding it by the
 // grid's size inside the kernel cost 10-25 % of the scalar steps.)
+__device__ __forceinline__ void let_next_kernel_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <bool LET_IN>
 __device__ __forceinline__ void after_previous_kernel() {
-    if constexpr (LET_IN) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if constexpr (LET_IN) let_next_kernel_in();
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
