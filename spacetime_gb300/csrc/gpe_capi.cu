@@ -63,6 +63,12 @@ cudaError_t launch_il_step_from(const StepArgs& a, const ILGrid& G, int deg, siz
 template <int C>
 unsigned il_blocks(const ILGrid& G, int deg, bool obs, size_t max_blocks);
 cudaError_t launch_il_convert(char* aos, const Grid& g, char* il, const ILGrid& G, bool to_il, bool beside, cudaStream_t s);
+cudaError_t launch_split_planes(const StepArgs& a, int part, char* const planes[4], const Grid& g, const int32_t* tab,
+                                cudaStream_t s);
+cudaError_t launch_split_planes_convert(char* psi, char* q, char* const planes[4], const Grid& g, bool to_planes, cudaStream_t s);
+size_t split_plane_bytes(const Grid& g, bool q);
+bool split_planes_fit(const Grid& g);
+bool split_plane_table(const Grid& g, const gpe_incidence* inc, const gpe_edge* edges, std::vector<int32_t>& tab);
 template <int C>
 cudaError_t launch_il_hyper(const StepArgs& a, const ILGrid& G, const ILGrid& Gq, const int32_t* tab, cudaStream_t s);
 enum HyperKind {
@@ -219,6 +225,9 @@ static void release(gpe_handle* h) {
     for (char* b : h->ilq)
         if (b) cudaFree(b);
     if (h->il_htab) cudaFree(h->il_htab);
+    for (char* b : h->planes)
+        if (b) cudaFree(b);
+    if (h->plane_tab) cudaFree(h->plane_tab);
     if (h->tev_ok)
         for (cudaEvent_t ev : h->tev) cudaEventDestroy(ev);
     adjoint_release(h);
@@ -1179,8 +1188,15 @@ extern "C" gpe_status gpe_start(gpe_handle* h, void* stream) {
     return GPE_OK;
 }
 
-// n steps in the handle's layout.
+// Calls shorter than this stay in the handle's layout: the two layout changes in
+// and the two out cost about as much as two steps.
+constexpr int32_t kIlMinSteps = 16;
+static bool split_planes_ready(gpe_handle* h, int32_t n, cudaStream_t s);
+static gpe_status split_plane_steps(gpe_handle* h, int32_t n, cudaStream_t s);
+
+// n steps of the handle's own kernels (not the interleaved psi and q slots of il_steps).
 static gpe_status plain_steps(gpe_handle* h, int32_t n, cudaStream_t s) {
+    if (split_planes_ready(h, n, s)) return split_plane_steps(h, n, s);
     if (h->p.scheme == GPE_SCHEME_SPLIT) {
         // update_psi(I) + update_q(q_I), then update_psi(R) + update_q(q_R)
         // (RelativisticGpeC15/GPUGrossPitaevskii_C15.cu:477-482), one launch each
@@ -1244,9 +1260,6 @@ struct StepTimer {
 
 // ---------------------------------------------------------- interleaved steps
 
-// Calls shorter than this stay in the handle's layout: the two layout changes in
-// and the two out cost about as much as two steps.
-constexpr int32_t kIlMinSteps = 16;
 
 // Rows the interleaved kernel takes: 4 entries in every row (BCC, A15, C15, Z), or
 // rows of 4 and 8 (FCC), every neighbour in an adjacent cell (|dx|, |dy|, |dz| <= 1);
@@ -1402,6 +1415,72 @@ static gpe_status ensure_il_hyper(gpe_handle* h, cudaStream_t s) {
     }
     h->il_htab = static_cast<int32_t*>(p);
     CUDA_TRY(cudaMemcpy(p, tab.data(), tab.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
+    return GPE_OK;
+}
+
+// Whether a split-scheme call of n steps runs on interleaved planes (gpe_split.cuh): FP32,
+// the automatic kernel choice, calls long enough for the layout changes (one change
+// in and one out cost about one step), 4 edges per node and 2 per node of a cell within
+// adjacent cells, and the planes' memory to be had now (twice the state's; not while the
+// stream is being captured, which takes no allocation).
+static bool split_planes_ready(gpe_handle* h, int32_t n, cudaStream_t s) {
+    const Grid& g = h->g;
+    if (h->p.scheme != GPE_SCHEME_SPLIT || h->real_bytes != 4 || h->tune_kernel != 0 || n < kIlMinSteps) return false;
+    if (h->plane_tab) return true;
+    if (h->lat.F != 4 || g.E != 2 * g.V || !split_planes_fit(g)) return false;
+    auto adj = [](int dx, int dy, int dz) { return dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1 && dz >= -1 && dz <= 1; };
+    for (const gpe_edge& e : h->lat.edges)
+        if (!adj(e.dx, e.dy, e.dz)) return false;
+    for (const gpe_incidence& r : h->lat.incidence)
+        if (!adj(r.dx, r.dy, r.dz)) return false;
+    std::vector<int32_t> tab;
+    if (!split_plane_table(g, h->lat.incidence.data(), h->lat.edges.data(), tab)) return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+    void* t = nullptr;
+    bool ok = cudaMalloc(&t, tab.size() * sizeof(int32_t)) == cudaSuccess &&
+              cudaMemcpy(t, tab.data(), tab.size() * sizeof(int32_t), cudaMemcpyHostToDevice) == cudaSuccess;
+    for (int k = 0; k < 4 && ok; ++k) {
+        const size_t bytes = split_plane_bytes(g, k >= 2);
+        void* p = nullptr;
+        ok = cudaMalloc(&p, bytes) == cudaSuccess;
+        h->planes[k] = static_cast<char*>(p);
+        // the halo rows and the padding cells stay zero
+        ok = ok && cudaMemsetAsync(p, 0, bytes, s) == cudaSuccess;
+    }
+    if (!ok) {
+        cudaGetLastError();
+        for (char*& p : h->planes) {
+            if (p) cudaFree(p);
+            p = nullptr;
+        }
+        if (t) cudaFree(t);
+        return false;
+    }
+    h->plane_tab = static_cast<int32_t*>(t);
+    return true;
+}
+
+// n steps of the split scheme on the planes: psi and q changed in, two half-step
+// launches per step, changed back.
+static gpe_status split_plane_steps(gpe_handle* h, int32_t n, cudaStream_t s) {
+    char *psi = h->interior[GPE_PSI_EVEN], *q = h->interior[GPE_Q_EVEN];
+    cudaError_t e = launch_split_planes_convert(psi, q, h->planes, h->g, true, s);
+    if (e != cudaSuccess) return cuda_fail(e, "layout change (in)");
+    gpe_fields zero;
+    std::memset(&zero, 0, sizeof zero);
+    for (int32_t k = 0; k < n; ++k) {
+        const StepArgs a = make_args(h, zero, h->t0 + (double)(h->nstep + 1) * h->p.dt);
+        for (int part = 0; part < 2; ++part)
+            if ((e = launch_split_planes(a, part, h->planes, h->g, h->plane_tab, s)) != cudaSuccess)
+                return cuda_fail(e, "split-scheme launch");
+        h->launches += 2;
+        h->epoch += 1;
+        h->nstep++;
+    }
+    e = launch_split_planes_convert(psi, q, h->planes, h->g, false, s);
+    if (e != cudaSuccess) return cuda_fail(e, "layout change (out)");
+    h->launches += 4;
     return GPE_OK;
 }
 

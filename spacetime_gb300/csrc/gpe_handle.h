@@ -95,6 +95,9 @@ struct gpe_handle {
     char* ilq[2] = {nullptr, nullptr};
     gpe::ILGrid ilgq{};
     int32_t* il_htab = nullptr;
+    // split-scheme handles: the interleaved planes R, I, q_R, q_I and their offset table
+    char* planes[4] = {nullptr, nullptr, nullptr, nullptr};
+    int32_t* plane_tab = nullptr;
     // device timing of gpe_step / gpe_step_observe calls (GPE_TUNE_TIMING)
     int tune_timing = 0;
     bool tev_ok = false;

@@ -1818,15 +1818,15 @@ __global__ void __launch_bounds__(256) split_step_kernel(StepArgs a, uint32_t no
 #pragma unroll
             for (int k = 0; k < 4; ++k) qv[k] = *reinterpret_cast<const R*>(qb + off[k]);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) d1q += w[k] * qv[k];
+            for (int k = 0; k < 4; ++k) d1q = fm(w[k], qv[k], d1q);
         } else {
-            for (int k = 0; k < F; ++k) d1q += sh.inc_w[l * F + k] * *reinterpret_cast<const R*>(qb + sh.inc_off[l * F + k]);
+            for (int k = 0; k < F; ++k) d1q = fm(sh.inc_w[l * F + k], *reinterpret_cast<const R*>(qb + sh.inc_off[l * F + k]), d1q);
         }
         R r[3];
         node_pos(P, x, y, z, sh.pos + 3 * l, r);
-        const R tp = trap<R>(P, r) + P.c0 * (v.x * v.x + v.y * v.y);
-        if constexpr (PART == 0) *reinterpret_cast<R*>(own + wr) = v.y - P.dt * (tp * v.x - d1q);
-        else *reinterpret_cast<R*>(own + wr) = v.x + P.dt * (tp * v.y - d1q);
+        const R tp = fm(P.c0, norm_sq(v), trap<R>(P, r));
+        if constexpr (PART == 0) *reinterpret_cast<R*>(own + wr) = fm(-P.dt, fm(tp, v.x, -d1q), v.y);
+        else *reinterpret_cast<R*>(own + wr) = fm(P.dt, fm(tp, v.y, -d1q), v.x);
     } else {
         const uint32_t eb = (kNodes ? group * ratio : 0) + (sub - 1);
         const uint32_t i = eb * blockDim.x + threadIdx.x;
@@ -1843,9 +1843,9 @@ __global__ void __launch_bounds__(256) split_step_kernel(StepArgs a, uint32_t no
         const R d0 = *reinterpret_cast<const R*>(pb + sh.e_to[e]) - *reinterpret_cast<const R*>(pb + sh.e_from[e]);
         char* qe = a.qnext + qcell_off + e * 2 * sizeof(R);
         const R qr = *reinterpret_cast<const R*>(qe + rd);
-        if constexpr (PART == 0) *reinterpret_cast<R*>(qe + wr) += P.dts * (qr + d0);
-        else if constexpr (PART == 1) *reinterpret_cast<R*>(qe + wr) -= P.dts * (qr + d0);
-        else *reinterpret_cast<R*>(qe) = qr + qinit * (qr + d0);
+        if constexpr (PART == 0) *reinterpret_cast<R*>(qe + wr) = fm(P.dts, qr + d0, *reinterpret_cast<R*>(qe + wr));
+        else if constexpr (PART == 1) *reinterpret_cast<R*>(qe + wr) = fm(-P.dts, qr + d0, *reinterpret_cast<R*>(qe + wr));
+        else *reinterpret_cast<R*>(qe) = fm(qinit, qr + d0, qr);
     }
     }
 }
@@ -3027,3 +3027,4 @@ cudaError_t launch_hyper_tile(const StepArgs& a, uint32_t T, cudaStream_t s) {
 
 #include "gpe_slab.cuh"
 #include "gpe_il.cuh"
+#include "gpe_split.cuh"
