@@ -563,8 +563,8 @@ gpe_status gpe_adjoint_backward(gpe_handle* h, const double* seed, double* grad,
  *   `steps` steps of up to four of its members on scratch copies of their
  *   buffers, on a grid scaled so that each block has the work it has in the
  *   whole batch, for item sizes of 4K..256K nodes, and keeps the fastest; the
- *   members' states are untouched.  Within a step the blocks take items from
- *   one counter, so a block that finishes early takes more.
+ *   members' states are untouched.  Within a step the blocks take the last of
+ *   their items from one counter, so a block that finishes early takes more.
  *   `report` receives a JSON list of the timings.
  * An FP32 batch keeps its members' per-node constants in constant memory, one of
  * 256 slots per device and member, held until gpe_batch_destroy.  A batch created
@@ -581,7 +581,9 @@ typedef struct gpe_batch gpe_batch;
  * cell-interleaved layout of gpe_step's interleaved kernel -- each call changes
  * their two psi slots in and back (4 layout-change launches per member, in the
  * captured graph too) and the states are those of the gather form bit for bit;
- * 0: every member in its handle's layout.  Changing it drops a captured run. */
+ * 0: every member in its handle's layout.  Until the key is set, calls (and captured
+ * runs) of fewer than 11 steps stay in the handles' layout as well: the layout changes
+ * would cost them more than the steps gain.  Changing it drops a captured run. */
 enum {
     GPE_BATCH_ITEM_NODES = 0,
     GPE_BATCH_STEPS_PER_LAUNCH = 1,

@@ -83,6 +83,7 @@ struct BatchArgs {
     const BatchItem* items;
     unsigned* next_item;       // one counter per step of the launch (zeroed before it)
     uint32_t nmembers, nitems;
+    uint32_t own;              // turns of a step that are a block's own (the rest go by the counter)
     uint32_t nsteps;           // steps of this launch
     uint32_t step_base;        // steps of this call taken by earlier launches
     unsigned* bar;             // grid barrier: arrivals, generation
@@ -167,6 +168,13 @@ __device__ __forceinline__ void set_fields(PhysR<R>& P, const StepFieldsD& f) {
     }
     P.trap_on = f.trap_on;
 }
+
+// 16 bytes from global to shared memory, in flight until copies_landed().
+__device__ __forceinline__ void copy16_async(void* shared, const void* global) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(shared)), "l"(global)
+                 : "memory");
+}
+__device__ __forceinline__ void copies_landed() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // Rows row0 .. row0 + rows - 1 of a member.  K: the member's grid and divisors
 // (BatchMember in shared memory, or MemberConst in constant memory); P its
@@ -338,34 +346,54 @@ __global__ void __launch_bounds__(kBatchThreads, sizeof(R) == 8 ? 1 : (CMASK & 4
     __shared__ SmemTables<R> st;
     __shared__ PhysR<R> P;
     __shared__ BatchMember M;
-    __shared__ uint32_t grabbed;
+    // the loop's state, in shared memory: the node loops need the registers
+    __shared__ __align__(16) BatchItem now, ahead;
+    __shared__ uint32_t step, turn, loaded;
+    __shared__ int cur;
     const uint32_t gtid = blockIdx.x * kBatchThreads + threadIdx.x;
     const uint32_t gthreads = gridDim.x * kBatchThreads;
     for (uint32_t m = gtid; m < A.nmembers; m += gthreads) batch_fields(A, m, A.step_base, A.fields);
+    if (threadIdx.x == 0) step = 0;
     if (!grid_barrier(A.bar, A.err, A.expect, A.timeout_ns)) return;
-    for (uint32_t s = 0; s < A.nsteps; ++s) {
-        const uint32_t k = A.step_base + s;
-        const StepFieldsD* F = A.fields + (size_t)(s & 1) * A.nmembers;
-        uint32_t loaded = 0xffffffffu;
+    for (;;) {
+        // Items go out in list order.  A block's first turns of a step are its own (turn j:
+        // item j gridDim.x + blockIdx.x), their descriptions copied to shared memory while
+        // the turn before is worked on; the list's last full round and what is left over go
+        // by one counter per step, so blocks that finish early take more and the step ends
+        // within about one item.  24 members of 33M nodes, 40 steps: the last round 18.34 ms,
+        // the last two 18.43, every item by the counter 18.53; with every thread holding the
+        // loop's state in registers and a counter for all 18.56 (28 bytes of spills).
+        if (threadIdx.x == 0) {
+            turn = 0;
+            loaded = 0xffffffffu;
+            if (A.own > 0) copy16_async(&ahead, A.items + blockIdx.x);
+        }
         for (;;) {
-            // items are handed out in list order by one counter per step, so blocks
-            // that finish early take more and the step ends within about one item
-            if (threadIdx.x == 0) grabbed = atomicAdd(A.next_item + s, 1u);
+            __syncthreads();  // every warp is done with the turn before
+            if (threadIdx.x == 0) {
+                const uint32_t j = turn++;
+                if (j < A.own) {
+                    copies_landed();
+                    now = ahead;
+                    if (j + 1 < A.own) copy16_async(&ahead, A.items + (j + 1) * gridDim.x + blockIdx.x);
+                } else {
+                    const uint32_t it = A.own * gridDim.x + atomicAdd(A.next_item + step, 1u);
+                    now = it < A.nitems ? A.items[it] : BatchItem{0, 0, 0, 0};
+                }
+            }
             __syncthreads();
-            const uint32_t it = grabbed;
-            __syncthreads();  // every thread has read `grabbed` before thread 0 rewrites it
-            if (it >= A.nitems) break;
-            const BatchItem w = A.items[it];
+            const BatchItem w = now;
+            if (w.rows == 0) break;
             // items of one member share the staged tables: the block synchronises
             // only where the member changes (w.member is the same in every thread)
             if (w.member != loaded) {
-                __syncthreads();  // every warp is done with the previous member's tables
                 // the member's description, a word per thread (one thread copying its 1.5 KB
                 // held the block for some 3 us)
                 static_assert(sizeof(BatchMember) % 4 == 0, "copied in words");
                 const uint32_t* src = reinterpret_cast<const uint32_t*>(A.members + w.member);
                 for (uint32_t i = threadIdx.x; i < sizeof(BatchMember) / 4; i += kBatchThreads)
                     reinterpret_cast<uint32_t*>(&M)[i] = src[i];
+                if (threadIdx.x == 0) cur = A.state[w.member].cur;
                 __syncthreads();
                 const int V = M.g.V, nent = M.tab.entries;
                 for (int i = threadIdx.x; i <= V; i += kBatchThreads) st.row_ptr[i] = M.tab.row_ptr[i];
@@ -387,11 +415,13 @@ __global__ void __launch_bounds__(kBatchThreads, sizeof(R) == 8 ? 1 : (CMASK & 4
                     for (uint32_t i = threadIdx.x; i < sizeof(P) / 4; i += kBatchThreads) reinterpret_cast<uint32_t*>(&P)[i] = ph[i];
                     __syncthreads();
                 }
-                if (threadIdx.x == 0) set_fields<R>(P, F[w.member]);
-                loaded = w.member;
+                if (threadIdx.x == 0) {
+                    set_fields<R>(P, A.fields[(size_t)(step & 1) * A.nmembers + w.member]);
+                    loaded = w.member;
+                }
                 __syncthreads();
             }
-            const int prev_slot = A.state[w.member].cur ^ (int)(k & 1);
+            const int prev_slot = cur ^ (int)((A.step_base + step) & 1);
             const char* prev = M.psi[prev_slot];
             char* next = M.psi[prev_slot ^ 1];
             if constexpr (CONSTP) {
@@ -401,11 +431,13 @@ __global__ void __launch_bounds__(kBatchThreads, sizeof(R) == 8 ? 1 : (CMASK & 4
                 batch_item<R, CMASK, IL>(M, M, st, P, nullptr, prev, next, w.row0, w.rows);
             }
         }
-        if (s + 1 < A.nsteps) {
-            StepFieldsD* G = A.fields + (size_t)((s + 1) & 1) * A.nmembers;
-            for (uint32_t m = gtid; m < A.nmembers; m += gthreads) batch_fields(A, m, k + 1, G);
+        const uint32_t done = step + 1;
+        if (done < A.nsteps) {
+            StepFieldsD* G = A.fields + (size_t)(done & 1) * A.nmembers;
+            for (uint32_t m = gtid; m < A.nmembers; m += gthreads) batch_fields(A, m, A.step_base + done, G);
         }
-        if (!grid_barrier(A.bar, A.err, A.expect, A.timeout_ns)) return;
+        if (!grid_barrier(A.bar, A.err, A.expect, A.timeout_ns) || done == A.nsteps) return;
+        if (threadIdx.x == 0) step = done;
     }
 }
 
@@ -486,6 +518,7 @@ struct gpe_batch {
     int32_t barrier_timeout_ms = 10000;
     int32_t extra_arrivals = 0;       // test hook: the barrier waits for arrivals that never come
     BatchMember* d_members = nullptr;
+    BatchMember* d_handle_members = nullptr;  // the same, every member in the handle's layout
     BatchState* d_state = nullptr;
     BatchState* h_state = nullptr;   // pinned
     StepFieldsD* d_fields = nullptr;
@@ -498,12 +531,14 @@ struct gpe_batch {
     int* d_err = nullptr;
     std::vector<int> cslots;         // FP32: one constant-memory slot per member, or none
     int32_t layout = 1;              // GPE_BATCH_LAYOUT
+    bool layout_set = false;         // GPE_BATCH_LAYOUT was set
     std::vector<int> il_deg;         // per member: 0, or the interleaved rows (4 or 8)
     std::vector<void*> il_off;       // per member: device interleaved entry offsets, or null
     bool any_il = false;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int32_t graph_steps = 0;
+    bool graph_il = false;           // the captured run changes layouts
     uint64_t launches = 0;
 };
 
@@ -563,7 +598,7 @@ int member_il_deg(const gpe_batch* b, const gpe_handle* h) {
 // Every member's BatchMember (constants, layout, constant-memory slot) into d_members.
 gpe_status upload_members(gpe_batch* b) {
     const size_t n = b->members.size();
-    std::vector<BatchMember> hm(n);
+    std::vector<BatchMember> hm(n), plain(n);
     b->il_deg.assign(n, 0);
     b->il_off.resize(n, nullptr);
     b->any_il = false;
@@ -571,6 +606,7 @@ gpe_status upload_members(gpe_batch* b) {
         gpe_handle* h = b->members[i];
         member_constants(h, hm[i]);
         if (!b->cslots.empty()) hm[i].cslot = b->cslots[i];
+        plain[i] = hm[i];
         const int deg = member_il_deg(b, h);
         const std::vector<int32_t> offs = deg ? il_offsets(h) : std::vector<int32_t>();
         if (deg && !offs.empty()) {
@@ -590,6 +626,7 @@ gpe_status upload_members(gpe_batch* b) {
         }
     }
     cudaError_t e = cudaMemcpy(b->d_members, hm.data(), n * sizeof(BatchMember), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(b->d_handle_members, plain.data(), n * sizeof(BatchMember), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(e, "batch members upload");
     return GPE_OK;
 }
@@ -618,6 +655,15 @@ uint64_t convert_launch_count(const gpe_batch* b) {
 
 // A lattice is told apart by its node and stencil-entry counts per cell.
 uint64_t lattice_key(const gpe_handle* h) { return ((uint64_t)h->g.V << 32) | (uint32_t)h->tab.entries; }
+
+// Calls of fewer steps leave every member in the handle's layout unless GPE_BATCH_LAYOUT
+// was set: a step costs the interleaved members less, but their states go in and out once
+// a call.  24 members of 33M nodes, half of the nodes in such members: 2 steps 1.02 ms (1.63
+// interleaved), 10 steps 4.89 (5.15), 20 steps 9.7 (9.6), 40 steps 19.4 (18.3).  Batches of
+// one lattice break even at 9 steps (11 x FCC 56^3), 13 (11 x BCC 56^3), 15 to 19 (8 x FCC or
+// BCC 40^3, 9 x A15 24^3) and, launch bound, 31 (36 x BCC 24^3).
+constexpr int32_t kIlBatchSteps = 11;
+bool call_is_il(const gpe_batch* b, int32_t n) { return b->any_il && (b->layout_set || n >= kIlBatchSteps); }
 
 // Nodes per work item: the autotuner's choice for the lattice, else the set size, else
 // what gives every block kItemsPerBlock items a step, at most 16384.  With three items
@@ -710,10 +756,14 @@ gpe_status fill_state(gpe_batch* b) {
 }
 
 gpe_status grid_size(gpe_batch* b) {
-    void* fn = batch_kernel_for(b->precision, b->cmask, !b->cslots.empty(), b->any_il);
     int occ = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kBatchThreads, 0);
-    if (e != cudaSuccess) return batch_fail_cuda(e, "occupancy of the batch kernel");
+    for (int il = 0; il <= (b->any_il ? 1 : 0); ++il) {
+        int o = 0;
+        void* fn = batch_kernel_for(b->precision, b->cmask, !b->cslots.empty(), il != 0);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, fn, kBatchThreads, 0);
+        if (e != cudaSuccess) return batch_fail_cuda(e, "occupancy of the batch kernel");
+        occ = il ? std::min(occ, o) : o;
+    }
     if (occ < 1) return fail(GPE_ERR_UNSUPPORTED, "the batch kernel does not fit on an SM");
     b->blocks_per_sm = occ;
     const int per = b->tune_blocks_per_sm > 0 ? std::min<int>(b->tune_blocks_per_sm, occ) : occ;
@@ -722,16 +772,16 @@ gpe_status grid_size(gpe_batch* b) {
 }
 
 // Enqueues n steps of every member: the state upload, the interleaved members'
-// layout change in (convert), ceil(n / K) persistent launches, and the layout
-// change back.  Capturable into a CUDA graph (the state copy reads the pinned host
+// layout change in (convert), ceil(n / K) persistent launches (il: some of the members
+// passed are interleaved), and the layout change back.  Capturable into a CUDA graph (the state copy reads the pinned host
 // array when the graph runs).
 gpe_status enqueue_steps(gpe_batch* b, int32_t n, cudaStream_t s, const BatchMember* members, uint32_t nmembers,
-                         const BatchState* h_state, int grid, bool convert) {
+                         const BatchState* h_state, int grid, bool il, bool convert) {
     cudaError_t e = cudaMemcpyAsync(b->d_state, h_state, nmembers * sizeof(BatchState), cudaMemcpyHostToDevice, s);
     if (e != cudaSuccess) return batch_fail_cuda(e, "batch state upload");
     if (convert)
         if (gpe_status st = convert_members(b, true, s)) return st;
-    void* fn = batch_kernel_for(b->precision, b->cmask, !b->cslots.empty(), b->any_il);
+    void* fn = batch_kernel_for(b->precision, b->cmask, !b->cslots.empty(), il);
     const int32_t K = std::min(b->steps_per_launch > 0 ? b->steps_per_launch : n, kMaxStepsPerLaunch);
     for (int32_t done = 0; done < n; done += K) {
         const int32_t steps = std::min(K, n - done);
@@ -746,6 +796,8 @@ gpe_status enqueue_steps(gpe_batch* b, int32_t n, cudaStream_t s, const BatchMem
         A.next_item = b->d_next;
         A.nmembers = nmembers;
         A.nitems = b->nitems;
+        const uint32_t rounds = b->nitems / (uint32_t)grid;
+        A.own = rounds > 1 ? rounds - 1 : 0;
         A.nsteps = (uint32_t)steps;
         A.step_base = (uint32_t)done;
         A.bar = b->d_bar;
@@ -798,6 +850,7 @@ void release_batch(gpe_batch* b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
     if (b->d_members) cudaFree(b->d_members);
+    if (b->d_handle_members) cudaFree(b->d_handle_members);
     if (b->d_state) cudaFree(b->d_state);
     if (b->h_state) cudaFreeHost(b->h_state);
     if (b->d_fields) cudaFree(b->d_fields);
@@ -876,6 +929,7 @@ extern "C" gpe_status gpe_batch_create(gpe_handle* const* members, int32_t count
         }
     }
     if (cudaMalloc(&b->d_members, count * sizeof(BatchMember)) != cudaSuccess ||
+        cudaMalloc(&b->d_handle_members, count * sizeof(BatchMember)) != cudaSuccess ||
         cudaMalloc(&b->d_state, count * sizeof(BatchState)) != cudaSuccess ||
         cudaMallocHost(&b->h_state, count * sizeof(BatchState)) != cudaSuccess ||
         cudaMalloc(&b->d_fields, 2 * (size_t)count * sizeof(StepFieldsD)) != cudaSuccess ||
@@ -915,7 +969,9 @@ extern "C" gpe_status gpe_batch_step(gpe_batch* b, int32_t n, void* stream) {
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return cuda_fail(e, "batch step");
     if (gpe_status st = fill_state(b)) return st;
-    gpe_status st = enqueue_steps(b, n, s, b->d_members, (uint32_t)b->members.size(), b->h_state, b->grid, true);
+    const bool il = call_is_il(b, n);
+    gpe_status st = enqueue_steps(b, n, s, il ? b->d_members : b->d_handle_members, (uint32_t)b->members.size(), b->h_state,
+                                  b->grid, il, il);
     if (st) return st;
     advance_members(b, n);
     return check_batch_error(b, s);
@@ -934,7 +990,9 @@ extern "C" gpe_status gpe_batch_capture(gpe_batch* b, int32_t n, void* stream) {
     cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_fail(e, "cudaStreamBeginCapture");
     const uint64_t launches = b->launches;
-    gpe_status st = enqueue_steps(b, n, s, b->d_members, (uint32_t)b->members.size(), b->h_state, b->grid, true);
+    const bool il = call_is_il(b, n);
+    gpe_status st = enqueue_steps(b, n, s, il ? b->d_members : b->d_handle_members, (uint32_t)b->members.size(), b->h_state,
+                                  b->grid, il, il);
     b->launches = launches;
     cudaGraph_t g = nullptr;
     e = cudaStreamEndCapture(s, &g);
@@ -950,6 +1008,7 @@ extern "C" gpe_status gpe_batch_capture(gpe_batch* b, int32_t n, void* stream) {
     }
     b->graph = g;
     b->graph_steps = n;
+    b->graph_il = il;
     return GPE_OK;
 }
 
@@ -963,7 +1022,7 @@ extern "C" gpe_status gpe_batch_replay(gpe_batch* b, void* stream) {
     e = cudaGraphLaunch(b->exec, s);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGraphLaunch");
     const int32_t K = std::min(b->steps_per_launch > 0 ? b->steps_per_launch : b->graph_steps, kMaxStepsPerLaunch);
-    b->launches += (uint64_t)((b->graph_steps + K - 1) / K) + convert_launch_count(b);
+    b->launches += (uint64_t)((b->graph_steps + K - 1) / K) + (b->graph_il ? convert_launch_count(b) : 0);
     advance_members(b, b->graph_steps);
     return check_batch_error(b, s);
 }
@@ -999,6 +1058,7 @@ extern "C" gpe_status gpe_batch_set_tuning(gpe_batch* b, int32_t key, int32_t va
     }
     if (key == GPE_BATCH_LAYOUT) {
         if (value < 0 || value > 1) return fail(GPE_ERR_INVALID_ARG, "batch layout (0 or 1)");
+        b->layout_set = true;
         if (value == b->layout) return GPE_OK;
         cudaError_t e = cudaDeviceSynchronize();
         if (e != cudaSuccess) return cuda_fail(e, "batch layout");
@@ -1124,12 +1184,12 @@ extern "C" gpe_status gpe_batch_autotune(gpe_batch* b, int32_t steps, char* repo
             // as many blocks as give each the work a block has in the whole batch
             const double share = (double)b->item_cost.back() / (double)full_cost;
             const int tgrid = std::max(1, std::min(b->grid, (int)std::lround(share * b->grid)));
-            if (enqueue_steps(b, 1, s, dm, (uint32_t)which.size(), ps, tgrid, false) != GPE_OK) {
+            if (enqueue_steps(b, 1, s, dm, (uint32_t)which.size(), ps, tgrid, b->any_il, false) != GPE_OK) {
                 ok = false;
                 break;
             }
             cudaEventRecord(e0, s);
-            gpe_status st = enqueue_steps(b, steps, s, dm, (uint32_t)which.size(), ps, tgrid, false);
+            gpe_status st = enqueue_steps(b, steps, s, dm, (uint32_t)which.size(), ps, tgrid, b->any_il, false);
             cudaEventRecord(e1, s);
             if (st != GPE_OK || cudaEventSynchronize(e1) != cudaSuccess) {
                 ok = false;
