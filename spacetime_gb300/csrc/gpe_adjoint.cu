@@ -501,6 +501,7 @@ template <typename R, int C>
 __global__ void __launch_bounds__(256) adjoint_final_kernel(StepArgs a) {
     using A = ObsArith<R>;
     typename A::S s[kFinalCount] = {}, f6[2] = {};
+    typename A::E re_sum{}, fz{};   // of one sign where T is near u, and in polarised clouds
     for (uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < a.total;
          gid += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t x, y, z, l;
@@ -512,7 +513,8 @@ __global__ void __launch_bounds__(256) adjoint_final_kernel(StepArgs a) {
         ld_node<R, C, true>(a.next + off, p);
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            A::add(s[0], A::dot2(t[c].x, p[c].x, t[c].y, p[c].y));
+            A::add_prod(re_sum, t[c].x, p[c].x);
+            A::add_prod(re_sum, t[c].y, p[c].y);
             A::add(s[1], A::cross2(t[c].x, p[c].y, t[c].y, p[c].x));
         }
         if constexpr (C > 1) {
@@ -525,19 +527,21 @@ __global__ void __launch_bounds__(256) adjoint_final_kernel(StepArgs a) {
             if constexpr (C == 3) {
                 A::add(s[2], re);
                 A::add(s[3], im);
-                A::add(s[4], n.n[0] - n.n[2]);
+                A::add(fz, n.template fz<0>());
             } else {
                 A::add(f6[0], re);
                 A::add(f6[1], im);
                 A::add(s[2], A::dot2(p[0].x, p[1].x, p[0].y, p[1].y) + A::dot2(p[3].x, p[4].x, p[3].y, p[4].y));
                 A::add(s[3], A::cross2(p[0].x, p[1].y, p[0].y, p[1].x) + A::cross2(p[3].x, p[4].y, p[3].y, p[4].x));
-                A::add(s[4], twice(n.n[0] - n.n[4]) + (n.n[1] - n.n[3]));
+                A::add(fz, n.template fz<0>());
             }
         }
     }
     double v[kFinalCount];
 #pragma unroll
     for (int k = 0; k < kFinalCount; ++k) v[k] = A::value(s[k]);
+    v[0] = A::value(re_sum);
+    v[4] = A::value(fz);
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         if constexpr (C == 3) v[2 + k] *= GPE_REF_SQRT_2;

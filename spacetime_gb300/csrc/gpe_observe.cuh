@@ -10,10 +10,15 @@
 //    per-node terms and multiplied in once per column, in FP64;
 //  - the per-node terms, products of stored values alone, are exact pairs of FP32
 //    values for FP32 storage (two-products and two-sums: Dekker 1971, Knuth; the
-//    sums are PairSum's), plain FP64 for FP64 storage.
+//    sums are PairSum's and, for terms of one sign, TripleSum's), plain FP64 for FP64
+//    storage.
 // A pair keeps 47 bits or more of each node's term, and the errors of different nodes
-// are independent, so that the sums carry the error of their FP64 additions: measured
-// against sums in 64 bits and more, 1e-16 to 1e-15 of the energy, as observe_kernel's.
+// are independent, so that the sums carry the error of their FP64 additions.  Measured
+// against sums in more than 64 bits on Thomas-Fermi clouds and noise (BCC 12^3 .. 24^3,
+// C15 9^3; root mean square, relative): norm 1e-16 to 2.5e-16, centre of mass 1e-16 to
+// 3e-16, energy 1e-16 to 3e-16, M_z 1e-16 to 2e-16, |F| 1e-16 -- observe_kernel's are 1e-16
+// to 2.5e-16, 1e-16 to 2.5e-16, 1e-16 to 3e-16, 1e-16 to 6e-16 and 1e-16 (spin-1, whose sqrt2
+// it takes from the reference's constant, 1e-15 to 3e-15).
 #pragma once
 
 namespace gpe {
@@ -59,12 +64,24 @@ __device__ __forceinline__ Pair twice(Pair a) {
     a.l = __fadd_rn(a.l, a.l);
     return a;
 }
-// Newton's step from the correctly rounded root: what it leaves out is below 2^-51.
+// a^2 with the term l^2, which a product of two pairs may leave out (its sign is random
+// there) but which has the same sign in every square: 6e-16 of the sum of squares.  Half
+// of it goes into h l, which is doubled exactly; added later it would fall to the rounding.
+__device__ __forceinline__ Pair square(Pair a) {
+    const Pair p = two_prod(a.h, a.h);
+    const float hl = __fmaf_rn(a.l, a.h, __fmul_rn(__fmul_rn(0.5f, a.l), a.l));
+    return pair_norm(p.h, __fmaf_rn(2.f, hl, p.l));
+}
+// sqrt(a) = s + d + d^2 / (2 sqrt(a)) + ..., s the correctly rounded root of the high word and
+// d = (a - s^2) / (2 sqrt(a)).  With i = 1 / (2 sqrt(a.h)) for the reciprocal the terms of
+// second order are i d (d - 2 i a.l): 5e-16 on average and always of one sign, so they are
+// added before the rounding of d.
 __device__ __forceinline__ Pair square_root(Pair a) {
     if (!(a.h > 0.f)) return Pair{a.h, 0.f};
-    const float s = __fsqrt_rn(a.h);
-    const float r = __fadd_rn(__fmaf_rn(-s, s, a.h), a.l);   // a - s^2
-    return pair_norm(s, __fmul_rn(__fmul_rn(0.5f, rsqrtf(a.h)), r));
+    const float s = __fsqrt_rn(a.h), i = __fmul_rn(0.5f, rsqrtf(a.h));
+    const float r = __fadd_rn(__fmaf_rn(-s, s, a.h), a.l);
+    const float d = __fmul_rn(i, r);
+    return pair_norm(s, __fmaf_rn(i, r, __fmul_rn(__fmul_rn(i, d), __fmaf_rn(-2.f * i, a.l, d))));
 }
 // sqrt(6) a: the constant in three parts, since two leave an error of 1e-15 that is the
 // same for every node
@@ -76,15 +93,69 @@ __device__ __forceinline__ Pair times_sqrt6(Pair a) {
 }
 __device__ __forceinline__ double times_sqrt6(double a) { return 2.449489742783178098 * a; }
 __device__ __forceinline__ double twice(double a) { return 2.0 * a; }
+__device__ __forceinline__ double square(double a) { return a * a; }
 __device__ __forceinline__ double square_root(double a) { return sqrt(a); }
 
-// The per-node arithmetic by storage type: T a node's term, S a running sum of terms.
+// A sum in three FP32 words, for terms that all have one sign: a pair's low word rounds,
+// and for sums of squares not evenly (the square of an odd integer is 1 modulo 8, so its
+// last bits are dropped downwards more often than upwards): 3e-16 to 8e-16 of the norm of
+// a Thomas-Fermi cloud, always too low, where sums in 64 bits are 1e-16 off.
+struct TripleSum {
+    float h, l, m;
+    __device__ __forceinline__ TripleSum() : h(0.f), l(0.f), m(0.f) {}
+    // a b
+    __device__ __forceinline__ TripleSum(float a, float b) : m(0.f) {
+        const Pair p = two_prod(a, b);
+        h = p.h;
+        l = p.l;
+    }
+    __device__ __forceinline__ void add_low(float v) {
+        const Pair s = two_sum(l, v);
+        l = s.h;
+        m = __fadd_rn(m, s.l);
+    }
+    __device__ __forceinline__ void add(float v) {
+        const Pair s = two_sum(h, v);
+        h = s.h;
+        add_low(s.l);
+    }
+    __device__ __forceinline__ void add_prod(float a, float b) {
+        const Pair p = two_prod(a, b);
+        add(p.h);
+        add_low(p.l);
+    }
+    __device__ __forceinline__ void add(const TripleSum& v) {
+        add(v.h);
+        add_low(v.l);
+        m = __fadd_rn(m, v.m);
+    }
+    __device__ __forceinline__ void add(Pair v) {
+        add(v.h);
+        add_low(v.l);
+    }
+    // += k v for a small integer k
+    __device__ __forceinline__ void add_times(float k, const TripleSum& v) {
+        add_prod(k, v.h);
+        const Pair p = two_prod(k, v.l);
+        add_low(p.h);
+        m = __fadd_rn(m, __fmaf_rn(k, v.m, p.l));
+    }
+    __device__ __forceinline__ Pair pair() const { return pair_norm(h, __fadd_rn(l, m)); }
+    // (an overflow or an infinity leaves NaN in l or m)
+    __device__ __forceinline__ double value() const {
+        return isfinite(__fadd_rn(l, m)) ? (double)h + ((double)l + (double)m) : (double)h;
+    }
+};
+
+// The per-node arithmetic by storage type: T a node's term, S a running sum of terms, E one
+// of terms of one sign.
 template <typename R>
 struct ObsArith;
 template <>
 struct ObsArith<float> {
     using T = Pair;
     using S = PairSum;
+    using E = TripleSum;
     // a b + c d and a b - c d
     __device__ static __forceinline__ T dot2(float a, float b, float c, float d) { return two_prod(a, b) + two_prod(c, d); }
     __device__ static __forceinline__ T cross2(float a, float b, float c, float d) { return two_prod(a, b) - two_prod(c, d); }
@@ -103,7 +174,37 @@ struct ObsArith<float> {
         s.add_prod(p, d.h);
         s.l = __fmaf_rn(p, d.l, s.l);
     }
+    __device__ static __forceinline__ void add_prod(E& s, float a, float b) { s.add_prod(a, b); }
+    // a a + b b; k (a - b) for k a power of two; a sum in E as a term
+    __device__ static __forceinline__ E norm2(float a, float b) {
+        E s(a, a);
+        s.add_prod(b, b);
+        return s;
+    }
+    __device__ static __forceinline__ E difference(float k, E a, E b) {
+        b.h = -b.h;
+        b.l = -b.l;
+        b.m = -b.m;
+        a.add(b);
+        a.h *= k;
+        a.l *= k;
+        a.m *= k;
+        return a;
+    }
+    __device__ static __forceinline__ T term(const E& s) { return s.pair(); }
+    // s^2 (rounding s to a pair first would leave 4e-16 of the interaction energy)
+    __device__ static __forceinline__ T square_of(const E& s) {
+        const Pair n = pair_norm(s.h, s.l), p = two_prod(n.h, n.h);
+        const float hl = __fmaf_rn(n.l, n.h, __fmaf_rn(s.m, n.h, __fmul_rn(__fmul_rn(0.5f, n.l), n.l)));
+        return pair_norm(p.h, __fmaf_rn(2.f, hl, p.l));
+    }
+    template <class V>
+    __device__ static __forceinline__ void add(E& s, const V& v) {
+        s.add(v);
+    }
+    __device__ static __forceinline__ void add_times(E& s, float k, const E& v) { s.add_times(k, v); }
     __device__ static __forceinline__ double value(const S& s) { return s.value(); }
+    __device__ static __forceinline__ double value(const E& s) { return s.value(); }
     __device__ static __forceinline__ bool less(T a, T b) { return a.h < b.h || (a.h == b.h && a.l < b.l); }
     __device__ static __forceinline__ T zero() { return Pair{0.f, 0.f}; }
     // the power of two that takes rho near 1 (1 where it is zero or subnormal), and v
@@ -118,6 +219,12 @@ template <>
 struct ObsArith<double> {
     using T = double;
     using S = double;
+    using E = double;
+    __device__ static __forceinline__ void add_prod(E& s, double a, double b) { s = fm(a, b, s); }
+    __device__ static __forceinline__ E norm2(double a, double b) { return fm(a, a, b * b); }
+    __device__ static __forceinline__ E difference(double k, E a, E b) { return k * (a - b); }
+    __device__ static __forceinline__ T term(E s) { return s; }
+    __device__ static __forceinline__ T square_of(E s) { return s * s; }
     __device__ static __forceinline__ T dot2(double a, double b, double c, double d) { return fm(a, b, c * d); }
     __device__ static __forceinline__ T cross2(double a, double b, double c, double d) { return fm(a, b, -(c * d)); }
     __device__ static __forceinline__ void add(S& s, T v) { s += v; }
@@ -141,13 +248,27 @@ template <typename R, int C>
 struct NodeTerms {
     using A = ObsArith<R>;
     using T = typename A::T;
-    T n[C], rho;
+    using E = typename A::E;
+    E n[C], density;
+    T rho;   // the density rounded to a term
     __device__ __forceinline__ explicit NodeTerms(const Cx<R>* p) {
 #pragma unroll
-        for (int s = 0; s < C; ++s) n[s] = A::dot2(p[s].x, p[s].x, p[s].y, p[s].y);
-        rho = n[0];
+        for (int s = 0; s < C; ++s) n[s] = A::norm2(p[s].x, p[s].y);
+        density = n[0];
 #pragma unroll
-        for (int s = 1; s < C; ++s) rho = rho + n[s];
+        for (int s = 1; s < C; ++s) A::add(density, n[s]);
+        rho = A::term(density);
+    }
+    // F_z of components b .. (spin-2: of all five)
+    template <int b>
+    __device__ __forceinline__ E fz() const {
+        if constexpr (b == 0 && C == 5) {
+            E f = A::difference((R)2, n[0], n[4]);
+            A::add(f, A::difference((R)1, n[1], n[3]));
+            return f;
+        } else {
+            return A::difference((R)1, n[b], n[b + 2]);
+        }
     }
     // Re and Im of conj(a) b + conj(b) c
     __device__ static __forceinline__ void chain(Cx<R> a, Cx<R> b, Cx<R> c, T& re, T& im) {
@@ -158,11 +279,13 @@ struct NodeTerms {
     // taken once per thread, in FP64)
     __device__ __forceinline__ void track_max(const Cx<R>* p, T& top, Cx<R>& at) const {
 #pragma unroll
-        for (int s = 0; s < C; ++s)
-            if (A::less(top, n[s])) {
-                top = n[s];
+        for (int s = 0; s < C; ++s) {
+            const T m = A::term(n[s]);
+            if (A::less(top, m)) {
+                top = m;
                 at = p[s];
             }
+        }
     }
 };
 
@@ -213,13 +336,15 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_k
         const uint32_t within = col - y * a.row_items;
         const uint32_t x = fdiv(within, a.divV);
         const uint32_t l = within - x * a.g.V;
-        const uint32_t z0 = chunk * zc, nz = min(zc, a.g.Z - z0);
+        // moments in z are taken about the column's middle
+        const uint32_t z0 = chunk * zc, nz = min(zc, a.g.Z - z0), mid = nz / 2;
         const char* base = a.prev + (size_t)z0 * a.g.slice + (size_t)y * a.g.pitch + (size_t)x * a.g.cell_bytes;
         const int f0 = st.row_ptr[l], nd = st.row_ptr[l + 1] - f0;
         int32_t off[D];
 #pragma unroll
         for (int k = 0; k < D; ++k) off[k] = k < nd ? st.nb_off[f0 + k] : (int32_t)(l * node_bytes);
-        S kin[D], s0{}, s1{}, s2{}, srr{}, mx{}, my{}, fz{}, fz1{}, sff{}, sabs{}, gx{}, gy{}, sth{};
+        S kin[D], mx{}, my{}, gx{}, gy{};
+        typename A::E s0{}, s1{}, s2{}, srr{}, sff{}, sth{}, sabs{}, fz{}, fz1{};
 #pragma unroll
         for (int k = 0; k < D; ++k) kin[k] = S{};
 #pragma unroll 1
@@ -247,20 +372,21 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_k
             nbad += count_nonfinite<R, C>(p);
             const NodeTerms<R, C> t(p);
             t.track_max(p, top, at);
-            const R zj = (R)j;
-            A::add(s0, t.rho);
-            A::add_times(s1, zj, t.rho);
-            A::add_times(s2, zj * zj, t.rho);
-            A::add(srr, t.rho * t.rho);
+            const R zj = (R)((int32_t)j - (int32_t)mid);
+            A::add(s0, t.density);
+            A::add_times(s1, zj, t.density);
+            A::add_times(s2, zj * zj, t.density);
+            A::add(srr, A::square_of(t.density));
             if constexpr (C == 3) {
                 T re, im;
                 t.chain(p[0], p[1], p[2], re, im);
-                const T f = t.n[0] - t.n[2];
-                const T ff = twice(re * re + im * im) + f * f;
+                const typename A::E fe = t.template fz<0>();
+                const T f = A::term(fe);
+                const T ff = twice(square(re) + square(im)) + square(f);
                 A::add(mx, re);
                 A::add(my, im);
-                A::add(fz, f);
-                A::add_times(fz1, zj, f);
+                A::add(fz, fe);
+                A::add_times(fz1, zj, fe);
                 A::add(sff, ff);
                 A::add(sabs, square_root(ff));
             } else if constexpr (C == 5) {
@@ -270,15 +396,16 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_k
                 t.chain(p[1], p[2], p[3], re6, im6);
                 const T re2 = A::dot2(p[0].x, p[1].x, p[0].y, p[1].y) + A::dot2(p[3].x, p[4].x, p[3].y, p[4].y);
                 const T im2 = A::cross2(p[0].x, p[1].y, p[0].y, p[1].x) + A::cross2(p[3].x, p[4].y, p[3].y, p[4].x);
-                const T f = twice(t.n[0] - t.n[4]) + (t.n[1] - t.n[3]);
+                const typename A::E fe = t.template fz<0>();
+                const T f = A::term(fe);
                 const T fx = twice(re2) + times_sqrt6(re6), fy = twice(im2) + times_sqrt6(im6);
-                const T ff = fx * fx + fy * fy + f * f;
+                const T ff = square(fx) + square(fy) + square(f);
                 A::add(mx, re2);
                 A::add(my, im2);
                 A::add(gx, re6);
                 A::add(gy, im6);
-                A::add(fz, f);
-                A::add_times(fz1, zj, f);
+                A::add(fz, fe);
+                A::add_times(fz1, zj, fe);
                 A::add(sff, ff);
                 A::add(sabs, square_root(ff));
                 // |theta|^2 of the singlet sum theta = psi_0^2 - 2 psi_1 psi_-1 + 2 psi_2 psi_-2
@@ -286,21 +413,27 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_k
                              twice(A::cross2(p[0].x, p[4].x, p[0].y, p[4].y) - A::cross2(p[1].x, p[3].x, p[1].y, p[3].y));
                 const T ty = twice(A::dot2(p[2].x, p[2].y, (R)0, (R)0) + A::dot2(p[0].x, p[4].y, p[0].y, p[4].x) -
                                    A::dot2(p[1].x, p[3].y, p[1].y, p[3].x));
-                A::add(sth, tx * tx + ty * ty);
+                A::add(sth, square(tx) + square(ty));
             }
         }
         // the column's sums with what is the same for all its nodes
         const double S0 = A::value(s0), S1 = A::value(s1), S2 = A::value(s2);
         const double rx = P.p0[0] + P.bs * ((double)x * P.bw[0] + st.pos[3 * l + 0]);
         const double ry = P.p0[1] + P.bs * ((double)y * P.bw[1] + st.pos[3 * l + 1]);
-        const double rz = P.p0[2] + P.bs * ((double)z0 * P.bw[2] + st.pos[3 * l + 2]), gz = P.bs * P.bw[2];
+        // the middle's height and the step, whose roundings are the same for all the column's
+        // nodes, with what they leave out (heights rounded as a whole put up to 1e-15 of the
+        // centre of mass)
+        const double zm = (double)(z0 + mid), hm = zm * P.bw[2], hl = fm(zm, P.bw[2], -hm);
+        const double rz = fm(P.bs, st.pos[3 * l + 2] + hl, fm(P.bs, hm, P.p0[2]));
+        const double gz = P.bs * P.bw[2], gl = fm(P.bs, P.bw[2], -gz);
         double hexp = 0.0, eint = P.c0 * A::value(srr);
 #pragma unroll
         for (int k = 0; k < D; ++k)
             if (k < nd) hexp += st.w[f0 + k] * A::value(kin[k]);
         if (P.trap_on) {
             const double tx = rx * P.lambda[0], ty = ry * P.lambda[1], hz = 0.5 * P.lambda[2] * P.lambda[2];
-            hexp += (0.5 * (tx * tx + ty * ty) + P.trap_offset) * S0 + hz * (rz * rz * S0 + gz * (2.0 * rz * S1 + gz * S2));
+            hexp += (0.5 * (tx * tx + ty * ty) + P.trap_offset) * S0 + 
+                    hz * (rz * rz * S0 + (gz * (2.0 * rz * S1 + gz * S2) + 2.0 * gl * (rz * S1 + gz * S2)));
         }
         if constexpr (C > 1) {
             double Mx, My;
@@ -329,7 +462,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_k
         acc[OBS_EINT] += eint;
         acc[OBS_COMX] += rx * S0;
         acc[OBS_COMY] += ry * S0;
-        acc[OBS_COMZ] += rz * S0 + gz * S1;
+        acc[OBS_COMZ] += rz * S0 + (gz * S1 + gl * S1);
     }
     acc[OBS_MAXABS] = sqrt((double)at.x * at.x + (double)at.y * at.y);
     acc[OBS_NONFINITE] = (double)nbad;
@@ -355,6 +488,7 @@ __global__ void __launch_bounds__(256) field_sums_kernel(StepArgs a) {
     using T = typename O::T;
     __shared__ double red[8][kFieldSums];
     typename O::S s[5] = {};
+    typename O::E spin{}, density{};
     A top = (A)0;
     bool empty = false;
     for (uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < a.total;
@@ -376,19 +510,19 @@ __global__ void __launch_bounds__(256) field_sums_kernel(StepArgs a) {
             if constexpr (sizeof(A) == 4) top = fmaxf(top, fmaxf(fabsf(p[c].x), fabsf(p[c].y)));
         }
         const NodeTerms<A, C> t(p);
-        O::add(s[SPIN ? 4 : 0], t.rho);
+        O::add(density, t.density);
         if constexpr (SPIN && C > 1) {
             constexpr int b = C == 5 ? 1 : 0;  // s1, s0, s_1
             T re, im;
             t.chain(p[b], p[b + 1], p[b + 2], re, im);
-            const T f = t.n[b] - t.n[b + 2];
+            const T f = O::term(t.template fz<b>());
             O::add(s[1], re);
             O::add(s[2], im);
             O::add(s[3], t.rho * f);
             // rho |s| with m and rho taken near 1, so that no square leaves the range
             const A u = O::unit(t.rho);
             const T rx = O::times(re, u), ry = O::times(im, u), rz = O::times(t.rho, u) * f;
-            O::add(s[0], O::times(square_root(twice(rx * rx + ry * ry) + rz * rz), (A)1 / u));
+            O::add(spin, O::times(square_root(twice(square(rx) + square(ry)) + square(rz)), (A)1 / u));
             bool none = true;
 #pragma unroll
             for (int c = 0; c < C; ++c) none = none && p[c].x == (A)0 && p[c].y == (A)0;
@@ -398,6 +532,8 @@ __global__ void __launch_bounds__(256) field_sums_kernel(StepArgs a) {
     double v[kFieldSums];
 #pragma unroll
     for (int k = 0; k < 5; ++k) v[k] = O::value(s[k]);
+    v[0] = O::value(SPIN && C > 1 ? spin : density);
+    if (SPIN) v[4] = O::value(density);
     if constexpr (SPIN) {
         v[1] *= GPE_REF_SQRT_2;
         v[2] *= GPE_REF_SQRT_2;

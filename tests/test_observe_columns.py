@@ -123,3 +123,48 @@ def test_empty_and_nonfinite_nodes(gpu, prec):
             with pytest.raises(capi.GpeError) as e:
                 s.observe(capi.PSI_ODD)
             assert e.value.status == 5  # GPE_ERR_NONFINITE
+
+
+@pytest.mark.parametrize("name,C,dims", [("bcc", 1, (12, 13, 14)), ("bcc", 3, (13, 12, 15)), ("bcc", 5, (12, 12, 13)),
+                                         ("c15", 3, (4, 5, 6))])
+def test_sums_of_one_sign_have_no_bias(gpu, name, C, dims):
+    """Norm, centre of mass and spin against sums in extended precision over eight clouds: what
+    is left is the rounding of the sums' last FP64 additions and of the product with the cell
+    volume, 2e-16 at most each time and of either sign (a bias of the pairs' low words, whose
+    squares round down more often than up, is 3e-16 to 8e-16)."""
+    lat = capi.Lattice(name)
+    p = _params(lat, C, capi.FP32, dims)
+    wide = np.longdouble
+    dv = wide(p.block_scale * p.block_scale * p.block_scale * lat.volume)
+    inner = (slice(1, -1),) * 3
+    errors = []
+    with Stepper(lat, p) as s:
+        for seed in range(8):
+            rng = np.random.default_rng(seed)
+            psi = np.zeros(capi.buffer_shape(lat, p))
+            shape = psi[inner].shape[:-1]
+            # densities of a cloud from its edge to its middle, every node's phases its own
+            phase = rng.uniform(-np.pi, np.pi, shape)
+            psi[inner] = 0.07 * np.sqrt(rng.uniform(0, 1, shape))[..., None] * np.stack([np.cos(phase), np.sin(phase)], -1)
+            psi = psi.astype(np.float32).astype(np.float64)
+            s.upload(capi.PSI_EVEN, psi)
+            got = s.observe(capi.PSI_EVEN)
+            re, im = psi[inner][..., 0].astype(wide), psi[inner][..., 1].astype(wide)
+            n = re * re + im * im
+            x = wide(p.p0[0]) + wide(p.block_scale) * (np.arange(dims[0]).astype(wide)[:, None] * wide(lat.block_width[0])
+                                                       + lat.pos[:, 0].astype(wide))
+            norm, com = n.sum() * dv, (n.sum(-1) * x).sum() * dv
+            e = [(wide(got["norm"]) - norm) / norm, (wide(got["com"][0]) - com) / ((n.sum(-1) * abs(x)).sum() * dv)]
+            if C > 1:
+                def pair(a, b):
+                    return np.stack([re[..., a] * re[..., b] + im[..., a] * im[..., b],
+                                     re[..., a] * im[..., b] - im[..., a] * re[..., b]])
+                if C == 3:
+                    across, along = np.sqrt(wide(2)) * (pair(0, 1) + pair(1, 2)), n[..., 0] - n[..., 2]
+                else:
+                    across = 2 * (pair(0, 1) + pair(3, 4)) + np.sqrt(wide(6)) * (pair(1, 2) + pair(2, 3))
+                    along = 2 * (n[..., 0] - n[..., 4]) + n[..., 1] - n[..., 3]
+                size = np.sqrt((across ** 2).sum(0) + along ** 2).sum() * dv
+                e.append((wide(got["spin_norm"]) - size) / size)
+            errors.append([float(v) for v in e])
+    assert np.all(np.abs(np.mean(errors, axis=0)) <= 2e-16), np.mean(errors, axis=0)
