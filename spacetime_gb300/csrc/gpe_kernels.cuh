@@ -680,6 +680,80 @@ struct PairSum {
     }
 };
 
+// A value as an unevaluated sum h + l of two FP32 values, |l| <= ulp(h) / 2.
+struct Pair {
+    float h, l;
+};
+__device__ __forceinline__ Pair pair_norm(float s, float e) {   // |s| >= |e|
+    Pair r;
+    r.h = __fadd_rn(s, e);
+    r.l = __fsub_rn(e, __fsub_rn(r.h, s));
+    return r;
+}
+__device__ __forceinline__ Pair two_sum(float a, float b) {
+    Pair r;
+    r.h = __fadd_rn(a, b);
+    const float t = __fsub_rn(r.h, a);
+    r.l = __fadd_rn(__fsub_rn(a, __fsub_rn(r.h, t)), __fsub_rn(b, t));
+    return r;
+}
+__device__ __forceinline__ Pair two_prod(float a, float b) {
+    Pair r;
+    r.h = __fmul_rn(a, b);
+    r.l = __fmaf_rn(a, b, -r.h);
+    return r;
+}
+// A sum in three FP32 words, for terms that all have one sign: a pair's low word rounds,
+// and for sums of squares not evenly (the square of an odd integer is 1 modulo 8, so its
+// last bits are dropped downwards more often than upwards): 3e-16 to 8e-16 of the norm of
+// a Thomas-Fermi cloud, always too low, where sums in 64 bits are 1e-16 off.
+struct TripleSum {
+    float h, l, m;
+    __device__ __forceinline__ TripleSum() : h(0.f), l(0.f), m(0.f) {}
+    // a b
+    __device__ __forceinline__ TripleSum(float a, float b) : m(0.f) {
+        const Pair p = two_prod(a, b);
+        h = p.h;
+        l = p.l;
+    }
+    __device__ __forceinline__ void add_low(float v) {
+        const Pair s = two_sum(l, v);
+        l = s.h;
+        m = __fadd_rn(m, s.l);
+    }
+    __device__ __forceinline__ void add(float v) {
+        const Pair s = two_sum(h, v);
+        h = s.h;
+        add_low(s.l);
+    }
+    __device__ __forceinline__ void add_prod(float a, float b) {
+        const Pair p = two_prod(a, b);
+        add(p.h);
+        add_low(p.l);
+    }
+    __device__ __forceinline__ void add(const TripleSum& v) {
+        add(v.h);
+        add_low(v.l);
+        m = __fadd_rn(m, v.m);
+    }
+    __device__ __forceinline__ void add(Pair v) {
+        add(v.h);
+        add_low(v.l);
+    }
+    // += k v for a small integer k
+    __device__ __forceinline__ void add_times(float k, const TripleSum& v) {
+        add_prod(k, v.h);
+        const Pair p = two_prod(k, v.l);
+        add_low(p.h);
+        m = __fadd_rn(m, __fmaf_rn(k, v.m, p.l));
+    }
+    __device__ __forceinline__ Pair pair() const { return pair_norm(h, __fadd_rn(l, m)); }
+    // (an overflow or an infinity leaves NaN in l or m)
+    __device__ __forceinline__ double value() const {
+        return isfinite(__fadd_rn(l, m)) ? (double)h + ((double)l + (double)m) : (double)h;
+    }
+};
+
 // Sum of |v|^2 over the records a thread passes to add(), the per-node terms in R
 // and their sum in FP64 (FP64 storage) or as a pair of FP32 values (PairSum: no FP64
 // operation per node), and the normalisation factor from the whole grid's sum: every
@@ -1929,13 +2003,13 @@ cudaError_t launch_scale(const StepArgs& a, cudaStream_t s) {
 namespace gpe {
 
 // sum_interior Re(conj(a) b) into scale_out->sum (innerProduct, Spin1GpeBCC.cu:
-// 213-233); a = StepArgs::prev, b = StepArgs::next.  FP32 storage: a pair sum per
+// 213-233); a = StepArgs::prev, b = StepArgs::next.  FP32 storage: a sum in three words per
 // thread.
 template <typename R, int C>
 __global__ void __launch_bounds__(256) dot_kernel(StepArgs a) {
     __shared__ double red[8];
     double acc = 0;
-    PairSum pair;
+    TripleSum sum;
     for (uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < a.total;
          gid += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t i = (uint32_t)gid;
@@ -1955,17 +2029,13 @@ __global__ void __launch_bounds__(256) dot_kernel(StepArgs a) {
         } else {
 #pragma unroll
             for (int s = 0; s < C; ++s) {
-                pair.add_prod(u[s].x, v[s].x);
-                pair.add_prod(u[s].y, v[s].y);
+                sum.add_prod(u[s].x, v[s].x);
+                sum.add_prod(u[s].y, v[s].y);
             }
         }
     }
-    if constexpr (sizeof(R) == 4) {
-        pair.warp_sum();
-        acc = pair.value();
-    } else {
-        acc = NormAcc<R>::warp_sum(acc);
-    }
+    if constexpr (sizeof(R) == 4) acc = sum.value();
+    acc = NormAcc<R>::warp_sum(acc);
     NormAcc<R>::grid_sum(acc, red, a.partials, a.dv, a.scale_out);
 }
 

@@ -23,29 +23,6 @@
 
 namespace gpe {
 
-// A value as an unevaluated sum h + l of two FP32 values, |l| <= ulp(h) / 2.
-struct Pair {
-    float h, l;
-};
-__device__ __forceinline__ Pair pair_norm(float s, float e) {   // |s| >= |e|
-    Pair r;
-    r.h = __fadd_rn(s, e);
-    r.l = __fsub_rn(e, __fsub_rn(r.h, s));
-    return r;
-}
-__device__ __forceinline__ Pair two_sum(float a, float b) {
-    Pair r;
-    r.h = __fadd_rn(a, b);
-    const float t = __fsub_rn(r.h, a);
-    r.l = __fadd_rn(__fsub_rn(a, __fsub_rn(r.h, t)), __fsub_rn(b, t));
-    return r;
-}
-__device__ __forceinline__ Pair two_prod(float a, float b) {
-    Pair r;
-    r.h = __fmul_rn(a, b);
-    r.l = __fmaf_rn(a, b, -r.h);
-    return r;
-}
 __device__ __forceinline__ Pair operator+(Pair a, Pair b) {
     const Pair s = two_sum(a.h, b.h);
     return pair_norm(s.h, __fadd_rn(s.l, __fadd_rn(a.l, b.l)));
@@ -95,57 +72,6 @@ __device__ __forceinline__ double times_sqrt6(double a) { return 2.4494897427831
 __device__ __forceinline__ double twice(double a) { return 2.0 * a; }
 __device__ __forceinline__ double square(double a) { return a * a; }
 __device__ __forceinline__ double square_root(double a) { return sqrt(a); }
-
-// A sum in three FP32 words, for terms that all have one sign: a pair's low word rounds,
-// and for sums of squares not evenly (the square of an odd integer is 1 modulo 8, so its
-// last bits are dropped downwards more often than upwards): 3e-16 to 8e-16 of the norm of
-// a Thomas-Fermi cloud, always too low, where sums in 64 bits are 1e-16 off.
-struct TripleSum {
-    float h, l, m;
-    __device__ __forceinline__ TripleSum() : h(0.f), l(0.f), m(0.f) {}
-    // a b
-    __device__ __forceinline__ TripleSum(float a, float b) : m(0.f) {
-        const Pair p = two_prod(a, b);
-        h = p.h;
-        l = p.l;
-    }
-    __device__ __forceinline__ void add_low(float v) {
-        const Pair s = two_sum(l, v);
-        l = s.h;
-        m = __fadd_rn(m, s.l);
-    }
-    __device__ __forceinline__ void add(float v) {
-        const Pair s = two_sum(h, v);
-        h = s.h;
-        add_low(s.l);
-    }
-    __device__ __forceinline__ void add_prod(float a, float b) {
-        const Pair p = two_prod(a, b);
-        add(p.h);
-        add_low(p.l);
-    }
-    __device__ __forceinline__ void add(const TripleSum& v) {
-        add(v.h);
-        add_low(v.l);
-        m = __fadd_rn(m, v.m);
-    }
-    __device__ __forceinline__ void add(Pair v) {
-        add(v.h);
-        add_low(v.l);
-    }
-    // += k v for a small integer k
-    __device__ __forceinline__ void add_times(float k, const TripleSum& v) {
-        add_prod(k, v.h);
-        const Pair p = two_prod(k, v.l);
-        add_low(p.h);
-        m = __fadd_rn(m, __fmaf_rn(k, v.m, p.l));
-    }
-    __device__ __forceinline__ Pair pair() const { return pair_norm(h, __fadd_rn(l, m)); }
-    // (an overflow or an infinity leaves NaN in l or m)
-    __device__ __forceinline__ double value() const {
-        return isfinite(__fadd_rn(l, m)) ? (double)h + ((double)l + (double)m) : (double)h;
-    }
-};
 
 // The per-node arithmetic by storage type: T a node's term, S a running sum of terms, E one
 // of terms of one sign.
