@@ -519,15 +519,18 @@ gpe_status gpe_observe_noalloc(const gpe_lattice_desc* lat, const gpe_params* p,
  * fields[j] at time t_j = t0 + j*dt (t0 from gpe_set_ramp, else 0) -- the same
  * steps gpe_start + gpe_step(n_steps-1) take with a ramp whose value at t_j is
  * fields[j].  It keeps checkpoints (u_{kS}, u_{kS+1}) every `stride` steps
- * (stride <= 0: ceil(sqrt(n_steps))) in device memory owned by the handle, and
- * writes out[5] = (Re <T|u_N>, Im <T|u_N>, M_x, M_y, M_z): the overlap with
+ * (stride <= 0: every state where those take at most 8 GiB and a quarter of the free
+ * memory and the run is stepped in the interleaved layout, else ceil(sqrt(n_steps)))
+ * in device memory owned by the handle (given back by a call with other needs and by
+ * gpe_destroy), and writes out[5] = (Re <T|u_N>, Im <T|u_N>, M_x, M_y, M_z): the overlap with
  * `target` (host FP64, file layout, `count` doubles) and the magnetization of
  * the final state, integrated with dv as gpe_observe does.  Synchronises.
  *
  * gpe_adjoint_backward takes seed[5] = dL/d(out[k]) for a loss L of those five
  * numbers and writes grad[4*j + m] = dL/d(field m of step j) for
- * m = 0: bq, 1..3: bb[0..2] (n_steps x 4 doubles).  It recomputes the states of
- * one checkpoint segment at a time with the forward kernel and runs the adjoint
+ * m = 0: bq, 1..3: bb[0..2] (n_steps x 4 doubles), the same for every stride, bit for
+ * bit.  It recomputes the states that were not kept, one checkpoint segment at a
+ * time, with the forward kernel and runs the adjoint
  * (reverse-time) kernel of the step back through it.  Valid while no other call
  * has written the handle's psi buffers since gpe_adjoint_forward; may be called
  * again with another seed.  Synchronises. */

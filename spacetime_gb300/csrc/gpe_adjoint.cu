@@ -691,6 +691,9 @@ void adjoint_release(gpe_handle* h) {
     for (void* p : A.seg) cudaFree(p);
     A.ckpt.clear();
     A.seg.clear();
+    if (A.kept) cudaFree(A.kept);
+    A.kept = nullptr;
+    A.kept_bytes = 0;
     for (void*& p : A.adj) {
         if (p) cudaFree(p);
         p = nullptr;
@@ -706,7 +709,7 @@ void adjoint_release(gpe_handle* h) {
     A.target = nullptr;
     A.grad = A.out = A.wT64 = nullptr;
     A.wT32 = nullptr;
-    A.valid = A.il = false;
+    A.valid = A.il = A.keeps = false;
     A.buf_bytes = 0;
     A.n = A.stride = A.segments = 0;
 }
@@ -754,12 +757,45 @@ static gpe_status build_transpose(gpe_handle* h) {
     return GPE_OK;
 }
 
-static gpe_status ensure_adjoint_buffers(gpe_handle* h, int n, int stride, bool il) {
+// Whether a run without a given stride keeps all its states instead of checkpoints: where
+// they take at most kKeepBytes (3 % of the memory) and a quarter of what is free.
+// Recomputing a state costs what its first computation did, and a state is written and read
+// once either way: spin-1 BCC 40^3, 200 steps (3.7 GB), one gradient 7.79 ms with
+// checkpoints, 6.01 with all states, the first one with its allocations 10.0 and 7.1.
+constexpr size_t kKeepBytes = (size_t)8 << 30;
+static size_t kept_step(const gpe_handle* h) { return (h->ilg.bytes + 255) & ~(size_t)255; }
+static bool keep_states(const gpe_handle* h, int n) {
+    const size_t need = kept_step(h) * (size_t)n;
+    if (need > kKeepBytes) return false;
+    if (h->adj.il && h->adj.kept_bytes >= need) return true;
+    size_t free_bytes = 0, total = 0;
+    if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) return false;
+    return need <= free_bytes / 4;
+}
+
+static gpe_status ensure_adjoint_buffers(gpe_handle* h, int n, int stride, bool il, bool keep) {
     AdjointStore& A = h->adj;
     const int segments = (n + stride - 1) / stride;
     const size_t bytes = il ? h->ilg.bytes : h->alloc_bytes[GPE_PSI_EVEN];
     if (A.il != il || A.buf_bytes != bytes) adjoint_release(h);
-    const size_t want_ckpt = (size_t)2 * segments, want_seg = stride > 2 ? (size_t)(stride - 2) : 0;
+    const size_t want_ckpt = keep ? 0 : (size_t)2 * segments, want_seg = !keep && stride > 2 ? (size_t)(stride - 2) : 0;
+    const size_t need = keep ? kept_step(h) * (size_t)n : 0;
+    if (A.kept && (!keep || A.kept_bytes < need)) {
+        cudaFree(A.kept);
+        A.kept = nullptr;
+        A.kept_bytes = 0;
+    }
+    if (keep && !A.kept) {
+        if (cudaMalloc(&A.kept, need) != cudaSuccess) {
+            A.kept = nullptr;
+            return fail(GPE_ERR_OOM, "cudaMalloc (adjoint states)");
+        }
+        A.kept_bytes = need;
+        // zero halos: the steps write the interior only
+        if (cudaMemset(A.kept, 0, need) != cudaSuccess) return fail(GPE_ERR_CUDA, "cudaMemset (adjoint states)");
+    }
+    A.kept_step = kept_step(h);
+    A.keeps = keep;
     auto resize = [&](std::vector<void*>& v, size_t want) -> bool {
         while (v.size() > want) {
             cudaFree(v.back());
@@ -830,24 +866,29 @@ extern "C" gpe_status gpe_adjoint_forward(gpe_handle* h, int32_t n_steps, const 
     if (h->exp_rate != 0) return fail(GPE_ERR_UNSUPPORTED, "the adjoint does not follow condensate expansion");
     if (n_steps < 1) return fail(GPE_ERR_INVALID_ARG, "n_steps must be at least 1");
     if (count != host_count(h, false)) return fail(GPE_ERR_INVALID_ARG, "target size does not match the grid");
-    if (stride <= 0) stride = (int32_t)std::ceil(std::sqrt((double)n_steps));
+    const bool any_stride = stride <= 0;
+    if (any_stride) stride = (int32_t)std::ceil(std::sqrt((double)n_steps));
     if (stride > n_steps) stride = n_steps;
     AdjointStore& A = h->adj;
     A.valid = false;
     cudaStream_t s = (cudaStream_t)stream;
-    // runs long enough for the interleaved step kernel keep all their states in its layout, where the memory for them can be had (its rows are padded to whole
-    // groups of cells); others in the handle's layout
+    // runs long enough for the interleaved step kernel have their states in its layout,
+    // where the memory for them can be had (its rows are padded to whole groups of
+    // cells); others in the handle's layout
     gpe_status st = GPE_ERR_OOM;
     if (n_steps > 1 && il_leapfrog_applies(h, n_steps)) {
         st = il_ensure(h, s);
-        if (!st) st = ensure_adjoint_buffers(h, n_steps, stride, true);
-        if (st && st != GPE_ERR_OOM) return st;
-        if (st) {
+        for (int keep = any_stride && !st && keep_states(h, n_steps) ? 1 : 0; !st && keep >= 0; --keep) {
+            st = ensure_adjoint_buffers(h, n_steps, stride, true, keep != 0);
+            if (st != GPE_ERR_OOM) break;
             adjoint_release(h);
             cudaGetLastError();
+            if (keep) st = GPE_OK;   // once more, with checkpoints
         }
+        if (st && st != GPE_ERR_OOM) return st;
+        if (st) cudaGetLastError();
     }
-    if (st) st = ensure_adjoint_buffers(h, n_steps, stride, false);
+    if (st) st = ensure_adjoint_buffers(h, n_steps, stride, false, false);
     if (st) return st;
     // target: host FP64 file layout -> device buffer in the handle's precision
     if ((st = ensure_stage(h, count))) return st;
@@ -868,11 +909,12 @@ extern "C" gpe_status gpe_adjoint_forward(gpe_handle* h, int32_t n_steps, const 
     if ((st = step_buffers(h, h->interior[GPE_PSI_EVEN], h->interior[GPE_PSI_ODD], fields[0], A.t0, GPE_MODE_EULER, s)))
         return st;
     if (A.il) {
-        // u_j goes where it is wanted: a checkpoint (u_{kS}, u_{kS+1}), or one of two work
-        // buffers, in place of u_{j-2} where that is no checkpoint
+        // u_j goes where it is wanted: its place among the kept states, a checkpoint (u_{kS},
+        // u_{kS+1}), or one of two work buffers, in place of u_{j-2} where that is neither
         auto il_buffer = [&](void* p) { return static_cast<char*>(p); };
         auto home = [&](int j) -> char* {
             if (j == n_steps) return nullptr;
+            if (A.keeps) return il_buffer(A.kept) + (size_t)j * A.kept_step;
             if (j % stride == 0) return il_buffer(A.ckpt[2 * (j / stride)]);
             if (j % stride == 1) return il_buffer(A.ckpt[2 * (j / stride) + 1]);
             return nullptr;
@@ -956,9 +998,13 @@ extern "C" gpe_status gpe_adjoint_backward(gpe_handle* h, const double* seed, do
     const bool oop = leapfrog_from_supported(h);
     for (int k = A.segments - 1; k >= 0; --k) {
         const int lo = k * S, hi = std::min(lo + S, n), len = hi - lo;
-        state[0] = A.ckpt[2 * k];
-        if (len > 1) state[1] = A.ckpt[2 * k + 1];
-        for (int m = 2; m < len; ++m) {
+        if (A.keeps) {
+            for (int m = 0; m < len; ++m) state[m] = static_cast<char*>(A.kept) + (size_t)(lo + m) * A.kept_step;
+        } else {
+            state[0] = A.ckpt[2 * k];
+            if (len > 1) state[1] = A.ckpt[2 * k + 1];
+        }
+        for (int m = 2; m < len && !A.keeps; ++m) {
             state[m] = A.seg[m - 2];
             const int jj = lo + m - 1;
             if (A.il) {

@@ -30,6 +30,9 @@ struct AdjointStore {
     std::vector<gpe_fields> fields; // per step
     std::vector<void*> ckpt;        // 2 per segment: (u_{kS}, u_{kS+1})
     std::vector<void*> seg;         // stride buffers for the recomputed segment
+    void* kept = nullptr;           // or all of u_0 .. u_{n-1}, kept_step bytes apart
+    size_t kept_bytes = 0, kept_step = 0;
+    bool keeps = false;             // the recorded run is in `kept`
     void* adj[2] = {nullptr, nullptr};
     void* target = nullptr;
     size_t buf_bytes = 0;           // bytes of each state buffer above

@@ -58,3 +58,29 @@ def test_interleaved_adjoint_strides(gpu, stride):
     got = _gradient(lat, capi.FP32, 3, (24, 3, 2), 17, stride, capi.KERNEL_AUTO)
     for a, b in zip(got, ref):
         assert np.array_equal(a, b)
+
+
+def test_one_handle_many_records(gpu):
+    """One handle's records one after the other -- every state kept (no stride given), more
+    of them, checkpoints, fewer states -- give what a handle of their own gives, bit for bit."""
+    lat = capi.Lattice("bcc")
+    p = capi.make_params(components=3, precision=capi.FP32, dims=(24, 3, 2), block_scale=0.3, dt=2e-4, trap_offset=10.0,
+                         c0=120.0, c2=-7.0, lattice=lat)
+    shape = capi.buffer_shape(lat, p)
+    psi = states.normalize(states.random_state(shape, seed=3), lat, p)
+    target = states.normalize(states.random_state(shape, seed=4), lat, p)
+
+    def run(s, n, stride):
+        fields = 0.5 * np.random.default_rng(n).standard_normal((n, 4))
+        s.upload(capi.PSI_ODD, psi)
+        out = s.adjoint_forward(fields, target, stride)
+        return out, s.adjoint_backward(SEED), s.adjoint_backward(2 * SEED), s.download(s.current)
+
+    records = [(17, 0), (40, 0), (40, 6), (19, 0), (7, 0), (18, 18), (40, 0)]
+    with Stepper(lat, p) as s:
+        got = [run(s, *r) for r in records]
+    for (n, _), g in zip(records, got):
+        with Stepper(lat, p) as s:
+            want = run(s, n, 1)
+        for a, b in zip(g, want):
+            assert np.array_equal(a, b), n
