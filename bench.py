@@ -65,7 +65,7 @@ LEGS["scalar-split-c15-64"] = dict(lattice="c15", C=1, dims=(64, 64, 64), c0=200
                                    scheme=2, sigma=0.00225, zeta=(1.0,), kappa=1, noise_abs=1e-3, noise_rel=0.0,
                                    bytes_fp32=72, seed=7)
 KERNEL_OF_SCHEME = {0: "leapfrog kernel (auto) C=%d", 1: "hyper_tile_kernel<float,%d> (fused tile)",
-                    2: "split_step_kernel<float,PART> (C=%d, two launches per step)"}
+                    2: "il_split_kernel<PART,CELLS> (C=%d, two launches per step)"}
 
 
 def workload(precision):
@@ -160,9 +160,9 @@ def time_leg(w, steps, inner, warmup, kernel=0, dims=None):
     if w["scheme"] == 0 and gather:
         name = "parabolic_fixed_kernel<float,%d,LEAPFROG,4>" % w["C"]
     if interleaved and w["scheme"] == 1:
-        name = "il_hyper_kernel<%d,%d>" % (w["C"], il_group_cells(p.dims[0]))
+        name = "il_hyper_kernel<%d,%d>" % (w["C"], il_group_cells(p.dims[0], w["C"]))
     elif interleaved:
-        name = "il_step_kernel<%d,%d,%d>" % (w["C"], 8 if w["lattice"] == "fcc" else 4, il_group_cells(p.dims[0]))
+        name = "il_step_kernel<%d,%d,%d>" % (w["C"], 8 if w["lattice"] == "fcc" else 4, il_group_cells(p.dims[0], w["C"]))
     return {"metric": "lattice-site-updates/s", "value": sites * inner * steps / (total_ms * 1e-3),
             "unit": "lattice-site-updates/s", "steps": steps, "inner_steps_per_step": inner, "sites": sites,
             "ms_per_step": total_ms / steps, "dims": list(p.dims),
@@ -175,10 +175,14 @@ def time_leg(w, steps, inner, warmup, kernel=0, dims=None):
             "norm_last": obs[-1]["norm"] if obs else None}
 
 
-def il_group_cells(x):
-    """Cells per group of the interleaved layout for an x edge (the library's rule:
-    32 unless 16 leaves fewer lanes idle)."""
-    return 32 if 32 * ((x + 31) // 32) <= 16 * ((x + 15) // 16) else 16
+def il_group_cells(x, components):
+    """Cells per group of the interleaved layout for an x edge (the library's rule: by the
+    lanes left idle and what narrower groups cost)."""
+    def cost(cells, percent):
+        return (x + cells - 1) // cells * cells * percent
+
+    wide = min((cost(32, 100), 0, 32), (cost(16, 103), 1, 16))
+    return 8 if cost(8, 115 if components == 3 else 106) < wide[0] else wide[2]
 
 
 def leg_e2e(w, steps, inner, dims=None, flight=1):

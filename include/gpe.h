@@ -394,17 +394,24 @@ gpe_status gpe_node_fields_reduce(gpe_handle* h, int32_t slot, int32_t kind, dou
  *                      slots (and q) into a cell-interleaved layout (node l,
  *                      component s of 32, 16 or 8 cells along x contiguous), steps
  *                      there and changes them back; the states are those of the
- *                      gather kernel, bit for bit.  Single explicit steps
- *                      (gpe_step_explicit, imaginary time) take the gather kernel.
+ *                      gather kernel, bit for bit.  gpe_itp follows the same rule for
+ *                      its iterations before the last (parabolic scheme), where the
+ *                      layout's buffers are there or can be had; gpe_step_explicit
+ *                      takes the gather kernel.
  *                  The automatic choice (0) is the interleaved kernel for calls of
  *                  16 or more steps on the parabolic spinor handles and the
- *                  hyperbolic handles it applies to (faster there by 12-50 %; not
+ *                  hyperbolic handles it applies to (faster there by 20-70 %; not
  *                  for parabolic scalars, whose 8-byte records already load as
  *                  coalesced runs; the layout changes cost a few steps per
  *                  call), else 1 (grid-stride gather, whole-record loads) -- which
  *                  gpe_get_tuning reports; 2-5 on request, and gpe_autotune may
  *                  pick any of 1-4 (it times single steps; its gather candidate is
- *                  recorded as 0).
+ *                  recorded as 0).  Under 0, FP32 split-scheme calls of 16 or more
+ *                  steps on lattices with 4 edges per node and 2 per node of a cell
+ *                  keep R, I, q_R and q_I in interleaved planes of their own (twice
+ *                  the state's memory, on first use; without it, or in a stream that
+ *                  is being captured before it, the call stays in the handle's
+ *                  layout), with the same states bit for bit.
  * GPE_TUNE_TILE_CELLS: cells per tile row (0 = automatic).
  * GPE_TUNE_TILE_ROWS: rows per tile along y (z-march TY, row-block RY; 0 = automatic).
  * GPE_TUNE_ZCHUNK: z-march planes per block, or row-block RZ (0 = automatic).
@@ -412,8 +419,10 @@ gpe_status gpe_node_fields_reduce(gpe_handle* h, int32_t slot, int32_t kind, dou
  *                   thread loops over the block's nodes; 0 = automatic).
  * GPE_TUNE_OBSERVE_ARITH: arithmetic of gpe_observe's per-node terms on an FP32
  *                   handle: 0 = FP64 (default; the same numbers as an FP64 run
- *                   on the stored values), 1 = FP32.  The sums over nodes are FP64
- *                   either way; mode 0 is bound by GB300's narrow FP64 pipe.
+ *                   on the stored values: sums over columns of nodes in exact pairs
+ *                   of FP32 values, as near to sums in extended precision as FP64
+ *                   terms are; FP64 terms where |psi| leaves 2^-20 .. 2^27), 1 = FP32
+ *                   terms.  The sums over nodes are FP64 either way.
  * GPE_TUNE_CARVEOUT: shared-memory share (percent) of the unified L1 / shared
  *                   memory for the row-tile kernel; the rest caches its off-row
  *                   gathers (0 = driver default).
@@ -441,7 +450,8 @@ gpe_status gpe_set_tuning(gpe_handle* h, int32_t key, int32_t value);
 gpe_status gpe_get_tuning(const gpe_handle* h, int32_t key, int32_t* value);
 
 /* Device time of the gpe_step / gpe_step_observe calls made while GPE_TUNE_TIMING
- * was 1, from CUDA events on the calls' streams: the plain step launches, the
+ * was 1, from CUDA events on the calls' streams: the plain step launches (a split
+ * call's layout changes among them), the
  * observed steps (their finalize included) and the layout changes of interleaved
  * calls.  `reset` non-zero zeroes the sums after reading.  No counterpart in the
  * reference (its programs time whole loops with host clocks). */

@@ -2,8 +2,8 @@
 ``torch.autograd.Function``.
 
 The forward and the reverse run happen in libgpe (``gpe_adjoint_forward`` /
-``gpe_adjoint_backward``: CUDA step and adjoint kernels, sqrt(N) checkpoints with
-recomputation).  torch only carries the chain rule from the per-step fields to
+``gpe_adjoint_backward``: CUDA step and adjoint kernels, every state kept or
+checkpoints with recomputation).  torch only carries the chain rule from the per-step fields to
 whatever parametrises them, here piecewise-linear knots of Bz(t) and of the
 quadrupole gradient Bq(t).  The reference has no differentiable path; its ramps
 are fixed tables (Spin1GpeBCC/AliceRingRamps.h:74-141, KnotRamps.h:64-135).

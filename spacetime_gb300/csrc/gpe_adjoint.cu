@@ -1,5 +1,6 @@
 // gpe_adjoint.cu -- reverse-mode (adjoint) derivative of the parabolic leapfrog
-// run with respect to the per-step magnetic fields, with sqrt(N) checkpointing.
+// run with respect to the per-step magnetic fields, with every state kept or
+// checkpoints.
 //
 // Forward run of N steps from u_0 (the reference's time loop, Spin1GpeBCC.cu:1428-1603):
 //     u_1     = u_0 + (1/2) F_0(u_0)                    forwardEuler, :667-791
@@ -21,9 +22,11 @@
 //
 // Checkpointing: the forward run keeps (u_{kS}, u_{kS+1}) for every segment k of
 // S steps; the reverse run recomputes one segment at a time from its pair with the
-// forward step kernel itself (bit-identical states; with the gather kernel out of
-// place, u_{j+1} = u_{j-1} + F(u_j) into a fresh buffer) and walks it backwards.
-// Memory: 2 ceil(N/S) + S - 2 state buffers; S = ceil(sqrt(N)) by default.
+// forward step kernel itself (bit-identical states: interleaved runs with
+// il_step_from_kernel, others with the gather kernel out of place, u_{j+1} = u_{j-1} +
+// F(u_j) into a fresh buffer) and walks it backwards.  Memory: 2 ceil(N/S) + S - 2 state
+// buffers.  Without a given S, all N states where they fit (keep_states), else S =
+// ceil(sqrt(N)).
 #include <algorithm>
 #include <cmath>
 #include <cstring>

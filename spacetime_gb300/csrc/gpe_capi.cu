@@ -1295,11 +1295,13 @@ static bool il_applies(const gpe_handle* h) {
 }
 
 // Where the automatic choice takes the interleaved kernel, by measurement (FP32
-// leapfrog, one launch, fraction of the measured copy peak, gather / interleaved;
-// BCC 96^3, A15 64^3, C15 48^3, Z 56^3): spin-1 BCC 0.68 / 0.85, A15 0.63 / 0.85,
-// C15 0.62 / 0.70, Z 0.66 / 0.77; spin-2 BCC 0.66 / 0.89, A15 0.59 / 0.88, C15
-// 0.60 / 0.72, Z 0.64 / 0.79.  Not for scalars (BCC 0.68 / 0.51, C15 0.64 / 0.40:
-// an 8-byte record already loads as one coalesced run in the handle's layout).
+// leapfrog, one step of forty, fraction of the measured copy peak, gather /
+// interleaved; BCC and FCC 96^3, A15 64^3, C15 48^3, Z 56^3): spin-1 BCC 0.71 / 0.92,
+// FCC 0.43 / 0.64, A15 0.64 / 0.91, C15 0.64 / 0.89, Z 0.69 / 0.83; spin-2 BCC 0.65 /
+// 0.93, FCC 0.47 / 0.68, A15 0.58 / 0.92, C15 0.59 / 0.88, Z 0.63 / 0.83.  Not for
+// scalars (BCC 0.73 / 0.64, FCC 0.49 / 0.39, A15 0.68 / 0.64, C15 0.68 / 0.61, Z 0.72 /
+// 0.59; BCC 32^3 4.1 / 4.2 us, C15 41^3 50 / 65 us: an 8-byte record already loads as
+// one coalesced run in the handle's layout).
 static bool il_auto(const gpe_handle* h) { return h->g.C >= 3; }
 
 // The q slots' geometry as a Grid whose "nodes" are the E edges of a cell.
@@ -1332,9 +1334,9 @@ static bool il_hyper_applies(const gpe_handle* h) {
 
 // Where the automatic choice takes the interleaved hyperbolic step: everywhere it
 // applies, by measurement (FP32, one fused launch, fraction of the measured copy
-// peak, gather / row tile / interleaved): scalar BCC 128^3 0.64 / 0.46 / 0.71,
-// spin-1 BCC 96^3 0.56 / 0.74 / 0.97, C15 40^3 0.57 / 0.51 / 0.80, spin-2 BCC 96^3
-// 0.77 / 0.69 / 0.99, C15 48^3 0.75 / 0.67 / 0.93, C15 128^3 0.69 / 0.69 / 0.86.
+// peak, gather / row tile / interleaved): scalar BCC 128^3 0.66 / 0.46 / 0.73, C15
+// 40^3 0.67 / 0.39 / 0.70, spin-1 BCC 96^3 0.51 / 0.74 / 0.99, C15 40^3 0.52 / 0.51 /
+// 0.90, spin-2 BCC 96^3 0.77 / 0.69 / 1.01, C15 48^3 0.73 / 0.68 / 0.97.
 static bool il_hyper_auto(const gpe_handle*) { return true; }
 
 static bool use_interleaved(const gpe_handle* h, int32_t n) {

@@ -224,9 +224,10 @@ struct ILWalk {
 // of prev go.  With a NormAcc for oa: an imaginary-time iteration (kModeItpNorm), next =
 // prev - dt H prev with prev read times inv.
 //
-// What bounds the plain step is the instruction count and the latency of the loads
-// together (spin-1 BCC 96^3: warps issue on 63 % of the cycles, DRAM at 72 %), so
-// nothing is computed here that is the same for the whole launch or row.
+// What bounds the plain step is the latency of the loads and the instructions between
+// them (spin-1 BCC 96^3: warps issue on 51 % of the cycles, on 63 % before the local terms
+// were multiply-adds, DRAM at 75 %), so nothing is computed here that is the same for the
+// whole launch or row.
 template <int C, int D, int CELLS, class OA>
 __device__ __forceinline__ void il_task(const PhysR<float>& P, const PhysR<float>* F, const char* prev, char* next,
                                         const char* old, uint32_t own, const int32_t* off, uint32_t outside, int32_t zero, const float* w,

@@ -4,7 +4,8 @@
 // GB300 runs one FP64 operation for every 64 FP32 ones, and a conversion from FP32
 // costs as much as an FP64 operation: with per-node terms in FP64, observe_kernel
 // spent 290 FP64 operations on a spin-1 node and ran at 87 % of the FP64 pipe with
-// DRAM at 1 % (1463 us on spin-1 BCC 64^3, whose state is read in 11 us).  Here
+// DRAM at 1 % (1463 us on spin-1 BCC 64^3, whose state is read in 11 us; this form
+// takes 140 us, bound by the FP32 instructions of the exact sums).  Here
 //  - everything that is the same for a column of cells -- the stencil weights, the
 //    trap, the fields, the coupling constants, the position -- is left out of the
 //    per-node terms and multiplied in once per column, in FP64;
@@ -13,7 +14,9 @@
 //    sums are PairSum's and, for terms of one sign, TripleSum's), plain FP64 for FP64
 //    storage.
 // A pair keeps 47 bits or more of each node's term, and the errors of different nodes
-// are independent, so that the sums carry the error of their FP64 additions.  Measured
+// are independent, so that the sums carry the error of their FP64 additions.  (Densities
+// in FP64 node by node instead of three FP32 words: observables, density and spin sums of
+// that state together 487 us against 335.)  Measured
 // against sums in more than 64 bits on Thomas-Fermi clouds and noise (BCC 12^3 .. 24^3,
 // C15 9^3; root mean square, relative): norm 1e-16 to 2.5e-16, centre of mass 1e-16 to
 // 3e-16, energy 1e-16 to 3e-16, M_z 1e-16 to 2e-16, |F| 1e-16 -- observe_kernel's are 1e-16
