@@ -65,7 +65,7 @@ LEGS["scalar-split-c15-64"] = dict(lattice="c15", C=1, dims=(64, 64, 64), c0=200
                                    scheme=2, sigma=0.00225, zeta=(1.0,), kappa=1, noise_abs=1e-3, noise_rel=0.0,
                                    bytes_fp32=72, seed=7)
 KERNEL_OF_SCHEME = {0: "leapfrog kernel (auto) C=%d", 1: "hyper_tile_kernel<float,%d> (fused tile)",
-                    2: "il_split_kernel<PART,CELLS> (C=%d, two launches per step)"}
+                    2: "line_split_kernel<PART> (C=%d, two launches per step)"}
 
 
 def workload(precision):

@@ -408,8 +408,8 @@ gpe_status gpe_node_fields_reduce(gpe_handle* h, int32_t slot, int32_t kind, dou
  *                  pick any of 1-4 (it times single steps; its gather candidate is
  *                  recorded as 0).  Under 0, FP32 split-scheme calls of 16 or more
  *                  steps on lattices with 4 edges per node and 2 per node of a cell
- *                  keep R, I, q_R and q_I in interleaved planes of their own (twice
- *                  the state's memory, on first use; without it, or in a stream that
+ *                  keep R, I, q_R and q_I in planes of their own (about the
+ *                  state's memory again, on first use; without it, or in a stream that
  *                  is being captured before it, the call stays in the handle's
  *                  layout), with the same states bit for bit.
  * GPE_TUNE_TILE_CELLS: cells per tile row (0 = automatic).

@@ -68,7 +68,7 @@ cudaError_t launch_split_planes(const StepArgs& a, int part, char* const planes[
 cudaError_t launch_split_planes_convert(char* psi, char* q, char* const planes[4], const Grid& g, bool to_planes, cudaStream_t s);
 size_t split_plane_bytes(const Grid& g, bool q);
 bool split_planes_fit(const Grid& g);
-bool split_plane_table(const Grid& g, const gpe_incidence* inc, const gpe_edge* edges, std::vector<int32_t>& tab);
+void split_plane_table(const Grid& g, const gpe_incidence* inc, const gpe_edge* edges, std::vector<int32_t>& tab);
 template <int C>
 cudaError_t launch_il_hyper(const StepArgs& a, const ILGrid& G, const ILGrid& Gq, const int32_t* tab, cudaStream_t s);
 enum HyperKind {
@@ -1420,7 +1420,7 @@ static gpe_status ensure_il_hyper(gpe_handle* h, cudaStream_t s) {
     return GPE_OK;
 }
 
-// Whether a split-scheme call of n steps runs on interleaved planes (gpe_split.cuh): FP32,
+// Whether a split-scheme call of n steps runs on planes (gpe_split.cuh): FP32,
 // the automatic kernel choice, calls long enough for the layout changes (one change
 // in and one out cost about one step), 4 edges per node and 2 per node of a cell within
 // adjacent cells, and the planes' memory to be had now (twice the state's; not while the
@@ -1436,7 +1436,7 @@ static bool split_planes_ready(gpe_handle* h, int32_t n, cudaStream_t s) {
     for (const gpe_incidence& r : h->lat.incidence)
         if (!adj(r.dx, r.dy, r.dz)) return false;
     std::vector<int32_t> tab;
-    if (!split_plane_table(g, h->lat.incidence.data(), h->lat.edges.data(), tab)) return false;
+    split_plane_table(g, h->lat.incidence.data(), h->lat.edges.data(), tab);
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
     void* t = nullptr;
@@ -1447,7 +1447,7 @@ static bool split_planes_ready(gpe_handle* h, int32_t n, cudaStream_t s) {
         void* p = nullptr;
         ok = cudaMalloc(&p, bytes) == cudaSuccess;
         h->planes[k] = static_cast<char*>(p);
-        // the halo rows and the padding cells stay zero
+        // the cells around the grid stay zero
         ok = ok && cudaMemsetAsync(p, 0, bytes, s) == cudaSuccess;
     }
     if (!ok) {

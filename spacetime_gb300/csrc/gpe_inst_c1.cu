@@ -47,39 +47,30 @@ cudaError_t launch_split_planes(const StepArgs& a, int part, char* const planes[
                                 cudaStream_t s) {
     // planes: R, I, q_R, q_I
     const SplitPlanes p = {planes[part], planes[1 - part], planes[2 + part], planes[3 - part]};
-    return launch_il_split(a, part, p, make_plane_grid(g, g.V), make_plane_grid(g, g.E), tab, s);
+    return launch_line_split(a, part, p, make_line_grid(g, g.V), make_line_grid(g, g.E), tab, s);
 }
 cudaError_t launch_split_planes_convert(char* psi, char* q, char* const planes[4], const Grid& g, bool to_planes, cudaStream_t s) {
-    const cudaError_t e = launch_split_convert(psi, g.pitch, g.slice, g.cell_bytes, planes[0], planes[1], make_plane_grid(g, g.V),
+    const cudaError_t e = launch_split_convert(psi, g.pitch, g.slice, g.cell_bytes, planes[0], planes[1], make_line_grid(g, g.V),
                                                to_planes, false, s);
     if (e != cudaSuccess) return e;
-    return launch_split_convert(q, g.qpitch, g.qslice, g.qcell_bytes, planes[2], planes[3], make_plane_grid(g, g.E), to_planes, true,
+    return launch_split_convert(q, g.qpitch, g.qslice, g.qcell_bytes, planes[2], planes[3], make_line_grid(g, g.E), to_planes, true,
                                 s);
 }
-size_t split_plane_bytes(const Grid& g, bool q) { return make_plane_grid(g, q ? g.E : g.V).bytes; }
-bool split_planes_fit(const Grid& g) {
-    const ILGrid G = make_plane_grid(g, g.V), Gq = make_plane_grid(g, g.E);
-    return il_offsets_fit(G) && il_offsets_fit(Gq) && (uint64_t)il_warp_tasks(G) * G.V <= 0xffffffffu;
-}
-bool split_plane_table(const Grid& g, const gpe_incidence* inc, const gpe_edge* edges, std::vector<int32_t>& tab) {
-    const ILGrid G = make_plane_grid(g, g.V), Gq = make_plane_grid(g, g.E);
-    const int64_t run = (int64_t)G.cells * 4;   // bytes between nodes (edges) of a group
+size_t split_plane_bytes(const Grid& g, bool q) { return make_line_grid(g, q ? g.E : g.V).bytes; }
+bool split_planes_fit(const Grid& g) { return line_fits(make_line_grid(g, g.V)) && line_fits(make_line_grid(g, g.E)); }
+void split_plane_table(const Grid& g, const gpe_incidence* inc, const gpe_edge* edges, std::vector<int32_t>& tab) {
+    const LineGrid G = make_line_grid(g, g.V);
+    auto cells = [&](int dx, int dy, int dz) { return (dz * (int32_t)G.Yp + dy) * (int32_t)G.Xp + dx; };
     tab.clear();
-    auto put = [&](int64_t b, int dx) {
-        tab.push_back((int32_t)b | (dx + 1));
-        return b <= INT32_MAX - 3 && b >= INT32_MIN;
-    };
-    bool ok = true;
     for (uint32_t i = 0; i < 4 * g.V; ++i) {
-        const gpe_incidence& r = inc[i];
-        ok = put(((int64_t)r.dz * (Gq.Y + 2) + r.dy) * (int64_t)Gq.row + (int64_t)r.edge * run + (int64_t)r.dx * 4, r.dx) && ok;
+        tab.push_back(cells(inc[i].dx, inc[i].dy, inc[i].dz));
+        tab.push_back((int32_t)inc[i].edge);
     }
     for (uint32_t i = 0; i < g.E; ++i) {
-        const gpe_edge& e = edges[i];
-        ok = put(((int64_t)e.dz * (G.Y + 2) + e.dy) * (int64_t)G.row + (int64_t)e.to * run + (int64_t)e.dx * 4, e.dx) && ok;
+        tab.push_back(cells(edges[i].dx, edges[i].dy, edges[i].dz));
+        tab.push_back((int32_t)edges[i].to);
     }
-    for (uint32_t i = 0; i < g.E; ++i) tab.push_back((int32_t)(edges[i].from * run));
-    return ok;
+    for (uint32_t i = 0; i < g.E; ++i) tab.push_back((int32_t)edges[i].from);
 }
 GPE_DEFINE_IL_CONVERT
 }  // namespace gpe

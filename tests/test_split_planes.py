@@ -1,4 +1,4 @@
-"""The split scheme's calls of 16 or more steps on interleaved planes against the same
+"""The split scheme's calls of 16 or more steps on planes of cells in a line against the same
 steps in the handle's layout (the gather kernel on request), bit for bit."""
 import numpy as np
 import pytest
@@ -9,7 +9,7 @@ from spacetime_gb300.stepper import Stepper
 pytestmark = pytest.mark.gpu
 
 
-# group widths 32, 16 and 8, rows that end on a group's edge and around it
+# rows that end on a group of 32 cells, before and after it; lines of less than a group
 @pytest.mark.parametrize("name,dims", [("c15", (36, 2, 2)), ("c15", (2, 3, 2)), ("bcc", (32, 3, 2)), ("bcc", (33, 2, 3)),
                                        ("bcc", (31, 2, 2)), ("bcc", (12, 3, 3)), ("bcc", (8, 2, 2)), ("bcc227", (40, 3, 2)),
                                        ("bcc", (1, 1, 1)), ("bcc", (64, 2, 2))])
