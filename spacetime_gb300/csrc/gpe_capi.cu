@@ -1002,12 +1002,17 @@ static cudaError_t dispatch_tile(const gpe_handle* h, const StepArgs& a, uint32_
 // Hyperbolic row-tile kernel eligibility and tile length (0 = gather kernel).
 static uint32_t hyper_tile_cells(const gpe_handle* h) {
     if (h->tune_kernel == 1 || h->g.E == 0) return 0;
-    // the automatic choice, by measurement (fraction of peak, gather against tile):
-    // scalars BCC 128^3 0.64 / 0.45, C15 40^3 0.60 / 0.39; spin-2 C15 128^3 0.69 /
-    // 0.69, C15 48^3 0.75 / 0.71, BCC 96^3 0.77 / 0.69; spin-1 C15 40^3 0.55 / 0.51
-    // -- the gather kernel; spin-1 BCC 96^3 0.56 / 0.74 -- the tile.  The tile
-    // is chosen for spin-1 on small cells (V <= 16) and on request.
-    if (h->tune_kernel != 2 && !(h->g.C == 3 && h->g.V <= 16)) return 0;
+    // the automatic choice, by measurement (us a step, gather against tile): FP32 scalars
+    // BCC 96^3 166 / 241, C15 40^3 136 / 240; spin-1 BCC 96^3 415 / 458, 64^3 125 / 135, 32^3
+    // 17 / 22, 12^3 3.7 / 7.7, BCC-227 40^3 33 / 46, C15 40^3 341 / 542; spin-2 BCC 96^3 720 /
+    // 813, C15 40^3 614 / 677; FP64 spin-1 C15 40^3 2169 / 3482, BCC 96^3 2650 / 3876, 20^3
+    // 36 / 39, 14^3 18.2 / 18.5 -- the gather kernel; FP64 spin-1 BCC 12^3 16.9 / 14.3, cube
+    // 120^3 1138 / 575, 40^3 54 / 40 -- the tile.  The tile is chosen for spin-1 on small
+    // cells (V <= 16) where the grid is small, FP64 below 25000 nodes and FP32 below 2048 (a
+    // step is all launch and latency there), for FP64 spin-1 on the cube, and on request.
+    const uint64_t nodes = (uint64_t)h->g.X * h->g.Y * h->g.Z * h->g.V;
+    const bool few = nodes < (h->real_bytes == 8 ? 25000u : 2048u);
+    if (h->tune_kernel != 2 && !(h->g.C == 3 && h->g.V <= 16 && (few || (h->real_bytes == 8 && h->g.V == 1)))) return 0;
     if (h->g.cell_bytes % 16 != 0 || h->g.qcell_bytes % 16 != 0) return 0;
     const uint32_t per = h->g.V + h->g.E;
     const size_t tables = (size_t)h->g.V * h->lat.F * (8 + h->real_bytes) + (size_t)(3 * h->g.E + 1) * 4 +

@@ -151,7 +151,10 @@ __device__ __forceinline__ void st_node(char* p, const Cx<R>* v) {
 // finish.  Measured per step, let in / not: gather kernel, scalar C15 41 x 37 x 35 39.3 /
 // 40.6 us, split C15 36^3 194 / 199, scalar BCC 32^3 3.97 / 3.85; interleaved kernels
 // (no tables to stage) equal or slower, imaginary time 2 % slower.  (Deciding it by the
-// grid's size inside the kernel cost 10-25 % of the scalar steps.)
+// grid's size inside the kernel cost 10-25 % of the scalar steps.)  Not in FP64, whose grids
+// of a wave or two then fall unevenly on the SMs, let in / not: scalar FCC 24^3 31.8 / 24.6
+// us, cube 40^3 15.4 / 8.9, spin-1 FCC 12^3 25.6 / 14.8, hyperbolic scalar BCC 16^3 13.2 / 8.3,
+// split BCC 16^3 20.0 / 12.9; larger grids equal.
 __device__ __forceinline__ void let_next_kernel_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <bool LET_IN>
 __device__ __forceinline__ void after_previous_kernel() {
@@ -1029,7 +1032,7 @@ __device__ __forceinline__ void parabolic_step_body(const StepArgs& a) {
     __shared__ SmemTables<R> st;
     load_tables<R>(st, a);
     __syncthreads();
-    after_previous_kernel<true>();
+    after_previous_kernel<sizeof(R) == 4>();
     const PhysR<R>& P = make_phys<R>(a);
     using OA = typename AccOf<MODE, OBS, R>::type;
     __shared__ double obs_sums[OBS ? kObsSums * 256 : 1];
@@ -1075,7 +1078,7 @@ __device__ __forceinline__ void parabolic_fixed_body(const StepArgs& a) {
     __shared__ SmemTables<R> st;
     load_tables<R>(st, a);
     __syncthreads();
-    after_previous_kernel<true>();
+    after_previous_kernel<sizeof(R) == 4>();
     const PhysR<R>& P = make_phys<R>(a);
     constexpr bool kAll = OBS || MODE == kModeItpNorm;   // every thread takes part in the block's sums
     using OA = typename AccOf<MODE, OBS, R>::type;
@@ -1118,7 +1121,7 @@ __global__ void __launch_bounds__(256) parabolic_columns_kernel(StepArgs a, uint
     __shared__ SmemTables<R> st;
     load_tables<R>(st, a);
     __syncthreads();
-    after_previous_kernel<true>();
+    after_previous_kernel<sizeof(R) == 4>();
     const PhysR<R>& P = make_phys<R>(a);
     using OA = typename AccOf<MODE, false, R>::type;
     OA oa = AccOf<MODE, false, R>::make(nullptr);
@@ -1262,6 +1265,11 @@ __device__ __forceinline__ void q_update(const StepArgs& a, const SmemHyper<R>& 
 // grid strides over these `vblocks` item blocks on one wave, so that each block
 // stages the tables once.
 // DO_PSI: psi update with MODE and HYPERB (-c_K scaling); QM < 0: no q update.
+//
+// Bound by the loads' latency: the old psi_next record is loaded with the others, not after
+// the local terms, which took the spin-1 step on C15 40^3 from 487 to 341 us (0.57 to 0.81
+// of the copy peak), BCC 96^3 from 603 to 414 (0.82), cube 120^3 165 to 160; scalar BCC 96^3
+// 172 to 166.
 template <typename R, int C, bool DO_PSI, int MODE, bool HYPERB, int QM>
 __global__ void __launch_bounds__(256) hyper_step_kernel(StepArgs a, uint32_t node_items, uint32_t edge_items,
                                                          uint32_t ratio, uint32_t vblocks) {
@@ -1282,7 +1290,11 @@ __global__ void __launch_bounds__(256) hyper_step_kernel(StepArgs a, uint32_t no
     }
     __syncthreads();
 
-    after_previous_kernel<true>();
+    // Old psi_next up front: FP32 scalars and spin-1 only.  Spin-2 on C15 40^3 went from 612 to
+    // 897 us with it, BCC 64^3 from 222 to 325 (cube 90^3 146 to 131), FP64 spin-1 BCC 64^3 from
+    // 925 to 1708.  Letting the next kernel in cost spin-2 2 %.
+    constexpr bool kEarly = MODE == GPE_MODE_LEAPFROG && sizeof(R) == 4 && C < 5;
+    after_previous_kernel<sizeof(R) == 4 && (C < 5)>();
     for (uint32_t vb = blockIdx.x; vb < vblocks; vb += gridDim.x) {
     uint32_t group, sub;
     if (DO_PSI && QM >= 0) {
@@ -1311,6 +1323,9 @@ __global__ void __launch_bounds__(256) hyper_step_kernel(StepArgs a, uint32_t no
         const char* own = a.prev + cell_off + l * node_bytes;
         Cx<R> prv[C], H[C];
         ld_node<R, C>(own, prv);
+        char* nxt = a.next + cell_off + l * node_bytes;
+        Cx<R> nv[C];
+        if constexpr (kEarly) ld_node<R, C>(nxt, nv);
 #pragma unroll
         for (int s = 0; s < C; ++s) H[s] = cx<R>((R)0, (R)0);
         // d1 of q (RelativisticSpin2Gpe.cu:1051-1066), whole edge records
@@ -1346,7 +1361,13 @@ __global__ void __launch_bounds__(256) hyper_step_kernel(StepArgs a, uint32_t no
             local_spin2<R>(P, r, pot, MODE != GPE_MODE_ITP, false, HYPERB, prv, H);
         }
         char* hp = (MODE == GPE_MODE_ITP && a.hpsi) ? a.hpsi + cell_off + l * node_bytes : nullptr;
-        write_update<R, C>(MODE, P.dt, a.next + cell_off + l * node_bytes, hp, prv, H);
+        if constexpr (kEarly) {
+#pragma unroll
+            for (int s = 0; s < C; ++s) add_scaled(nv[s], (R)2 * P.dt, cx<R>(H[s].y, -H[s].x));
+            st_node<R, C>(nxt, nv);
+        } else {
+            write_update<R, C>(MODE, P.dt, nxt, hp, prv, H);
+        }
     } else if constexpr (QM >= 0) {
         const uint32_t eb = (DO_PSI ? group * ratio : 0) + (sub - 1);
         const uint32_t i = eb * blockDim.x + threadIdx.x;
@@ -1854,7 +1875,7 @@ __global__ void __launch_bounds__(256) split_step_kernel(StepArgs a, uint32_t no
         else sh.pos[i] = a.tab.pos64[i];
     }
     __syncthreads();
-    after_previous_kernel<true>();
+    after_previous_kernel<sizeof(R) == 4>();
     constexpr bool kNodes = PART != 2;
     const PhysR<R>& P = make_phys<R>(a);
     // the half read by the psi update and by d0 (R for PARTs 0 and 2, I for PART 1)
