@@ -1338,10 +1338,12 @@ static bool il_hyper_applies(const gpe_handle* h) {
 }
 
 // Where the automatic choice takes the interleaved hyperbolic step: everywhere it
-// applies, by measurement (FP32, one fused launch, fraction of the measured copy
-// peak, gather / row tile / interleaved): scalar BCC 128^3 0.66 / 0.46 / 0.73, C15
-// 40^3 0.67 / 0.39 / 0.70, spin-1 BCC 96^3 0.51 / 0.74 / 0.99, C15 40^3 0.52 / 0.51 /
-// 0.90, spin-2 BCC 96^3 0.77 / 0.69 / 1.01, C15 48^3 0.73 / 0.68 / 0.97.
+// applies, by measurement (FP32; us a step, gather / interleaved + a call's layout
+// changes): spin-2 BCC 96^3 720 / 559 + 1689, C15 40^3 615 / 500 + 1363, 24^3 137 / 114 + 299
+// (even at 8 to 13 steps); spin-1 BCC 96^3 414 / 341 + 1008, C15 40^3 341 / 309 + 810, 32^3 177 /
+// 150 + 448 (14 to 25); scalars BCC 96^3 166 / 157 + 431, C15 40^3 136 / 132 + 303 (47 and 76).
+// Calls that lose by it: spin-1 of 16 to 25 steps up to 10 %, scalars of 16 to 47 steps and
+// small grids (BCC 20^3 3.5 / 6.2, 6.0 / 8.2, 9.7 / 10.2); GPE_TUNE_KERNEL 1 avoids it there.
 static bool il_hyper_auto(const gpe_handle*) { return true; }
 
 static bool use_interleaved(const gpe_handle* h, int32_t n) {
