@@ -218,6 +218,14 @@ struct NodeTerms {
     }
 };
 
+// The largest |re|, |im| of the records so far (a NaN is none).
+template <typename R, int C>
+__device__ __forceinline__ R largest(R top, const Cx<R>* p) {
+#pragma unroll
+    for (int s = 0; s < C; ++s) top = fmax(top, fmax(fabs(p[s].x), fabs(p[s].y)));
+    return top;
+}
+
 template <typename R, int C>
 __device__ __forceinline__ uint32_t count_nonfinite(const Cx<R>* p) {
     uint32_t n = 0;
@@ -256,6 +264,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_k
     for (int k = 0; k < OBS_COUNT; ++k) acc[k] = 0.0;
     T top = A::zero();
     Cx<R> at = cx<R>((R)0, (R)0);
+    R big = (R)0;
     uint32_t nbad = 0;
     const uint32_t node_bytes = C * 2 * sizeof(R);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
@@ -299,6 +308,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_k
                 }
             }
             nbad += count_nonfinite<R, C>(p);
+            if constexpr (sizeof(R) == 4) big = largest<R, C>(big, p);
             const NodeTerms<R, C> t(p);
             t.track_max(p, top, at);
             const R zj = (R)((int32_t)j - (int32_t)mid);
@@ -393,7 +403,9 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_k
         acc[OBS_COMY] += ry * S0;
         acc[OBS_COMZ] += rz * S0 + (gz * S1 + gl * S1);
     }
-    acc[OBS_MAXABS] = sqrt((double)at.x * at.x + (double)at.y * at.y);
+    // FP32: densities that overflow, or all vanish, leave no record to track; the largest
+    // |re|, |im| (never above the modulus) then takes the state out of the pairs' range
+    acc[OBS_MAXABS] = fmax(sqrt((double)at.x * at.x + (double)at.y * at.y), (double)big);
     acc[OBS_NONFINITE] = (double)nbad;
     block_observables(acc, red, a.partials);
 }
@@ -434,10 +446,8 @@ __global__ void __launch_bounds__(256) field_sums_kernel(StepArgs a) {
                                 l * (C * 2 * sizeof(R)), v);
         Cx<A> p[C];
 #pragma unroll
-        for (int c = 0; c < C; ++c) {
-            p[c] = cx<A>((A)v[c].x, (A)v[c].y);
-            if constexpr (sizeof(A) == 4) top = fmaxf(top, fmaxf(fabsf(p[c].x), fabsf(p[c].y)));
-        }
+        for (int c = 0; c < C; ++c) p[c] = cx<A>((A)v[c].x, (A)v[c].y);
+        if constexpr (sizeof(A) == 4) top = largest<A, C>(top, p);
         const NodeTerms<A, C> t(p);
         O::add(density, t.density);
         if constexpr (SPIN && C > 1) {
