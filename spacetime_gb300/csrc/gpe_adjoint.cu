@@ -497,58 +497,75 @@ __global__ void __launch_bounds__(kSumThreads) adjoint_sum_kernel(const double* 
 
 constexpr int kFinalCount = 5;  // Re <T|u>, Im <T|u>, Mx, My, Mz
 
-// Final-state quantities: the overlap sum conj(T) u and the spin density sums, to FP64's
-// precision in pairs of FP32 values (gpe_observe.cuh) for FP32 storage.  a.prev = target
-// T, a.next = u_N.
-template <typename R, int C>
-__global__ void __launch_bounds__(256) adjoint_final_kernel(StepArgs a) {
-    using A = ObsArith<R>;
-    typename A::S s[kFinalCount] = {}, f6[2] = {};
-    typename A::E re_sum{}, fz{};   // of one sign where T is near u, and in polarised clouds
+// Final-state quantities of the thread's nodes: the overlap sum conj(T) u and the spin density
+// sums.  a.prev = target T, a.next = u_N.  A: the arithmetic's type; top_t, top_u: the largest
+// |re|, |im| of T and u.
+template <typename R, typename A, int C>
+__device__ __forceinline__ void final_sums(const StepArgs& a, double (&v)[kFinalCount], R& top_t, R& top_u) {
+    using O = ObsArith<A>;
+    typename O::S s[kFinalCount] = {}, f6[2] = {};
+    typename O::E re_sum{}, fz{};   // of one sign where T is near u, and in polarised clouds
     for (uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < a.total;
          gid += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t x, y, z, l;
         node_coords(a, (uint32_t)gid, x, y, z, l);
         const size_t off = (size_t)z * a.g.slice + (size_t)y * a.g.pitch + (size_t)x * a.g.cell_bytes +
                            l * (C * 2 * sizeof(R));
-        Cx<R> t[C], p[C];
-        ld_node<R, C, true>(a.prev + off, t);
-        ld_node<R, C, true>(a.next + off, p);
+        Cx<R> tr[C], pr[C];
+        ld_node<R, C, true>(a.prev + off, tr);
+        ld_node<R, C, true>(a.next + off, pr);
+        top_t = largest<R, C>(top_t, tr);
+        top_u = largest<R, C>(top_u, pr);
+        Cx<A> t[C], p[C];
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            A::add_prod(re_sum, t[c].x, p[c].x);
-            A::add_prod(re_sum, t[c].y, p[c].y);
-            A::add(s[1], A::cross2(t[c].x, p[c].y, t[c].y, p[c].x));
+            t[c] = cx<A>((A)tr[c].x, (A)tr[c].y);
+            p[c] = cx<A>((A)pr[c].x, (A)pr[c].y);
+            O::add_prod(re_sum, t[c].x, p[c].x);
+            O::add_prod(re_sum, t[c].y, p[c].y);
+            O::add(s[1], O::cross2(t[c].x, p[c].y, t[c].y, p[c].x));
         }
         if constexpr (C > 1) {
             // the spin densities' sums: spin-1 sqrt2 (chain of its components), spin-2 twice its outer
             // pairs and sqrt6 times its inner chain
-            const NodeTerms<R, C> n(p);
-            typename A::T re, im;
+            const NodeTerms<A, C> n(p);
+            typename O::T re, im;
             constexpr int b = C == 5 ? 1 : 0;
             n.chain(p[b], p[b + 1], p[b + 2], re, im);
             if constexpr (C == 3) {
-                A::add(s[2], re);
-                A::add(s[3], im);
-                A::add(fz, n.template fz<0>());
+                O::add(s[2], re);
+                O::add(s[3], im);
+                O::add(fz, n.template fz<0>());
             } else {
-                A::add(f6[0], re);
-                A::add(f6[1], im);
-                A::add(s[2], A::dot2(p[0].x, p[1].x, p[0].y, p[1].y) + A::dot2(p[3].x, p[4].x, p[3].y, p[4].y));
-                A::add(s[3], A::cross2(p[0].x, p[1].y, p[0].y, p[1].x) + A::cross2(p[3].x, p[4].y, p[3].y, p[4].x));
-                A::add(fz, n.template fz<0>());
+                O::add(f6[0], re);
+                O::add(f6[1], im);
+                O::add(s[2], O::dot2(p[0].x, p[1].x, p[0].y, p[1].y) + O::dot2(p[3].x, p[4].x, p[3].y, p[4].y));
+                O::add(s[3], O::cross2(p[0].x, p[1].y, p[0].y, p[1].x) + O::cross2(p[3].x, p[4].y, p[3].y, p[4].x));
+                O::add(fz, n.template fz<0>());
             }
         }
     }
-    double v[kFinalCount];
 #pragma unroll
-    for (int k = 0; k < kFinalCount; ++k) v[k] = A::value(s[k]);
-    v[0] = A::value(re_sum);
-    v[4] = A::value(fz);
+    for (int k = 0; k < kFinalCount; ++k) v[k] = O::value(s[k]);
+    v[0] = O::value(re_sum);
+    v[4] = O::value(fz);
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         if constexpr (C == 3) v[2 + k] *= GPE_REF_SQRT_2;
-        if constexpr (C == 5) v[2 + k] = 2.0 * v[2 + k] + 2.449489742783178098 * A::value(f6[k]);
+        if constexpr (C == 5) v[2 + k] = 2.0 * v[2 + k] + 2.449489742783178098 * O::value(f6[k]);
+    }
+}
+
+// To FP64's precision in words of FP32 (gpe_observe.cuh) for FP32 storage; a thread whose values
+// leave their range adds its nodes once more in FP64.
+template <typename R, int C>
+__global__ void __launch_bounds__(256) adjoint_final_kernel(StepArgs a) {
+    double v[kFinalCount];
+    R top_t = (R)0, top_u = (R)0;
+    final_sums<R, R, C>(a, v, top_t, top_u);
+    if constexpr (sizeof(R) == 4) {
+        if (!products_hold(top_t, top_u) || (C > 1 && !products_hold(top_u, top_u)))
+            final_sums<R, double, C>(a, v, top_t, top_u);
     }
     block_partials<kFinalCount, double>(v, 1.0, a.partials);
 }

@@ -706,6 +706,13 @@ __device__ __forceinline__ Pair two_prod(float a, float b) {
     r.l = __fmaf_rn(a, b, -r.h);
     return r;
 }
+// Whether exact products of two FP32 factors (two_prod) of up to a and b in magnitude keep their
+// low words and stay finite when they are summed: from 2^-100, whose low word's last bit is 2^-147,
+// to 2^100.
+__device__ __forceinline__ bool products_hold(float a, float b) {
+    const float p = a * b;
+    return (p >= 0x1p-100f && p <= 0x1p100f) || a == 0.f || b == 0.f;
+}
 // A sum in three FP32 words, for terms that all have one sign: a pair's low word rounds,
 // and for sums of squares not evenly (the square of an odd integer is 1 modulo 8, so its
 // last bits are dropped downwards more often than upwards): 3e-16 to 8e-16 of the norm of
