@@ -2030,12 +2030,10 @@ cudaError_t launch_scale(const StepArgs& a, cudaStream_t s) {
 
 namespace gpe {
 
-// sum_interior Re(conj(a) b) into scale_out->sum (innerProduct, Spin1GpeBCC.cu:
-// 213-233); a = StepArgs::prev, b = StepArgs::next.  FP32 storage: a sum in three words per
-// thread.
-template <typename R, int C>
-__global__ void __launch_bounds__(256) dot_kernel(StepArgs a) {
-    __shared__ double red[8];
+// sum Re(conj(a) b) over the thread's nodes; a = StepArgs::prev, b = StepArgs::next.  FP64: in
+// FP64, else a sum in three FP32 words.  top_a, top_b: the largest |re|, |im| of a and b.
+template <typename R, int C, bool FP64>
+__device__ __forceinline__ double dot_sum(const StepArgs& a, R& top_a, R& top_b) {
     double acc = 0;
     TripleSum sum;
     for (uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < a.total;
@@ -2051,18 +2049,31 @@ __global__ void __launch_bounds__(256) dot_kernel(StepArgs a) {
         Cx<R> u[C], v[C];
         ld_node<R, C, true>(a.prev + off, u);
         ld_node<R, C, true>(a.next + off, v);
-        if constexpr (sizeof(R) == 8) {
 #pragma unroll
-            for (int s = 0; s < C; ++s) acc += u[s].x * v[s].x + u[s].y * v[s].y;
-        } else {
-#pragma unroll
-            for (int s = 0; s < C; ++s) {
+        for (int s = 0; s < C; ++s) {
+            if constexpr (FP64) {
+                acc += (double)u[s].x * (double)v[s].x + (double)u[s].y * (double)v[s].y;
+            } else {
                 sum.add_prod(u[s].x, v[s].x);
                 sum.add_prod(u[s].y, v[s].y);
+                top_a = fmax(top_a, fmax(fabs(u[s].x), fabs(u[s].y)));
+                top_b = fmax(top_b, fmax(fabs(v[s].x), fabs(v[s].y)));
             }
         }
     }
-    if constexpr (sizeof(R) == 4) acc = sum.value();
+    return FP64 ? acc : sum.value();
+}
+
+// sum_interior Re(conj(a) b) into scale_out->sum (innerProduct, Spin1GpeBCC.cu:213-233).  A
+// thread whose FP32 products leave the range of their sum adds its nodes once more in FP64.
+template <typename R, int C>
+__global__ void __launch_bounds__(256) dot_kernel(StepArgs a) {
+    __shared__ double red[8];
+    R top_a = (R)0, top_b = (R)0;
+    double acc = dot_sum<R, C, sizeof(R) == 8>(a, top_a, top_b);
+    if constexpr (sizeof(R) == 4) {
+        if (!products_hold(top_a, top_b)) acc = dot_sum<R, C, true>(a, top_a, top_b);
+    }
     acc = NormAcc<R>::warp_sum(acc);
     NormAcc<R>::grid_sum(acc, red, a.partials, a.dv, a.scale_out);
 }
