@@ -243,6 +243,7 @@ __device__ __forceinline__ void il_task(const PhysR<float>& P, const PhysR<float
         prv[s] = ldc<float>(pp + s * kComp);
         if constexpr (!kItp) nv[s] = ldc<float>(old + own + s * kComp);
     }
+    if constexpr (kItp) scale_record(prv, C, inv);
 #pragma unroll
     for (int s = 0; s < C; ++s) H[s] = cx<float>(0.f, 0.f);
     // DEC Laplacian, sum_f w_f (psi_nb - psi) in entry order (Spin1GpeBCC.cu:835-865),
@@ -259,13 +260,10 @@ __device__ __forceinline__ void il_task(const PhysR<float>& P, const PhysR<float
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
+            if constexpr (kItp) scale_record(v[k], C, inv);
 #pragma unroll
             for (int s = 0; s < C; ++s) add_scaled(H[s], w[k0 + k], v[k][s] - prv[s]);
         }
-    }
-    if constexpr (kItp) {
-        scale_record(prv, C, inv);
-        scale_record(H, C, inv);
     }
     // local terms and the leapfrog update, as node_finish
     float rr[3];
