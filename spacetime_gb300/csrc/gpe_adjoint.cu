@@ -503,8 +503,9 @@ constexpr int kFinalCount = 5;  // Re <T|u>, Im <T|u>, Mx, My, Mz
 template <typename R, typename A, int C>
 __device__ __forceinline__ void final_sums(const StepArgs& a, double (&v)[kFinalCount], R& top_t, R& top_u) {
     using O = ObsArith<A>;
-    typename O::S s[kFinalCount] = {}, f6[2] = {};
-    typename O::E re_sum{}, fz{};   // of one sign where T is near u, and in polarised clouds
+    typename O::S mx{}, my{};
+    // of one sign where T is near u, and in polarised clouds; Im <T|u> is what is left of its products
+    typename O::E re_sum{}, im_sum{}, fz{};
     for (uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < a.total;
          gid += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t x, y, z, l;
@@ -523,37 +524,25 @@ __device__ __forceinline__ void final_sums(const StepArgs& a, double (&v)[kFinal
             p[c] = cx<A>((A)pr[c].x, (A)pr[c].y);
             O::add_prod(re_sum, t[c].x, p[c].x);
             O::add_prod(re_sum, t[c].y, p[c].y);
-            O::add(s[1], O::cross2(t[c].x, p[c].y, t[c].y, p[c].x));
+            O::add_prod(im_sum, t[c].x, p[c].y);
+            O::add_prod(im_sum, -t[c].y, p[c].x);
         }
         if constexpr (C > 1) {
-            // the spin densities' sums: spin-1 sqrt2 (chain of its components), spin-2 twice its outer
-            // pairs and sqrt6 times its inner chain
             const NodeTerms<A, C> n(p);
             typename O::T re, im;
-            constexpr int b = C == 5 ? 1 : 0;
-            n.chain(p[b], p[b + 1], p[b + 2], re, im);
-            if constexpr (C == 3) {
-                O::add(s[2], re);
-                O::add(s[3], im);
-                O::add(fz, n.template fz<0>());
-            } else {
-                O::add(f6[0], re);
-                O::add(f6[1], im);
-                O::add(s[2], O::dot2(p[0].x, p[1].x, p[0].y, p[1].y) + O::dot2(p[3].x, p[4].x, p[3].y, p[4].y));
-                O::add(s[3], O::cross2(p[0].x, p[1].y, p[0].y, p[1].x) + O::cross2(p[3].x, p[4].y, p[3].y, p[4].x));
-                O::add(fz, n.template fz<0>());
-            }
+            if constexpr (C == 3) n.chain(p[0], p[1], p[2], re, im);
+            else n.transverse(p, re, im);
+            O::add(mx, re);
+            O::add(my, im);
+            O::add(fz, n.template fz<0>());
         }
     }
-#pragma unroll
-    for (int k = 0; k < kFinalCount; ++k) v[k] = O::value(s[k]);
+    const double q = C == 3 ? GPE_REF_SQRT_2 : 1.0;
     v[0] = O::value(re_sum);
+    v[1] = O::value(im_sum);
+    v[2] = q * O::value(mx);
+    v[3] = q * O::value(my);
     v[4] = O::value(fz);
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        if constexpr (C == 3) v[2 + k] *= GPE_REF_SQRT_2;
-        if constexpr (C == 5) v[2 + k] = 2.0 * v[2 + k] + 2.449489742783178098 * O::value(f6[k]);
-    }
 }
 
 // To FP64's precision in words of FP32 (gpe_observe.cuh) for FP32 storage; a thread whose values

@@ -65,13 +65,23 @@ __device__ __forceinline__ Pair square_root(Pair a) {
 }
 // sqrt(6) a: the constant in three parts, since two leave an error of 1e-15 that is the
 // same for every node
-__device__ __forceinline__ Pair times_sqrt6(Pair a) {
+__device__ __forceinline__ TripleSum times_sqrt6(const TripleSum& a) {
     constexpr double c = 2.449489742783178098;
     constexpr float c1 = (float)c, c2 = (float)(c - (double)c1), c3 = (float)(c - (double)c1 - (double)c2);
-    const Pair p = two_prod(c1, a.h);
-    return pair_norm(p.h, __fadd_rn(p.l, __fmaf_rn(c3, a.h, __fmaf_rn(c2, a.h, __fmul_rn(c1, a.l)))));
+    TripleSum r(c1, a.h);
+    const Pair p = two_prod(c1, a.l), q = two_prod(c2, a.h);
+    r.add_low(p.h);
+    r.add_low(q.h);
+    r.m = __fadd_rn(r.m, __fadd_rn(__fadd_rn(p.l, q.l), __fmaf_rn(c3, a.h, __fmaf_rn(c2, a.l, __fmul_rn(c1, a.m)))));
+    return r;
 }
 __device__ __forceinline__ double times_sqrt6(double a) { return 2.449489742783178098 * a; }
+__device__ __forceinline__ TripleSum twice(TripleSum a) {
+    a.h = __fadd_rn(a.h, a.h);
+    a.l = __fadd_rn(a.l, a.l);
+    a.m = __fadd_rn(a.m, a.m);
+    return a;
+}
 __device__ __forceinline__ double twice(double a) { return 2.0 * a; }
 __device__ __forceinline__ double square(double a) { return a * a; }
 __device__ __forceinline__ double square_root(double a) { return sqrt(a); }
@@ -104,6 +114,24 @@ struct ObsArith<float> {
         s.l = __fmaf_rn(p, d.l, s.l);
     }
     __device__ static __forceinline__ void add_prod(E& s, float a, float b) { s.add_prod(a, b); }
+    // a0 b0 + a1 b1 + a2 b2 + a3 b3 and the same with the second and fourth product subtracted
+    __device__ static __forceinline__ E dot4(float a0, float b0, float a1, float b1, float a2, float b2, float a3, float b3) {
+        const Pair p0 = two_prod(a0, b0), p1 = two_prod(a1, b1), p2 = two_prod(a2, b2), p3 = two_prod(a3, b3);
+        const Pair s0 = two_sum(p0.h, p1.h), s1 = two_sum(p2.h, p3.h), t = two_sum(s0.h, s1.h);
+        E s;
+        s.h = t.h;
+        s.l = p0.l;
+        s.add_low(p1.l);
+        s.add_low(p2.l);
+        s.add_low(p3.l);
+        s.add_low(s0.l);
+        s.add_low(s1.l);
+        s.add_low(t.l);
+        return s;
+    }
+    __device__ static __forceinline__ E cross4(float a0, float b0, float a1, float b1, float a2, float b2, float a3, float b3) {
+        return dot4(a0, b0, -a1, b1, a2, b2, -a3, b3);
+    }
     // a a + b b; k (a - b) for k a power of two; a sum in E as a term
     __device__ static __forceinline__ E norm2(float a, float b) {
         E s(a, a);
@@ -120,7 +148,20 @@ struct ObsArith<float> {
         a.m *= k;
         return a;
     }
+    __device__ static __forceinline__ E product(const E& a, const E& b) {
+        E r(a.h, b.h);
+        const Pair p = two_prod(a.h, b.l), q = two_prod(a.l, b.h);
+        r.add_low(p.h);
+        r.add_low(q.h);
+        r.m = __fadd_rn(r.m, __fadd_rn(__fadd_rn(p.l, q.l), __fmaf_rn(a.l, b.l, __fmaf_rn(a.h, b.m, __fmul_rn(a.m, b.h)))));
+        return r;
+    }
     __device__ static __forceinline__ T term(const E& s) { return s.pair(); }
+    // as a term where the words may cancel: h + l exactly first
+    __device__ static __forceinline__ T rest(const E& s) {
+        const Pair p = two_sum(s.h, s.l);
+        return pair_norm(p.h, __fadd_rn(p.l, s.m));
+    }
     // s^2 (rounding s to a pair first would leave 4e-16 of the interaction energy)
     __device__ static __forceinline__ T square_of(const E& s) {
         const Pair n = pair_norm(s.h, s.l), p = two_prod(n.h, n.h);
@@ -152,7 +193,16 @@ struct ObsArith<double> {
     __device__ static __forceinline__ void add_prod(E& s, double a, double b) { s = fm(a, b, s); }
     __device__ static __forceinline__ E norm2(double a, double b) { return fm(a, a, b * b); }
     __device__ static __forceinline__ E difference(double k, E a, E b) { return k * (a - b); }
+    __device__ static __forceinline__ E product(E a, E b) { return a * b; }
     __device__ static __forceinline__ T term(E s) { return s; }
+    __device__ static __forceinline__ T rest(E s) { return s; }
+    __device__ static __forceinline__ E dot4(double a0, double b0, double a1, double b1, double a2, double b2, double a3, double b3) {
+        return fm(a0, b0, a1 * b1) + fm(a2, b2, a3 * b3);
+    }
+    __device__ static __forceinline__ E cross4(double a0, double b0, double a1, double b1, double a2, double b2, double a3,
+                                               double b3) {
+        return fm(a0, b0, -(a1 * b1)) + fm(a2, b2, -(a3 * b3));
+    }
     __device__ static __forceinline__ T square_of(E s) { return s * s; }
     __device__ static __forceinline__ T dot2(double a, double b, double c, double d) { return fm(a, b, c * d); }
     __device__ static __forceinline__ T cross2(double a, double b, double c, double d) { return fm(a, b, -(c * d)); }
@@ -199,10 +249,33 @@ struct NodeTerms {
             return A::difference((R)1, n[b], n[b + 2]);
         }
     }
-    // Re and Im of conj(a) b + conj(b) c
+    // Re and Im of conj(a) b + conj(c) d
+    __device__ static __forceinline__ void pairs(Cx<R> a, Cx<R> b, Cx<R> c, Cx<R> d, E& re, E& im) {
+        re = A::dot4(a.x, b.x, a.y, b.y, c.x, d.x, c.y, d.y);
+        im = A::cross4(a.x, b.y, a.y, b.x, c.x, d.y, c.y, d.x);
+    }
+    // the transverse spin of three neighbouring components over sqrt2, conj(a) b + conj(b) c.  In
+    // three words until its products are summed: in nematic and cyclic states they cancel, and
+    // what pairs left of |F| there was 30 to 60 times as far off as FP64 terms (a polar cloud turned
+    // by its texture, 1e-3 noise, relative: 4.5e-15 for 1e-16; with 1e-6 noise 4e-12 for 6e-14).
     __device__ static __forceinline__ void chain(Cx<R> a, Cx<R> b, Cx<R> c, T& re, T& im) {
-        re = A::dot2(a.x, b.x, a.y, b.y) + A::dot2(b.x, c.x, b.y, c.y);
-        im = A::cross2(a.x, b.y, a.y, b.x) + A::cross2(b.x, c.y, b.y, c.x);
+        E er, ei;
+        pairs(a, b, b, c, er, ei);
+        re = A::rest(er);
+        im = A::rest(ei);
+    }
+    // spin-2: <F_+> = 2 (conj(psi_2) psi_1 + conj(psi_-1) psi_-2) + sqrt6 (conj(psi_1) psi_0 +
+    // conj(psi_0) psi_-1), likewise
+    __device__ static __forceinline__ void transverse(const Cx<R>* p, T& fx, T& fy) {
+        E re2, im2, re6, im6;
+        pairs(p[0], p[1], p[3], p[4], re2, im2);
+        pairs(p[1], p[2], p[2], p[3], re6, im6);
+        re6 = times_sqrt6(re6);
+        im6 = times_sqrt6(im6);
+        A::add(re6, twice(re2));
+        A::add(im6, twice(im2));
+        fx = A::rest(re6);
+        fy = A::rest(im6);
     }
     // the record whose |psi_s| is the largest so far, kept by its value (its modulus is
     // taken once per thread, in FP64)
@@ -281,7 +354,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_k
         int32_t off[D];
 #pragma unroll
         for (int k = 0; k < D; ++k) off[k] = k < nd ? st.nb_off[f0 + k] : (int32_t)(l * node_bytes);
-        S kin[D], mx{}, my{}, gx{}, gy{};
+        S kin[D], mx{}, my{};
         typename A::E s0{}, s1{}, s2{}, srr{}, sff{}, sth{}, sabs{}, fz{}, fz1{};
 #pragma unroll
         for (int k = 0; k < D; ++k) kin[k] = S{};
@@ -320,7 +393,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_k
                 T re, im;
                 t.chain(p[0], p[1], p[2], re, im);
                 const typename A::E fe = t.template fz<0>();
-                const T f = A::term(fe);
+                const T f = A::rest(fe);
                 const T ff = twice(square(re) + square(im)) + square(f);
                 A::add(mx, re);
                 A::add(my, im);
@@ -329,20 +402,13 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_k
                 A::add(sff, ff);
                 A::add(sabs, square_root(ff));
             } else if constexpr (C == 5) {
-                // <F_+> = 2 (conj(psi_2) psi_1 + conj(psi_-1) psi_-2) + sqrt6 (conj(psi_1) psi_0 +
-                // conj(psi_0) psi_-1)
-                T re6, im6;
-                t.chain(p[1], p[2], p[3], re6, im6);
-                const T re2 = A::dot2(p[0].x, p[1].x, p[0].y, p[1].y) + A::dot2(p[3].x, p[4].x, p[3].y, p[4].y);
-                const T im2 = A::cross2(p[0].x, p[1].y, p[0].y, p[1].x) + A::cross2(p[3].x, p[4].y, p[3].y, p[4].x);
+                T fx, fy;
+                t.transverse(p, fx, fy);
                 const typename A::E fe = t.template fz<0>();
-                const T f = A::term(fe);
-                const T fx = twice(re2) + times_sqrt6(re6), fy = twice(im2) + times_sqrt6(im6);
+                const T f = A::rest(fe);
                 const T ff = square(fx) + square(fy) + square(f);
-                A::add(mx, re2);
-                A::add(my, im2);
-                A::add(gx, re6);
-                A::add(gy, im6);
+                A::add(mx, fx);
+                A::add(my, fy);
                 A::add(fz, fe);
                 A::add_times(fz1, zj, fe);
                 A::add(sff, ff);
@@ -375,14 +441,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_k
                     hz * (rz * rz * S0 + (gz * (2.0 * rz * S1 + gz * S2) + 2.0 * gl * (rz * S1 + gz * S2)));
         }
         if constexpr (C > 1) {
-            double Mx, My;
-            if constexpr (C == 3) {
-                Mx = GPE_REF_SQRT_2 * A::value(mx);
-                My = GPE_REF_SQRT_2 * A::value(my);
-            } else {
-                Mx = 2.0 * A::value(mx) + 2.449489742783178098 * A::value(gx);
-                My = 2.0 * A::value(my) + 2.449489742783178098 * A::value(gy);
-            }
+            const double q = C == 3 ? GPE_REF_SQRT_2 : 1.0, Mx = q * A::value(mx), My = q * A::value(my);
             const double Mz = A::value(fz), Mz1 = A::value(fz1);
             const bool qo = P.flags & GPE_FLAG_QUADRUPOLE_OFFSET;
             const double bx = P.bq * (rx - (qo ? P.qc[0] : 0.0)) + P.bb[0], by = P.bq * (ry - (qo ? P.qc[1] : 0.0)) + P.bb[1];
@@ -428,8 +487,8 @@ __global__ void __launch_bounds__(256) field_sums_kernel(StepArgs a) {
     using O = ObsArith<A>;
     using T = typename O::T;
     __shared__ double red[8][kFieldSums];
-    typename O::S s[5] = {};
-    typename O::E spin{}, density{};
+    typename O::S sx{}, sy{};
+    typename O::E spin{}, density{}, sz{};
     A top = (A)0;
     bool empty = false;
     for (uint64_t gid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gid < a.total;
@@ -454,10 +513,11 @@ __global__ void __launch_bounds__(256) field_sums_kernel(StepArgs a) {
             constexpr int b = C == 5 ? 1 : 0;  // s1, s0, s_1
             T re, im;
             t.chain(p[b], p[b + 1], p[b + 2], re, im);
-            const T f = O::term(t.template fz<b>());
-            O::add(s[1], re);
-            O::add(s[2], im);
-            O::add(s[3], t.rho * f);
+            const typename O::E fe = t.template fz<b>();
+            const T f = O::rest(fe);
+            O::add(sx, re);
+            O::add(sy, im);
+            O::add(sz, O::product(t.density, fe));
             // rho |s| with m and rho taken near 1, so that no square leaves the range
             const A u = O::unit(t.rho);
             const T rx = O::times(re, u), ry = O::times(im, u), rz = O::times(t.rho, u) * f;
@@ -468,17 +528,14 @@ __global__ void __launch_bounds__(256) field_sums_kernel(StepArgs a) {
             empty = empty || none;
         }
     }
-    double v[kFieldSums];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) v[k] = O::value(s[k]);
-    v[0] = O::value(SPIN && C > 1 ? spin : density);
-    if (SPIN) v[4] = O::value(density);
+    double v[kFieldSums] = {O::value(SPIN && C > 1 ? spin : density), 0.0, 0.0, 0.0, 0.0, (double)top};
     if constexpr (SPIN) {
-        v[1] *= GPE_REF_SQRT_2;
-        v[2] *= GPE_REF_SQRT_2;
+        v[1] = GPE_REF_SQRT_2 * O::value(sx);
+        v[2] = GPE_REF_SQRT_2 * O::value(sy);
+        v[3] = O::value(sz);
+        v[4] = O::value(density);
         if (empty) v[0] = v[1] = v[2] = nan("");
     }
-    v[5] = (double)top;
 #pragma unroll
     for (int k = 0; k < kFieldSums; ++k)
         for (int o = 16; o > 0; o >>= 1) {
