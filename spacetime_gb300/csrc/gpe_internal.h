@@ -39,6 +39,16 @@ constexpr int kMaxEntries = 640;
 constexpr int kMaxEdges = 320;
 constexpr int kMaxFaces = 8;
 
+// The items first, first + stride, ... below total, one thread's share of a grid.  A grid
+// may have up to 2^32 - 1 sites, so a plain 32-bit index could step past 2^32 and start over
+// in a loop that never ends; this one stops at total.
+struct Strided {
+    uint32_t i, stride, total;
+    __host__ __device__ Strided(uint32_t first, uint32_t stride, uint32_t total) : i(first), stride(stride), total(total) {}
+    __host__ __device__ bool more() const { return i < total; }
+    __host__ __device__ void next() { i = stride < total - i ? i + stride : total; }
+};
+
 // Unsigned division by a run-time constant: q = umulhi(n, mul) >> shift
 // (Granlund & Montgomery, "Division by invariant integers using multiplication", 1994).
 struct FastDiv {

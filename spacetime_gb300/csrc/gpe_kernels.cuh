@@ -1133,7 +1133,8 @@ __global__ void __launch_bounds__(256) parabolic_columns_kernel(StepArgs a, uint
     const PhysR<R>& P = make_phys<R>(a);
     using OA = typename AccOf<MODE, false, R>::type;
     OA oa = AccOf<MODE, false, R>::make(nullptr);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    for (Strided it(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, total); it.more(); it.next()) {
+        const uint32_t i = it.i;
         const uint32_t chunk = fdiv(i, dcol);
         const uint32_t col = i - chunk * columns;   // (y X + x) V + l
         const uint32_t y = fdiv(col, a.divRow);

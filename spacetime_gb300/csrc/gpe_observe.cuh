@@ -340,7 +340,8 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_k
     R big = (R)0;
     uint32_t nbad = 0;
     const uint32_t node_bytes = C * 2 * sizeof(R);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    for (Strided it(blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, total); it.more(); it.next()) {
+        const uint32_t i = it.i;
         const uint32_t chunk = fdiv(i, dcol);
         const uint32_t col = i - chunk * columns;   // (y X + x) V + l
         const uint32_t y = fdiv(col, a.divRow);
