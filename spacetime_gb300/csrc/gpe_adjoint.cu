@@ -782,7 +782,9 @@ static bool keep_states(const gpe_handle* h, int n) {
     return need <= free_bytes / 4;
 }
 
-static gpe_status ensure_adjoint_buffers(gpe_handle* h, int n, int stride, bool il, bool keep) {
+// What is cleared is cleared on the call's stream: a clear on the default stream is not ordered
+// before the kernels of a non-blocking one.
+static gpe_status ensure_adjoint_buffers(gpe_handle* h, int n, int stride, bool il, bool keep, cudaStream_t s) {
     AdjointStore& A = h->adj;
     const int segments = (n + stride - 1) / stride;
     const size_t bytes = il ? h->ilg.bytes : h->alloc_bytes[GPE_PSI_EVEN];
@@ -801,7 +803,7 @@ static gpe_status ensure_adjoint_buffers(gpe_handle* h, int n, int stride, bool 
         }
         A.kept_bytes = need;
         // zero halos: the steps write the interior only
-        if (cudaMemset(A.kept, 0, need) != cudaSuccess) return fail(GPE_ERR_CUDA, "cudaMemset (adjoint states)");
+        if (cudaMemsetAsync(A.kept, 0, need, s) != cudaSuccess) return fail(GPE_ERR_CUDA, "cudaMemset (adjoint states)");
     }
     A.kept_step = kept_step(h);
     A.keeps = keep;
@@ -815,7 +817,7 @@ static gpe_status ensure_adjoint_buffers(gpe_handle* h, int n, int stride, bool 
             if (cudaMalloc(&p, bytes) != cudaSuccess) return false;
             v.push_back(p);
             // zero halos: the out-of-place recomputation writes only the interior
-            if (cudaMemset(p, 0, bytes) != cudaSuccess) return false;
+            if (cudaMemsetAsync(p, 0, bytes, s) != cudaSuccess) return false;
         }
         return true;
     };
@@ -831,7 +833,7 @@ static gpe_status ensure_adjoint_buffers(gpe_handle* h, int n, int stride, bool 
     if (!A.target) {
         const size_t tb = h->alloc_bytes[GPE_PSI_EVEN];   // the target stays in the handle's layout
         if (cudaMalloc(&A.target, tb) != cudaSuccess) return fail(GPE_ERR_OOM, "cudaMalloc (target)");
-        if (cudaMemset(A.target, 0, tb) != cudaSuccess) return fail(GPE_ERR_CUDA, "cudaMemset (target)");
+        if (cudaMemsetAsync(A.target, 0, tb, s) != cudaSuccess) return fail(GPE_ERR_CUDA, "cudaMemset (target)");
     }
     if (A.grad && A.n < n) {
         cudaFree(A.grad);
@@ -888,7 +890,7 @@ extern "C" gpe_status gpe_adjoint_forward(gpe_handle* h, int32_t n_steps, const 
     if (n_steps > 1 && il_leapfrog_applies(h, n_steps)) {
         st = il_ensure(h, s);
         for (int keep = any_stride && !st && keep_states(h, n_steps) ? 1 : 0; !st && keep >= 0; --keep) {
-            st = ensure_adjoint_buffers(h, n_steps, stride, true, keep != 0);
+            st = ensure_adjoint_buffers(h, n_steps, stride, true, keep != 0, s);
             if (st != GPE_ERR_OOM) break;
             adjoint_release(h);
             cudaGetLastError();
@@ -897,7 +899,7 @@ extern "C" gpe_status gpe_adjoint_forward(gpe_handle* h, int32_t n_steps, const 
         if (st && st != GPE_ERR_OOM) return st;
         if (st) cudaGetLastError();
     }
-    if (st) st = ensure_adjoint_buffers(h, n_steps, stride, false, false);
+    if (st) st = ensure_adjoint_buffers(h, n_steps, stride, false, false, s);
     if (st) return st;
     // target: host FP64 file layout -> device buffer in the handle's precision
     if ((st = ensure_stage(h, count))) return st;

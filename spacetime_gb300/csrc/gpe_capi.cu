@@ -436,11 +436,18 @@ extern "C" gpe_status gpe_destroy(gpe_handle* h) {
 
 static bool slot_ok(const gpe_handle* h, int slot) { return slot >= 0 && slot < 5 && h->alloc[slot] != nullptr; }
 
-static gpe_status ensure_hpsi(gpe_handle* h) {
+// Cleared on the call's stream: a clear on the default stream is not ordered before the kernels
+// of a non-blocking one.
+static gpe_status ensure_hpsi(gpe_handle* h, cudaStream_t s) {
     if (h->alloc[GPE_HPSI]) return GPE_OK;
     const size_t bytes = h->g.slice * (h->g.Z + 2);
-    if (cudaMalloc(&h->alloc[GPE_HPSI], bytes) != cudaSuccess) return fail(GPE_ERR_OOM, "cudaMalloc (H psi)");
-    cudaMemset(h->alloc[GPE_HPSI], 0, bytes);
+    void* p = nullptr;
+    if (cudaMalloc(&p, bytes) != cudaSuccess) return fail(GPE_ERR_OOM, "cudaMalloc (H psi)");
+    if (cudaError_t e = cudaMemsetAsync(p, 0, bytes, s); e != cudaSuccess) {
+        cudaFree(p);
+        return cuda_fail(e, "cudaMemset (H psi)");
+    }
+    h->alloc[GPE_HPSI] = p;
     h->alloc_bytes[GPE_HPSI] = bytes;
     h->interior[GPE_HPSI] = static_cast<char*>(h->alloc[GPE_HPSI]) + h->g.slice + h->g.pitch + h->g.cell_bytes;
     return GPE_OK;
@@ -492,7 +499,7 @@ static gpe_status transfer(gpe_handle* h, int32_t slot, double* host, size_t cou
     if (!h || !host) return fail(GPE_ERR_INVALID_ARG, "null argument");
     if (up) h->epoch += 1;
     if (up && slot == GPE_HPSI) {
-        gpe_status st = ensure_hpsi(h);
+        gpe_status st = ensure_hpsi(h, (cudaStream_t)stream);
         if (st) return st;
     }
     if (!slot_ok(h, slot)) return fail(GPE_ERR_INVALID_ARG, "slot not allocated");
@@ -1136,7 +1143,7 @@ extern "C" gpe_status gpe_step_explicit(gpe_handle* h, int32_t next_slot, int32_
     if (mode < 0 || mode > 2) return fail(GPE_ERR_INVALID_ARG, "mode");
     if (h->p.scheme == GPE_SCHEME_SPLIT) return fail(GPE_ERR_UNSUPPORTED, "the split scheme steps in place: use gpe_step");
     if (mode == GPE_MODE_ITP) {
-        gpe_status st = ensure_hpsi(h);
+        gpe_status st = ensure_hpsi(h, (cudaStream_t)stream);
         if (st) return st;
     }
     gpe_fields B;
@@ -1819,7 +1826,7 @@ static gpe_status itp_iterations(gpe_handle* h, int32_t n, cudaStream_t s) {
 extern "C" gpe_status gpe_itp(gpe_handle* h, int32_t n, double* mu_out, void* stream) {
     if (!h) return fail(GPE_ERR_INVALID_ARG, "null handle");
     if (h->p.scheme == GPE_SCHEME_SPLIT) return fail(GPE_ERR_UNSUPPORTED, "imaginary time is not built for the split scheme");
-    gpe_status st = ensure_hpsi(h);
+    gpe_status st = ensure_hpsi(h, (cudaStream_t)stream);
     if (st) return st;
     cudaStream_t s = (cudaStream_t)stream;
     gpe_fields zero;
