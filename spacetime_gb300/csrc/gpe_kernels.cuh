@@ -1662,31 +1662,36 @@ __global__ void __launch_bounds__(256) scale_kernel(StepArgs a) {
 inline unsigned nblocks(uint64_t items, unsigned bs) { return (unsigned)((items + bs - 1) / bs); }
 
 // The launch of a kernel whose threads walk up columns of cells (256 threads a block,
-// occ blocks per SM): the cells of z per column that leave the busiest thread the least
-// work, with what is done once per column counted as `overhead` nodes.
+// occ blocks per SM).
 struct ColumnGrid {
-    uint32_t zc, columns, total;   // total: columns times chunks of z
+    uint32_t zc, columns, total;   // cells of z per column; total: columns times chunks of z
     unsigned blocks;
 };
-inline ColumnGrid column_grid(const StepArgs& a, unsigned occ, uint32_t overhead) {
-    constexpr uint32_t kMost = 64;   // cells per column
+inline ColumnGrid column_grid(const StepArgs& a, unsigned occ, uint32_t zc) {
     const uint64_t threads = (uint64_t)occ * (unsigned)device_sm_count() * 256;
     ColumnGrid g;
+    g.zc = zc;
     g.columns = a.row_items * a.g.Y;
-    g.zc = std::min(kMost, a.g.Z);
-    uint64_t best = ~0ull;
-    for (uint32_t c = (a.g.Z + kMost - 1) / kMost; c <= a.g.Z && c <= 4 * kMost; ++c) {
-        const uint32_t z = (a.g.Z + c - 1) / c;
-        const uint64_t cost = ((uint64_t)g.columns * c + threads - 1) / threads * (z + overhead);
-        if (cost < best) {
-            best = cost;
-            g.zc = z;
-        }
-    }
-    const uint64_t total = (uint64_t)g.columns * ((a.g.Z + g.zc - 1) / g.zc);
+    const uint64_t total = (uint64_t)g.columns * ((a.g.Z + zc - 1) / zc);
     g.total = (uint32_t)total;   // at most the grid's sites
     g.blocks = (unsigned)std::min<uint64_t>((total + 255) / 256, threads / 256);
     return g;
+}
+// A kernel that needs every warp of the grid to be busy: the cells per column that leave the
+// busiest thread the least work, with what is done once per column counted as `overhead` nodes.
+inline uint32_t cells_by_thread(const StepArgs& a, unsigned occ, uint32_t overhead) {
+    const uint64_t threads = (uint64_t)occ * (unsigned)device_sm_count() * 256, columns = (uint64_t)a.row_items * a.g.Y;
+    uint32_t zc = std::min(kMostCells, a.g.Z);
+    uint64_t best = ~0ull;
+    for (uint32_t c = (a.g.Z + kMostCells - 1) / kMostCells; c <= a.g.Z && c <= 4 * kMostCells; ++c) {
+        const uint32_t z = (a.g.Z + c - 1) / c;
+        const uint64_t cost = (columns * c + threads - 1) / threads * (z + overhead);
+        if (cost < best) {
+            best = cost;
+            zc = z;
+        }
+    }
+    return zc;
 }
 
 // One wave of resident blocks (the kernel's occupancy x SMs), fewer for small grids.
@@ -1700,7 +1705,7 @@ cudaError_t launch_parabolic_m(const StepArgs& a, cudaStream_t s, unsigned* grid
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, kc, 256, 0);
             if (occ_c < 1) occ_c = 1;
         }
-        const ColumnGrid g = column_grid(a, (unsigned)occ_c, 1);
+        const ColumnGrid g = column_grid(a, (unsigned)occ_c, cells_by_sm((uint64_t)a.row_items * a.g.Y, a.g.Z, (unsigned)occ_c, (unsigned)device_sm_count()));
         const cudaError_t e = launch_overlapped(kc, g.blocks, 256, 0, s, a, g.zc, g.columns, g.total, make_fastdiv(g.columns));
         if (e != cudaSuccess) return e;
         if (grid) *grid = g.blocks;

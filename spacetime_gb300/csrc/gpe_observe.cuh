@@ -567,7 +567,7 @@ cudaError_t launch_observe_columns_d(const StepArgs& a, double* out, cudaStream_
         occ = std::max(occ, 1);
     }
     // a column's FP64 part, about 100 operations, costs what 9 nodes cost
-    const ColumnGrid g = column_grid(a, (unsigned)occ, 9);
+    const ColumnGrid g = column_grid(a, (unsigned)occ, cells_by_thread(a, (unsigned)occ, 9));
     k<<<g.blocks, 256, 0, s>>>(a, g.zc, g.columns, g.total, make_fastdiv(g.columns));
     finalize_observables(a.partials, g.blocks, out, s);
     return cudaGetLastError();
