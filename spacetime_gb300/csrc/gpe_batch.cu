@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(kBatchThreads, sizeof(R) == 8 ? 1 : (CMASK & 4
         // item j gridDim.x + blockIdx.x), their descriptions copied to shared memory while
         // the turn before is worked on; the list's last full round and what is left over go
         // by one counter per step, so blocks that finish early take more and the step ends
-        // within about one item.  24 members of 33M nodes, 40 steps: the last round 18.34 ms,
+        // within about one item (long lists: all of it, own_turns).  24 members of 33M nodes, 40 steps: the last round 18.34 ms,
         // the last two 18.43, every item by the counter 18.53; with every thread holding the
         // loop's state in registers and a counter for all 18.56 (28 bytes of spills).
         if (threadIdx.x == 0) {
@@ -681,6 +681,16 @@ int32_t target_nodes(const gpe_batch* b, const gpe_handle* h) {
     return (int32_t)std::min<uint64_t>(b->item_nodes, std::max<uint64_t>(share, 1024));
 }
 
+// The turns of a step that are a block's own, of `rounds` full rounds of the item list.  A turn by
+// the counter costs its latency; own turns let the blocks drift apart as their items differ, by
+// more than the last round makes up for where there are many (and blocks then read neighbouring
+// rows at different times).  A step in us, by the counter and with own turns but the last round:
+// 5 rounds 91.0 / 88.7, 6 rounds 104.0 / 101.3, 7 rounds 474 / 466, 9 rounds 70.8 / 64.7; 20 rounds 1535 / 1566,
+// 23 rounds 6720 / 6614, 34 rounds 1511 / 1530, 55 rounds 22939 / 23487, 91 rounds 6148 / 6463, 282
+// rounds 21676 / 23433.
+constexpr uint32_t kOwnRounds = 16;
+uint32_t own_turns(uint32_t rounds) { return rounds > 1 && rounds <= kOwnRounds ? rounds - 1 : 0; }
+
 // Work items of the members `which` (indices into b->members), sorted by lattice
 // (V) and spin so that consecutive items share tables.
 std::vector<BatchItem> build_items(const gpe_batch* b, const std::vector<uint32_t>& which) {
@@ -796,8 +806,7 @@ gpe_status enqueue_steps(gpe_batch* b, int32_t n, cudaStream_t s, const BatchMem
         A.next_item = b->d_next;
         A.nmembers = nmembers;
         A.nitems = b->nitems;
-        const uint32_t rounds = b->nitems / (uint32_t)grid;
-        A.own = rounds > 1 ? rounds - 1 : 0;
+        A.own = own_turns(b->nitems / (uint32_t)grid);
         A.nsteps = (uint32_t)steps;
         A.step_base = (uint32_t)done;
         A.bar = b->d_bar;
