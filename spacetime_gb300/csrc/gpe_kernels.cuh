@@ -1279,8 +1279,17 @@ __device__ __forceinline__ void q_update(const StepArgs& a, const SmemHyper<R>& 
 // the local terms, which took the spin-1 step on C15 40^3 from 487 to 341 us (0.57 to 0.81
 // of the copy peak), BCC 96^3 from 603 to 414 (0.82), cube 120^3 165 to 160; scalar BCC 96^3
 // 172 to 166.
+//
+// FP64 imaginary time at 8 (scalar) and 4 (spin-1) blocks per SM: left to itself the compiler
+// takes registers for 6 and 3.  An iteration in us, then / now: scalar C15 32^3 727 / 534, BCC 64^3 521 /
+// 383; spin-1 C15 32^3 2033 / 1489, BCC 48^3 620 / 464.  Spin-2 is the faster for its registers (2
+// blocks; at 3 C15 24^3 1180 / 1706).
+template <typename R, int C, int MODE>
+constexpr int hyper_min_blocks() {
+    return sizeof(R) == 8 && MODE == GPE_MODE_ITP ? (C == 1 ? 8 : (C == 3 ? 4 : 0)) : 0;
+}
 template <typename R, int C, bool DO_PSI, int MODE, bool HYPERB, int QM>
-__global__ void __launch_bounds__(256) hyper_step_kernel(StepArgs a, uint32_t node_items, uint32_t edge_items,
+__global__ void __launch_bounds__(256, hyper_min_blocks<R, C, MODE>()) hyper_step_kernel(StepArgs a, uint32_t node_items, uint32_t edge_items,
                                                          uint32_t ratio, uint32_t vblocks) {
     __shared__ SmemHyper<R> sh;
     const int V = a.g.V, E = a.g.E, F = a.tab.faces;
