@@ -160,7 +160,8 @@ def time_leg(w, steps, inner, warmup, kernel=0, dims=None):
     if w["scheme"] == 0 and gather:
         name = "parabolic_fixed_kernel<float,%d,LEAPFROG,4>" % w["C"]
     if interleaved and w["scheme"] == 1:
-        name = "il_hyper_kernel<%d,%d>" % (w["C"], il_group_cells(p.dims[0], w["C"]))
+        small = w["C"] > 1 and sites * w["C"] * 8 < 9e6
+        name = "il_hyper_kernel<%d,%d>" % (w["C"], il_group_cells(p.dims[0], w["C"], small))
     elif interleaved:
         name = "il_step_kernel<%d,%d,%d>" % (w["C"], 8 if w["lattice"] == "fcc" else 4, il_group_cells(p.dims[0], w["C"]))
     return {"metric": "lattice-site-updates/s", "value": sites * inner * steps / (total_ms * 1e-3),
@@ -175,14 +176,14 @@ def time_leg(w, steps, inner, warmup, kernel=0, dims=None):
             "norm_last": obs[-1]["norm"] if obs else None}
 
 
-def il_group_cells(x, components):
+def il_group_cells(x, components, small_hyperbolic=False):
     """Cells per group of the interleaved layout for an x edge (the library's rule: by the
     lanes left idle and what narrower groups cost)."""
     def cost(cells, percent):
         return (x + cells - 1) // cells * cells * percent
 
     wide = min((cost(32, 100), 0, 32), (cost(16, 103), 1, 16))
-    return 8 if cost(8, 115 if components == 3 else 106) < wide[0] else wide[2]
+    return 8 if cost(8, 135 if small_hyperbolic else 115 if components == 3 else 106) < wide[0] else wide[2]
 
 
 def leg_e2e(w, steps, inner, dims=None, flight=1):

@@ -378,6 +378,7 @@ extern "C" gpe_status gpe_create(const gpe_lattice* lat, const gpe_params* p, gp
     g.slice = g.pitch * (g.Y + 2);
     g.qpitch = g.E ? round_up((size_t)(g.X + 2) * g.qcell_bytes, 256) : 0;
     g.qslice = g.qpitch * (g.Y + 2);
+    g.cost8 = il_cost8(g.C, p->scheme == GPE_SCHEME_HYPERBOLIC, sites * g.C * 8);
 
     const bool hyper = p->scheme != GPE_SCHEME_PARABOLIC;  // q buffers
     for (int slot = 0; slot < 5; ++slot) {

@@ -152,6 +152,7 @@ struct Grid {
     size_t pitch, slice;         // psi buffers
     size_t qpitch, qslice;       // q buffers
     uint32_t cell_bytes, qcell_bytes;
+    uint32_t cost8;              // il_cost8
 };
 
 // Geometry of an FP32 state in the cell-interleaved layout.  Rows (y, z) run from
@@ -178,11 +179,22 @@ struct ILGrid {
 // lanes' count.  Where lanes are idle: spin-1 C15 40^3 141.6 / 124.3 / 120.9, Z 40^3
 // 85.9 / 75.9 / 71.6, BCC 72^3 67.3 / 62.6 / 63.6; hyperbolic spin-2 C15 40^3 620.5 /
 // 545.4 / 501.3, 48^3 923.7 / 818.3 / 863.9.
-inline uint32_t il_group_cells(uint32_t X, uint32_t C) {
+// The hyperbolic step of spinors whose psi and q stay in L2 is bound by L1 requests, where the
+// four lines of an 8-cell run count in full: below 9 MB a psi slot they are taken as 35 %, and
+// only rows of less than half a group of 16 are cut in them.  A step in us, 8 cells / wider: spin-2 BCC
+// 24^3 (6.6 MB) 12.3 / 10.3, 36 x 16 x 16 (4.4 MB) 10.2 / 9.0, C15 24 x 8 x 8 (8.4 MB) 14.3 / 12.3, spin-1 BCC 40 x 24 x 24
+// (6.6 MB) 12.3 / 10.2; above, spin-2 BCC 20 x 32 x 32 (9.8 MB) 16.4 / 18.5, 23 x 32 x 32 (11.3 MB) 16.5 / 20.1,
+// C15 36 x 8 x 8 (12.5 MB) 20.5 / 24.1, spin-1 BCC 20 x 48 x 48 (13.3 MB) 23.0 / 31.0; rows of 5 and 8 cells
+// gain at any size (8.8 MB 14.3 / 24.6).  Scalars and the parabolic step (its launches overlap): no such
+// loss.
+inline uint32_t il_cost8(uint32_t C, bool hyperbolic, uint64_t slot_bytes) {
+    return hyperbolic && C > 1 && slot_bytes < 9000000 ? 135 : (C == 3 ? 115 : 106);
+}
+inline uint32_t il_group_cells(uint32_t X, uint32_t cost8) {
     auto cost = [X](uint32_t cells, uint32_t percent) { return (uint64_t)((X + cells - 1) / cells) * cells * percent; };
     uint32_t best = 32;
     if (cost(16, 103) < cost(32, 100)) best = 16;
-    if (cost(8, C == 3 ? 115 : 106) < (best == 32 ? cost(32, 100) : cost(16, 103))) best = 8;
+    if (cost(8, cost8) < (best == 32 ? cost(32, 100) : cost(16, 103))) best = 8;
     return best;
 }
 
@@ -199,7 +211,7 @@ inline ILGrid make_il_grid(const Grid& g) {
     G.Z = g.Z;
     G.V = g.V;
     G.C = g.C;
-    G.cells = il_group_cells(g.X, g.C);
+    G.cells = il_group_cells(g.X, g.cost8);
     G.GX = (g.X + G.cells - 1) / G.cells;
     G.gb = (size_t)g.V * g.C * G.cells * 8;
     G.row = G.GX * G.gb;
