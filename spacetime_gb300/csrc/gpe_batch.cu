@@ -563,7 +563,7 @@ void member_constants(const gpe_handle* h, BatchMember& M) {
     M.C = h->g.C;
     M.cslot = -1;
     M.il_deg = 0;
-    M.ilg = make_il_grid(h->g);
+    M.ilg = make_il_grid(h->g, h->il_cost8);
     M.divGX = make_fastdiv(M.ilg.GX);
     M.il_off = nullptr;
 }
@@ -572,7 +572,7 @@ void member_constants(const gpe_handle* h, BatchMember& M) {
 // a group's base, for the group's first cell: the rows (dz, dy), the node and dx,
 // with dx + 1 (|dx| <= 1) in the two low bits.  Empty if one does not fit 32 bits.
 std::vector<int32_t> il_offsets(const gpe_handle* h) {
-    const ILGrid G = make_il_grid(h->g);
+    const ILGrid G = make_il_grid(h->g, h->il_cost8);
     const int64_t node_run = (int64_t)G.C * G.cells * 8;
     std::vector<int32_t> out;
     for (const gpe_stencil_entry& e : h->lat.stencil) {

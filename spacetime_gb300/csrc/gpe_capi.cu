@@ -378,7 +378,7 @@ extern "C" gpe_status gpe_create(const gpe_lattice* lat, const gpe_params* p, gp
     g.slice = g.pitch * (g.Y + 2);
     g.qpitch = g.E ? round_up((size_t)(g.X + 2) * g.qcell_bytes, 256) : 0;
     g.qslice = g.qpitch * (g.Y + 2);
-    g.cost8 = il_cost8(g.C, p->scheme == GPE_SCHEME_HYPERBOLIC, sites * g.C * 8);
+    h->il_cost8 = il_cost8(g.C, p->scheme == GPE_SCHEME_HYPERBOLIC, sites * g.C * 8);
 
     const bool hyper = p->scheme != GPE_SCHEME_PARABOLIC;  // q buffers
     for (int slot = 0; slot < 5; ++slot) {
@@ -1279,7 +1279,7 @@ struct StepTimer {
 // 0 otherwise.
 namespace gpe {
 int il_stencil_deg(const gpe_handle* h) {
-    if (!il_offsets_fit(make_il_grid(h->g))) return 0;
+    if (!il_offsets_fit(make_il_grid(h->g, h->il_cost8))) return 0;
     for (const gpe_stencil_entry& e : h->lat.stencil)
         if (e.dx < -1 || e.dx > 1 || e.dy < -1 || e.dy > 1 || e.dz < -1 || e.dz > 1) return 0;
     if (h->tab.uniform_deg == 4) return 4;
@@ -1291,7 +1291,7 @@ int il_stencil_deg(const gpe_handle* h) {
 static int il_deg(const gpe_handle* h) { return il_stencil_deg(h); }
 
 static unsigned il_grid_blocks(const gpe_handle* h, bool obs) {
-    const ILGrid G = make_il_grid(h->g);
+    const ILGrid G = make_il_grid(h->g, h->il_cost8);
     const int deg = il_deg(h);
     switch (h->g.C) {
         case 1: return il_blocks<1>(G, deg, obs, h->partial_blocks);
@@ -1336,7 +1336,7 @@ static bool il_hyper_applies(const gpe_handle* h) {
     if (h->p.scheme != GPE_SCHEME_HYPERBOLIC || h->real_bytes != 4 || h->lat.F != 4 || g.E != 2 * g.V) return false;
     if ((g.V * g.C) % 2 || (g.E * g.C) % 2) return false;
     if (g.cell_bytes != g.V * g.C * 8 || g.qcell_bytes != g.E * g.C * 8) return false;
-    if (!il_offsets_fit(make_il_grid(g)) || !il_offsets_fit(make_il_grid(q_grid(h)))) return false;
+    if (!il_offsets_fit(make_il_grid(g, h->il_cost8)) || !il_offsets_fit(make_il_grid(q_grid(h), h->il_cost8))) return false;
     auto adj = [](int dx, int dy, int dz) { return dx >= -1 && dx <= 1 && dy >= -1 && dy <= 1 && dz >= -1 && dz <= 1; };
     for (const gpe_edge& e : h->lat.edges)
         if (!adj(e.dx, e.dy, e.dz)) return false;
@@ -1366,7 +1366,7 @@ static bool use_interleaved(const gpe_handle* h, int32_t n) {
 
 namespace gpe {
 gpe_status il_ensure(gpe_handle* h, cudaStream_t s) {
-    const ILGrid G = make_il_grid(h->g);
+    const ILGrid G = make_il_grid(h->g, h->il_cost8);
     void* fresh[2] = {nullptr, nullptr};
     for (int k = 0; k < 2; ++k) {
         if (h->il[k]) continue;
@@ -1398,7 +1398,7 @@ static gpe_status ensure_il_hyper(gpe_handle* h, cudaStream_t s) {
     gpe_status st = ensure_il(h, s);
     if (st) return st;
     const ILGrid G = h->ilg;
-    const ILGrid Gq = make_il_grid(q_grid(h));
+    const ILGrid Gq = make_il_grid(q_grid(h), h->il_cost8);
     for (int k = 0; k < 2; ++k) {
         if (h->ilq[k]) continue;
         void* p = nullptr;

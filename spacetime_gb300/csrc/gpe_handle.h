@@ -97,6 +97,7 @@ struct gpe_handle {
     // and the interleaved offset tables of the fused step (il_hyper_tables)
     char* ilq[2] = {nullptr, nullptr};
     gpe::ILGrid ilgq{};
+    uint32_t il_cost8 = 106;
     int32_t* il_htab = nullptr;
     // split-scheme handles: the interleaved planes R, I, q_R, q_I and their offset table
     char* planes[4] = {nullptr, nullptr, nullptr, nullptr};

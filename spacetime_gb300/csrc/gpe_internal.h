@@ -152,7 +152,6 @@ struct Grid {
     size_t pitch, slice;         // psi buffers
     size_t qpitch, qslice;       // q buffers
     uint32_t cell_bytes, qcell_bytes;
-    uint32_t cost8;              // il_cost8
 };
 
 // Geometry of an FP32 state in the cell-interleaved layout.  Rows (y, z) run from
@@ -204,14 +203,14 @@ inline bool il_offsets_fit(const ILGrid& G) {
     return (uint64_t)(G.Y + 3) * G.row + 2 * (uint64_t)G.gb < (uint64_t)INT32_MAX;
 }
 
-inline ILGrid make_il_grid(const Grid& g) {
+inline ILGrid make_il_grid(const Grid& g, uint32_t cost8) {
     ILGrid G;
     G.X = g.X;
     G.Y = g.Y;
     G.Z = g.Z;
     G.V = g.V;
     G.C = g.C;
-    G.cells = il_group_cells(g.X, g.cost8);
+    G.cells = il_group_cells(g.X, cost8);
     G.GX = (g.X + G.cells - 1) / G.cells;
     G.gb = (size_t)g.V * g.C * G.cells * 8;
     G.row = G.GX * G.gb;
