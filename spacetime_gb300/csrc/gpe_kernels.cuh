@@ -1723,20 +1723,21 @@ cudaError_t launch_parabolic_m(const StepArgs& a, cudaStream_t s, unsigned* grid
     } else if constexpr (D > 0) {
         // the largest multiple of V / gcd(V, 256) blocks within one wave: the grid
         // stride is then a multiple of V
-        // The FP32 spin-2 step takes 80 registers, 3 blocks per SM.  Where the states do not stay in
-        // L2 a fourth block hides more latency than its 64 registers cost; where they do it does not.
-        // A step in us at 3 / 4 blocks: C15 16^3 (557k nodes) 18.0 / 19.1, 24^3 (1.9M) 61.6 / 59.4, 40^3 262.6 /
-        // 257.1; BCC 24^3 (166k) 8.3 / 9.7, 48^3 (1.3M) 41.2 / 40.0, 80^3 167.2 / 163.8; A15 24^3 (636k) 21.4 /
-        // 22.9, 40^3 (2.9M) 95.2 / 88.9; Z 16^3 11.4 / 13.6, 40^3 145.6 / 138.5.
-        constexpr bool kFourth = sizeof(R) == 4 && C == 5 && D == 4 && !MORE && MODE == GPE_MODE_LEAPFROG && !OBS;
-        const bool fourth = kFourth && a.total >= (1u << 20);
+        // The FP32 spin-2 step takes 80 registers, 3 blocks per SM (rows of 6: 90, 2 blocks).  Where the
+        // states do not stay in L2 one more block hides more latency than its registers cost; where they do
+        // it does not.  A step in us, without it / with it: C15 16^3 (557k nodes) 18.0 / 19.1, 24^3 (1.9M) 61.6 /
+        // 59.4, 40^3 262.6 / 257.1; BCC 24^3 (166k) 8.3 / 9.7, 48^3 (1.3M) 41.2 / 40.0, 80^3 167.2 / 163.8; A15 24^3
+        // (636k) 21.4 / 22.9, 40^3 (2.9M) 95.2 / 88.9; Z 16^3 11.4 / 13.6, 40^3 145.6 / 138.5; cube 41^3 (69k) 4.1 / 4.7,
+        // 50^3 (125k) 6.1 / 5.9, 96^3 25.8 / 23.1, 228^3 353.9 / 319.1.
+        constexpr bool kOneMore = sizeof(R) == 4 && C == 5 && (D == 4 || D == 6) && !MORE && MODE == GPE_MODE_LEAPFROG && !OBS;
+        const bool more = kOneMore && a.total >= (D == 4 ? 1u << 20 : 100000u);
         auto kf = [&] {
             if constexpr (OBS) return &parabolic_fixed_obs_kernel<R, C, MODE, D, G, MORE>;
-            else return fourth ? &parabolic_fixed_kernel<R, C, MODE, D, G, MORE, kFourth ? 4 : 0>
-                               : &parabolic_fixed_kernel<R, C, MODE, D, G, MORE>;
+            else return more ? &parabolic_fixed_kernel<R, C, MODE, D, G, MORE, kOneMore ? (D == 4 ? 4 : 3) : 0>
+                             : &parabolic_fixed_kernel<R, C, MODE, D, G, MORE>;
         }();
         static int occs[2] = {0, 0};
-        int& occ_f = occs[fourth];
+        int& occ_f = occs[more];
         if (occ_f == 0) {
             // a small shared-memory share leaves the rest of L1 to cache the gathers; the
             // observed step also holds its FP64 sums there (20 KB per block)
