@@ -1309,7 +1309,8 @@ __global__ void __launch_bounds__(256, hyper_min_blocks<R, C, MODE>()) hyper_ste
     }
     __syncthreads();
 
-    // Old psi_next up front: FP32 scalars and spin-1 only.  Spin-2 on C15 40^3 went from 612 to
+    // Old psi_next up front: FP32 scalars, and spin-1 but on the cube (180^3 559 / 556 us up front / after the
+    // local terms, 228^3 1334 / 1256).  Spin-2 on C15 40^3 went from 612 to
     // 897 us with it, BCC 64^3 from 222 to 325 (cube 90^3 146 to 131), FP64 spin-1 BCC 64^3 from
     // 925 to 1708.  Letting the next kernel in cost spin-2 2 %.
     constexpr bool kEarly = MODE == GPE_MODE_LEAPFROG && sizeof(R) == 4 && C < 5;
@@ -1344,7 +1345,10 @@ __global__ void __launch_bounds__(256, hyper_min_blocks<R, C, MODE>()) hyper_ste
         ld_node<R, C>(own, prv);
         char* nxt = a.next + cell_off + l * node_bytes;
         Cx<R> nv[C];
-        if constexpr (kEarly) ld_node<R, C>(nxt, nv);
+        const bool early = kEarly && (C == 1 || F == 4);
+        if constexpr (kEarly) {
+            if (early) ld_node<R, C>(nxt, nv);
+        }
 #pragma unroll
         for (int s = 0; s < C; ++s) H[s] = cx<R>((R)0, (R)0);
         // d1 of q (RelativisticSpin2Gpe.cu:1051-1066), whole edge records
@@ -1381,6 +1385,7 @@ __global__ void __launch_bounds__(256, hyper_min_blocks<R, C, MODE>()) hyper_ste
         }
         char* hp = (MODE == GPE_MODE_ITP && a.hpsi) ? a.hpsi + cell_off + l * node_bytes : nullptr;
         if constexpr (kEarly) {
+            if (!early) ld_node<R, C>(nxt, nv);
 #pragma unroll
             for (int s = 0; s < C; ++s) add_scaled(nv[s], (R)2 * P.dt, cx<R>(H[s].y, -H[s].x));
             st_node<R, C>(nxt, nv);
