@@ -893,6 +893,15 @@ __device__ __forceinline__ void node_finish(const PhysR<R>& P, const R pos[3], u
     }
 }
 
+// The FP32 spin-1 step that sums observables starts when everything before it is done, so that it
+// may read the state by the read-only path, whose loads the compiler moves past the sums' stores:
+// with plain loads, overlapped, BCC 99^3 takes 287 us for 261, A15 63^3 302 / 268, C15 44^3 306 / 276, Z 52^3
+// 287 / 258, cube 228^3 326 / 304; spin-2 is up to 2 % faster with plain loads, scalars are equal.
+template <typename R, int C, class OA>
+constexpr bool in_order_launch() {
+    return std::is_same<OA, ObsAcc<R>>::value && sizeof(R) == 4 && C == 3;
+}
+
 // One node of a parabolic step whose first D (> 0) stencil entries are given in t:
 // the DEC Laplacian gather, the neighbour loads issued G at a time, then the local
 // terms and the time update.  MORE: the node's further entries f_more .. f_end - 1
@@ -911,7 +920,7 @@ __device__ __forceinline__ void parabolic_node_t(const Grid& g, const NodeTab<R,
     const char* base = prev + cell_off;
     const uint32_t node_bytes = C * 2 * sizeof(R);
     Cx<R> prv[C], H[C], nv[C];
-    ld_node<R, C>(base + l * node_bytes, prv);
+    ld_node<R, C, in_order_launch<R, C, OA>()>(base + l * node_bytes, prv);
     if constexpr (kScale) scale_record(prv, C, inv);
     char* nxt = next + cell_off + l * node_bytes;
     // leapfrog: the old next record is loaded up front, in flight with the gathers
@@ -925,7 +934,7 @@ __device__ __forceinline__ void parabolic_node_t(const Grid& g, const NodeTab<R,
         Cx<R> v[G][C];
 #pragma unroll
         for (int k = 0; k < G; ++k)
-            if (k0 + k < D) ld_node<R, C>(base + t.off[k0 + k], v[k]);
+            if (k0 + k < D) ld_node<R, C, in_order_launch<R, C, OA>()>(base + t.off[k0 + k], v[k]);
 #pragma unroll
         for (int k = 0; k < G; ++k) {
             if (k0 + k < D) {
@@ -953,7 +962,7 @@ __device__ __forceinline__ void parabolic_node_t(const Grid& g, const NodeTab<R,
             for (int h = 0; h < 4; h += G) {
                 Cx<R> v[G][C];
 #pragma unroll
-                for (int k = 0; k < G; ++k) ld_node<R, C>(base + o[h + k], v[k]);
+                for (int k = 0; k < G; ++k) ld_node<R, C, in_order_launch<R, C, OA>()>(base + o[h + k], v[k]);
 #pragma unroll
                 for (int k = 0; k < G; ++k) {
                     if constexpr (kScale) scale_record(v[k], C, inv);
@@ -990,7 +999,7 @@ __device__ __forceinline__ void parabolic_node(const Grid& g, const SmemTables<R
         const char* base = prev + cell_off;
         const uint32_t node_bytes = C * 2 * sizeof(R);
         Cx<R> prv[C], H[C], nv[C];
-        ld_node<R, C>(base + l * node_bytes, prv);
+        ld_node<R, C, in_order_launch<R, C, OA>()>(base + l * node_bytes, prv);
         if constexpr (kScale) scale_record(prv, C, inv);
 #pragma unroll
         for (int s = 0; s < C; ++s) H[s] = cx<R>((R)0, (R)0);
@@ -1006,7 +1015,7 @@ __device__ __forceinline__ void parabolic_node(const Grid& g, const SmemTables<R
                 Cx<R> v[4][C];
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                    if (f + k < f1) ld_node<R, C>(base + st.nb_off[f + k], v[k]);
+                    if (f + k < f1) ld_node<R, C, in_order_launch<R, C, OA>()>(base + st.nb_off[f + k], v[k]);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     if (f + k < f1) {
@@ -1020,7 +1029,7 @@ __device__ __forceinline__ void parabolic_node(const Grid& g, const SmemTables<R
         } else {
             for (int f = f0; f < f1; ++f) {
                 Cx<R> v[C];
-                ld_node<R, C>(base + st.nb_off[f], v);
+                ld_node<R, C, in_order_launch<R, C, OA>()>(base + st.nb_off[f], v);
                 if constexpr (kScale) scale_record(v, C, inv);
                 const R w = st.w[f];
 #pragma unroll
@@ -1160,9 +1169,10 @@ template <typename R, int C, int MODE, int D, int G, bool MORE, int BLOCKS = 0>
 __global__ void __launch_bounds__(256, BLOCKS) parabolic_fixed_kernel(StepArgs a) {
     parabolic_fixed_body<R, C, MODE, D, G, MORE, false>(a);
 }
-// The same with the observables of the state it reads (three blocks per SM).
+// The same with the observables of the state it reads (three blocks per SM; two for spin-1 on
+// FCC, whose 80 registers had 40 bytes of spills: with the loads in order 48^3 102 -> 93 us, 99^3 414 -> 380).
 template <typename R, int C, int MODE, int D, int G, bool MORE>
-__global__ void __launch_bounds__(256, 3) parabolic_fixed_obs_kernel(StepArgs a) {
+__global__ void __launch_bounds__(256, C == 3 && MORE ? 2 : 3) parabolic_fixed_obs_kernel(StepArgs a) {
     parabolic_fixed_body<R, C, MODE, D, G, MORE, true>(a);
 }
 
@@ -1761,7 +1771,12 @@ cudaError_t launch_parabolic_m(const StepArgs& a, cudaStream_t s, unsigned* grid
         const unsigned nb = (unsigned)(wave / m * m);
         if (nb > 0) {
             if (grid) *grid = nb;
-            return launch_overlapped(kf, nb, 256, 0, s, a);
+            if constexpr (in_order_launch<R, C, typename ObsOf<OBS, R>::type>()) {
+                kf<<<nb, 256, 0, s>>>(a);
+                return cudaGetLastError();
+            } else {
+                return launch_overlapped(kf, nb, 256, 0, s, a);
+            }
         }
     }
     // grids smaller than V / gcd(V, 256) blocks: the grid-stride kernel (the
@@ -1780,7 +1795,13 @@ cudaError_t launch_parabolic_m(const StepArgs& a, cudaStream_t s, unsigned* grid
     }
     const unsigned nb = std::min<unsigned>(nblocks(a.total, 256), (unsigned)occ * (unsigned)device_sm_count());
     if (grid) *grid = nb;
-    return nb ? launch_overlapped(ks, nb, 256, 0, s, a) : cudaSuccess;
+    if (nb == 0) return cudaSuccess;
+    if constexpr (in_order_launch<R, C, typename ObsOf<OBS, R>::type>()) {
+        ks<<<nb, 256, 0, s>>>(a);
+        return cudaGetLastError();
+    } else {
+        return launch_overlapped(ks, nb, 256, 0, s, a);
+    }
 }
 
 template <typename R, int C, int D, int G = D, bool MORE = false>
