@@ -1287,8 +1287,8 @@ __device__ __forceinline__ void q_update(const StepArgs& a, const SmemHyper<R>& 
 // DO_PSI: psi update with MODE and HYPERB (-c_K scaling); QM < 0: no q update.
 //
 // Bound by the loads' latency: the old psi_next record is loaded with the others, not after
-// the local terms, which took the spin-1 step on C15 40^3 from 487 to 341 us (0.57 to 0.81
-// of the copy peak), BCC 96^3 from 603 to 414 (0.82), cube 120^3 165 to 160; scalar BCC 96^3
+// the local terms, which took the spin-1 step on C15 40^3 from 487 to 330 us (0.57 to 0.84
+// of the copy peak), BCC 96^3 from 603 to 412 (0.82); scalar BCC 96^3
 // 172 to 166.
 //
 // FP64 imaginary time at 8 (scalar) and 4 (spin-1) blocks per SM: left to itself the compiler
@@ -1319,8 +1319,8 @@ __global__ void __launch_bounds__(256, hyper_min_blocks<R, C, MODE>()) hyper_ste
     }
     __syncthreads();
 
-    // Old psi_next up front: FP32 scalars, and spin-1 but on the cube (180^3 559 / 556 us up front / after the
-    // local terms, 228^3 1334 / 1256).  Spin-2 on C15 40^3 went from 612 to
+    // Old psi_next up front: FP32 scalars, and spin-1 but on the cube (up front / component by component after
+    // the local terms, 130^3 207 / 190 us, 228^3 1342 / 1111).  Spin-2 on C15 40^3 went from 612 to
     // 897 us with it, BCC 64^3 from 222 to 325 (cube 90^3 146 to 131), FP64 spin-1 BCC 64^3 from
     // 925 to 1708.  Letting the next kernel in cost spin-2 2 %.
     constexpr bool kEarly = MODE == GPE_MODE_LEAPFROG && sizeof(R) == 4 && C < 5;
@@ -1395,7 +1395,10 @@ __global__ void __launch_bounds__(256, hyper_min_blocks<R, C, MODE>()) hyper_ste
         }
         char* hp = (MODE == GPE_MODE_ITP && a.hpsi) ? a.hpsi + cell_off + l * node_bytes : nullptr;
         if constexpr (kEarly) {
-            if (!early) ld_node<R, C>(nxt, nv);
+            if (!early) {
+                write_update<R, C>(MODE, P.dt, nxt, hp, prv, H);
+                continue;
+            }
 #pragma unroll
             for (int s = 0; s < C; ++s) add_scaled(nv[s], (R)2 * P.dt, cx<R>(H[s].y, -H[s].x));
             st_node<R, C>(nxt, nv);
