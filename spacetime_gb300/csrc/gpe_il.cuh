@@ -548,8 +548,9 @@ cudaError_t launch_il_itp(const StepArgs& a, const ILGrid& G, int deg, size_t ma
 // incidences relative to the q group base, E to-nodes relative to the psi group
 // base, both with dx + 1 in the two low bits, and E from-nodes).  The arithmetic
 // and its order are hyper_step_kernel's (fused leapfrog), so the states are its
-// states bit for bit.
-template <int C, int CELLS>
+// states bit for bit.  EDGES edges are loaded before the first of them is stored
+// (IlHyperEdges).
+template <int C, int CELLS, int EDGES>
 __device__ __forceinline__ void il_hyper_body(const StepArgs& a, const ILGrid& G, const ILGrid& Gq, const int32_t* tab,
                                               FastDiv dGX) {
     const uint32_t V = G.V, E = Gq.V;
@@ -633,26 +634,34 @@ __device__ __forceinline__ void il_hyper_body(const StepArgs& a, const ILGrid& G
                 stc<float>(a.next + own + s * kComp, nv[s]);
             }
         }
+        // edges 2j and 2j + 1: q_update, hyperbolic leapfrog: next_q += i 2 (dt/sigma)(prev_q + d0 psi)
 #pragma unroll 1
-        for (int e = 0; e < 2; ++e) {
-            // edge 2j + e: q_update, hyperbolic leapfrog: next_q += i 2 (dt/sigma)(prev_q + d0 psi)
-            const size_t own = qbase + (size_t)(2 * j + e) * (C * kComp) + (size_t)sub * 8;
-            Cx<float> to[C], fr[C], pq[C], v[C];
-            const bool in = !((outside >> (4 + e)) & 1);
-            const char* pt = a.prev + gbase + eto[e];
+        for (int e0 = 0; e0 < 2; e0 += EDGES) {
+            Cx<float> to[EDGES][C], fr[EDGES][C], pq[EDGES][C], v[EDGES][C];
 #pragma unroll
-            for (int s = 0; s < C; ++s) {
-                to[s] = in ? ldc_nc<float>(pt + s * kComp) : cx<float>(0.f, 0.f);
-                fr[s] = ldc_nc<float>(a.prev + gbase + efrom[e] + s * kComp);
-                pq[s] = ldc_nc<float>(a.q + own + s * kComp);
-                v[s] = ldc<float>(a.qnext + own + s * kComp);
+            for (int i = 0; i < EDGES; ++i) {
+                const int e = e0 + i;
+                const size_t own = qbase + (size_t)(2 * j + e) * (C * kComp) + (size_t)sub * 8;
+                const bool in = !((outside >> (4 + e)) & 1);
+                const char* pt = a.prev + gbase + eto[e];
+#pragma unroll
+                for (int s = 0; s < C; ++s) {
+                    to[i][s] = in ? ldc_nc<float>(pt + s * kComp) : cx<float>(0.f, 0.f);
+                    fr[i][s] = ldc_nc<float>(a.prev + gbase + efrom[e] + s * kComp);
+                    pq[i][s] = ldc_nc<float>(a.q + own + s * kComp);
+                    v[i][s] = ldc<float>(a.qnext + own + s * kComp);
+                }
             }
 #pragma unroll
-            for (int s = 0; s < C; ++s) {
-                const Cx<float> d0psi = to[s] - fr[s];
-                const Cx<float> qq = pq[s] + d0psi;
-                add_scaled(v[s], 2.f * dts, cx<float>(-qq.y, qq.x));
-                stc<float>(a.qnext + own + s * kComp, v[s]);
+            for (int i = 0; i < EDGES; ++i) {
+                const size_t own = qbase + (size_t)(2 * j + e0 + i) * (C * kComp) + (size_t)sub * 8;
+#pragma unroll
+                for (int s = 0; s < C; ++s) {
+                    const Cx<float> d0psi = to[i][s] - fr[i][s];
+                    const Cx<float> qq = pq[i][s] + d0psi;
+                    add_scaled(v[i][s], 2.f * dts, cx<float>(-qq.y, qq.x));
+                    stc<float>(a.qnext + own + s * kComp, v[i][s]);
+                }
             }
         }
     }
@@ -668,19 +677,32 @@ struct IlHyperBounds {
     static constexpr int kMin = C == 5 ? 5 : (C == 3 ? 6 : 8);
 };
 
-template <int C, int CELLS>
+// The edges of a node that are in flight together.  On small grids a step is one wave: the
+// node's loads, then each edge's behind the store before it, and both edges at once take a
+// round trip off that (spin-1 BCC 8^3 4.8 -> 4.3 us a step, 6^3 6.3 -> 4.3, scalar C15 5^3 6.4 -> 4.3;
+// such steps follow each other in quanta of 2 us).  On large ones it is more bytes in flight:
+// scalar BCC 64^3 57.7 -> 50.1 us, C15 40^3 144 -> 131, spin-1 BCC 64^3 120 -> 116, C15 32^3 156 -> 152.
+// Not where spin-1 groups are of 8 cells and the state is beyond il_cost8's line, whose short
+// runs C15 then reads 0.4 to 1.4 % slower (40^3 338 -> 340 us; 22-cell rows of 13 MB 9 %), and not
+// for spin-2, whose records would not fit the registers.
+template <int C>
+struct IlHyperEdges {
+    static constexpr int kMost = C <= 3 ? 2 : 1;
+};
+
+template <int C, int CELLS, int EDGES>
 __global__ void __launch_bounds__(kIlPlainThreads, IlHyperBounds<C>::kMin)
     il_hyper_kernel(StepArgs a, ILGrid G, ILGrid Gq, const int32_t* tab, FastDiv dGX) {
-    il_hyper_body<C, CELLS>(a, G, Gq, tab, dGX);
+    il_hyper_body<C, CELLS, EDGES>(a, G, Gq, tab, dGX);
 }
 
-template <int C, int CELLS>
+template <int C, int CELLS, int EDGES>
 unsigned il_hyper_blocks_c(const ILGrid& G, const ILGrid& Gq) {
     static int occ = 0;
     const unsigned wpb = kIlPlainThreads / 32;
     if (occ == 0) {
-        cudaFuncSetAttribute(il_hyper_kernel<C, CELLS>, cudaFuncAttributePreferredSharedMemoryCarveout, 25);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, il_hyper_kernel<C, CELLS>, (int)kIlPlainThreads, 0);
+        cudaFuncSetAttribute(il_hyper_kernel<C, CELLS, EDGES>, cudaFuncAttributePreferredSharedMemoryCarveout, 25);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, il_hyper_kernel<C, CELLS, EDGES>, (int)kIlPlainThreads, 0);
         if (occ < 1) occ = 1;
     }
     const uint32_t items = G.V;
@@ -704,15 +726,17 @@ cudaError_t launch_il_hyper(const StepArgs& a, const ILGrid& G, const ILGrid& Gq
     const uint64_t tasks64 = (uint64_t)il_warp_tasks(G) * G.V;
     if (tasks64 > 0xffffffffu || G.cells != Gq.cells || G.GX != Gq.GX || Gq.V != 2 * G.V) return cudaErrorInvalidValue;
     const FastDiv dGX = make_fastdiv(G.GX);
+    constexpr int kEdges = IlHyperEdges<C>::kMost;
+    auto launch = [&](auto kernel, unsigned blocks) { kernel<<<blocks, kIlPlainThreads, 0, s>>>(a, G, Gq, tab, dGX); };
     switch (G.cells) {
-        case 32:
-            il_hyper_kernel<C, 32><<<il_hyper_blocks_c<C, 32>(G, Gq), kIlPlainThreads, 0, s>>>(a, G, Gq, tab, dGX);
-            break;
-        case 16:
-            il_hyper_kernel<C, 16><<<il_hyper_blocks_c<C, 16>(G, Gq), kIlPlainThreads, 0, s>>>(a, G, Gq, tab, dGX);
-            break;
+        case 32: launch(il_hyper_kernel<C, 32, kEdges>, il_hyper_blocks_c<C, 32, kEdges>(G, Gq)); break;
+        case 16: launch(il_hyper_kernel<C, 16, kEdges>, il_hyper_blocks_c<C, 16, kEdges>(G, Gq)); break;
         case 8:
-            il_hyper_kernel<C, 8><<<il_hyper_blocks_c<C, 8>(G, Gq), kIlPlainThreads, 0, s>>>(a, G, Gq, tab, dGX);
+            if (C == 3 && !hyper_state_in_l2((uint64_t)G.X * G.Y * G.Z * G.V * C * 8)) {
+                launch(il_hyper_kernel<C, 8, C == 3 ? 1 : kEdges>, il_hyper_blocks_c<C, 8, C == 3 ? 1 : kEdges>(G, Gq));
+            } else {
+                launch(il_hyper_kernel<C, 8, kEdges>, il_hyper_blocks_c<C, 8, kEdges>(G, Gq));
+            }
             break;
         default: return cudaErrorInvalidValue;
     }

@@ -186,8 +186,9 @@ struct ILGrid {
 // C15 36 x 8 x 8 (12.5 MB) 20.5 / 24.1, spin-1 BCC 20 x 48 x 48 (13.3 MB) 23.0 / 31.0; rows of 5 and 8 cells
 // gain at any size (8.8 MB 14.3 / 24.6).  Scalars and the parabolic step (its launches overlap): no such
 // loss.
+inline bool hyper_state_in_l2(uint64_t slot_bytes) { return slot_bytes < 9000000; }
 inline uint32_t il_cost8(uint32_t C, bool hyperbolic, uint64_t slot_bytes) {
-    return hyperbolic && C > 1 && slot_bytes < 9000000 ? 135 : (C == 3 ? 115 : 106);
+    return hyperbolic && C > 1 && hyper_state_in_l2(slot_bytes) ? 135 : (C == 3 ? 115 : 106);
 }
 inline uint32_t il_group_cells(uint32_t X, uint32_t cost8) {
     auto cost = [X](uint32_t cells, uint32_t percent) { return (uint64_t)((X + cells - 1) / cells) * cells * percent; };
