@@ -400,10 +400,15 @@ gpe_status gpe_node_fields_reduce(gpe_handle* h, int32_t slot, int32_t kind, dou
  *                      takes the gather kernel.
  *                  The automatic choice (0) is the interleaved kernel for calls of
  *                  16 or more steps on the parabolic spinor handles and the
- *                  hyperbolic handles it applies to (faster there by 20-70 %; not
- *                  for parabolic scalars, whose 8-byte records already load as
- *                  coalesced runs; the layout changes cost a few steps per
- *                  call), else 1 (grid-stride gather, whole-record loads) -- which
+ *                  hyperbolic handles it applies to (a step is faster by 20-60 %
+ *                  for the parabolic spinors, by 7-30 % for hyperbolic ones and by
+ *                  13-24 % for hyperbolic scalars; hyperbolic grids of a few
+ *                  thousand cells are slower;
+ *                  not for parabolic scalars, whose 8-byte records already load as
+ *                  coalesced runs; a call's layout changes cost some three steps,
+ *                  which hyperbolic calls earn back in 8 to 13 steps with spin 2, 13
+ *                  to 37 with spin 1 and 13 to 19 with scalars: shorter ones are
+ *                  faster under 1), else 1 (grid-stride gather, whole-record loads) -- which
  *                  gpe_get_tuning reports; 2-5 on request, and gpe_autotune may
  *                  pick any of 1-4 (it times single steps; its gather candidate is
  *                  recorded as 0).  Under 0, FP32 split-scheme calls of 16 or more
@@ -420,8 +425,9 @@ gpe_status gpe_node_fields_reduce(gpe_handle* h, int32_t slot, int32_t kind, dou
  * GPE_TUNE_OBSERVE_ARITH: arithmetic of gpe_observe's per-node terms on an FP32
  *                   handle: 0 = FP64 (default; the same numbers as an FP64 run
  *                   on the stored values: sums over columns of nodes in exact pairs
- *                   of FP32 values, as near to sums in extended precision as FP64
- *                   terms are; FP64 terms where |psi| leaves 2^-20 .. 2^27), 1 = FP32
+ *                   of FP32 values (spins and sums of one sign in three), as near to
+ *                   sums in extended precision as FP64 terms are; FP64 terms where
+ *                   the largest |re|, |im| or |psi_s| is outside 2^-20 .. 2^27), 1 = FP32
  *                   terms.  The sums over nodes are FP64 either way.
  * GPE_TUNE_CARVEOUT: shared-memory share (percent) of the unified L1 / shared
  *                   memory for the row-tile kernel; the rest caches its off-row
@@ -577,7 +583,8 @@ gpe_status gpe_adjoint_backward(gpe_handle* h, const double* seed, double* grad,
  *   buffers, on a grid scaled so that each block has the work it has in the
  *   whole batch, for item sizes of 4K..256K nodes, and keeps the fastest; the
  *   members' states are untouched.  Within a step the blocks take the last of
- *   their items from one counter, so a block that finishes early takes more.
+ *   their items (all of them where the list is long) from one counter, so a block
+ *   that finishes early takes more.
  *   `report` receives a JSON list of the timings.
  * An FP32 batch keeps its members' per-node constants in constant memory, one of
  * 256 slots per device and member, held until gpe_batch_destroy.  A batch created

@@ -378,8 +378,8 @@ __global__ void __launch_bounds__(256, (sizeof(R) == 4 && C <= 3) ? 4 : 1) adjoi
 // in registers, and every load and store is one run of full lines.  The handle-layout
 // form above spends its time on L1 (67 %), index arithmetic and table reads.  Spin-1 BCC
 // 40^3, 200 steps forward and back: 10.7 ms with every state in the handle's layout, 7.75
-// with all of them in this one (a reverse step 20.4 -> 16 us, a forward or recomputed
-// step 15.0 -> 11.9).  Registers: 6 blocks per SM (80) 7.75 ms, 5 (96) 7.85, 7 (72) 7.85.
+// with all of them in this one (a reverse step 20.4 -> 15.4 us, a forward or recomputed
+// step 15.0 -> 11.1).  Registers: 6 blocks per SM (80) 7.75 ms, 5 (96) 7.85, 7 (72) 7.85.
 constexpr unsigned kIlAdjThreads = 128;
 template <int C, int D, int CELLS>
 __global__ void __launch_bounds__(kIlAdjThreads, C == 5 ? 3 : D == 8 ? 4 : 6) il_adjoint_kernel(StepArgs a, AdjArgs j, ILGrid G,

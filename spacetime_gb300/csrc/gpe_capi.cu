@@ -1201,8 +1201,9 @@ extern "C" gpe_status gpe_start(gpe_handle* h, void* stream) {
     return GPE_OK;
 }
 
-// Calls shorter than this stay in the handle's layout: the two layout changes in
-// and the two out cost about as much as two steps.
+// Calls shorter than this stay in the handle's layout: the two layout changes in and the two
+// out cost some three steps (BCC 96^3 354 us a call against 122 a step, hyperbolic spin-1 1014 / 336);
+// the hyperbolic calls' break-evens are at il_hyper_auto.
 constexpr int32_t kIlMinSteps = 16;
 static bool split_planes_ready(gpe_handle* h, int32_t n, cudaStream_t s);
 static gpe_status split_plane_steps(gpe_handle* h, int32_t n, cudaStream_t s);
@@ -1348,10 +1349,11 @@ static bool il_hyper_applies(const gpe_handle* h) {
 // Where the automatic choice takes the interleaved hyperbolic step: everywhere it
 // applies, by measurement (FP32; us a step, gather / interleaved + a call's layout
 // changes): spin-2 BCC 96^3 720 / 559 + 1689, C15 40^3 615 / 500 + 1363, 24^3 137 / 114 + 299
-// (even at 8 to 13 steps); spin-1 BCC 96^3 414 / 341 + 1008, C15 40^3 341 / 309 + 810, 32^3 177 /
-// 150 + 448 (14 to 25); scalars BCC 96^3 166 / 157 + 431, C15 40^3 136 / 132 + 303 (47 and 76).
-// Calls that lose by it: spin-1 of 16 to 25 steps up to 10 %, scalars of 16 to 47 steps and
-// small grids (BCC 20^3 3.5 / 6.2, 6.0 / 8.2, 9.7 / 10.2); GPE_TUNE_KERNEL 1 avoids it there.
+// (even at 8 to 13 steps); spin-1 BCC 96^3 412 / 336 + 1014, C15 40^3 330 / 308 + 824, 32^3 168 /
+// 147 + 453 (13 to 37); scalars BCC 96^3 166 / 134 + 436, C15 40^3 136 / 120 + 301 (13 and 19).
+// Calls that lose by it: spin-1 of 16 to 37 steps up to 10 % and small grids, scalar, spin-1
+// and spin-2 BCC 8^3 1.8 / 4.1, 2.8 / 4.1, 3.8 / 6.0, 16^3 2.9 / 4.3, 4.8 / 6.1, 6.6 / 6.1;
+// GPE_TUNE_KERNEL 1 avoids it there.
 static bool il_hyper_auto(const gpe_handle*) { return true; }
 
 static bool use_interleaved(const gpe_handle* h, int32_t n) {

@@ -5,18 +5,19 @@
 // costs as much as an FP64 operation: with per-node terms in FP64, observe_kernel
 // spent 290 FP64 operations on a spin-1 node and ran at 87 % of the FP64 pipe with
 // DRAM at 1 % (1463 us on spin-1 BCC 64^3, whose state is read in 11 us; this form
-// takes 140 us, bound by the FP32 instructions of the exact sums).  Here
+// takes 146 us, bound by the FP32 instructions of the exact sums).  Here
 //  - everything that is the same for a column of cells -- the stencil weights, the
 //    trap, the fields, the coupling constants, the position -- is left out of the
 //    per-node terms and multiplied in once per column, in FP64;
 //  - the per-node terms, products of stored values alone, are exact pairs of FP32
 //    values for FP32 storage (two-products and two-sums: Dekker 1971, Knuth; the
-//    sums are PairSum's and, for terms of one sign, TripleSum's), plain FP64 for FP64
-//    storage.
+//    sums are PairSum's and, for terms of one sign and for the products of a spin,
+//    which cancel within a node of an unpolarised state, TripleSum's), plain FP64 for
+//    FP64 storage.
 // A pair keeps 47 bits or more of each node's term, and the errors of different nodes
 // are independent, so that the sums carry the error of their FP64 additions.  (Densities
 // in FP64 node by node instead of three FP32 words: observables, density and spin sums of
-// that state together 487 us against 335.)  Measured
+// that state together 487 us against 335; the spins' third words are 25 us more.)  Measured
 // against sums in more than 64 bits on Thomas-Fermi clouds and noise (BCC 12^3 .. 24^3,
 // C15 9^3; root mean square, relative): norm 1e-16 to 2.5e-16, centre of mass 1e-16 to
 // 3e-16, energy 1e-16 to 3e-16, M_z 1e-16 to 2e-16, |F| 1e-16 -- observe_kernel's are 1e-16
