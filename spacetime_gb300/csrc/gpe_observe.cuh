@@ -313,7 +313,9 @@ __device__ __forceinline__ uint32_t count_nonfinite(const Cx<R>* p) {
 // consecutive threads consecutive nodes along x, so that the rows are read as in the
 // step kernels and the neighbours in z come from the thread's own recent reads.  D: the
 // longest row (4, 6 or 8 entries).  The sums of a column's nodes are combined in FP64
-// once per column of zc cells.
+// once per column of zc cells.  FP32 has two blocks per SM (128 registers): spin-1 without
+// spills, spin-2 with 84 to 184 bytes of them.  gpe_observe as a whole, before (FP64 terms) and
+// now: spin-1 BCC 64^3 1527 -> 191 us, spin-2 BCC 64^3 3512 -> 310, C15 32^3 4964 -> 434.
 template <typename R, int C, int D>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) observe_columns_kernel(StepArgs a, uint32_t zc, uint32_t columns,
                                                                                     uint32_t total, FastDiv dcol) {
